@@ -77,3 +77,34 @@ def test_training_reduces_loss():
         net.train_step(Xd, Td, Md, lr=2e-3)
     last = net.grad(Xd, Td, Md)[0]
     assert last < first / 10.0, (first, last)
+
+
+@pytest.mark.parametrize("B", [1, 15, 64, 129, 4095, 4096, 4097])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_gradients_at_tile_edges(B, offset):
+    """Batches around the row tiles, the batch splits and the switch of tile
+    size, with rows that start off a 16-byte boundary.  Each gradient is a sum
+    of float32 products; its rounding error is bounded by the summed magnitudes
+    times 2^-24 per operation of a chain, far below GRAD_TOL of its norm."""
+    import torch
+    from zhenmode_b200.closure import ClosureMLP, init_params
+    rng = np.random.default_rng(B + 31)
+    p = init_params(seed=8, out_bias=0.0)
+    X = rng.standard_normal((B, 256)).astype(np.float32)
+    T = rng.standard_normal((B, 64)).astype(np.float32)
+    M = (rng.random((B, 64)) < 0.7).astype(np.float32)
+    M[0, 0] = 1.0
+
+    def dev(a):
+        flat = torch.zeros(a.size + offset, device="cuda")
+        flat[offset:] = torch.as_tensor(a.ravel(), device="cuda")
+        return flat[offset:].view(a.shape)
+
+    net = ClosureMLP(p)
+    loss, g = net.grad(dev(X), dev(T), dev(M))
+    want_loss, want_g = omlp.loss_and_grad(p, X, T, M)
+    assert abs(loss - want_loss) <= GRAD_TOL * want_loss
+    g = g.cpu().numpy()
+    for name in omlp.OFF:
+        sl = slice(omlp.OFF[name], omlp.OFF[name] + int(np.prod(omlp.SHAPES[name])))
+        assert _rel(g[sl], want_g[sl]) < GRAD_TOL, (name, _rel(g[sl], want_g[sl]))

@@ -405,99 +405,278 @@ __global__ void k_mlp_pack(const float* __restrict__ params, __nv_bfloat16* __re
 }
 
 // ---------------------------------------------------------------- training (float32)
+//
+// A training step is seven launches: the two hidden layers with their bias and
+// GELU, the output layer with the loss and its derivative, the two input
+// gradients with the GELU derivative, every weight and bias gradient at once,
+// and the fold of the gradient's partial sums with the Adam update.  The
+// products are float32 FMA (6.2 GFLOP a step at 8192 rows: 84 us at the FP32
+// rate of 148 SMs), so what bounds them is the FMA pipe once every SM has a
+// tile:
+//  * a block of 256 threads forms a BM x BN tile from K slabs of 16 held in
+//    shared memory, two buffers, the next slab loaded into registers during
+//    the current one; a thread holds BM/16 x BN/16 sums and runs the paired
+//    FP32 instructions;
+//  * the gradients of the weights are sums over the batch (16 output tiles of
+//    64 x 64 with a serial chain of 8192 rows filled 16 of 148 SMs): the batch
+//    is split over blockIdx.z, each split writes its partial sums and k_fold
+//    adds them in split order; the bias gradients are the column sums of the
+//    same slabs (they took 0.47 ms each as one block's serial sums).
+// At 8192 rows a step went from 4.00 to 0.24 ms (one B200), 0.022 ms of it the host's
+// read of the mask count.
 
-// C[M][N] = op(A) op(B) (+ bias[n]) with op(A) [M][K], op(B) [K][N]; A is
-// [M][K] (ta = 0) or [K][M] (ta = 1), B is [K][N] (tb = 0) or [N][K] (tb = 1).
-__global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, const float* __restrict__ A, int ta,
-                                               const float* __restrict__ B, int tb, const float* __restrict__ bias,
-                                               float* __restrict__ C) {
-  __shared__ float As[16][64 + 1], Bs[16][64 + 1];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += 16) {
-    for (int e = threadIdx.x; e < 16 * 64; e += 256) {
-      const int kk = e / 64, mm = e - kk * 64;
-      const int m = m0 + mm, k = k0 + kk;
-      As[kk][mm] = (m < M && k < K) ? (ta ? A[(size_t)k * M + m] : A[(size_t)m * K + k]) : 0.f;
-      const int n = n0 + mm;
-      Bs[kk][mm] = (n < N && k < K) ? (tb ? B[(size_t)n * K + k] : B[(size_t)k * N + n]) : 0.f;
+constexpr int GK = 16;  // K slab
+
+// Four consecutive floats, by one load where the pointer allows.
+__device__ __forceinline__ float4 load4(const float* p, bool vec) {
+  if (vec) return __ldg(reinterpret_cast<const float4*>(p));
+  return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+}
+
+// One operand's slab: T = 0 reads rows of [R][K] (K contiguous), T = 1 rows of
+// [K][R] (R contiguous); into s[k][r].  R0 is the tile's first r, Rn the
+// extent of r; K runs to k1.  Each thread moves BR / 64 float4.
+template <int BR, int T>
+struct Slab {
+  static constexpr int Q = BR / 64;
+  float4 v[Q];
+  __device__ __forceinline__ void fetch(const float* __restrict__ p, int ldp, int R0, int Rn, int k0, int k1, bool vec) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int e = threadIdx.x + q * 256;
+      v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (T == 0) {
+        const int r = R0 + e / 4, k = k0 + (e % 4) * 4;
+        if (r < Rn && k < k1) v[q] = load4(p + (size_t)r * ldp + k, vec);
+      } else {
+        const int k = k0 + e / (BR / 4), r = R0 + (e % (BR / 4)) * 4;
+        if (r < Rn && k < k1) v[q] = load4(p + (size_t)k * ldp + r, vec);
+      }
     }
-    __syncthreads();
+  }
+  __device__ __forceinline__ void put(float (*s)[BR + 4]) const {
 #pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-      float a[4], b[4];
+    for (int q = 0; q < Q; ++q) {
+      const int e = threadIdx.x + q * 256;
+      if (T == 0) {
+        const int r = e / 4, k = (e % 4) * 4;
+        s[k][r] = v[q].x;
+        s[k + 1][r] = v[q].y;
+        s[k + 2][r] = v[q].z;
+        s[k + 3][r] = v[q].w;
+      } else {
+        const int k = e / (BR / 4), r = (e % (BR / 4)) * 4;
+        *reinterpret_cast<float4*>(&s[k][r]) = v[q];
+      }
+    }
+  }
+};
+
+// acc += A B over K in [k0, k1), tile rows from m0, columns from n0.  A is
+// [M][K] (TA = 0) or [K][M] (TA = 1), B is [N][K] (TB = 0) or [K][N] (TB = 1);
+// M, N and, where K is the contiguous index, K are multiples of 4 or the rows
+// of an operand whose rows are whole.  Thread (tx, ty) holds rows ty * 4 + 64 a
+// + 0..3 and columns tx * 4 + 64 b + 0..3 as column pairs.  With CS the sums
+// over k of A's columns come back in colsum of thread m < BM.
+template <int BM, int BN>
+struct GemmSmem {
+  float a[2][GK][BM + 4], b[2][GK][BN + 4];
+};
+
+template <int BM, int BN, int TA, int TB, bool CS>
+__device__ __forceinline__ void gemm_tile(GemmSmem<BM, BN>& sm, const float* __restrict__ A, int lda, int M, int m0,
+                                          bool va, const float* __restrict__ B, int ldb, int N, int n0, bool vb,
+                                          int k0, int k1, float2 (&acc)[BM / 16][BN / 32], float& colsum) {
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        a[q] = As[kk][ty * 4 + q];
-        b[q] = Bs[kk][tx * 4 + q];
+  for (int q = 0; q < BM / 16; ++q)
+#pragma unroll
+    for (int r = 0; r < BN / 32; ++r) acc[q][r] = make_float2(0.f, 0.f);
+  colsum = 0.f;
+  Slab<BM, TA> sa;
+  Slab<BN, TB> sb;
+  sa.fetch(A, lda, m0, M, k0, k1, va);
+  sb.fetch(B, ldb, n0, N, k0, k1, vb);
+  sa.put(sm.a[0]);
+  sb.put(sm.b[0]);
+  __syncthreads();
+  int p = 0;
+  for (int k = k0; k < k1; k += GK, p ^= 1) {
+    const bool more = k + GK < k1;
+    if (more) {
+      sa.fetch(A, lda, m0, M, k + GK, k1, va);
+      sb.fetch(B, ldb, n0, N, k + GK, k1, vb);
+    }
+#pragma unroll
+    for (int kk = 0; kk < GK; ++kk) {
+      float a[BM / 16];
+      float2 b[BN / 32];
+#pragma unroll
+      for (int q = 0; q < BM / 64; ++q) {
+        const float4 v = *reinterpret_cast<const float4*>(&sm.a[p][kk][q * 64 + ty * 4]);
+        a[4 * q] = v.x; a[4 * q + 1] = v.y; a[4 * q + 2] = v.z; a[4 * q + 3] = v.w;
       }
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
+      for (int r = 0; r < BN / 64; ++r) {
+        const float4 v = *reinterpret_cast<const float4*>(&sm.b[p][kk][r * 64 + tx * 4]);
+        b[2 * r] = make_float2(v.x, v.y);
+        b[2 * r + 1] = make_float2(v.z, v.w);
+      }
 #pragma unroll
-        for (int r = 0; r < 4; ++r) acc[q][r] += a[q] * b[r];
+      for (int q = 0; q < BM / 16; ++q)
+#pragma unroll
+        for (int r = 0; r < BN / 32; ++r) acc[q][r] = __ffma2_rn(make_float2(a[q], a[q]), b[r], acc[q][r]);
+    }
+    if (CS && threadIdx.x < BM) {
+#pragma unroll
+      for (int kk = 0; kk < GK; ++kk) colsum += sm.a[p][kk][threadIdx.x];
+    }
+    if (more) {
+      sa.put(sm.a[p ^ 1]);
+      sb.put(sm.b[p ^ 1]);
     }
     __syncthreads();
   }
+}
+
+// Walks the thread's outputs four columns at a time: f(m, n, float4).
+template <int BM, int BN, class F>
+__device__ __forceinline__ void tile_rows(const float2 (&acc)[BM / 16][BN / 32], int m0, int n0, int M, int N, F f) {
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
+  for (int q = 0; q < BM / 16; ++q) {
+    const int m = m0 + (q / 4) * 64 + ty * 4 + (q % 4);
+    if (m >= M) continue;
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int m = m0 + ty * 4 + q, n = n0 + tx * 4 + r;
-      if (m < M && n < N) C[(size_t)m * N + n] = acc[q][r] + (bias ? bias[n] : 0.f);
+    for (int r = 0; r < BN / 64; ++r) {
+      const int n = n0 + r * 64 + tx * 4;
+      if (n < N) f(m, n, make_float4(acc[q][2 * r].x, acc[q][2 * r].y, acc[q][2 * r + 1].x, acc[q][2 * r + 1].y));
     }
+  }
 }
 
-__global__ void k_gelu_fwd(const float* __restrict__ Z, float* __restrict__ H, long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    H[i] = gelu(Z[i]);
+// Z = A W^T + b and H = gelu(Z): a hidden layer over `rows` rows, 256 -> 256.
+template <int BT>
+__global__ void __launch_bounds__(256) k_layer_fwd(int rows, const float* __restrict__ A, bool va,
+                                                   const float* __restrict__ W, bool vw,
+                                                   const float* __restrict__ bias, float* __restrict__ Z,
+                                                   float* __restrict__ H) {
+  __shared__ GemmSmem<BT, BT> sm;
+  float2 acc[BT / 16][BT / 32];
+  float cs;
+  const int m0 = blockIdx.y * BT, n0 = blockIdx.x * BT;
+  gemm_tile<BT, BT, 0, 0, false>(sm, A, MK, rows, m0, va, W, MK, MK, n0, vw, 0, MK, acc, cs);
+  tile_rows<BT, BT>(acc, m0, n0, rows, MK, [&](int m, int n, float4 z) {
+    z.x += __ldg(bias + n); z.y += __ldg(bias + n + 1); z.z += __ldg(bias + n + 2); z.w += __ldg(bias + n + 3);
+    const size_t o = (size_t)m * MK + n;
+    *reinterpret_cast<float4*>(Z + o) = z;
+    *reinterpret_cast<float4*>(H + o) = make_float4(gelu(z.x), gelu(z.y), gelu(z.z), gelu(z.w));
+  });
 }
 
-__global__ void k_gelu_bwd(const float* __restrict__ Z, float* __restrict__ G, long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    G[i] *= gelu_grad(Z[i]);
-}
-
-// masked mean-square error over the valid outputs: dY = 2 m (Y - T) / sum(m),
-// per-block partial losses and mask counts
-__global__ void k_mse(const float* __restrict__ Y, const float* __restrict__ T, const float* __restrict__ Mk,
-                      float* __restrict__ dY, long long n, float inv_count, double* __restrict__ part) {
-  __shared__ double red[256];
+// The output layer with the masked mean-square error: Y = H W^T + b,
+// e = (Y - T) m, dY = 2 e / sum(m); part[block] = the block's sum of e^2.
+__global__ void __launch_bounds__(256) k_layer_out(int rows, const float* __restrict__ H, const float* __restrict__ W,
+                                                   bool vw, const float* __restrict__ bias,
+                                                   const float* __restrict__ T, bool vt, const float* __restrict__ Mk,
+                                                   bool vm, float inv_count, float* __restrict__ dY,
+                                                   double* __restrict__ part) {
+  __shared__ GemmSmem<64, 64> sm;
+  __shared__ double red[8];
+  float2 acc[4][2];
+  float cs;
+  const int m0 = blockIdx.x * 64;
+  gemm_tile<64, 64, 0, 0, false>(sm, H, MK, rows, m0, true, W, MK, MO, 0, vw, 0, MK, acc, cs);
   double s = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float e = (Y[i] - T[i]) * Mk[i];
-    dY[i] = 2.f * e * inv_count;
-    s += (double)e * (double)e;
-  }
-  red[threadIdx.x] = s;
+  tile_rows<64, 64>(acc, m0, 0, rows, MO, [&](int m, int n, float4 y) {
+    const size_t o = (size_t)m * MO + n;
+    const float4 t = load4(T + o, vt), k = load4(Mk + o, vm);
+    const float4 e = make_float4((y.x + __ldg(bias + n) - t.x) * k.x, (y.y + __ldg(bias + n + 1) - t.y) * k.y,
+                                 (y.z + __ldg(bias + n + 2) - t.z) * k.z, (y.w + __ldg(bias + n + 3) - t.w) * k.w);
+    *reinterpret_cast<float4*>(dY + o) =
+        make_float4(2.f * e.x * inv_count, 2.f * e.y * inv_count, 2.f * e.z * inv_count, 2.f * e.w * inv_count);
+    s += (double)e.x * e.x + (double)e.y * e.y + (double)e.z * e.z + (double)e.w * e.w;
+  });
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) s += red[w];
+    part[blockIdx.x] = s;
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
-// column sums of G [rows][cols] -> out[cols]
-__global__ void k_colsum(const float* __restrict__ G, int rows, int cols, float* __restrict__ out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  float s = 0.f;
-  for (int r = 0; r < rows; ++r) s += G[(size_t)r * cols + c];
-  out[c] = s;
+// G = (D W) gelu'(Z): the gradient of a hidden layer's pre-activation from the
+// gradient D [rows][K] of the next one, W [K][256].
+template <int BT>
+__global__ void __launch_bounds__(256) k_layer_bwd(int rows, int K, const float* __restrict__ D,
+                                                   const float* __restrict__ W, bool vw, const float* __restrict__ Z,
+                                                   float* __restrict__ G) {
+  __shared__ GemmSmem<BT, BT> sm;
+  float2 acc[BT / 16][BT / 32];
+  float cs;
+  const int m0 = blockIdx.y * BT, n0 = blockIdx.x * BT;
+  gemm_tile<BT, BT, 0, 1, false>(sm, D, K, rows, m0, true, W, MK, MK, n0, vw, 0, K, acc, cs);
+  tile_rows<BT, BT>(acc, m0, n0, rows, MK, [&](int m, int n, float4 g) {
+    const size_t o = (size_t)m * MK + n;
+    const float4 z = *reinterpret_cast<const float4*>(Z + o);
+    *reinterpret_cast<float4*>(G + o) = make_float4(g.x * gelu_grad(z.x), g.y * gelu_grad(z.y), g.z * gelu_grad(z.z),
+                                                    g.w * gelu_grad(z.w));
+  });
 }
 
-__global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, long long n, float lr, float b1, float b2, float eps, float c1,
-                       float c2) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+// Every weight and bias gradient over the rows of one split (blockIdx.y):
+// dW = D^T A and db = column sums of D, layer by layer; the tiles of the three
+// layers are consecutive in blockIdx.x.  ws[split] has the parameters' layout.
+struct GradLayer {
+  const float *D, *A;  // [rows][out], [rows][256]
+  int out;             // outputs (rows of the weight)
+  bool va;             // A allows 16-byte loads
+  long long w, b;      // offsets of the weight and the bias
+};
+struct GradArgs {
+  GradLayer l[3];
+  int rows, per_split;
+  float* ws;
+};
+constexpr int GRAD_TILES = 4 + 4 + 2;  // 128 x 128 tiles of the 256 x 256, 256 x 256 and 64 x 256 weights
+
+__global__ void __launch_bounds__(256) k_layer_grads(GradArgs g) {
+  __shared__ GemmSmem<128, 128> sm;
+  float2 acc[8][4];
+  float cs;
+  const int layer = blockIdx.x < 4 ? 0 : (blockIdx.x < 8 ? 1 : 2);
+  const int t = blockIdx.x - 4 * layer;
+  const GradLayer L = g.l[layer];
+  const int m0 = (t >> 1) * 128, n0 = (t & 1) * 128;
+  const int k0 = blockIdx.y * g.per_split, k1 = min(g.rows, k0 + g.per_split);
+  gemm_tile<128, 128, 1, 1, true>(sm, L.D, L.out, L.out, m0, true, L.A, MK, MK, n0, L.va, k0, k1, acc, cs);
+  float* ws = g.ws + (size_t)blockIdx.y * ZM_MLP_NPARAMS;
+  tile_rows<128, 128>(acc, m0, n0, L.out, MK, [&](int m, int n, float4 v) {
+    *reinterpret_cast<float4*>(ws + L.w + (size_t)m * MK + n) = v;
+  });
+  if (n0 == 0 && threadIdx.x < 128 && m0 + threadIdx.x < L.out) ws[L.b + m0 + threadIdx.x] = cs;
+}
+
+// The gradient: partial sums added in split order; then either written to
+// grad or taken as one Adam step (grad null).
+__global__ void __launch_bounds__(256) k_fold(const float* __restrict__ ws, int splits, float* __restrict__ grad,
+                                              float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
+                                              float lr, float b1, float b2, float eps, float c1, float c2) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= ZM_MLP_NPARAMS) return;
+  float gi = 0.f;
+#pragma unroll 8
+  for (int s = 0; s < splits; ++s) gi += ws[(size_t)s * ZM_MLP_NPARAMS + i];
+  if (grad) {
+    grad[i] = gi;
+    return;
   }
+  const float mi = b1 * m[i] + (1.f - b1) * gi;
+  const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
+  m[i] = mi;
+  v[i] = vi;
+  p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
 }
 
 }  // namespace zm
@@ -523,19 +702,20 @@ bool launch_ok(const char* what) {
   return true;
 }
 
-void sgemm(cudaStream_t s, int M, int N, int K, const float* A, int ta, const float* B, int tb, const float* bias,
-           float* C) {
-  k_sgemm<<<dim3((N + 63) / 64, (M + 63) / 64), 256, 0, s>>>(M, N, K, A, ta, B, tb, bias, C);
-}
+bool vec16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
+
+// splits of the weight gradients' batch sums: with 14 the 10 tiles fill the 148 SMs once
+constexpr int GRAD_SPLITS = 14;
 
 }  // namespace
 
 struct zm_mlp_trainer {
   int batch_max = 0;
-  float *Z1 = nullptr, *H1 = nullptr, *Z2 = nullptr, *H2 = nullptr, *Y = nullptr, *dY = nullptr;
-  float *G1 = nullptr, *G2 = nullptr, *grad = nullptr;
-  double* part = nullptr;
-  int nparts = 0;
+  void* base = nullptr;  // the allocation that holds the arrays
+  float *Z1 = nullptr, *H1 = nullptr, *Z2 = nullptr, *H2 = nullptr, *dY = nullptr;
+  float *G1 = nullptr, *G2 = nullptr;
+  float* ws = nullptr;     // [GRAD_SPLITS][parameters] partial gradients
+  double* part = nullptr;  // loss partials, one per 64 rows
 };
 
 extern "C" int zm_mlp_forward_bf16(void* stream, int32_t ncol, const void* X, const void* W1, const float* b1,
@@ -562,74 +742,86 @@ extern "C" int zm_mlp_trainer_create(int32_t batch_max, zm_mlp_trainer** out) {
   if (!out || batch_max < 1) return ZM_ERR_INVALID;
   zm_mlp_trainer* tr = new zm_mlp_trainer();
   tr->batch_max = batch_max;
-  tr->nparts = 256;
-  const size_t h = (size_t)batch_max * MK, o = (size_t)batch_max * MO;
-  float** bufs[] = {&tr->Z1, &tr->H1, &tr->Z2, &tr->H2, &tr->G1, &tr->G2};
-  bool ok = true;
-  for (float** b : bufs) ok = ok && cudaMalloc(b, h * sizeof(float)) == cudaSuccess;
-  ok = ok && cudaMalloc(&tr->Y, o * sizeof(float)) == cudaSuccess;
-  ok = ok && cudaMalloc(&tr->dY, o * sizeof(float)) == cudaSuccess;
-  ok = ok && cudaMalloc(&tr->grad, (size_t)ZM_MLP_NPARAMS * sizeof(float)) == cudaSuccess;
-  ok = ok && cudaMalloc(&tr->part, (size_t)tr->nparts * sizeof(double)) == cudaSuccess;
-  if (!ok) {
-    zm_mlp_trainer_destroy(tr);
+  // one allocation, each array a multiple of 16 bytes: separate ones made a new trainer's first step slower
+  const size_t h = (size_t)batch_max * MK, o = (size_t)batch_max * MO, w = (size_t)GRAD_SPLITS * ZM_MLP_NPARAMS;
+  const size_t np = ((size_t)batch_max + 63) / 64;
+  if (cudaMalloc(&tr->base, (6 * h + o + w) * sizeof(float) + np * sizeof(double)) != cudaSuccess) {
+    delete tr;
     return ZM_ERR_CUDA;
   }
+  float* f = static_cast<float*>(tr->base);
+  float** bufs[] = {&tr->Z1, &tr->H1, &tr->Z2, &tr->H2, &tr->G1, &tr->G2};
+  for (float** b : bufs) {
+    *b = f;
+    f += h;
+  }
+  tr->dY = f;
+  tr->ws = f + o;
+  tr->part = reinterpret_cast<double*>(tr->ws + w);
   *out = tr;
   return ZM_OK;
 }
 
 extern "C" void zm_mlp_trainer_destroy(zm_mlp_trainer* tr) {
   if (!tr) return;
-  float* bufs[] = {tr->Z1, tr->H1, tr->Z2, tr->H2, tr->G1, tr->G2, tr->Y, tr->dY, tr->grad};
-  for (float* b : bufs) cudaFree(b);
-  cudaFree(tr->part);
+  cudaFree(tr->base);
   delete tr;
 }
 
-// forward pass of one batch (float32), keeping the pre-activations for the
-// backward pass
-static int mlp_forward_train(zm_mlp_trainer* tr, cudaStream_t st, int B, const float* X, const float* P) {
-  const long long nh = (long long)B * MK;
-  sgemm(st, B, MK, MK, X, 0, P + Off::W1, 1, P + Off::b1, tr->Z1);
-  k_gelu_fwd<<<512, 256, 0, st>>>(tr->Z1, tr->H1, nh);
-  sgemm(st, B, MK, MK, tr->H1, 0, P + Off::W2, 1, P + Off::b2, tr->Z2);
-  k_gelu_fwd<<<512, 256, 0, st>>>(tr->Z2, tr->H2, nh);
-  sgemm(st, B, MO, MK, tr->H2, 0, P + Off::W3, 1, P + Off::b3, tr->Y);
-  return launch_ok("mlp forward") ? ZM_OK : ZM_ERR_CUDA;
+// Forward and backward pass of one batch into the partial gradients.  A
+// 128-row tile where its blocks come near the SM count, else 64-row tiles
+// (four times the blocks; at 500 rows 128-row tiles fill 8 SMs).  Returns the
+// split count, or 0 after a launch failure.
+static int mlp_passes(zm_mlp_trainer* tr, cudaStream_t st, int B, const float* X, const float* T, const float* Mk,
+                      const float* P, double count) {
+  const bool vx = vec16(X), vp = vec16(P);
+  const float *W1 = P + Off::W1, *W2 = P + Off::W2, *W3 = P + Off::W3;
+  const float *b1 = P + Off::b1, *b2 = P + Off::b2, *b3 = P + Off::b3;
+  const bool big = B >= 4096;
+  const int bt = big ? 128 : 64;
+  const dim3 g(MK / bt, (B + bt - 1) / bt);
+  const float ic = (float)(1.0 / count);
+  if (big) {
+    k_layer_fwd<128><<<g, 256, 0, st>>>(B, X, vx, W1, vp, b1, tr->Z1, tr->H1);
+    k_layer_fwd<128><<<g, 256, 0, st>>>(B, tr->H1, true, W2, vp, b2, tr->Z2, tr->H2);
+  } else {
+    k_layer_fwd<64><<<g, 256, 0, st>>>(B, X, vx, W1, vp, b1, tr->Z1, tr->H1);
+    k_layer_fwd<64><<<g, 256, 0, st>>>(B, tr->H1, true, W2, vp, b2, tr->Z2, tr->H2);
+  }
+  k_layer_out<<<(B + 63) / 64, 256, 0, st>>>(B, tr->H2, W3, vp, b3, T, vec16(T), Mk, vec16(Mk), ic, tr->dY, tr->part);
+  if (big) {
+    k_layer_bwd<128><<<g, 256, 0, st>>>(B, MO, tr->dY, W3, vp, tr->Z2, tr->G2);
+    k_layer_bwd<128><<<g, 256, 0, st>>>(B, MK, tr->G2, W2, vp, tr->Z1, tr->G1);
+  } else {
+    k_layer_bwd<64><<<g, 256, 0, st>>>(B, MO, tr->dY, W3, vp, tr->Z2, tr->G2);
+    k_layer_bwd<64><<<g, 256, 0, st>>>(B, MK, tr->G2, W2, vp, tr->Z1, tr->G1);
+  }
+  // splits of whole slabs, none empty
+  const int per = ((B + GRAD_SPLITS - 1) / GRAD_SPLITS + GK - 1) / GK * GK;
+  const int splits = (B + per - 1) / per;
+  GradArgs a{};
+  a.l[0] = GradLayer{tr->G1, X, MK, vx, Off::W1, Off::b1};
+  a.l[1] = GradLayer{tr->G2, tr->H1, MK, true, Off::W2, Off::b2};
+  a.l[2] = GradLayer{tr->dY, tr->H2, MO, true, Off::W3, Off::b3};
+  a.rows = B;
+  a.per_split = per;
+  a.ws = tr->ws;
+  k_layer_grads<<<dim3(GRAD_TILES, splits), 256, 0, st>>>(a);
+  return launch_ok("mlp passes") ? splits : 0;
 }
 
-// masked mean-square loss and the gradient of every parameter into tr->grad
-static int mlp_backward(zm_mlp_trainer* tr, cudaStream_t st, int B, const float* X, const float* T, const float* Mk,
-                        const float* P, double count, double* loss) {
-  const float *W2 = P + Off::W2, *W3 = P + Off::W3;
-  float* g = tr->grad;
-  const long long nh = (long long)B * MK, no = (long long)B * MO;
-  k_mse<<<tr->nparts, 256, 0, st>>>(tr->Y, T, Mk, tr->dY, no, (float)(1.0 / count), tr->part);
-  // layer 3
-  sgemm(st, MO, MK, B, tr->dY, 1, tr->H2, 0, nullptr, g + Off::W3);
-  k_colsum<<<1, MO, 0, st>>>(tr->dY, B, MO, g + Off::b3);
-  sgemm(st, B, MK, MO, tr->dY, 0, W3, 0, nullptr, tr->G2);
-  k_gelu_bwd<<<512, 256, 0, st>>>(tr->Z2, tr->G2, nh);
-  // layer 2
-  sgemm(st, MK, MK, B, tr->G2, 1, tr->H1, 0, nullptr, g + Off::W2);
-  k_colsum<<<1, MK, 0, st>>>(tr->G2, B, MK, g + Off::b2);
-  sgemm(st, B, MK, MK, tr->G2, 0, W2, 0, nullptr, tr->G1);
-  k_gelu_bwd<<<512, 256, 0, st>>>(tr->Z1, tr->G1, nh);
-  // layer 1
-  sgemm(st, MK, MK, B, tr->G1, 1, X, 0, nullptr, g + Off::W1);
-  k_colsum<<<1, MK, 0, st>>>(tr->G1, B, MK, g + Off::b1);
-  if (!launch_ok("mlp backward")) return ZM_ERR_CUDA;
-  if (loss) {
-    double parts[256];
-    if (cudaMemcpyAsync(parts, tr->part, (size_t)tr->nparts * sizeof(double), cudaMemcpyDeviceToHost, st) !=
-            cudaSuccess ||
+// the batch loss from the blocks' partial sums (synchronizes the stream)
+static int mlp_loss(zm_mlp_trainer* tr, cudaStream_t st, int B, double count, double* loss) {
+  double parts[1024], s = 0.0;
+  const int n = (B + 63) / 64;
+  for (int q = 0; q < n; q += 1024) {
+    const int c = n - q < 1024 ? n - q : 1024;
+    if (cudaMemcpyAsync(parts, tr->part + q, c * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
       return ZM_ERR_CUDA;
-    double s = 0.0;
-    for (int q = 0; q < tr->nparts; ++q) s += parts[q];
-    *loss = s / count;
+    for (int e = 0; e < c; ++e) s += parts[e];
   }
+  *loss = s / count;
   return ZM_OK;
 }
 
@@ -638,13 +830,12 @@ extern "C" int zm_mlp_grad(zm_mlp_trainer* tr, void* stream, int32_t batch, cons
   if (!tr || batch < 1 || batch > tr->batch_max || !X || !T || !M || !params || !grad_out || !(mask_count > 0))
     return ZM_ERR_INVALID;
   cudaStream_t st = (cudaStream_t)stream;
-  int rc = mlp_forward_train(tr, st, batch, X, params);
-  if (rc == ZM_OK) rc = mlp_backward(tr, st, batch, X, T, M, params, mask_count, loss);
-  if (rc == ZM_OK &&
-      cudaMemcpyAsync(grad_out, tr->grad, (size_t)ZM_MLP_NPARAMS * sizeof(float), cudaMemcpyDeviceToDevice, st) !=
-          cudaSuccess)
-    rc = ZM_ERR_CUDA;
-  return rc;
+  const int splits = mlp_passes(tr, st, batch, X, T, M, params, mask_count);
+  if (splits == 0) return ZM_ERR_CUDA;
+  k_fold<<<(ZM_MLP_NPARAMS + 255) / 256, 256, 0, st>>>(tr->ws, splits, grad_out, nullptr, nullptr, nullptr, 0.f, 0.f,
+                                                       0.f, 0.f, 1.f, 1.f);
+  if (!launch_ok("zm_mlp_grad")) return ZM_ERR_CUDA;
+  return loss ? mlp_loss(tr, st, batch, mask_count, loss) : ZM_OK;
 }
 
 extern "C" int zm_mlp_train_step(zm_mlp_trainer* tr, void* stream, int32_t batch, const float* X, const float* T,
@@ -654,10 +845,11 @@ extern "C" int zm_mlp_train_step(zm_mlp_trainer* tr, void* stream, int32_t batch
       !(mask_count > 0))
     return ZM_ERR_INVALID;
   cudaStream_t st = (cudaStream_t)stream;
-  int rc = mlp_forward_train(tr, st, batch, X, params);
-  if (rc == ZM_OK) rc = mlp_backward(tr, st, batch, X, T, M, params, mask_count, loss);
-  if (rc != ZM_OK) return rc;
+  const int splits = mlp_passes(tr, st, batch, X, T, M, params, mask_count);
+  if (splits == 0) return ZM_ERR_CUDA;
   const float c1 = 1.f - powf(beta1, (float)step), c2 = 1.f - powf(beta2, (float)step);
-  k_adam<<<512, 256, 0, st>>>(params, tr->grad, adam_m, adam_v, ZM_MLP_NPARAMS, lr, beta1, beta2, eps, c1, c2);
-  return launch_ok("zm_mlp_train_step") ? ZM_OK : ZM_ERR_CUDA;
+  k_fold<<<(ZM_MLP_NPARAMS + 255) / 256, 256, 0, st>>>(tr->ws, splits, nullptr, params, adam_m, adam_v, lr, beta1,
+                                                       beta2, eps, c1, c2);
+  if (!launch_ok("zm_mlp_train_step")) return ZM_ERR_CUDA;
+  return loss ? mlp_loss(tr, st, batch, mask_count, loss) : ZM_OK;
 }
