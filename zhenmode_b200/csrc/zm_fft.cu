@@ -136,12 +136,11 @@ __global__ void __launch_bounds__(256) k_dealias_lon(Dev d, FftPlan plan, const 
   const int n = plan.n;
   float2* bufa = fsm;
   float2* bufb = bufa + (size_t)lines_per_block * n;
-  const int total = d.ny * d.nz;
   const int first = blockIdx.x * lines_per_block;
-  const int lines = min(lines_per_block, total - first);
+  const int lines = min(lines_per_block, plan.nlines - first);
   if (lines <= 0) return;
   for (int l = 0; l < lines; ++l) {
-    const int line = first + l;
+    const int line = __ldg(plan.lines + first + l);
     const int k = line / d.ny, j = line - k * d.ny;
     const long long row = idx3(d, k, j, 0);
     for (int i = threadIdx.x; i < n; i += blockDim.x) bufa[l * n + i] = make_float2(ld(Ayu, row + i), ld(Ayv, row + i));
@@ -163,7 +162,7 @@ __global__ void __launch_bounds__(256) k_dealias_lon(Dev d, FftPlan plan, const 
   const float wind_s = 1.f / (kRho0 * d.dz_surface);
   const float wind_bt = 1.f / (kRho0 * d.H_sw);
   for (int l = 0; l < lines; ++l) {
-    const int line = first + l;
+    const int line = __ldg(plan.lines + first + l);
     const int k = line / d.ny, j = line - k * d.ny;
     const long long row = idx3(d, k, j, 0);
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -316,8 +315,9 @@ __global__ void __launch_bounds__(reg_threads<N1, N2, N3>() * 4) k_dealias_reg(D
   extern __shared__ float2 xsm[];
   float2* ex = xsm + threadIdx.y * N;  // this line's exchange buffer
   const int t = threadIdx.x;
-  const int line = blockIdx.x * blockDim.y + threadIdx.y;
-  const bool live = line < d.ny * d.nz;
+  const int slot = blockIdx.x * blockDim.y + threadIdx.y;
+  const bool live = slot < plan.nlines;
+  const int line = live ? __ldg(plan.lines + slot) : 0;
   const int k = live ? line / d.ny : 0, j = live ? line - k * d.ny : 0;
   const long long row = idx3(d, k, j, 0);
   const float2* tw = plan.tw_full;
@@ -435,8 +435,7 @@ template <int N1, int N2, int N3>
 static cudaError_t launch_reg(cudaStream_t s, const Dev& d, const FftPlan& plan, const float* Ayu, const float* Ayv,
                               float* Au, float* Av, int lines, bool pdl) {
   constexpr int T = reg_threads<N1, N2, N3>();
-  const int nlines = d.ny * d.nz;
-  const dim3 g((nlines + lines - 1) / lines), b(T, lines);
+  const dim3 g((plan.nlines + lines - 1) / lines), b(T, lines);
   const size_t smem = (size_t)lines * N1 * N2 * N3 * sizeof(float2);
   if (pdl) return launch_pdl(k_dealias_reg<N1, N2, N3>, g, b, smem, s, d, plan, Ayu, Ayv, Au, Av);
   k_dealias_reg<N1, N2, N3><<<g, b, smem, s>>>(d, plan, Ayu, Ayv, Au, Av);
@@ -445,6 +444,7 @@ static cudaError_t launch_reg(cudaStream_t s, const Dev& d, const FftPlan& plan,
 
 cudaError_t launch_dealias(cudaStream_t s, const Dev& d, const FftPlan& plan, const float* Ayu, const float* Ayv,
                            float* Au, float* Av, int lines, size_t stockham_smem, bool pdl) {
+  if (plan.nlines == 0) return cudaSuccess;
   if (plan.r1 > 0) {
     const int l = lines >= 4 ? 4 : (lines >= 2 ? 2 : 1);
     if (plan.n == 720) return launch_reg<8, 9, 10>(s, d, plan, Ayu, Ayv, Au, Av, l, pdl);
@@ -452,8 +452,7 @@ cudaError_t launch_dealias(cudaStream_t s, const Dev& d, const FftPlan& plan, co
     if (plan.n == 360) return launch_reg<4, 9, 10>(s, d, plan, Ayu, Ayv, Au, Av, l, pdl);
     if (plan.n == 180) return launch_reg<4, 9, 5>(s, d, plan, Ayu, Ayv, Au, Av, l, pdl);
   }
-  const int nlines = d.ny * d.nz;
-  const dim3 g((nlines + lines - 1) / lines), b(256);
+  const dim3 g((plan.nlines + lines - 1) / lines), b(256);
   if (pdl) return launch_pdl(k_dealias_lon, g, b, stockham_smem, s, d, plan, Ayu, Ayv, Au, Av, lines);
   k_dealias_lon<<<g, b, stockham_smem, s>>>(d, plan, Ayu, Ayv, Au, Av, lines);
   return cudaGetLastError();

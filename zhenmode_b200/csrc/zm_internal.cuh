@@ -61,6 +61,11 @@ struct Dev {
   const float* wet2;           // 2-D wet mask (barotropic mode)
   const uint64_t* wbits;       // 3-D wet mask, one word per column
   const unsigned char* nu_gate; // 3-D [nz][ny][P] face gates of the nu_h Laplacian (k_nu_gates)
+  const unsigned char* nu_class; // class of each strip of the nu_h tiles (k_nu_class)
+  // wet levels of column tiles, one word per tile: the union of the columns' words over the tile and
+  // a two-cell ring.  A level whose bit is clear has no wet point that a tile cell could reach.
+  const uint64_t* tile8;       // 32 x 8 tiles [(ny + 7) / 8][(nx + 31) / 32]
+  const uint64_t* tile4;       // 32 x 4 tiles
   const float* kh2;            // kappa_h + coastal kappa_h
   const float* kv2;            // kappa_v + coastal kappa_v
   const float* tau_x;
@@ -85,6 +90,7 @@ struct Dev {
   // block of the tracer-advection and linear-step column marches, tile rows
   // of the pressure-gradient and vertical-transport marches
   int ta_kc, lt_kc, pg_rows, fz_rows;
+  int dx_rows;                 // 1: dx is constant along every row (inv_dx2 of a row is its first value)
   Vert vc;
 };
 
@@ -99,6 +105,8 @@ __device__ __forceinline__ int south(int j) { return j > 0 ? j - 1 : 0; }
 __device__ __forceinline__ float wetf(uint64_t bits, int k) { return (float)((bits >> k) & 1ull); }
 __device__ __forceinline__ bool wetb(uint64_t bits, int k) { return (bits >> k) & 1ull; }
 __device__ __forceinline__ int kbot_of(uint64_t bits) { return bits ? 63 - __clzll((long long)bits) : 0; }
+// levels of a tile down to its deepest wet one (0: no wet level)
+__device__ __forceinline__ int levels_of(uint64_t bits) { return bits ? 64 - __clzll((long long)bits) : 0; }
 __device__ __forceinline__ uint64_t wb(const Dev& d, int j, int i) { return __ldg(d.wbits + idx2(d, j, i)); }
 __device__ __forceinline__ float ld(const float* p, long long i) { return __ldg(p + i); }
 

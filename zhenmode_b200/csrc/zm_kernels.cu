@@ -118,29 +118,58 @@ __device__ __forceinline__ float colv(const float* __restrict__ a, long long bas
 // The Laplacian of numerics/horizontal.py:181-215 is rewritten per point as
 //   lap = aE (uE - u0) + aW (uW - u0) + aN (uN - u0) + aS (uS - u0)
 // with aE/aW the gated x faces times 1/dx^2, aN = cN - t, aS = cS + t
-// (cN/cS the gated y faces times 1/dy^2, t = tan(lat)/(2 R dy) from the
+// (cN/cS the gated y faces times 1/dy^2, t = tan(lat)/(2R dy) from the
 // metric term -(tan(lat)/R) du/dy), and the mirror ghost of the closed
 // walls folded in: at j = ny-1 the north neighbour equals u0, so aN = 0; at
-// j = 0, aS = 0.  The coefficients, scaled by nu_h dt_sub, are formed once
-// per pass from the face gates of the cell (k_nu_gates, built once per
-// solver: one byte per point) and per-row constants, so the set-up needs
-// no neighbour wet flags.  Longitude wraps.  The lane's two columns are held
-// as packed pairs, so the update runs on the paired FP32 instructions
-// (__ffma2_rn, __fadd2_rn; the same roundings as the scalar form).  Points
-// of the tile edge see their own values as the missing neighbours (their
-// results are discarded with the halo).
+// j = 0, aS = 0.  Longitude wraps.  The lane's two columns are held as packed
+// pairs, so the update runs on the paired FP32 instructions (__ffma2_rn).
+// Points of the tile edge see their own values as the missing neighbours
+// (their results are discarded with the halo).
+//
+// What bounds the kernel is instruction issue and the latency of its short
+// phases (set-up, a barrier per subcycle), so each warp does only what its strip
+// needs, by a class formed once per solver and launch shape (k_nu_class):
+//  * open: every face of the strip's cells is open and dx is constant along
+//    the rows.  The coefficients are then three numbers a row, read from shared
+//    memory; the second difference in x takes two operations and the
+//    difference in y is shared by the two rows it joins: 6 paired operations a
+//    row and field where the gated form takes 9, and no coefficient set-up;
+//  * gated: the general form, coefficients from the face gates of the cell
+//    (k_nu_gates, one byte per point);
+//  * dead: no cell is within reach of a wet cell in the subcycles left.  A dry
+//    cell's value moves only along its column of latitudes (its faces are
+//    closed; the metric term reads the rows above and below), one row per
+//    subcycle, so a strip whose cells are all at least `left` rows from the
+//    next wet one cannot change a wet point any more: it keeps its values and
+//    its warp leaves the barriers.
+// At 720x360x50 (40 % of the points dry: 37 % of the strips dead, 47 % open) a
+// launch of 6 subcycles went from 150 to 127 us, 98 to 72 M warp instructions;
+// issue-active fell from 60 to 47 %, barrier and shared-memory waits lead.
+// Strips of 4 rows with twice the warps took 138 us, coefficients formed from
+// gate bits at 64 registers (4 blocks per SM) 131 us: occupancy is not the bound.
+constexpr unsigned NU_OPEN = 16u;  // class byte: bits 0-3 the strip's distance class, bit 4 open
+
 template <int NW>
 __global__ void __launch_bounds__(32 * NW, 16 / NW)
 k_nu_tb(Dev d, const float* __restrict__ u, const float* __restrict__ v, float* __restrict__ uo,
-        float* __restrict__ vo, float c, int nsub, int halo) {
+        float* __restrict__ vo, float c, int nsub, int halo, int left) {
   constexpr int NH = NW * NB_R;                   // tile rows
   const int TI = NB_W - 2 * halo, TJ = NH - 2 * halo;
-  __shared__ float4 edge[2][NW][2][32];           // [parity][warp][0 bottom row, 1 top row][lane]
+  extern __shared__ float4 nu_smem[];
+  auto edge = reinterpret_cast<float4 (*)[NW][2][32]>(nu_smem);  // [parity][warp][0 bottom row, 1 top row][lane]
+  // open faces of a row: aE = aW and aN as pairs, then -aS as a pair
+  float4* rowc = nu_smem + 2 * NW * 2 * 32;
+  float2* rows = reinterpret_cast<float2*>(rowc + NH);
   pdl_trigger();
   const int lane = threadIdx.x, wp = threadIdx.y;
   const int k = blockIdx.z;
   const int gx0 = blockIdx.x * TI - halo, gy0 = blockIdx.y * TJ - halo;
   const int c0 = 2 * lane, r0 = wp * NB_R;
+  const unsigned char* tile_cls = d.nu_class + ((k * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * NW;
+  const unsigned cls = __ldg(tile_cls + wp);
+  const bool dead = 2 * (int)(cls & 15u) >= left, open = !dead && (cls & NU_OPEN) != 0u;
+  // the threads that meet at the barriers: the warps of strips that are not dead
+  const int live = 32 * __popc(__ballot_sync(0xffffffffu, lane < NW && 2 * (int)(__ldg(tile_cls + lane % NW) & 15u) < left));
   int gi[2];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -148,81 +177,126 @@ k_nu_tb(Dev d, const float* __restrict__ u, const float* __restrict__ v, float* 
     gi[h] = g < 0 ? g + d.nx : g;
   }
   const long long kb = (long long)k * d.plane;
-  const float cn = d.nu_h * c;
-  // face coefficients, paired like the state: (column 2l, column 2l+1).  The
-  // west and south ones are held negated (nW = -aW, nS = -aS) and negated back
-  // in the update, an exact round trip: ptxas 12.9 allocates this form's
-  // registers differently, and it ran 4 % faster than holding aW, aS.
-  float2 kE[NB_R], nW[NB_R], kN[NB_R], nS[NB_R];
-#pragma unroll
-  for (int q = 0; q < NB_R; ++q) {
-    const int gj = gy0 + r0 + q;
-    const int gjc = gj < 0 ? 0 : (gj >= d.ny ? d.ny - 1 : gj);
-    const bool n_in = gj < d.ny - 1;  // north neighbour inside the domain
-    const bool s_in = gj > 0;
-    const float t = 0.5f * d.inv_dy * __ldg(d.tanR + gjc);
-    // aN with the north face open / closed, aS likewise (0 beyond the walls)
-    const float n1 = n_in ? (d.inv_dy2 - t) * cn : 0.f, n0 = n_in ? (0.f - t) * cn : 0.f;
-    const float s1 = s_in ? (d.inv_dy2 + t) * cn : 0.f, s0 = s_in ? (0.f + t) * cn : 0.f;
-    float ce[2], cw[2], cnn[2], cs[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int id2 = idx2(d, gjc, gi[h]);
-      const unsigned g = __ldg(d.nu_gate + kb + id2);
-      const float ax = __ldg(d.inv_dx2 + id2) * cn;
-      ce[h] = (g & 1u) ? ax : 0.f;
-      cw[h] = (g & 2u) ? ax : 0.f;
-      cnn[h] = (g & 4u) ? n1 : n0;
-      cs[h] = (g & 8u) ? s1 : s0;
-    }
-    kE[q] = make_float2(ce[0], ce[1]);
-    nW[q] = make_float2(-cw[0], -cw[1]);
-    kN[q] = make_float2(cnn[0], cnn[1]);
-    nS[q] = make_float2(-cs[0], -cs[1]);
-  }
   const unsigned full = 0xffffffffu;
+  // every lane's column pair starts on an even column and does not straddle the seam: 8-byte accesses
+  const bool pairs = ((gx0 | d.nx | halo) & 1) == 0;
   pdl_wait();  // u, v come from the preceding kernel
   // the lane's two columns as pairs: au[q] = (u[2l], u[2l+1]) of row q, av likewise
   float2 au[NB_R], av[NB_R];
 #pragma unroll
   for (int q = 0; q < NB_R; ++q) {
-    int gj = gy0 + r0 + q;
-    gj = gj < 0 ? 0 : (gj >= d.ny ? d.ny - 1 : gj);
-    const long long id0 = kb + (long long)gj * d.P + gi[0], id1 = kb + (long long)gj * d.P + gi[1];
-    au[q] = make_float2(ld(u, id0), ld(u, id1));
-    av[q] = make_float2(ld(v, id0), ld(v, id1));
+    const int gj = min(max(gy0 + r0 + q, 0), d.ny - 1);
+    const float *ru = u + kb + gj * d.P, *rv = v + kb + gj * d.P;
+    if (pairs) {
+      au[q] = __ldg(reinterpret_cast<const float2*>(ru + gi[0]));
+      av[q] = __ldg(reinterpret_cast<const float2*>(rv + gi[0]));
+    } else {
+      au[q] = make_float2(__ldg(ru + gi[0]), __ldg(ru + gi[1]));
+      av[q] = make_float2(__ldg(rv + gi[0]), __ldg(rv + gi[1]));
+    }
   }
-  const float2 m1 = make_float2(-1.f, -1.f);
-  for (int s = 0; s < nsub; ++s) {
+  const float cn = d.nu_h * c;
+  if (lane < NB_R) {  // this warp's rows
+    const int gj = min(max(gy0 + r0 + lane, 0), d.ny - 1);
+    const float t = 0.5f * d.inv_dy * __ldg(d.tanR + gj);
+    const float ax = __ldg(d.inv_dx2 + idx2(d, gj, 0)) * cn, an = (d.inv_dy2 - t) * cn, as = -((d.inv_dy2 + t) * cn);
+    rowc[r0 + lane] = make_float4(ax, ax, an, an);
+    rows[r0 + lane] = make_float2(as, as);
+  }
+  __syncwarp();
+  // gated form: face coefficients, paired like the state: (column 2l, column 2l+1)
+  float2 kE[NB_R], kW[NB_R], kN[NB_R], kS[NB_R];
+  if (!dead && !open) {
+#pragma unroll
+    for (int q = 0; q < NB_R; ++q) {
+      const int gj = gy0 + r0 + q;
+      const int gjc = gj < 0 ? 0 : (gj >= d.ny ? d.ny - 1 : gj);
+      const bool n_in = gj < d.ny - 1;  // north neighbour inside the domain
+      const bool s_in = gj > 0;
+      const float t = 0.5f * d.inv_dy * __ldg(d.tanR + gjc);
+      // aN with the north face open / closed, aS likewise (0 beyond the walls)
+      const float n1 = n_in ? (d.inv_dy2 - t) * cn : 0.f, n0 = n_in ? (0.f - t) * cn : 0.f;
+      const float s1 = s_in ? (d.inv_dy2 + t) * cn : 0.f, s0 = s_in ? (0.f + t) * cn : 0.f;
+      float ce[2], cw[2], cnn[2], cs[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int id2 = idx2(d, gjc, gi[h]);
+        const unsigned g = __ldg(d.nu_gate + kb + id2);
+        const float ax = __ldg(d.inv_dx2 + id2) * cn;
+        ce[h] = (g & 1u) ? ax : 0.f;
+        cw[h] = (g & 2u) ? ax : 0.f;
+        cnn[h] = (g & 4u) ? n1 : n0;
+        cs[h] = (g & 8u) ? s1 : s0;
+      }
+      kE[q] = make_float2(ce[0], ce[1]);
+      kW[q] = make_float2(cw[0], cw[1]);
+      kN[q] = make_float2(cnn[0], cnn[1]);
+      kS[q] = make_float2(cs[0], cs[1]);
+    }
+  }
+  const float2 m1 = make_float2(-1.f, -1.f), m2 = make_float2(-2.f, -2.f);
+  if (dead) {  // its neighbours read the same edge rows in every subcycle
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      edge[p][wp][0][lane] = make_float4(au[0].x, au[0].y, av[0].x, av[0].y);
+      edge[p][wp][1][lane] = make_float4(au[NB_R - 1].x, au[NB_R - 1].y, av[NB_R - 1].x, av[NB_R - 1].y);
+    }
+  }
+  if (live < 32 * NW) __syncthreads();
+  for (int s = 0; s < (dead ? 0 : nsub); ++s) {
     const int p = s & 1;
     edge[p][wp][0][lane] = make_float4(au[0].x, au[0].y, av[0].x, av[0].y);
     edge[p][wp][1][lane] = make_float4(au[NB_R - 1].x, au[NB_R - 1].y, av[NB_R - 1].x, av[NB_R - 1].y);
-    __syncthreads();
+    asm volatile("bar.sync 1, %0;" ::"r"(live) : "memory");
     // rows just outside the strip (the tile edge reuses the strip's own row)
     const float4 nt = edge[p][wp + 1 < NW ? wp + 1 : wp][wp + 1 < NW ? 0 : 1][lane];
     const float4 sb = edge[p][wp > 0 ? wp - 1 : wp][wp > 0 ? 1 : 0][lane];
+    if (open) {
+      float2 du = __ffma2_rn(make_float2(sb.x, sb.y), m1, au[0]), dv = __ffma2_rn(make_float2(sb.z, sb.w), m1, av[0]);
+#pragma unroll
+      for (int q = 0; q < NB_R; ++q) {
+        const float4 rc = rowc[r0 + q];
+        const float2 ax = make_float2(rc.x, rc.y), an = make_float2(rc.z, rc.w), as = rows[r0 + q];
+        // east of (2l, 2l+1) is (2l+1, 2l+2), west is (2l-1, 2l); the outside columns come from the neighbouring
+        // lanes (lanes 0 and 31 get their own values: tile-edge error)
+        const float2 xu = __fadd2_rn(make_float2(au[q].y, __shfl_down_sync(full, au[q].x, 1)),
+                                     make_float2(__shfl_up_sync(full, au[q].y, 1), au[q].x));
+        const float2 xv = __fadd2_rn(make_float2(av[q].y, __shfl_down_sync(full, av[q].x, 1)),
+                                     make_float2(__shfl_up_sync(full, av[q].y, 1), av[q].x));
+        const float2 nu = q + 1 < NB_R ? au[q + 1 < NB_R ? q + 1 : q] : make_float2(nt.x, nt.y);
+        const float2 nv = q + 1 < NB_R ? av[q + 1 < NB_R ? q + 1 : q] : make_float2(nt.z, nt.w);
+        // u0 + ax (uE + uW - 2 u0) + aN (uN - u0) - aS (u0 - uS)
+        const float2 gu = __ffma2_rn(au[q], m1, nu), gv = __ffma2_rn(av[q], m1, nv);
+        float2 ou = __ffma2_rn(ax, __ffma2_rn(m2, au[q], xu), au[q]);
+        float2 ov = __ffma2_rn(ax, __ffma2_rn(m2, av[q], xv), av[q]);
+        ou = __ffma2_rn(as, du, ou);
+        ov = __ffma2_rn(as, dv, ov);
+        au[q] = __ffma2_rn(an, gu, ou);
+        av[q] = __ffma2_rn(an, gv, ov);
+        du = gu;
+        dv = gv;
+      }
+      continue;
+    }
     float2 su = make_float2(sb.x, sb.y), sv = make_float2(sb.z, sb.w);
 #pragma unroll
     for (int q = 0; q < NB_R; ++q) {
       const float2 nu = q + 1 < NB_R ? au[q + 1] : make_float2(nt.x, nt.y);
       const float2 nv = q + 1 < NB_R ? av[q + 1] : make_float2(nt.z, nt.w);
-      // east of (2l, 2l+1) is (2l+1, 2l+2), west is (2l-1, 2l); the outside
-      // columns come from the neighbouring lanes (lanes 0 and 31 get their
-      // own values: tile-edge error)
       const float2 eu = make_float2(au[q].y, __shfl_down_sync(full, au[q].x, 1));
       const float2 wu = make_float2(__shfl_up_sync(full, au[q].y, 1), au[q].x);
       const float2 ev = make_float2(av[q].y, __shfl_down_sync(full, av[q].x, 1));
       const float2 wv = make_float2(__shfl_up_sync(full, av[q].y, 1), av[q].x);
-      // u0 + aE (uE - u0) + aW (uW - u0) + aN (uN - u0) + aS (uS - u0) on packed pairs
+      // u0 + aE (uE - u0) + aW (uW - u0) + aN (uN - u0) + aS (uS - u0)
       const float2 ncu = __fmul2_rn(au[q], m1), ncv = __fmul2_rn(av[q], m1);
       float2 ou = __ffma2_rn(kE[q], __fadd2_rn(eu, ncu), au[q]);
       float2 ov = __ffma2_rn(kE[q], __fadd2_rn(ev, ncv), av[q]);
-      ou = __ffma2_rn(make_float2(-nW[q].x, -nW[q].y), __fadd2_rn(wu, ncu), ou);
-      ov = __ffma2_rn(make_float2(-nW[q].x, -nW[q].y), __fadd2_rn(wv, ncv), ov);
+      ou = __ffma2_rn(kW[q], __fadd2_rn(wu, ncu), ou);
+      ov = __ffma2_rn(kW[q], __fadd2_rn(wv, ncv), ov);
       ou = __ffma2_rn(kN[q], __fadd2_rn(nu, ncu), ou);
       ov = __ffma2_rn(kN[q], __fadd2_rn(nv, ncv), ov);
-      ou = __ffma2_rn(make_float2(-nS[q].x, -nS[q].y), __fadd2_rn(su, ncu), ou);
-      ov = __ffma2_rn(make_float2(-nS[q].x, -nS[q].y), __fadd2_rn(sv, ncv), ov);
+      ou = __ffma2_rn(kS[q], __fadd2_rn(su, ncu), ou);
+      ov = __ffma2_rn(kS[q], __fadd2_rn(sv, ncv), ov);
       su = au[q];
       sv = av[q];
       au[q] = ou;
@@ -230,21 +304,74 @@ k_nu_tb(Dev d, const float* __restrict__ u, const float* __restrict__ v, float* 
     }
   }
   // write the exact interior
+  const bool in0 = c0 >= halo && c0 < NB_W - halo && gx0 + c0 < d.nx;
+  const bool in1 = c0 + 1 >= halo && c0 + 1 < NB_W - halo && gx0 + c0 + 1 < d.nx;
 #pragma unroll
   for (int q = 0; q < NB_R; ++q) {
-    const int r = r0 + q;
-    const int gj = gy0 + r;
+    const int r = r0 + q, gj = gy0 + r;
     if (r < halo || r >= NH - halo || gj >= d.ny) continue;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int col = c0 + h;
-      const int ix = gx0 + col;
-      if (col < halo || col >= NB_W - halo || ix >= d.nx) continue;
-      const long long id = kb + (long long)gj * d.P + ix;
-      uo[id] = h == 0 ? au[q].x : au[q].y;
-      vo[id] = h == 0 ? av[q].x : av[q].y;
+    float *ru = uo + kb + gj * d.P + gx0 + c0, *rv = vo + kb + gj * d.P + gx0 + c0;
+    if (pairs) {
+      if (in0) {
+        *reinterpret_cast<float2*>(ru) = au[q];
+        *reinterpret_cast<float2*>(rv) = av[q];
+      }
+    } else {
+      if (in0) {
+        ru[0] = au[q].x;
+        rv[0] = av[q].x;
+      }
+      if (in1) {
+        ru[1] = au[q].y;
+        rv[1] = av[q].y;
+      }
     }
   }
+}
+
+// Class of every strip (NB_R rows of NB_W columns) of the nu_h tiles of one
+// launch shape: bits 0-3 half the distance in rows, rounded down and at most
+// 15, from the strip's nearest cell to the next wet cell of its column and
+// level (0: the strip holds a wet cell); bit 4 set when every face of its cells
+// is open and dx is constant along the rows.  One warp per strip; built once
+// per solver and launch shape.
+__global__ void k_nu_class(Dev d, unsigned char* __restrict__ cls, int nw, int halo, int gxn, int gyn) {
+  const int strip = blockIdx.x * blockDim.y + threadIdx.y;
+  if (strip >= d.nz * gyn * gxn * nw) return;
+  const int wp = strip % nw, bx = strip / nw % gxn, by = strip / nw / gxn % gyn, k = strip / nw / gxn / gyn;
+  const int gx0 = bx * (NB_W - 2 * halo) - halo, gy0 = by * (nw * NB_R - 2 * halo) - halo + wp * NB_R;
+  int dist = 30;
+  bool open = d.dx_rows != 0;
+  for (int h = 0; h < 2; ++h) {
+    int i = (gx0 + 2 * threadIdx.x + h) % d.nx;
+    if (i < 0) i += d.nx;
+    for (int q = 0; q < NB_R; ++q) {
+      const int gj = gy0 + q, j = min(max(gj, 0), d.ny - 1);
+      open = open && gj == j && (__ldg(d.nu_gate + idx3(d, k, j, i)) & 15u) == 15u;
+      for (int m = 0; m < dist; ++m)
+        if (wetb(wb(d, max(j - m, 0), i), k) || wetb(wb(d, min(j + m, d.ny - 1), i), k)) dist = m;
+    }
+  }
+  dist = __reduce_min_sync(0xffffffffu, dist);
+  open = __all_sync(0xffffffffu, open);
+  if (threadIdx.x == 0) cls[strip] = (unsigned char)((dist / 2) | (open ? NU_OPEN : 0u));
+}
+
+// Union of the wet words over RY-row tiles of 32 columns and their two-cell
+// ring (rows clamped, longitude wrapped); one warp per tile.
+__global__ void k_tile_bits(Dev d, uint64_t* __restrict__ out, int ry, int ntx, int nty) {
+  const int tile = blockIdx.x * blockDim.y + threadIdx.y;
+  if (tile >= ntx * nty) return;
+  const int i0 = tile % ntx * 32, j0 = tile / ntx * ry;
+  uint64_t any = 0ull;
+  for (int j = max(j0 - 2, 0); j < min(j0 + ry + 2, d.ny); ++j)
+    for (int o = threadIdx.x; o < 36; o += 32) {
+      int i = (i0 - 2 + o) % d.nx;
+      if (i < 0) i += d.nx;
+      any |= wb(d, j, i);
+    }
+  for (int o = 16; o > 0; o >>= 1) any |= __shfl_xor_sync(0xffffffffu, any, o);
+  if (threadIdx.x == 0) out[tile] = any;
 }
 
 // Face gates of the nu_h Laplacian, one byte per point (built once per
@@ -423,8 +550,11 @@ __global__ void __launch_bounds__(LT_X * LT_Y, 4) k_lin_t(Dev d, const float* __
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int tid = ty * LT_X + tx, nt = LT_X * LT_Y;
   const int i0 = blockIdx.x * LT_X, j0 = blockIdx.y * LT_Y;
-  const int k0 = blockIdx.z * d.lt_kc, k1 = min(d.nz, k0 + d.lt_kc);  // this block's levels
+  const int k0 = blockIdx.z * d.lt_kc, ke = min(d.nz, k0 + d.lt_kc);  // this block's levels
   const int i = i0 + tx, j = j0 + ty;
+  // the levels with a wet point in reach; below them only the dry velocities pass through
+  const int nk = levels_of(__ldg(d.tile8 + blockIdx.y * gridDim.x + blockIdx.x));
+  const int k1 = min(ke, nk);
   // threads outside the grid copy their tile cells, form their wet flags and
   // meet the barriers, nothing else
   const bool in = i < d.nx && j < d.ny;
@@ -440,6 +570,27 @@ __global__ void __launch_bounds__(LT_X * LT_Y, 4) k_lin_t(Dev d, const float* __
     (&t.ix[0][0])[e1] = __ldg(d.inv_dx + s1);
     (&t.ix2[0][0])[e1] = __ldg(d.inv_dx2 + s1);
   }
+  const int ic = in ? i : 0, jc = in ? j : 0;
+  const long long base = idx2(d, jc, ic);
+  const float rc = IMPL ? 0.f : __ldg(d.rot_c + base), rs = IMPL ? 0.f : __ldg(d.rot_s + base);
+  // dry levels below: u, v held and rotated (k_implicit_vdiff does both where it follows)
+  auto dry_levels = [&]() {
+    if constexpr (!IMPL) {
+      if (!in) return;
+#pragma unroll 5
+      for (int k = max(k0, nk); k < ke; ++k) {
+        const long long id = (long long)k * d.plane + base;
+        const float u = ld(u0, id), v = ld(v0, id);
+        uo[id] = rc * u + rs * v;
+        vo[id] = -rs * u + rc * v;
+      }
+    }
+  };
+  if (k0 >= nk) {
+    pdl_wait();
+    dry_levels();
+    return;
+  }
   if (tid < LT_PY) {
     const int gj = min(max(j0 - LT_H + tid, 0), d.ny - 1);
     t.gj[tid] = gj;
@@ -448,7 +599,7 @@ __global__ void __launch_bounds__(LT_X * LT_Y, 4) k_lin_t(Dev d, const float* __
     t.icos[tid] = __ldg(d.inv_cos + gj);
   }
   auto issue = [&](int k) {  // level k into buffer k % LT_NB; one commit group per call
-    if (k < d.nz && k <= k1) {  // level k1 only for the column neighbour below the chunk
+    if (k <= k1 && k < nk) {  // level k1 only for the column neighbour below the chunk
       const long long off = (long long)k * d.plane;
       const int q = k % LT_NB;
       cp_async4(&t.u[q][0][0] + e0, u0 + off + s0);
@@ -479,12 +630,9 @@ __global__ void __launch_bounds__(LT_X * LT_Y, 4) k_lin_t(Dev d, const float* __
   issue(k0);
   issue(k0 + 1);
   wet_level(k0);
-  const int ic = in ? i : 0, jc = in ? j : 0;
-  const long long base = idx2(d, jc, ic);
   const uint64_t bits = __ldg(d.wbits + base);
   const int kbt = kbot_of(bits);
   const float kv = __ldg(d.kv2 + base);
-  const float rc = IMPL ? 0.f : __ldg(d.rot_c + base), rs = IMPL ? 0.f : __ldg(d.rot_s + base);
   // u0, v0, T0, S0 of the level above
   float um = 0.f, vm = 0.f, Tm = 0.f, Sm = 0.f;
   if (k0 > 0) {
@@ -527,13 +675,8 @@ __global__ void __launch_bounds__(LT_X * LT_Y, 4) k_lin_t(Dev d, const float* __
     const long long id = (long long)k * d.plane + base;
     const bool wet = wetb(bits, k);
     const float uc = t.u[q][r][cc], vc = t.v[q][r][cc], Tc = t.T[q][r][cc], Sc = t.S[q][r][cc];
-    float u, v, T, S;
-    if (!wet) {
-      u = uc;
-      v = vc;
-      T = Tc;
-      S = Sc;
-    } else {
+    float u = uc, v = vc, T = Tc, S = Sc;
+    if (wet) {
       float2 ts = __ffma2_rn(hdiff2(d, t, w, t.T[q], t.S[q], r, cc, false), f2(dth), make_float2(Tc, Sc));
       if (do_ts) ts = __ffma2_rn(hdiff2(d, t, w, t.LT, t.LS, r, cc, true), f2(-d.kappa_bi * dth), ts);
       float2 uv = make_float2(ld(usub, id), ld(vsub, id));
@@ -543,7 +686,7 @@ __global__ void __launch_bounds__(LT_X * LT_Y, 4) k_lin_t(Dev d, const float* __
       u = uv.x;
       v = uv.y;
       if (!IMPL) {
-        const bool below = k + 1 < d.nz;  // level k + 1 sits in buffer qn
+        const bool below = k + 1 < nk;  // level k + 1 sits in buffer qn; no column of the tile is wet beyond nk
         const float up = below ? t.u[qn][r][cc] : uc, vp = below ? t.v[qn][r][cc] : vc;
         const float Tp = below ? t.T[qn][r][cc] : Tc, Sp = below ? t.S[qn][r][cc] : Sc;
         u = u + d.nu_v * d2z_c(d, k, kbt, um, uc, up) * dth;
@@ -552,11 +695,18 @@ __global__ void __launch_bounds__(LT_X * LT_Y, 4) k_lin_t(Dev d, const float* __
         S = S + vdiff_c(d, k, bits, kv, Sm, Sc, Sp) * dth;
       }
     }
-    To[id] = T;
-    So[id] = S;
-    if (IMPL) {  // the column solve and the rotation follow
-      uo[id] = u;
-      vo[id] = v;
+    // T, S below a column's deepest wet level are never read (k_final restores
+    // them from the step's input); dry levels above it are, by the column stencils
+    const bool reach = bits != 0ull && k <= kbt;
+    if (reach) {
+      To[id] = T;
+      So[id] = S;
+    }
+    if (IMPL) {  // the column solve, the hold and the rotation follow
+      if (reach) {
+        uo[id] = u;
+        vo[id] = v;
+      }
     } else {
       uo[id] = rc * u + rs * v;
       vo[id] = -rs * u + rc * v;
@@ -566,6 +716,7 @@ __global__ void __launch_bounds__(LT_X * LT_Y, 4) k_lin_t(Dev d, const float* __
     Tm = Tc;
     Sm = Sc;
   }
+  dry_levels();
 }
 
 // The biharmonic and implicit-diffusion options are template arguments: a
@@ -698,7 +849,7 @@ __global__ void __launch_bounds__(IV_T, 32) k_implicit_vdiff(Dev d, float* __res
   // 4. back substitution of the correction; x + e, land hold, rotation
   const float rc = tracers ? 0.f : __ldg(d.rot_c + base), rs = tracers ? 0.f : __ldg(d.rot_s + base);
   float en = 0.f;
-  for (int k = d.nz - 1; k >= 0; --k) {
+  for (int k = (tracers ? n : d.nz) - 1; k >= 0; --k) {  // dry T, S are never read (u, v: every lane runs all levels)
     const long long id = base + k * pl;
     const bool wet = wetb(bits, k);
     float val = 0.f;
@@ -716,7 +867,7 @@ __global__ void __launch_bounds__(IV_T, 32) k_implicit_vdiff(Dev d, float* __res
     }
     if (!wet) val = ld(hold, id);
     if (tracers) {
-      if (in && (k < n || !wet)) fld[id] = val;
+      if (in && wet) fld[id] = val;
     } else {
       const float other = __shfl_xor_sync(0xffffffffu, val, 1);
       const float uu = f ? other : val, vv = f ? val : other;
@@ -758,9 +909,15 @@ __global__ void __launch_bounds__(FZ_X * RY) k_fz(Dev d, const float* __restrict
   const int e0 = tid, e1 = tid + FZ_X * RY;
   const bool has1 = e1 < FZ_CELLS;
   const int s0 = tile_cell<FZ_PX>(d, e0, i0, j0), s1 = has1 ? tile_cell<FZ_PX>(d, e1, i0, j0) : 0;
-  auto issue = [&](int q) {  // the q-th level from the bottom into buffer q % FZ_NB; one commit group per call
-    if (q < d.nz) {
-      const long long off = (long long)(d.nz - 1 - q) * d.plane;
+  // levels with a wet point in the tile; below them Fz is 0, as allocated
+  const int nk = levels_of(__ldg((RY == 8 ? d.tile8 : d.tile4) + blockIdx.y * gridDim.x + blockIdx.x));
+  if (nk == 0) {
+    pdl_wait();
+    return;
+  }
+  auto issue = [&](int q) {  // the q-th of them from the bottom into buffer q % FZ_NB; one commit group per call
+    if (q < nk) {
+      const long long off = (long long)(nk - 1 - q) * d.plane;
       float* bu = &su[q % FZ_NB][0][0];
       float* bv = &sv[q % FZ_NB][0][0];
       cp_async4(bu + e0, u + off + s0);
@@ -781,19 +938,19 @@ __global__ void __launch_bounds__(FZ_X * RY) k_fz(Dev d, const float* __restrict
   const float cf_n = __ldg(d.cfp + jc), cf_s = jc > 0 ? __ldg(d.cfp + jc - 1) : 0.f;
   const float yscale = d.inv_dy * __ldg(d.inv_cos + jc);
   float acc = 0.f;
-  // wet flags with level nz - 1 in bit 63, shifted up one level per iteration (the march runs upwards)
-  const int up = 64 - d.nz;
+  // wet flags with level nk - 1 in bit 63, shifted up one level per iteration (the march runs upwards)
+  const int up = 64 - nk;
   uint64_t f0 = m0 << up, fe = me << up, fw = mw << up, fn = mn << up, fs = ms << up;
   pdl_wait();  // u, v come from the preceding kernel
 #pragma unroll
   for (int q = 0; q < FZ_NB - 1; ++q) issue(q);
   const int r = ty + 1, c = tx + 1;
-  for (int q = 0; q < d.nz; ++q) {
+  for (int q = 0; q < nk; ++q) {
     cp_async_wait<FZ_NB - 2>();  // this thread's copies of level q are done
     __syncthreads();             // everyone's are, and level q - 1's buffer is free
     issue(q + FZ_NB - 1);
     if (!in) continue;
-    const int k = d.nz - 1 - q, bq = q % FZ_NB;
+    const int k = nk - 1 - q, bq = q % FZ_NB;
     const float uc = su[bq][r][c], ue = su[bq][r][c + 1], uw = su[bq][r][c - 1];
     const float w0 = (float)(unsigned)(f0 >> 63), we = (float)(unsigned)(fe >> 63),
                 ww = (float)(unsigned)(fw >> 63), wn = (float)(unsigned)(fn >> 63),
@@ -812,11 +969,11 @@ __global__ void __launch_bounds__(FZ_X * RY) k_fz(Dev d, const float* __restrict
 }
 
 cudaError_t launch_nu_tb(cudaStream_t s, const Dev& d, int warps, const float* u, const float* v, float* uo,
-                         float* vo, float c, int nsub, int halo) {
-  const int TI = NB_W - 2 * halo, TJ = warps * NB_R - 2 * halo;
-  const dim3 grd((d.nx + TI - 1) / TI, (d.ny + TJ - 1) / TJ, d.nz);
-  if (warps == 16) return launch_pdl(k_nu_tb<16>, grd, dim3(32, 16), 0, s, d, u, v, uo, vo, c, nsub, halo);
-  return launch_pdl(k_nu_tb<8>, grd, dim3(32, 8), 0, s, d, u, v, uo, vo, c, nsub, halo);
+                         float* vo, float c, int nsub, int halo, int left) {
+  const dim3 grd = nu_grid(d, warps, halo);
+  const size_t sm = nu_smem_bytes(warps);
+  if (warps == 16) return launch_pdl(k_nu_tb<16>, grd, dim3(32, 16), sm, s, d, u, v, uo, vo, c, nsub, halo, left);
+  return launch_pdl(k_nu_tb<8>, grd, dim3(32, 8), sm, s, d, u, v, uo, vo, c, nsub, halo, left);
 }
 
 void launch_fz(cudaStream_t s, const Dev& d, const float* u, const float* v, float* Fz) {
@@ -885,6 +1042,14 @@ __global__ void __launch_bounds__(256) k_madv(Dev d, const float* __restrict__ u
   const int i = blockIdx.x * 32 + threadIdx.x;
   const int j0 = blockIdx.y * MADV_TY;
   const int k = blockIdx.z;
+  {  // no wet point within two rows of the tile: the result is 0 everywhere, as allocated
+    uint64_t any = 0ull;
+    for (int r = j0 / 8; r <= min(j0 + MADV_TY - 1, d.ny - 1) / 8; ++r) any |= __ldg(d.tile8 + r * gridDim.x + blockIdx.x);
+    if (!wetb(any, k)) {
+      pdl_wait();
+      return;
+    }
+  }
   pdl_wait();  // u, v, Fz come from the preceding kernels
   for (int r = threadIdx.y; r < MADV_TY + 4; r += blockDim.y) {
     int jj = j0 - 2 + r;
@@ -1033,6 +1198,13 @@ __global__ void __launch_bounds__(TA_X * TA_Y, 5) k_tracer_adv_t(Dev d, const fl
                                                                  float* __restrict__ topS) {
   pdl_trigger();
   __shared__ TaTile t;
+  // this block's levels, down to the deepest one with a wet point in reach of the tile
+  const int nk = levels_of(__ldg(d.tile8 + blockIdx.y * gridDim.x + blockIdx.x));
+  const int k0 = blockIdx.z * d.ta_kc, k1 = min(nk, k0 + d.ta_kc);
+  if (k0 >= k1) {
+    pdl_wait();
+    return;
+  }
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TA_X + tx;
   const int i0 = blockIdx.x * TA_X, j0 = blockIdx.y * TA_Y;
   const int i = i0 + tx, j = j0 + ty;
@@ -1043,9 +1215,8 @@ __global__ void __launch_bounds__(TA_X * TA_Y, 5) k_tracer_adv_t(Dev d, const fl
   const bool has1 = e1 < TA_CELLS;
   const int s0 = tile_cell<TA_PX, TA_H>(d, e0, i0, j0), s1 = has1 ? tile_cell<TA_PX, TA_H>(d, e1, i0, j0) : 0;
   const uint64_t b0 = __ldg(d.wbits + s0), b1 = has1 ? __ldg(d.wbits + s1) : 0ull;
-  const int k0 = blockIdx.z * d.ta_kc, k1 = min(d.nz, k0 + d.ta_kc);  // this block's levels
   auto issue = [&](int k) {  // level k into buffer k % TA_NB; one commit group per call
-    if (k < d.nz && k <= k1) {  // level k1 only for the column neighbour below the chunk
+    if (k <= k1 && k < nk) {  // level k1 only for the column neighbour below the chunk
       const long long off = (long long)k * d.plane;
       const int q = k % TA_NB;
       float* ts = &t.ts[q][0][0].x;
@@ -1097,7 +1268,7 @@ __global__ void __launch_bounds__(TA_X * TA_Y, 5) k_tracer_adv_t(Dev d, const fl
     issue(k + 2);
     wet_level(k + 1);
     const long long id = (long long)k * d.plane + base;
-    const float fzn = k + 1 < d.nz ? ld(Fz, id + d.plane) : 0.f;
+    const float fzn = k + 1 < nk ? ld(Fz, id + d.plane) : 0.f;  // 0 below the wet levels
     if (!in) continue;
     const int q = k % TA_NB, qn = (k + 1) % TA_NB, wq = k & 1;
     const float w0 = t.w[wq][r][cc];
@@ -1106,7 +1277,7 @@ __global__ void __launch_bounds__(TA_X * TA_Y, 5) k_tracer_adv_t(Dev d, const fl
       topT[base] = (first ? 0.f : topT[base]) + fzk * ck.x;
       topS[base] = (first ? 0.f : topS[base]) + fzk * ck.y;
     }
-    float2 a = f2(0.f);
+    // dry points: the rate is 0 as allocated, and their tracers are never read with a weight
     if (w0 != 0.f) {
       const float2 m1 = f2(-1.f);
       const float2 fxe = ta_faces_x<LIM>(t, q, wq, r, cc), fxw = ta_faces_x<LIM>(t, q, wq, r, cc - 1);
@@ -1121,19 +1292,19 @@ __global__ void __launch_bounds__(TA_X * TA_Y, 5) k_tracer_adv_t(Dev d, const fl
       } else {
         up = __fmul2_rn(f2(fzk * (wup * w0)), fzk > 0.f ? cm : ck);
       }
-      if (k + 1 < d.nz) {
+      if (k + 1 < nk) {
         // ghost fill below the deepest wet level: node k+1 carries node k's value
         const float2 cn = k + 1 <= kbt ? t.ts[qn][r][cc] : ck;
         dn = __fmul2_rn(f2(fzn * (w0 * (float)(unsigned)((cb >> 1) & 1ull))), fzn > 0.f ? ck : cn);
       }
-      a = __fmul2_rn(__ffma2_rn(__ffma2_rn(up, m1, dn), f2(d.vc.inv_dz_node[k]), h), f2(-w0));
-    }
-    accT[id] = first ? a.x : accT[id] + a.x;
-    accS[id] = first ? a.y : accS[id] + a.y;
-    if (!last) {
-      const float2 cnew = __ffma2_rn(a, f2(dts), ck);
-      Tn[id] = cnew.x;
-      Sn[id] = cnew.y;
+      const float2 a = __fmul2_rn(__ffma2_rn(__ffma2_rn(up, m1, dn), f2(d.vc.inv_dz_node[k]), h), f2(-w0));
+      accT[id] = first ? a.x : accT[id] + a.x;
+      accS[id] = first ? a.y : accS[id] + a.y;
+      if (!last) {
+        const float2 cnew = __ffma2_rn(a, f2(dts), ck);
+        Tn[id] = cnew.x;
+        Sn[id] = cnew.y;
+      }
     }
     cm = ck;
     fzk = fzn;
@@ -1311,8 +1482,9 @@ __global__ void __launch_bounds__(128) k_tracer_rest(Dev d, RestArgs a) {
   if (i >= d.nx || j >= d.ny) return;
   const long long base = idx2(d, j, i);
   const uint64_t bits = wb(d, j, i);
+  const int nz = levels_of(bits);  // dry levels below keep their values: nothing reads them
   pdl_wait();  // the evaluation state and the advection rates come from the preceding kernels
-  const int nz = d.nz;
+  if (nz == 0) return;
   // static-instability gates of the evaluation state, in difference form:
   // rho[m] > rho[m+1]  <=>  beta (S[m]-S[m+1]) > alpha (T[m]-T[m+1]).
   uint64_t unstable = 0ull, wetpair = 0ull;
@@ -1493,8 +1665,10 @@ __global__ void __launch_bounds__(PG_X * RY) k_pgf(Dev d, PgfArgs a) {
   const int e0 = tid, e1 = tid + PG_X * RY;
   const bool has1 = e1 < PG_CELLS;
   const int s0 = tile_cell<PG_PX>(d, e0, i0, j0), s1 = has1 ? tile_cell<PG_PX>(d, e1, i0, j0) : 0;
+  // levels with a wet point in the tile: below them every density difference is 0
+  const int nk = levels_of(__ldg((RY == 8 ? d.tile8 : d.tile4) + blockIdx.y * gridDim.x + blockIdx.x));
   auto issue = [&](int k) {  // level k into buffer k % PG_NB; one commit group per call
-    if (k < d.nz) {
+    if (k < nk) {
       const long long off = (long long)k * d.plane;
       float* ts = &sTS[k % PG_NB][0][0].x;
       cp_async4(ts + 2 * e0, a.T + off + s0);
@@ -1526,18 +1700,18 @@ __global__ void __launch_bounds__(PG_X * RY) k_pgf(Dev d, PgfArgs a) {
   double su = 0.0, sv = 0.0;
   float u_prev = 0.f, v_prev = 0.f;
   float u_next = 0.f, v_next = 0.f;
+  constexpr float kInvRho0 = 1.f / kRho0;
+  pdl_wait();  // T, S, u, v and the momentum parts come from the preceding kernels
   if (MODE == 0 && in) {
     u_next = ld(a.u1, cc);
     v_next = ld(a.v1, cc);
   }
-  constexpr float kInvRho0 = 1.f / kRho0;
-  pdl_wait();  // T, S and the momentum parts come from the preceding kernels
 #pragma unroll
   for (int q = 0; q < PG_NB - 1; ++q) issue(q);
   const int r = ty + 1, c = tx + 1;
   float* gsx = MODE != 0 ? a.gsx + cc : nullptr;  // this column's gradient scratch, one plane per level
   float* gsy = MODE != 0 ? a.gsy + cc : nullptr;
-  for (int k = 0; k < d.nz; ++k) {
+  for (int k = 0; k < nk; ++k) {
     cp_async_wait<PG_NB - 2>();  // this thread's copies of level k are done
     __syncthreads();             // everyone's are, and level k - 1's buffer is free
     issue(k + PG_NB - 1);
@@ -1594,6 +1768,19 @@ __global__ void __launch_bounds__(PG_X * RY) k_pgf(Dev d, PgfArgs a) {
     }
   }
   if (!in) return;
+  if (MODE == 0) {  // the depth mean takes the dry levels too
+#pragma unroll 4
+    for (int k = nk; k < d.nz; ++k) {
+      const float uk = k == nk ? u_next : ld(a.u1, (long long)k * d.plane + cc);
+      const float vk = k == nk ? v_next : ld(a.v1, (long long)k * d.plane + cc);
+      if (k > 0) {
+        su += (double)(0.5f * (u_prev + uk) * d.vc.dznorm[k - 1]);
+        sv += (double)(0.5f * (v_prev + vk) * d.vc.dznorm[k - 1]);
+      }
+      u_prev = uk;
+      v_prev = vk;
+    }
+  }
   const float Fx = -fx / (kRho0 * d.H_sw);
   const float Fy = -fy / (kRho0 * d.H_sw);
   if (MODE == 0) {
@@ -1632,6 +1819,14 @@ __global__ void __launch_bounds__(256) k_pgf_out(Dev d, PgfArgs a) {
   const ulonglong2 b23 = __ldg(reinterpret_cast<const ulonglong2*>(d.wbits + c + 2));
   const float4 w = make_float4(wetf(b01.x, k), wetf(b01.y, k), wetf(b23.x, k), wetf(b23.y, k));
   pdl_wait();  // the gradient scratch and the momentum parts come from the preceding kernels
+  if (w.x + w.y + w.z + w.w == 0.f) {
+    // four dry points: u, v pass through; the first stage's are never read with a weight
+    if (MODE == 2) {
+      *reinterpret_cast<float4*>(a.uo + id) = __ldg(reinterpret_cast<const float4*>(a.u1 + id));
+      *reinterpret_cast<float4*>(a.vo + id) = __ldg(reinterpret_cast<const float4*>(a.v1 + id));
+    }
+    return;
+  }
   const float4 gx = *reinterpret_cast<const float4*>(a.gsx + id), gy = *reinterpret_cast<const float4*>(a.gsy + id);
   const float4 Fx = *reinterpret_cast<const float4*>(a.Fxs + c), Fy = *reinterpret_cast<const float4*>(a.Fys + c);
   const float4 Au = __ldg(reinterpret_cast<const float4*>(a.Au + id));

@@ -44,6 +44,9 @@ struct FftPlan {
   // register-resident form for n = r1 r2 r3 (0 when n has no supported split)
   int r1, r2, r3;
   const float2* tw_full;        // exp(-2 pi i j / n), j < n (float64-derived)
+  // the lines with a wet point, k * ny + j, in order: the others come out 0 (the filter's output is wet-masked)
+  const int* lines;
+  int nlines;
 };
 
 struct PgfArgs {
@@ -136,9 +139,17 @@ __global__ void k_budget_final(const double* partial, int nblocks, double* out);
 __global__ void k_forcing_blend(Dev d, const float* stack, int prev, int cur, int next, float w_prev, float w_cur,
                                 float w_next, float* out);
 __global__ void k_barrier_probe(unsigned* bar, unsigned* err, unsigned expected, unsigned max_polls);
-// the temporally blocked nu_h subcycles with 8 or 16 warps per tile (NB_W x 8 warps * NB_R)
+// the temporally blocked nu_h subcycles with 8 or 16 warps per tile (NB_W x 8 warps * NB_R); `left` counts the
+// subcycles of the half step from this pass on.  d.nu_class holds the strip classes of this shape.
+inline dim3 nu_grid(const Dev& d, int warps, int halo) {
+  const int TI = NB_W - 2 * halo, TJ = warps * NB_R - 2 * halo;
+  return dim3((d.nx + TI - 1) / TI, (d.ny + TJ - 1) / TJ, d.nz);
+}
+inline size_t nu_smem_bytes(int warps) { return (size_t)warps * (2 * 2 * 32 * 16 + NB_R * 24); }
 cudaError_t launch_nu_tb(cudaStream_t s, const Dev& d, int warps, const float* u, const float* v, float* uo,
-                         float* vo, float c, int nsub, int halo);
+                         float* vo, float c, int nsub, int halo, int left);
+__global__ void k_nu_class(Dev d, unsigned char* cls, int nw, int halo, int gxn, int gyn);
+__global__ void k_tile_bits(Dev d, uint64_t* out, int ry, int ntx, int nty);
 __global__ void k_nu_gates(Dev d, unsigned char* gate);
 void launch_lin_t(cudaStream_t s, const Dev& d, const float* usub, const float* vsub, const float* u0,
                   const float* v0, const float* T0, const float* S0, float* uo, float* vo, float* To, float* So,

@@ -59,6 +59,11 @@ struct zm_solver {
   float* eta[2] = {nullptr, nullptr};
   int cur = 0;
   // work fields
+  // A dry point's T and S below its column's deepest wet level are not written in
+  // s1, s2 and the tracer work fields of the N step, and their rates, Fz and the
+  // filtered advection keep the 0 they were allocated with; no wet point reads them
+  // with a weight.  So only the step's kernels write those fields: states from
+  // outside it (diagnostics, closure rows) go to L.
   Fields4 s1, s2, W1, W2, L;
   float *Fz = nullptr, *Ayu = nullptr, *Ayv = nullptr, *Au = nullptr, *Av = nullptr;
   float *accT = nullptr, *accS = nullptr, *TsA = nullptr, *SsA = nullptr, *TsB = nullptr, *SsB = nullptr;
@@ -178,6 +183,30 @@ struct zm_solver {
     if (e != cudaSuccess) throw Err{ZM_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e)};
   }
 
+  // Set the nu_h launch shape and form its strip classes.  Runs at creation and
+  // between the autotuner's trials; waits, so that any stream sees the table.
+  unsigned char* nu_class_buf = nullptr;
+  void set_nu_shape(int halo, int warps) {
+    nu_halo = halo;
+    nu_warps = warps;
+    if (!nu_class_buf) {
+      size_t most = 0;
+      for (int w : {8, 16})
+        for (int h = 3; h <= NB_T; ++h) {
+          const dim3 g = nu_grid(d, w, h);
+          most = std::max(most, (size_t)g.x * g.y * g.z * w);
+        }
+      nu_class_buf = alloc<unsigned char>(most);
+      d.nu_class = nu_class_buf;
+    }
+    const dim3 g = nu_grid(d, warps, halo);
+    const unsigned strips = g.x * g.y * g.z * warps;
+    ZM_CUDA(cudaDeviceSynchronize());  // no launch reads the old table any more
+    k_nu_class<<<(strips + 7) / 8, dim3(32, 8)>>>(d, nu_class_buf, warps, halo, (int)g.x, (int)g.y);
+    check_launch();
+    ZM_CUDA(cudaDeviceSynchronize());
+  }
+
   // ---------------------------------------------------------------- stages
   // Linear half step L(dt/2): src -> dst (dst must not alias src).
   void linear_half(cudaStream_t s, const Fields4& src, const Fields4& dst) {
@@ -193,7 +222,7 @@ struct zm_solver {
         const int nsub = std::min(nu_halo, n_nu - done);
         const Fields4& o = (pass % 2 == 0) ? W1 : W2;
         pb(ZM_K_NU_SUB, s);
-        ZM_CUDA(launch_nu_tb(s, d, nu_warps, a, c, o.u, o.v, dts, nsub, nu_halo));
+        ZM_CUDA(launch_nu_tb(s, d, nu_warps, a, c, o.u, o.v, dts, nsub, nu_halo, n_nu - done));
         pe(s);
         a = o.u;
         c = o.v;
@@ -574,8 +603,7 @@ struct zm_solver {
         int pick = nu_halo, pick_w = nu_warps;
         for (int wq : {8, 16})
           for (int h = 3; h <= NB_T; ++h) {
-            nu_halo = h;
-            nu_warps = wq;
+            set_nu_shape(h, wq);
             const float ms = time_ms([&] { linear_half(s, in, s1); });
             if (ms < best) {
               best = ms;
@@ -583,8 +611,7 @@ struct zm_solver {
               pick_w = wq;
             }
           }
-        nu_halo = pick;
-        nu_warps = pick_w;
+        set_nu_shape(pick, pick_w);
       }
       float best = 1e30f;
       int pick = fft_lines;
@@ -813,6 +840,31 @@ void build(zm_solver* s, const zm_grid* g, const zm_params* p) {
     ZM_CUDA(cudaGetLastError());
     ZM_CUDA(cudaDeviceSynchronize());
     d.nu_gate = gate;
+    d.dx_rows = 1;
+    for (int j = 0; j < ny && d.dx_rows; ++j)
+      for (int i = 1; i < nx; ++i)
+        if (inv_dx2[(size_t)j * P + i] != inv_dx2[(size_t)j * P]) d.dx_rows = 0;
+    s->set_nu_shape(s->nu_halo, s->nu_warps);
+    // wet levels of the column tiles
+    const int ntx = (nx + 31) / 32;
+    for (int ry : {8, 4}) {
+      const int nty = (ny + ry - 1) / ry;
+      uint64_t* t = s->alloc<uint64_t>((size_t)ntx * nty);
+      k_tile_bits<<<(ntx * nty + 7) / 8, dim3(32, 8)>>>(d, t, ry, ntx, nty);
+      ZM_CUDA(cudaGetLastError());
+      (ry == 8 ? d.tile8 : d.tile4) = t;
+    }
+    // the lines of the longitude filter with a wet point
+    std::vector<int> lines;
+    std::vector<uint64_t> row(ny, 0ull);
+    for (int j = 0; j < ny; ++j)
+      for (int i = 0; i < nx; ++i) row[j] |= bits[(size_t)j * P + i];
+    for (int k = 0; k < nz; ++k)
+      for (int j = 0; j < ny; ++j)
+        if (row[j] >> k & 1ull) lines.push_back(k * ny + j);
+    plan.nlines = (int)lines.size();
+    if (lines.empty()) lines.push_back(0);
+    plan.lines = s->upload(lines);
   }
   d.ta_kc = 10;
   d.lt_kc = 10;
@@ -1523,6 +1575,10 @@ int zm_run_stage(zm_solver* s, void* stream, int32_t stage, const zm_state* in, 
   try {
     s->load(st, in, s->st[s->cur], s->eta[s->cur]);
     const int a = s->cur, b = 1 - s->cur;
+    if (stage <= 2) {  // the stages leave dry tracers alone; here they are part of the result
+      ZM_CUDA(cudaMemcpyAsync(s->st[b].T, s->st[a].T, s->n3 * sizeof(float), cudaMemcpyDeviceToDevice, st));
+      ZM_CUDA(cudaMemcpyAsync(s->st[b].S, s->st[a].S, s->n3 * sizeof(float), cudaMemcpyDeviceToDevice, st));
+    }
     if (stage == 1) {
       s->linear_half(st, s->st[a], s->st[b]);
     } else if (stage == 2) {
@@ -1616,15 +1672,15 @@ int zm_diagnostics(zm_solver* s, void* stream, const zm_state* in, const float* 
   cudaStream_t st = (cudaStream_t)stream;
   try {
     // the caller's state goes to work buffers that are idle between steps
-    s->load(st, in, s->s2, s->frx);
+    s->load(st, in, s->L, s->frx);
     const float* sp = nullptr;
     const dim3 c(32, 4);
     if (surface_pressure_pa) {
       k_ref_to_int2<<<s->grid2(dim3(32, 8)), dim3(32, 8), 0, st>>>(s->d, surface_pressure_pa, s->fry);
       sp = s->fry;
     }
-    launch_fz(st, s->d, s->s2.u, s->s2.v, s->Fz);
-    k_diagnostics<<<s->grid2(c), c, 0, st>>>(s->d, s->s2.T, s->s2.S, s->frx, s->Fz, sp, s->W1.u, s->W1.v, s->W2.u);
+    launch_fz(st, s->d, s->L.u, s->L.v, s->Fz);
+    k_diagnostics<<<s->grid2(c), c, 0, st>>>(s->d, s->L.T, s->L.S, s->frx, s->Fz, sp, s->W1.u, s->W1.v, s->W2.u);
     s->check_launch();
     s->to_ref3(st, s->W1.u, rho, 0.f);
     s->to_ref3(st, s->W1.v, pressure, 0.f);
@@ -1642,9 +1698,9 @@ int zm_tracer_terms(zm_solver* s, void* stream, const zm_state* in, float* terms
   const size_t nref = (size_t)s->nx * s->ny * s->nz;
   try {
     // the caller's state goes to work buffers that are idle between steps
-    s->load(st, in, s->s2, s->frx);
-    launch_fz(st, s->d, s->s2.u, s->s2.v, s->Fz);
-    launch_tracer_terms(st, s->d, s->s2.T, s->s2.S, s->s2.u, s->s2.v, s->Fz, s->W1.u, s->W1.v, s->W1.T, s->W1.S);
+    s->load(st, in, s->L, s->frx);
+    launch_fz(st, s->d, s->L.u, s->L.v, s->Fz);
+    launch_tracer_terms(st, s->d, s->L.T, s->L.S, s->L.u, s->L.v, s->Fz, s->W1.u, s->W1.v, s->W1.T, s->W1.S);
     s->check_launch();
     const float* src[4] = {s->W1.u, s->W1.v, s->W1.T, s->W1.S};
     for (int q = 0; q < 4; ++q) s->to_ref3(st, src[q], terms + q * nref, 0.f);
@@ -1767,8 +1823,8 @@ int zm_closure_kappa(zm_solver* s, void* stream, const zm_state* in, float* kapp
   if (!s->closure_on) return fail(s, Err{ZM_ERR_INVALID, "zm_closure_kappa: no closure set"});
   cudaStream_t st = (cudaStream_t)stream;
   try {
-    s->load(st, in, s->s2, s->frx);
-    s->closure(st, s->s2);
+    s->load(st, in, s->L, s->frx);
+    s->closure(st, s->L);
     const long long ncol = (long long)s->nx * s->ny;
     k_kappa_rows<<<(unsigned)((ncol + 127) / 128), 128, 0, st>>>(s->d, s->kappa3, kappa);
     s->check_launch();
@@ -1783,9 +1839,9 @@ int zm_closure_features(zm_solver* s, void* stream, const zm_state* in, float* X
   if (s->nz > 51) return fail(s, Err{ZM_ERR_UNSUPPORTED, "the learned closure covers at most 50 levels"});
   cudaStream_t st = (cudaStream_t)stream;
   try {
-    s->load(st, in, s->s2, s->frx);
+    s->load(st, in, s->L, s->frx);
     ClosureArgs a{};
-    a.T = s->s2.T; a.S = s->s2.S; a.u = s->s2.u; a.v = s->s2.v; a.X = X; a.Tt = T; a.Mt = M;
+    a.T = s->L.T; a.S = s->L.S; a.u = s->L.u; a.v = s->L.v; a.X = X; a.Tt = T; a.Mt = M;
     const long long ncol = (long long)s->nx * s->ny;
     k_closure_features<<<(unsigned)((ncol + 127) / 128), 128, 0, st>>>(s->d, a);
     s->check_launch();
