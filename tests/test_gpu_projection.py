@@ -129,3 +129,30 @@ def test_projection_is_deterministic_at_full_size():
     after = np.linalg.norm(ostep.column_divergence(a["u"], a["v"], p))
     assert after < 0.5 * before, (after, before)
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("shape,iters", [((1000, 400, 3), 10), ((800, 400, 3), 10), ((75, 47, 8), 150)])
+@pytest.mark.parametrize("pre", ["none", "jacobi"])
+def test_every_solver_form(shape, iters, pre):
+    """The projection stage at sizes that take the streamed solver (more cells
+    than the resident tiles hold), the largest tiles (three rows per thread)
+    and one small ragged grid, against the oracle with the same tolerances;
+    both solvers are float64, so the bound is the other tight comparison's."""
+    nx, ny, nz = shape
+    grid = workloads.build_grid(nx, ny, nz)
+    kw = dict(workloads.PLAIN_OPTIONS, forcing=workloads.wind_forcing(grid), dt_bt=75.0, project_adv_vel=True,
+              projection_niter=iters, projection_preconditioner=pre, projection_max_refinements=1)
+    step = make_solver_global(grid, workloads.PLAIN_PHYSICS, 1800.0, dtype="float32", **kw)[0]
+    p = oparams.build_params(grid, workloads.PLAIN_PHYSICS, 1800.0, dtype="float32", **kw)
+    rng = np.random.default_rng(5)
+    wet = np.asarray(grid.wet_mask_3d)
+    T, S = workloads.initial_fields(grid)
+    lon, lat = np.meshgrid(np.radians(grid.lon), np.radians(grid.lat), indexing="ij")
+    noise = 0.01 * rng.standard_normal(wet.shape)
+    st = gu.f32(dict(u=((0.1 * np.cos(3 * lon) * np.cos(2 * lat))[:, :, None] + noise) * wet,
+                     v=(0.1 * np.sin(2 * lon) * np.cos(3 * lat))[:, :, None] * wet, T=T, S=S, eta=np.zeros((nx, ny))))
+    got = gu.run_stage(step, 8, st)
+    u, v = ostep.project_column_divergence(st["u"], st["v"], p, 1800.0)
+    assert gu.rel_l2(got["u"], u, wet) < TIGHT and gu.rel_l2(got["v"], v, wet) < TIGHT
+    again = gu.run_stage(step, 8, st)
+    assert np.array_equal(got["u"], again["u"]) and np.array_equal(got["v"], again["v"])

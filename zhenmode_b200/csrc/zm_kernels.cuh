@@ -202,7 +202,20 @@ struct ProjArgs {
   double tol2, trtol2;  // tol^2, transport rtol^2
   double dtg;           // dt g
   int niter, refinements;
+  // resident form: tile; 16-byte words of the exchanged values [2][ny][P] and sums [2][ZM_PJ_SUMS][blocks]; the
+  // sequence number of the last exchange
+  int tile_x, tile_y, tiles_x;
+  void *pub, *words;
+  unsigned long long* seq;
+  unsigned max_polls;
 };
+struct ProjTile {
+  int x, y, tiles_x, tiles_y, cpt, blocks, threads;  // blocks 0: no tile fits
+  size_t smem;
+};
+bool proj_res_tile(int nx, int ny, int sms, size_t smem_max, int least, ProjTile& best);
+void (*proj_res_kernel(int cpt))(Dev, ProjArgs);
+constexpr int PJ_RES_THREADS = 512;
 __global__ void k_proj_coef(Dev d, const double* dzn, const double* cosd, const double* area, double* cx, double* cy,
                             double* sxy, double* minv, double* rarea);
 __global__ void k_proj_rhs(Dev d, const float* u, const float* v, const double* dzn, const double* cosd,

@@ -29,6 +29,8 @@
 //    (dt g)^2 sum res^2 / area.  The refinements therefore need no pass over
 //    the 3-D fields: k_proj_rhs reads (u, v) once and k_proj_correct applies
 //    the summed potential once.
+//  * k_proj_res, for grids whose tiles fit in the SMs' shared memory, runs every
+//    solve resident on the chip (below); k_proj_cg takes the larger grids.
 //  * k_proj_cg runs every solve in one cooperative launch in float64, with the
 //    loop of jax's cg: x = 0, r = b, z = M r, p = z, gamma = <r, z>; while the
 //    squared residual (gamma without a preconditioner, <r, r> with one) is
@@ -40,6 +42,8 @@
 //    a fixed tree and over blocks in block order by every block, so all blocks
 //    take the same branches and the result does not depend on timing.  The
 //    whole working set (a dozen 2-D float64 fields) stays in L2.
+#include <algorithm>
+
 #include "zm_kernels.cuh"
 #include "zm_sync.cuh"
 
@@ -278,7 +282,8 @@ __global__ void __launch_bounds__(256) k_proj_rhs(Dev d, const float* __restrict
   const double cfn = has_n ? 0.5 * (c + cosd[j + 1]) : 0.0;
   const double cfs = has_s ? 0.5 * (cosd[j - 1] + c) : 0.0;
   double sum = 0.0;
-  for (int k = 0; k < d.nz; ++k) {
+  const int nk = levels_of(wc);  // a face of the column is open only where the column is wet
+  for (int k = 0; k < nk; ++k) {
     const long long o = (long long)k * d.plane;
     const double uc = ld(u, o + g), ue = ld(u, o + idx2(d, j, ie)), uw = ld(u, o + idx2(d, j, iw));
     const double vc = ld(v, o + g), vn = ld(v, o + idx2(d, jn, i)), vs = ld(v, o + idx2(d, js, i));
@@ -403,13 +408,484 @@ __global__ void __launch_bounds__(256) k_proj_correct(Dev d, float* __restrict__
   const double cp = 0.5 * (c + cosd[(j + 1) % d.ny]), cm = 0.5 * (c + cosd[(j - 1 + d.ny) % d.ny]);
   const double hx = d.inv_dx_d[g] * 0.5, hy = (d.inv_dy_d / c) * 0.5;
   const double dxe = pe - pc, dxw = pc - pw, dyn = (pn - pc) * cp, dys = (pc - ps) * cm;
-  for (int k = 0; k < d.nz; ++k) {
+  const int nk = levels_of(wc);  // every face of a dry point is closed
+  for (int k = 0; k < nk; ++k) {
     const long long o = (long long)k * d.plane + g;
     const double gx = hx * (dxe * bitd(e_c, k) + dxw * bitd(e_w, k));
     const double gy = hy * (dyn * bitd(pos, k) + dys * bitd(neg, k));
     u[o] = (float)((double)u[o] - dtg * gx);
     v[o] = (float)((double)v[o] - dtg * gy);
   }
+}
+
+// ---------------------------------------------------------------- resident form
+//
+// One block owns a tile of the grid.  The direction of steepest descent z
+// and s = A p stay in shared memory with a two-cell halo, the face weights of
+// the tile too, x, p and r in registers; the loop touches global memory only
+// for what the blocks exchange.  What bounds an iteration is the latency of
+// its grid-wide sums, so there is one exchange per iteration: with w = A z,
+//   gamma = <r, z>, delta = <w, z>,  beta = gamma / gamma_old,
+//   alpha = gamma / (delta - beta gamma / alpha_old),
+//   p = z + beta p, s = w + beta s, x += alpha p, r -= alpha s, z = M r,
+// the recurrences of Chronopoulos and Gear (1989), equal to the loop above in
+// exact arithmetic; both sums are formed before either scalar is needed.  The
+// halo needs no second exchange: each block publishes its w along the tile's
+// edges with the sums, and carries s and z of its halo cells with the same
+// recurrences.
+//
+// Everything the blocks exchange is a 16-byte {value, sequence number} word,
+// stored and loaded whole: a reader polls the word itself, so no fence, atomic
+// or second load stands between a value and its use.  A block's partial sums
+// go to every block's own list of words, one copy per reader: one list that
+// all blocks poll is a few cache lines with up to 148 readers each, and cost
+// 1.8 us more per exchange.  The lists are added in block order, so every
+// block gets the same bits.
+// Per iteration, against the streamed form's two barriers and two passes over
+// L2 (10.0 us at 360x180 cells, 14.5 us at 720x360): 4.0 and 5.7 us; without
+// the wait for the sums the loop takes 3.3 and 5.3 us, so what is left is the
+// latency of the FP64 chains and of one store and load across the chip.
+
+namespace {
+
+struct alignas(16) SumWord {
+  double v;
+  unsigned long long seq;
+};
+
+__device__ __forceinline__ void st_word(SumWord* p, double v, unsigned long long seq) {
+  asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}\n" ::"l"(p),
+               "l"(__double_as_longlong(v)), "l"(seq)
+               : "memory");
+}
+
+__device__ __forceinline__ SumWord ld_word(const SumWord* p) {
+  long long v;
+  unsigned long long q;
+  asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}\n"
+               : "=l"(v), "=l"(q)
+               : "l"(p)
+               : "memory");
+  return SumWord{__longlong_as_double(v), q};
+}
+
+// Polls a word until it carries seq; bounded, false after the limit or when another block gave up.
+__device__ __forceinline__ bool wait_word(const SumWord* p, unsigned long long seq, const ProjArgs& a, double& v) {
+  SumWord w = ld_word(p);
+  for (unsigned polls = 0; w.seq != seq; w = ld_word(p))
+    if (++polls > a.max_polls || ((polls & 255u) == 0u && ld_acquire(a.err) != 0u)) {
+      atomicOr(a.err, ZM_BT_ERR_BARRIER);
+      return false;
+    }
+  v = w.v;
+  return true;
+}
+
+template <int N>
+struct PjInt {
+  static constexpr int value = N;
+};
+
+constexpr int PJ_CHUNKS = 5;  // at most 32 * PJ_CHUNKS blocks
+
+struct ResShared {  // fixed part of the block's shared memory
+  double red[ZM_PJ_SUMS][32];
+  double tot[ZM_PJ_SUMS], part[ZM_PJ_SUMS][PJ_CHUNKS];
+  double pad;  // an even number of doubles, for what follows
+};
+
+}  // namespace
+
+// Shared memory of a tile of tx x ty cells.
+size_t proj_res_smem(int tx, int ty) {
+  const size_t halo = (size_t)(tx + 4) * (ty + 4), own = (size_t)tx * ty;
+  return sizeof(ResShared) + sizeof(double) * (4 * (size_t)(tx + ty) + 2 * halo + 3 * (size_t)(tx + 1) * ty +
+                                               3 * (size_t)tx * (ty + 1) + 2 * own);
+}
+
+// Thread (lx, chunk) owns CPT consecutive rows of column lx of the tile; with
+// one row per thread the face weights of its cell stay in registers.  The
+// index arithmetic is done before the loop.
+template <int CPT>
+__global__ void __launch_bounds__(PJ_RES_THREADS, 1) k_proj_res(Dev d, ProjArgs a) {
+  extern __shared__ double pr_smem[];
+  constexpr bool REGS = CPT == 1;
+  constexpr int HS = 2;  // halo cells per thread held ready (the others are found again each time)
+  const int tx = a.tile_x, ty = a.tile_y, PX = tx + 4, PY = ty + 4, nb = gridDim.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  ResShared& sh = *reinterpret_cast<ResShared*>(pr_smem);
+  double* hv = pr_smem + sizeof(ResShared) / sizeof(double);  // gathered halo values
+  double* z = hv + 4 * (tx + ty);          // [PY][PX]
+  double* sv = z + PX * PY;                // [PY][PX]
+  double* cx = sv + PX * PY;               // [3][ty][tx + 1]: east faces of columns -1 .. tx - 1
+  double* cy = cx + 3 * (tx + 1) * ty;     // [3][ty + 1][tx]: north faces of rows -1 .. ty - 1
+  double* sx = cy + 3 * tx * (ty + 1);     // [ty][tx] area / dx
+  double* sy = sx + tx * ty;               // [ty][tx] area / (dy cos)
+  SumWord* words = reinterpret_cast<SumWord*>(a.words);
+  const bool ident = a.minv == nullptr;
+  const long long n2 = d.plane;
+  const int i0 = (int)(blockIdx.x % a.tiles_x) * tx, j0 = (int)(blockIdx.x / a.tiles_x) * ty;
+  const int w_own = min(tx, d.nx - i0), h_own = min(ty, d.ny - j0);
+  auto wrap = [&](int i) {
+    i %= d.nx;
+    return i < 0 ? i + d.nx : i;
+  };
+  for (int e = threadIdx.x; e < (tx + 1) * ty; e += blockDim.x) {
+    const int r = e / (tx + 1), c = e - r * (tx + 1) - 1;
+    const bool in = r < h_own && c < w_own;
+    const int g = in ? idx2(d, j0 + r, wrap(i0 + c)) : 0;
+    for (int q = 0; q < 3; ++q) cx[q * (tx + 1) * ty + e] = in ? __ldg(a.cx + q * n2 + g) : 0.0;
+  }
+  for (int e = threadIdx.x; e < tx * (ty + 1); e += blockDim.x) {
+    const int r = e / tx - 1, c = e - (r + 1) * tx;
+    const bool in = r < h_own && c < w_own && j0 + r >= 0;  // no face south of the first row
+    const int g = in ? idx2(d, j0 + r, i0 + c) : 0;
+    for (int q = 0; q < 3; ++q) cy[q * tx * (ty + 1) + e] = in ? __ldg(a.cy + q * n2 + g) : 0.0;
+  }
+  for (int e = threadIdx.x; e < tx * ty; e += blockDim.x) {
+    const int r = e / tx, c = e - r * tx;
+    const bool in = r < h_own && c < w_own;
+    const int g = in ? idx2(d, j0 + r, i0 + c) : 0;
+    sx[e] = in ? __ldg(a.sxy + g) : 0.0;
+    sy[e] = in ? __ldg(a.sxy + n2 + g) : 0.0;
+  }
+  // ---- the thread's own cells
+  const int lx = threadIdx.x % tx, ly0 = (int)(threadIdx.x / tx) * CPT;
+  const int rows = lx < w_own ? min(CPT, h_own - ly0) : 0;  // owned rows, none where <= 0
+  const int o0 = (ly0 + 2) * PX + lx + 2, g0 = idx2(d, j0 + ly0, i0 + lx);
+  auto own = [&](int q) { return q < rows; };
+  auto edge = [&](int q) { return lx < 2 || lx >= w_own - 2 || ly0 + q < 2 || ly0 + q >= h_own - 2; };
+  SumWord* const pub0 = reinterpret_cast<SumWord*>(a.pub) + g0;
+  // ---- halo: the cells two deep around the tile that the stencil reads, two
+  // columns west and east, two rows south and north (none beyond the walls);
+  // cell h as its place e in the padded tile and its 2-D index g
+  const int n_halo = 4 * (h_own + w_own);
+  auto halo_cell = [&](int h, int& e, int& g) {
+    if (h >= n_halo) return false;
+    int r, c;
+    if (h < 4 * h_own) {
+      const int s = h / h_own;
+      r = h - s * h_own;
+      c = s < 2 ? s - 2 : w_own + s - 2;
+    } else {
+      const int m = h - 4 * h_own, s = m / w_own;
+      c = m - s * w_own;
+      r = s < 2 ? s - 2 : h_own + s - 2;
+    }
+    if (j0 + r < 0 || j0 + r >= d.ny) return false;
+    e = (r + 2) * PX + c + 2;
+    g = idx2(d, j0 + r, wrap(i0 + c));
+    return true;
+  };
+  // from the last thread down: the first warps gather the sums
+  const int h0 = (int)(blockDim.x - 1 - threadIdx.x), hstep = (int)blockDim.x;
+  int he[HS], hg[HS];  // place -1: no cell
+#pragma unroll
+  for (int s = 0; s < HS; ++s)
+    if (h0 < 0 || !halo_cell(h0 + s * hstep, he[s], hg[s])) he[s] = -1;
+  // f(e, g, h) over this thread's halo cells
+  auto each_halo = [&](auto&& f) {
+#pragma unroll
+    for (int s = 0; s < HS; ++s)
+      if (he[s] >= 0) f(he[s], hg[s], h0 + s * hstep);
+    for (int h = h0 < 0 ? n_halo : h0 + HS * hstep; h < n_halo; h += hstep) {
+      int e, g;
+      if (halo_cell(h, e, g)) f(e, g, h);
+    }
+  };
+  unsigned long long seq = *reinterpret_cast<volatile unsigned long long*>(a.seq) + 1;
+  // Publishes own(q)'s value along the tile's edges; before exchange().
+  auto publish = [&](int q, double v) {
+    if (edge(q)) st_word(pub0 + (seq & 1) * n2 + q * d.P, v, seq);
+  };
+  // Sums of NQ values over the grid into `out`, the same bits in every block,
+  // and the published values of the halo cells into hv.  Words alternate
+  // between two sets: a block writes those of exchange n + 2 only after it has
+  // seen every block's sums n + 1, which follow that block's reads of n.
+  // False if a word did not come within the poll limit or a block gave up.
+  const int nchunk = (nb + 31) / 32;
+  auto exchange = [&](auto& v, auto& out) {
+    constexpr int NQ = sizeof(v) / sizeof(double);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
+    if (lane == 0) {
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) sh.red[q][warp] = v[q];
+    }
+    __syncthreads();
+    bool ok = true;
+    if (warp == 0) {
+      double x[NQ];
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) x[q] = lane < nw ? sh.red[q][lane] : 0.0;
+#pragma unroll
+      for (int o = PJ_RES_THREADS / 64; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) x[q] += __shfl_down_sync(0xffffffffu, x[q], o);
+      if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) sh.tot[q] = x[q];
+      }
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < NQ * nb; t += blockDim.x) {
+      const int q = t / nb, dst = t - q * nb;
+      st_word(words + ((size_t)((seq & 1) * nb + dst) * ZM_PJ_SUMS + q) * nb + blockIdx.x, sh.tot[q], seq);
+    }
+    const SumWord* mine = words + (size_t)((seq & 1) * nb + blockIdx.x) * ZM_PJ_SUMS * nb;
+    for (int c = warp; c < NQ * nchunk; c += nw) {
+      const int q = c / nchunk, blk = (c - q * nchunk) * 32 + lane;
+      double y = 0.0;
+      if (blk < nb) ok = wait_word(mine + q * nb + blk, seq, a, y) && ok;
+      __syncwarp();
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) y += __shfl_down_sync(0xffffffffu, y, o);
+      if (lane == 0) sh.part[q][c - q * nchunk] = y;
+    }
+    const SumWord* pub = reinterpret_cast<const SumWord*>(a.pub) + (seq & 1) * n2;
+    each_halo([&](int, int g, int h) { ok = ok && wait_word(pub + g, seq, a, hv[h]); });
+    ++seq;
+    if (__syncthreads_or(!ok)) return false;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      double y = sh.part[q][0];
+      for (int c = 1; c < nchunk; ++c) y += sh.part[q][c];
+      out[q] = y;
+    }
+    return true;
+  };
+  // ---- A f on the thread's cells, f a padded array
+  const int fy = tx * (ty + 1), fx = (tx + 1) * ty;
+  const int ey0 = ly0 * tx + lx, ex0 = ly0 * (tx + 1) + lx + 1;  // the face south of the first row, the one east of it
+  __syncthreads();
+  double k_[REGS ? 14 : 1];
+  if (REGS && rows > 0) {
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      k_[q] = cx[q * fx + ex0];
+      k_[3 + q] = cx[q * fx + ex0 - 1];
+      k_[6 + q] = cy[q * fy + ey0 + tx];
+      k_[9 + q] = cy[q * fy + ey0];
+    }
+    k_[12] = sx[ey0];
+    k_[13] = sy[ey0];
+  }
+  auto apply = [&](const double* f, double (&out)[CPT]) {
+#pragma unroll
+    for (int q = 0; q < CPT; ++q) out[q] = 0.0;
+    if (rows <= 0) return;
+    const double* c = f + o0;
+    if (REGS) {
+      const double pc = c[0], pw = c[-1], pe = c[1], pn = c[PX], ps = c[-PX];
+      const double dw = pc - pw, de = pe - pc, ds = pc - ps, dn = pn - pc;
+      const double fe = k_[0] * dw + k_[1] * de + k_[2] * (c[2] - pe);
+      const double fw = k_[3] * (pw - c[-2]) + k_[4] * dw + k_[5] * de;
+      const double fn = k_[6] * ds + k_[7] * dn + k_[8] * (c[2 * PX] - pn);
+      const double fs = k_[9] * (ps - c[-2 * PX]) + k_[10] * ds + k_[11] * dn;
+      out[0] = -(k_[12] * (fe - fw) + k_[13] * (fn - fs));
+      return;
+    }
+    const double* ky = cy + ey0;
+    const double* kx = cx + ex0;
+    // north flux of the row below the chunk
+    double fs = ky[0] * (c[-PX] - c[-2 * PX]) + ky[fy] * (c[0] - c[-PX]) + ky[2 * fy] * (c[PX] - c[0]);
+#pragma unroll
+    for (int q = 0; q < CPT; ++q) {
+      if (q >= rows) break;
+      ky += tx;
+      const double pc = c[0], pw = c[-1], pe = c[1], pn = c[PX];
+      const double dw = pc - pw, de = pe - pc;
+      const double fe = kx[0] * dw + kx[fx] * de + kx[2 * fx] * (c[2] - pe);
+      const double fw = kx[-1] * (pw - c[-2]) + kx[fx - 1] * dw + kx[2 * fx - 1] * de;
+      const double fn = ky[0] * (pc - c[-PX]) + ky[fy] * (pn - pc) + ky[2 * fy] * (c[2 * PX] - pn);
+      out[q] = -(sx[ey0 + q * tx] * (fe - fw) + sy[ey0 + q * tx] * (fn - fs));
+      fs = fn;
+      c += PX;
+      kx += tx + 1;
+    }
+  };
+  for (int e = threadIdx.x; e < PX * PY; e += blockDim.x) z[e] = sv[e] = 0.0;
+  __syncthreads();
+  // z = M b, r = b; psi = 0
+  double psi[CPT], x[CPT], r[CPT], p[CPT], w[CPT];
+  double s2[2] = {0.0, 0.0}, t2[2];
+#pragma unroll
+  for (int q = 0; q < CPT; ++q) {
+    psi[q] = r[q] = 0.0;
+    if (own(q)) {
+      const int g = g0 + q * d.P;
+      r[q] = __ldcg(a.b + g);
+      z[o0 + q * PX] = ident ? r[q] : r[q] * __ldg(a.minv + g);
+      s2[0] += r[q] * r[q];
+      s2[1] += r[q] * r[q] * __ldg(a.rarea + g);
+      publish(q, r[q]);
+    }
+  }
+  if (!exchange(s2, t2)) return;
+  each_halo([&](int e, int g, int h) { z[e] = ident ? hv[h] : hv[h] * __ldg(a.minv + g); });
+  __syncthreads();
+  const double floor2 = a.tol2 * t2[0], thresh = a.trtol2 * t2[1], norm_in = t2[1];
+  int it[3] = {0, 0, 0}, nref = 0;
+
+  // one CG solve from r and z into x; NQ 2 without a preconditioner, where
+  // <r, r> is gamma, else 3; returns the iterations, -1 after a timeout
+  auto solve_n = [&](auto nq, double atol2) {
+    constexpr int NQ = decltype(nq)::value;
+    double gamma_old = 1.0, alpha_old = 1.0;
+#pragma unroll
+    for (int q = 0; q < CPT; ++q) x[q] = p[q] = 0.0;
+    for (int k = 0;; ++k) {
+      apply(z, w);
+      double s[NQ], t[NQ];
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) s[q] = 0.0;
+#pragma unroll
+      for (int q = 0; q < CPT; ++q) {
+        if (!own(q)) continue;
+        publish(q, w[q]);
+        const double zq = NQ == 2 ? r[q] : z[o0 + q * PX];
+        s[0] += r[q] * zq;
+        s[1] += w[q] * zq;
+        if (NQ > 2) s[NQ - 1] += r[q] * r[q];
+      }
+      if (!exchange(s, t)) return -1;
+      if (!(t[NQ > 2 ? NQ - 1 : 0] > atol2) || k >= a.niter) return k;
+      const double beta = k > 0 ? t[0] / gamma_old : 0.0;
+      const double alpha = k > 0 ? t[0] / (t[1] - beta * t[0] / alpha_old) : t[0] / t[1];
+      gamma_old = t[0];
+      alpha_old = alpha;
+      each_halo([&](int e, int g, int h) {
+        const double sq = k > 0 ? fma(beta, sv[e], hv[h]) : hv[h];
+        sv[e] = sq;
+        z[e] -= alpha * (NQ == 2 ? sq : sq * __ldg(a.minv + g));
+      });
+#pragma unroll
+      for (int q = 0; q < CPT; ++q) {
+        if (!own(q)) continue;
+        const int o = o0 + q * PX;
+        p[q] = fma(beta, p[q], NQ == 2 ? r[q] : z[o]);
+        const double sq = k > 0 ? fma(beta, sv[o], w[q]) : w[q];
+        sv[o] = sq;
+        x[q] += alpha * p[q];
+        r[q] -= alpha * sq;
+        z[o] = NQ == 2 ? r[q] : r[q] * __ldg(a.minv + g0 + q * d.P);
+      }
+      __syncthreads();
+    }
+  };
+  auto solve = [&](double atol2) {
+    return ident ? solve_n(PjInt<2>{}, atol2) : solve_n(PjInt<3>{}, atol2);
+  };
+  // w = A psi (through z, which the caller sets again)
+  auto apply_psi = [&]() {
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < CPT; ++q)
+      if (own(q)) {
+        z[o0 + q * PX] = psi[q];
+        publish(q, psi[q]);
+      }
+    double s[1] = {0.0}, t[1];
+    if (!exchange(s, t)) return false;
+    each_halo([&](int e, int, int h) { z[e] = hv[h]; });
+    __syncthreads();
+    apply(z, w);
+    __syncthreads();
+    return true;
+  };
+
+  it[0] = solve(a.tol2 * t2[0]);
+  if (it[0] < 0) return;
+#pragma unroll
+  for (int q = 0; q < CPT; ++q) psi[q] = x[q];
+  for (int n = 0; n < a.refinements; ++n) {
+    // residual of the corrected velocity: res = b - A psi
+    if (!apply_psi()) return;
+    double s[2] = {0.0, 0.0}, t[2];
+#pragma unroll
+    for (int q = 0; q < CPT; ++q) {
+      if (!own(q)) continue;
+      const int g = g0 + q * d.P;
+      const double res = __ldcg(a.b + g) - w[q];
+      r[q] = res;
+      z[o0 + q * PX] = ident ? res : res * __ldg(a.minv + g);
+      s[0] += res * res;
+      s[1] += res * res * __ldg(a.rarea + g);
+      publish(q, res);
+    }
+    if (!exchange(s, t)) return;
+    if (!(t[1] > thresh)) break;
+    each_halo([&](int e, int g, int h) { z[e] = ident ? hv[h] : hv[h] * __ldg(a.minv + g); });
+    __syncthreads();
+    ++nref;
+    it[1 + n] = solve(fmax(a.tol2 * t[0], floor2));
+    if (it[1 + n] < 0) return;
+#pragma unroll
+    for (int q = 0; q < CPT; ++q) psi[q] += x[q];
+  }
+#pragma unroll
+  for (int q = 0; q < CPT; ++q)
+    if (own(q)) a.psi[g0 + q * d.P] = psi[q];
+  if (a.norms) {  // ledger mode, as in k_proj_cg
+    if (!apply_psi()) return;
+    double s[1] = {0.0}, t[1];
+#pragma unroll
+    for (int q = 0; q < CPT; ++q)
+      if (own(q)) {
+        const double res = __ldcg(a.b + g0 + q * d.P) - w[q];
+        s[0] += res * res * __ldg(a.rarea + g0 + q * d.P);
+        publish(q, 0.0);
+      }
+    if (!exchange(s, t)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      a.norms[0] = a.dtg * a.dtg * norm_in;
+      a.norms[1] = a.dtg * a.dtg * t[0];
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    a.stats[0] = it[0];
+    a.stats[1] = it[1];
+    a.stats[2] = it[2];
+    a.stats[3] = nref;
+    *a.seq = seq - 1;  // every block has read it: it took part in the last exchange
+  }
+}
+
+void (*proj_res_kernel(int cpt))(Dev, ProjArgs) {
+  return cpt <= 1 ? k_proj_res<1> : cpt == 2 ? k_proj_res<2> : cpt == 3 ? k_proj_res<3> : cpt == 4 ? k_proj_res<4> : k_proj_res<5>;
+}
+
+// The tile of the resident solver: at most one block per SM, a block's cells in
+// PJ_RES_THREADS threads of at most five rows and its arrays in shared memory.  Fewest
+// cells per block first (an iteration's work), but no fewer than `least`: below
+// that the exchange grows with every block and the work is hidden (at 96x48
+// cells 2.6 us per iteration with at least 256, 3.3 with 128, 2.9 with 512).
+bool proj_res_tile(int nx, int ny, int sms, size_t smem_max, int least, ProjTile& best) {
+  best = ProjTile{};
+  for (int nty = 1; nty <= ny; ++nty)
+    for (int ntx = 1; ntx <= nx && ntx * nty <= std::min(sms, 32 * PJ_CHUNKS); ++ntx) {
+      ProjTile t{};
+      t.x = (nx + ntx - 1) / ntx;
+      t.y = (ny + nty - 1) / nty;
+      // no empty tiles, and edges wide enough that a halo lies in the next tile alone
+      t.tiles_x = (nx + t.x - 1) / t.x;
+      t.tiles_y = (ny + t.y - 1) / t.y;
+      if (t.x > PJ_RES_THREADS) continue;
+      t.cpt = 1;
+      while (t.cpt <= 5 && t.x * ((t.y + t.cpt - 1) / t.cpt) > PJ_RES_THREADS) ++t.cpt;
+      if (t.cpt > 5) continue;
+      t.blocks = t.tiles_x * t.tiles_y;
+      t.threads = (t.x * ((t.y + t.cpt - 1) / t.cpt) + 31) / 32 * 32;
+      t.smem = proj_res_smem(t.x, t.y);
+      if (t.smem > smem_max) continue;
+      const int cells = t.x * t.y;
+      if (t.blocks > 1 && cells < least) continue;
+      const int cost = cells * 8 + t.x + t.y;
+      if (best.blocks == 0 || cost < best.x * best.y * 8 + best.x + best.y) best = t;
+    }
+  return best.blocks > 0;
 }
 
 }  // namespace zm

@@ -93,6 +93,7 @@ struct zm_solver {
   bool proj_on = false;
   ProjArgs pj{};
   int pj_blocks = 0;
+  ProjTile pj_tile{};   // resident form of the solves (blocks 0: the grid does not fit)
   double pj_dtg = 0.0;
   double *pj_dzn = nullptr, *pj_cos = nullptr, *pj_area = nullptr;
   float *up = nullptr, *vp = nullptr;
@@ -414,7 +415,11 @@ struct zm_solver {
     pe(s);
     ProjArgs pa = pj;
     pa.norms = ledger_on ? led_norms : nullptr;
-    coop_launch(s, ZM_K_PROJECTION, k_proj_cg, pj_blocks, PJ_THREADS, 0, d, pa);
+    if (pj_tile.blocks > 0)
+      coop_launch(s, ZM_K_PROJECTION, proj_res_kernel(pj_tile.cpt), pj_tile.blocks, pj_tile.threads, pj_tile.smem, d,
+                  pa);
+    else
+      coop_launch(s, ZM_K_PROJECTION, k_proj_cg, pj_blocks, PJ_THREADS, 0, d, pa);
     if (ledger_on) {
       k_led_proj<<<1, 32, 0, s>>>(led_norms, led_acc);
       check_launch();
@@ -1220,6 +1225,23 @@ void build(zm_solver* s, const zm_grid* g, const zm_params* p) {
     a.trtol2 = trtol * trtol;
     a.niter = p->projection_niter;
     a.refinements = p->projection_max_refinements;
+    int optin = 0;
+    ZM_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
+    if (proj_res_tile(nx, ny, sms, (size_t)optin, 256, s->pj_tile)) {
+      auto kern = proj_res_kernel(s->pj_tile.cpt);
+      ZM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+      ZM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, s->pj_tile.threads, s->pj_tile.smem));
+      if (per_sm < 1) s->pj_tile.blocks = 0;
+    }
+    if (s->pj_tile.blocks > 0) {
+      a.tile_x = s->pj_tile.x;
+      a.tile_y = s->pj_tile.y;
+      a.tiles_x = s->pj_tile.tiles_x;
+      a.pub = s->alloc<double>(4 * s->n2);
+      a.words = s->alloc<double>((size_t)2 * ZM_PJ_SUMS * s->pj_tile.blocks * s->pj_tile.blocks * 2);
+      a.seq = s->alloc<unsigned long long>(1);
+      a.max_polls = ZM_BT_BARRIER_POLLS;
+    }
     s->pj_dtg = p->dt * 9.81;
     a.dtg = s->pj_dtg;
     s->proj_on = true;
