@@ -2,23 +2,30 @@
 // legacy branch; _subcycle of timestepping/subcycles.py:6-26).
 //
 // Resident path (k_bt_loop): one cooperative kernel runs all subcycles.  Each
-// block owns one BT_TX x BT_TY tile and keeps its float64 state (eta, ubt,
-// vbt) plus the static fields it stencils over (wet mask, 1/dx) in shared
-// memory, with a two-cell halo, and the forcing and Coriolis parameter of its
-// owned cells, for the whole loop.  Per subcycle:
-//   1  refresh the halo from the neighbours' published values of the previous
-//      subcycle (and apply the polar cap to the velocities);
+// block owns one tile and keeps its float64 state (eta, ubt, vbt) with a
+// two-cell halo, the static fields it stencils over and the forcing of its
+// cells in shared memory for the whole loop.  Per subcycle:
+//   1  the halo of eta, ubt, vbt from the neighbours' words of the previous
+//      subcycle (and the polar cap of the velocities);
 //   2  continuity eta* = (eta - dt H div(ubt wm, vbt wm)) wm on the tile and,
-//      redundantly, on its one-cell ring, so the gradient needs no exchange;
-//   3  (cap active only) publish band-row partial sums, grid barrier, cap eta*;
+//      redundantly, on the four sides of its one-cell ring, so the gradient
+//      needs no exchange;
+//   3  sponge and relaxation of eta* with their volume refill; (cap active)
+//      band-row partial sums, grid barrier, cap of eta*;
 //   4  momentum: adjoint gradient of eta*, u* = ubt + dt (-g grad eta* + F),
-//      backward-Euler Coriolis, implicit drag, wet mask; publish eta*, u, v;
-//   5  grid barrier.
+//      backward-Euler Coriolis, implicit drag, wet mask; the cells within two
+//      of the tile's edge publish eta*, u, v as exchange words.
+// What bounds the loop is the latency of a subcycle (at 180x90 the work of one
+// is 16200 cells).  A block waits only for its neighbours' words: no grid
+// barrier, no fence, and a block may run ahead of far ones.  The counter barrier
+// and the separate halo loads this replaces took 7.3 us per subcycle at every
+// grid size up to 360x180 (9.5 at 720x360); a subcycle takes 2.0 us at 180x90,
+// 3.2 at 360x180 and 4.7 at 720x360.  Grids between 300 and 480 thousand
+// cells streamed before (three launches per subcycle, 0.49 ms at 800x400; now 0.165).
 // The polar cap (numerics/horizontal.py:387-451) needs the wet-point zonal mean
 // of each band row; blocks write per-tile partial row sums and every reader
 // folds them in tile order, so the result does not depend on timing.  When no
-// band row has a wet point the cap is the identity and step 3 is skipped.
-// Published fields and partial sums are double-buffered by subcycle parity.
+// band row has a wet point the cap is the identity and its steps are skipped.
 //
 // Streaming path (k_bt_eta / k_bt_vel / k_cap2d): for grids whose tiles cannot
 // all be resident, three plain kernels per subcycle in the same arithmetic.
@@ -40,326 +47,417 @@ __device__ __forceinline__ int band_of(int ny, int nb, int j) {
   return -1;
 }
 
-constexpr int BT_PX = BT_TX + 2 * BT_H, BT_PY = BT_TY + 2 * BT_H;
-
 // Backward-Euler Coriolis with the implicit linear drag
 // (barotropic.py:86-265): u = (u* + fd v*) drag / (1 + fd^2), fd = f dt_bt.
 // The factor drag / (1 + fd^2) is static per cell; both paths form it here.
 __device__ __forceinline__ double bt_drag_factor(double fd, double drag) { return drag / (1.0 + fd * fd); }
 
-struct BtTile {
-  double U[BT_PY][BT_PX], V[BT_PY][BT_PX];  // velocities (capped at the subcycle start)
-  double E[BT_PY][BT_PX];                   // eta; overwritten in place by eta* on the tile + ring
-  double ix[BT_PY][BT_PX];                  // 1/dx
-  float w[BT_PY][BT_PX];                    // 2-D wet mask
-  double cosl[BT_PY], cfp[BT_PY], cfm[BT_PY];
-  double iyc[BT_PY];                        // 1/(dy cos(lat)) of the row
-  double mean[3][2 * ZM_BT_MAX_NB];         // band-row means: eta*, u, v
-  double red[BT_THREADS];
-  double fx[BT_TY][BT_TX], fy[BT_TY][BT_TX];  // forcing of the owned cells
-  double fd[BT_TY][BT_TX], rd[BT_TY][BT_TX];  // f dt and drag / (1 + (f dt)^2) of the owned cells
-  int gj[BT_PY];                            // global row, -1 beyond the walls
-  int gx[BT_PX];                            // global column (periodic wrap)
-  unsigned char own_c[BT_PX];               // column owned by this block
+constexpr int BT_H = 2;      // halo width
+constexpr int BT_HS = 2;     // halo words per thread held ready
+constexpr int BT_FIELDS = 3; // eta, ubt, vbt
+
+// item flags: open faces, wet cell, owned cell, owned cell within two of the tile's edge
+constexpr unsigned BT_E = 1u, BT_W = 2u, BT_N = 4u, BT_S = 8u, BT_WET = 16u, BT_OWN = 32u, BT_PUB = 64u, BT_LIVE = 128u;
+constexpr int BT_ROW = 8;    // above the flags: the cell's padded row
+
+struct BtFixed {  // the part of a block's shared memory whose size does not depend on the tile
+  double mean[3][2 * ZM_BT_MAX_NB];  // band-row means: eta*, u, v
+  double red[32];
+  double part[WORD_CHUNKS];
+  double tot;
 };
-
-// Continuity at padded cell (r, c); numerics/horizontal.py:69-97 flux form.
-__device__ __forceinline__ double eta_new(const Dev& d, const BtArgs& a, const BtTile& t, int r, int c) {
-  const int j = t.gj[r];
-  const double w0 = t.w[r][c], we = t.w[r][c + 1], ww = t.w[r][c - 1];
-  const double u0 = t.U[r][c] * w0, ue = t.U[r][c + 1] * we, uw = t.U[r][c - 1] * ww;
-  const double fe = 0.5 * (u0 + ue) * (w0 * we);
-  const double fw = 0.5 * (uw + u0) * (ww * w0);
-  const double div_x = (fe - fw) * t.ix[r][c];
-  const double v0 = t.V[r][c] * w0;
-  double fn = 0.0, fs = 0.0;
-  if (j < d.ny - 1) {
-    const double wn = t.w[r + 1][c];
-    fn = 0.5 * (v0 + t.V[r + 1][c] * wn) * (w0 * wn) * t.cfp[r];
-  }
-  if (j > 0) {
-    const double ws = t.w[r - 1][c];
-    fs = 0.5 * (t.V[r - 1][c] * ws + v0) * (ws * w0) * t.cfp[r - 1];
-  }
-  const double div = div_x + (fn - fs) * t.iyc[r];
-  return (t.E[r][c] - a.dtH * div) * w0;
-}
-
-// wet-point partial sums of a padded tile field over the owned cells of each band row
-__device__ void band_partials(const Dev& d, const BtArgs& a, BtTile& t, const double (*f)[BT_PX], double* part,
-                              int xt) {
-  for (int r = BT_H; r < BT_H + BT_TY; ++r) {
-    const int j = t.gj[r];
-    if (j < 0) continue;  // uniform over the block
-    const int b = band_of(d.ny, a.nb, j);
-    if (b < 0) continue;
-    double s = 0.0;
-    for (int c = BT_H + threadIdx.x; c < BT_H + BT_TX; c += blockDim.x)
-      if (t.own_c[c]) s += f[r][c] * (double)t.w[r][c];
-    t.red[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-      if (threadIdx.x < o) t.red[threadIdx.x] += t.red[threadIdx.x + o];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) part[b * a.ntx + xt] = t.red[0];
-    __syncthreads();
-  }
-}
-
-__device__ void band_means(const BtArgs& a, BtTile& t, int q, const double* part) {
-  for (int b = threadIdx.x; b < 2 * a.nb; b += blockDim.x) {
-    double s = 0.0;
-    for (int xt = 0; xt < a.ntx; ++xt) s += part[b * a.ntx + xt];
-    t.mean[q][b] = s / a.count[b];
-  }
-}
-
-// polar-cap blend of value f at row j with wet weight w
-__device__ __forceinline__ double cap_val(const BtArgs& a, const BtTile& t, int ny, int q, int j, double w, double f) {
-  const int b = band_of(ny, a.nb, j);
-  if (b < 0) return f;
-  const double wt = (double)a.wts[b < a.nb ? b : 2 * a.nb - 1 - b];
-  return wt * (t.mean[q][b] * w) + (1.0 - wt) * (f * w);
-}
-
-// Decay of eta* by fac on the tile and its ring with the uniform refill of the
-// removed volume (barotropic.py:22-31): the owned cells' sum of
-// area (eta fac - eta) is published per block, and after a grid barrier every
-// block folds the partials in block order.
-__device__ bool refill(const Dev& d, const BtArgs& a, BtTile& t, const double* fac, double* part, unsigned nblocks) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  constexpr int NT = BT_TX * BT_TY;
-  constexpr int NR = (BT_TX + 2) * (BT_TY + 2);
-  double s = 0.0;
-  for (int e = tid; e < NT; e += nt) {
-    const int r = BT_H + e / BT_TX, c = BT_H + e % BT_TX;
-    const int j = t.gj[r];
-    if (j < 0 || !t.own_c[c]) continue;
-    const int g = idx2(d, j, t.gx[c]);
-    const double e0 = t.E[r][c];
-    s += a.area[g] * (e0 * fac[g] - e0);
-  }
-  t.red[tid] = s;
-  __syncthreads();
-  for (int o = nt / 2; o > 0; o >>= 1) {
-    if (tid < o) t.red[tid] += t.red[tid + o];
-    __syncthreads();
-  }
-  if (tid == 0) part[blockIdx.x] = t.red[0];
-  if (!grid_barrier(a.bar, a.err, nblocks, ZM_BT_BARRIER_POLLS)) return false;
-  if (tid < 32) {
-    double x = 0.0;
-    for (unsigned b = tid; b < nblocks; b += 32) x += __ldcg(part + b);
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (tid == 0) t.red[0] = x;
-  }
-  __syncthreads();
-  const double shift = -t.red[0] / a.ocean;
-  for (int e = tid; e < NR; e += nt) {
-    const int r = 1 + e / (BT_TX + 2), c = 1 + e % (BT_TX + 2);
-    const int j = t.gj[r];
-    if (j < 0) continue;
-    const int g = idx2(d, j, t.gx[c]);
-    t.E[r][c] = t.E[r][c] * fac[g] + shift * (double)t.w[r][c];
-  }
-  __syncthreads();
-  return true;
-}
 
 }  // namespace
 
-size_t bt_tile_smem() { return sizeof(BtTile); }
+// Shared memory of a tile of tx x ty cells: eta, ubt, vbt, 1/dx on the padded
+// tile, forcing and Coriolis factors of the owned cells, row factors, wet flags.
+size_t bt_tile_smem(int tx, int ty) {
+  const size_t pad = (size_t)(tx + 2 * BT_H) * (ty + 2 * BT_H), own = (size_t)tx * ty;
+  return sizeof(BtFixed) + sizeof(double) * (4 * pad + 4 * own + 3 * (size_t)(ty + 2 * BT_H)) + (pad + 7) / 8 * 8;
+}
 
-__global__ void __launch_bounds__(BT_THREADS, 4) k_bt_loop(Dev d, BtArgs a) {
-  grid_barrier_begin(a.bar);
+// K: cells of continuity (tile and ring sides) per thread.
+template <int K>
+__global__ void __launch_bounds__(BT_THREADS, 1) k_bt_loop(Dev d, BtArgs a) {
   extern __shared__ double bt_smem[];
-  BtTile& t = *reinterpret_cast<BtTile*>(bt_smem);
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int xt = blockIdx.x % a.ntx, yt = blockIdx.x / a.ntx;
-  const int i0 = xt * BT_TX, j0 = yt * BT_TY;
+  const int tx = a.tile_x, ty = a.tile_y, PX = tx + 2 * BT_H, PY = ty + 2 * BT_H, PP = PX * PY;
+  BtFixed& sh = *reinterpret_cast<BtFixed*>(bt_smem);
+  double* E = bt_smem + sizeof(BtFixed) / sizeof(double);  // eta, then eta*
+  double* U = E + PP;
+  double* V = U + PP;
+  double* ixs = V + PP;             // 1/dx
+  double* fxs = ixs + PP;           // owned cells: forcing, f dt, drag / (1 + (f dt)^2)
+  double* fys = fxs + tx * ty;
+  double* fds = fys + tx * ty;
+  double* rds = fds + tx * ty;
+  double* iyc = rds + tx * ty;      // rows: 1 / (dy cos), cosine of the north and the south face
+  double* cfp = iyc + PY;
+  double* cfm = cfp + PY;
+  unsigned char* wet = reinterpret_cast<unsigned char*>(cfm + PY);
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
   const unsigned nblocks = gridDim.x;
+  const int bx = blockIdx.x % a.ntx, by = blockIdx.x / a.ntx;
+  const int i0 = bx * tx, j0 = by * ty;
+  const int w_own = min(tx, d.nx - i0), h_own = min(ty, d.ny - j0), n_own = w_own * h_own;
   const bool cap = a.cap_active != 0;
-  constexpr int NC = BT_PX * BT_PY;
-  constexpr int NR = (BT_TX + 2) * (BT_TY + 2);  // tile + one-cell ring
-  constexpr int NT = BT_TX * BT_TY;
-  // ---- geometry, static fields and the initial state on the padded tile
-  for (int c = tid; c < BT_PX; c += nt) {
-    const int gi = i0 - BT_H + c;
-    t.gx[c] = ((gi % d.nx) + d.nx) % d.nx;
-    t.own_c[c] = (c >= BT_H && c < BT_H + BT_TX && gi < d.nx) ? 1 : 0;
+  if (cap) grid_barrier_begin(a.bar);
+  auto wrap = [&](int i) {
+    i %= d.nx;
+    return i < 0 ? i + d.nx : i;
+  };
+  // ---- static fields and the initial state on the padded tile; beyond the walls only zero masks
+  for (int r = tid; r < PY; r += nt) {
+    const int j = min(max(j0 - BT_H + r, 0), d.ny - 1);
+    iyc[r] = d.inv_dy_d / (double)__ldg(d.cosl + j);
+    cfp[r] = (double)__ldg(d.cfp + j);
+    cfm[r] = (double)__ldg(d.cfm + j);
   }
-  for (int r = tid; r < BT_PY; r += nt) {
-    const int gj = j0 - BT_H + r;
-    t.gj[r] = (gj < 0 || gj >= d.ny) ? -1 : gj;
-    const int jc = gj < 0 ? 0 : (gj >= d.ny ? d.ny - 1 : gj);
-    t.cosl[r] = (double)__ldg(d.cosl + jc);
-    t.cfp[r] = (double)__ldg(d.cfp + jc);
-    t.cfm[r] = (double)__ldg(d.cfm + jc);
-    t.iyc[r] = d.inv_dy_d / t.cosl[r];
+  for (int e = tid; e < PP; e += nt) {
+    const int r = e / PX - BT_H, c = e - (r + BT_H) * PX - BT_H, j = j0 + r;
+    const bool in = j >= 0 && j < d.ny && r < h_own + BT_H && c < w_own + BT_H;
+    const int g = in ? idx2(d, j, wrap(i0 + c)) : 0;
+    E[e] = in ? (double)__ldg(a.eta_in + g) : 0.0;
+    U[e] = in ? a.ubt0[g] : 0.0;
+    V[e] = in ? a.vbt0[g] : 0.0;
+    ixs[e] = in ? __ldg(d.inv_dx_d + g) : 0.0;
+    wet[e] = in && __ldg(d.wet2 + g) != 0.f;
   }
-  __syncthreads();
-  for (int e = tid; e < NC; e += nt) {
-    const int r = e / BT_PX, c = e - r * BT_PX;
-    const int gj = t.gj[r];
-    if (gj < 0) {  // beyond a closed wall: only ever multiplied by a zero mask
-      t.U[r][c] = t.V[r][c] = t.E[r][c] = t.ix[r][c] = 0.0;
-      t.w[r][c] = 0.f;
-      continue;
-    }
-    const int g = idx2(d, gj, t.gx[c]);
-    t.U[r][c] = a.ubt0[g];
-    t.V[r][c] = a.vbt0[g];
-    t.E[r][c] = a.eta0[g];
-    t.w[r][c] = __ldg(d.wet2 + g);
-    t.ix[r][c] = __ldg(d.inv_dx_d + g);
-  }
-  for (int e = tid; e < NT; e += nt) {
-    const int r = e / BT_TX, c = e - r * BT_TX;
-    const int gj = t.gj[r + BT_H];
-    if (gj < 0 || !t.own_c[c + BT_H]) {
-      t.fx[r][c] = t.fy[r][c] = t.fd[r][c] = t.rd[r][c] = 0.0;
-      continue;
-    }
-    const int g = idx2(d, gj, t.gx[c + BT_H]);
-    t.fx[r][c] = a.Fx[g];
-    t.fy[r][c] = a.Fy[g];
+  const double fscale = 1.0 / (1025.0 * (double)d.H_sw);
+  for (int e = tid; e < n_own; e += nt) {
+    const int r = e / w_own, c = e - r * w_own, g = idx2(d, j0 + r, i0 + c);
+    // total barotropic forcing F_rho + tau / (rho0 H)
+    fxs[e] = (double)a.frx[g] + (double)__ldg(d.tau_x + g) * fscale;
+    fys[e] = (double)a.fry[g] + (double)__ldg(d.tau_y + g) * fscale;
     const double fd = __ldg(d.fcor_d + g) * a.dtb;
-    t.fd[r][c] = fd;
-    t.rd[r][c] = bt_drag_factor(fd, a.drag);
+    fds[e] = fd;
+    rds[e] = bt_drag_factor(fd, a.drag);
   }
   __syncthreads();
-  const double g9 = 9.81;
-  for (int n = 0; n < a.nsub; ++n) {
-    const int pin = n & 1, pout = pin ^ 1;
-    if (n > 0) {
-      // 1: halo from the neighbours' published fields; caps on every cell
-      if (cap) {
-        band_means(a, t, 1, a.part_u[pin]);
-        band_means(a, t, 2, a.part_v[pin]);
-        __syncthreads();
-      }
-      for (int e = tid; e < NC; e += nt) {
-        const int r = e / BT_PX, c = e - r * BT_PX;
-        const int gj = t.gj[r];
-        if (gj < 0) continue;
-        const bool own = r >= BT_H && r < BT_H + BT_TY && t.own_c[c];
-        if (own && !cap) continue;
-        double u, v;
-        if (own) {
-          u = t.U[r][c];
-          v = t.V[r][c];
-        } else {
-          const int g = idx2(d, gj, t.gx[c]);
-          u = a.pub_u[pin][g];
-          v = a.pub_v[pin][g];
-          t.E[r][c] = a.pub_e[pin][g];
-        }
-        if (cap) {
-          const double w = t.w[r][c];
-          u = cap_val(a, t, d.ny, 1, gj, w, u);
-          v = cap_val(a, t, d.ny, 2, gj, w, v);
-        }
-        t.U[r][c] = u;
-        t.V[r][c] = v;
-      }
-      __syncthreads();
-    }
-    // 2: continuity on the tile and its ring; each cell reads its own eta only,
-    // so eta* overwrites eta in place (after all threads computed)
-    double en[(NR + BT_THREADS - 1) / BT_THREADS];
+  // ---- this thread's cells: the owned ones first, then the ring's sides
+  const int n_eta = n_own + 2 * (w_own + h_own);
+  int at[K], gi[K];
+  unsigned fl[K];
 #pragma unroll
-    for (int q = 0; q < (NR + BT_THREADS - 1) / BT_THREADS; ++q) {
-      const int e = tid + q * BT_THREADS;
-      en[q] = 0.0;
-      if (e < NR) {
-        const int r = 1 + e / (BT_TX + 2), c = 1 + e % (BT_TX + 2);
-        if (t.gj[r] >= 0) en[q] = eta_new(d, a, t, r, c);
+  for (int q = 0; q < K; ++q) {
+    const int e = tid + q * nt;
+    at[q] = 0;
+    gi[q] = 0;
+    fl[q] = 0u;
+    if (e >= n_eta) continue;
+    int r, c;
+    if (e < n_own) {
+      r = e / w_own;
+      c = e - r * w_own;
+    } else {
+      const int m = e - n_own;
+      if (m < 2 * h_own) {
+        r = m % h_own;
+        c = m < h_own ? -1 : w_own;
+      } else {
+        c = (m - 2 * h_own) % w_own;
+        r = m - 2 * h_own < w_own ? -1 : h_own;
       }
+    }
+    const int j = j0 + r;
+    if (j < 0 || j >= d.ny) continue;
+    const int o = (r + BT_H) * PX + c + BT_H;
+    at[q] = o;
+    gi[q] = idx2(d, j, wrap(i0 + c));
+    unsigned f = BT_LIVE | (unsigned)(r + BT_H) << BT_ROW;
+    if (wet[o]) {
+      f |= BT_WET;
+      if (wet[o + 1]) f |= BT_E;
+      if (wet[o - 1]) f |= BT_W;
+      if (j < d.ny - 1 && wet[o + PX]) f |= BT_N;
+      if (j > 0 && wet[o - PX]) f |= BT_S;
+    }
+    if (e < n_own) {
+      f |= BT_OWN;
+      if (r < BT_H || r >= h_own - BT_H || c < BT_H || c >= w_own - BT_H) f |= BT_PUB;
+    }
+    fl[q] = f;
+  }
+  // ---- the halo words the stencils read: eta on the ring's sides, u and v there
+  // and on its corners, u two columns and v two rows out.  Word h as its place
+  // (field * PP + cell) in shared memory and its index (field * plane + cell)
+  const int n_halo = 8 * (w_own + h_own) + 8;
+  auto halo_word = [&](int h, int& place, long long& index) {
+    if (h >= n_halo) return false;
+    int r, c, f;
+    if (h < 8 * h_own) {  // west, east: eta, u, v at distance 1, u at distance 2
+      const int s = h / h_own, k = s >> 1;
+      r = h - s * h_own;
+      const int dist = k == 3 ? 2 : 1;
+      c = (s & 1) ? w_own - 1 + dist : -dist;
+      f = k == 3 ? 1 : k;
+    } else if (h < 8 * (h_own + w_own)) {  // south, north: eta, u, v at distance 1, v at distance 2
+      const int m = h - 8 * h_own, s = m / w_own, k = s >> 1;
+      c = m - s * w_own;
+      const int dist = k == 3 ? 2 : 1;
+      r = (s & 1) ? h_own - 1 + dist : -dist;
+      f = k == 3 ? 2 : k;
+    } else {  // corners: u and v
+      const int m = h - 8 * (h_own + w_own);
+      r = (m & 1) ? h_own : -1;
+      c = (m & 2) ? w_own : -1;
+      f = 1 + (m >> 2);
+    }
+    const int j = j0 + r;
+    if (j < 0 || j >= d.ny) return false;
+    place = f * PP + (r + BT_H) * PX + c + BT_H;
+    index = f * d.plane + idx2(d, j, wrap(i0 + c));
+    return true;
+  };
+  int hp[BT_HS];
+  long long hx[BT_HS];
+#pragma unroll
+  for (int s = 0; s < BT_HS; ++s)
+    if (!halo_word(tid + s * nt, hp[s], hx[s])) hp[s] = -1;
+  Word* const words = reinterpret_cast<Word*>(a.pub);
+  const long long set = BT_FIELDS * d.plane;
+  const unsigned long long base = *a.seq;  // k_final advances it when every block is done
+  unsigned long long sums = base;  // sequence number of the last grid-wide sum
+
+  // Sum over the grid, the same bits in every block: each block stores its
+  // partial sum into every block's own list (one copy per reader: a single
+  // list would be a few cache lines that all blocks poll).
+  auto grid_sum = [&](double v, double& out) {
+    ++sums;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) sh.red[warp] = v;
+    __syncthreads();
+    if (warp == 0) {
+      double x = lane < nw ? sh.red[lane] : 0.0;
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      if (lane == 0) sh.tot = x;
     }
     __syncthreads();
+    Word* lists = reinterpret_cast<Word*>(a.sums) + (size_t)(sums & 1) * nblocks * nblocks;
+    for (int t = tid; t < (int)nblocks; t += nt) st_word(lists + (size_t)t * nblocks + blockIdx.x, sh.tot, sums);
+    bool ok = true;
+    const int chunks = ((int)nblocks + 31) / 32;
+    for (int c = warp; c < chunks; c += nw) {
+      const int b = 32 * c + lane;
+      double y = 0.0;
+      if (b < (int)nblocks) ok = wait_word(lists + (size_t)blockIdx.x * nblocks + b, sums, a.err, ZM_BT_BARRIER_POLLS, y) && ok;
+      __syncwarp();
+      for (int o = 16; o > 0; o >>= 1) y += __shfl_down_sync(0xffffffffu, y, o);
+      if (lane == 0) sh.part[c] = y;
+    }
+    if (__syncthreads_or(!ok)) return false;
+    out = sh.part[0];
+    for (int c = 1; c < chunks; ++c) out += sh.part[c];
+    return true;
+  };
+  // Decay of eta* by fac on the tile and its ring with the uniform refill of
+  // the removed volume (barotropic.py:22-31).
+  auto refill = [&](const double* fac) {
+    double s = 0.0;
 #pragma unroll
-    for (int q = 0; q < (NR + BT_THREADS - 1) / BT_THREADS; ++q) {
-      const int e = tid + q * BT_THREADS;
-      if (e < NR) {
-        const int r = 1 + e / (BT_TX + 2), c = 1 + e % (BT_TX + 2);
-        t.E[r][c] = en[q];
+    for (int q = 0; q < K; ++q)
+      if (fl[q] & BT_OWN) {
+        const double e0 = E[at[q]];
+        s += a.area[gi[q]] * (e0 * fac[gi[q]] - e0);
       }
+    double dv;
+    if (!grid_sum(s, dv)) return false;
+    const double shift = -dv / a.ocean;
+#pragma unroll
+    for (int q = 0; q < K; ++q)
+      if (fl[q] & BT_LIVE) E[at[q]] = E[at[q]] * fac[gi[q]] + ((fl[q] & BT_WET) ? shift : 0.0);
+    __syncthreads();
+    return true;
+  };
+  // wet-point partial sums of a padded field over the owned cells of each band row, one warp per row
+  auto band_partials = [&](const double* f, double* part) {
+    for (int r = warp; r < h_own; r += nw) {
+      const int b = band_of(d.ny, a.nb, j0 + r);
+      if (b < 0) continue;
+      double s = 0.0;
+      for (int c = lane; c < w_own; c += 32) {
+        const int o = (r + BT_H) * PX + c + BT_H;
+        if (wet[o]) s += f[o];
+      }
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+      if (lane == 0) part[b * a.ntx + bx] = s;
+    }
+  };
+  auto band_means = [&](int q, const double* part) {
+    for (int b = tid; b < 2 * a.nb; b += nt) {
+      double s = 0.0;
+      for (int t = 0; t < a.ntx; ++t) s += __ldcg(part + b * a.ntx + t);
+      sh.mean[q][b] = s / a.count[b];
+    }
+  };
+  // polar-cap blend of value f at row j
+  auto cap_val = [&](int q, int j, bool w, double f) {
+    const int b = band_of(d.ny, a.nb, j);
+    if (b < 0) return f;
+    const double wt = (double)a.wts[b < a.nb ? b : 2 * a.nb - 1 - b], m = w ? 1.0 : 0.0;
+    return wt * (sh.mean[q][b] * m) + (1.0 - wt) * (f * m);
+  };
+
+  const double g9 = 9.81;
+  for (int n = 0; n < a.nsub; ++n) {
+    const int pout = n & 1;
+    if (n > 0) {
+      // 1: halo from the neighbours' words; caps on every cell
+      const unsigned long long seq = base + n;
+      const Word* in = words + (seq & 1) * set;
+      bool ok = true;
+#pragma unroll
+      for (int s = 0; s < BT_HS; ++s)
+        if (hp[s] >= 0) ok = wait_word(in + hx[s], seq, a.err, ZM_BT_BARRIER_POLLS, E[hp[s]]) && ok;
+      for (int h = tid + BT_HS * nt; h < n_halo && ok; h += nt) {
+        int place;
+        long long index;
+        if (halo_word(h, place, index)) ok = wait_word(in + index, seq, a.err, ZM_BT_BARRIER_POLLS, E[place]);
+      }
+      if (cap) {
+        band_means(1, a.part_u[pout ^ 1]);
+        band_means(2, a.part_v[pout ^ 1]);
+      }
+      if (__syncthreads_or(!ok)) return;
+      if (cap) {
+        for (int e = tid; e < PP; e += nt) {
+          const int r = e / PX - BT_H, j = j0 + r;
+          if (j < 0 || j >= d.ny || r >= h_own + BT_H) continue;
+          U[e] = cap_val(1, j, wet[e], U[e]);
+          V[e] = cap_val(2, j, wet[e], V[e]);
+        }
+        __syncthreads();
+      }
+    }
+    // 2: continuity (numerics/horizontal.py:69-97 flux form); a cell reads its own eta only
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+      const unsigned f = fl[q];
+      if (!(f & BT_LIVE)) continue;
+      const int o = at[q];
+      double en = 0.0;
+      if (f & BT_WET) {
+        const int r = (int)(f >> BT_ROW);
+        const double uc = U[o], vc = V[o];
+        const double fe = (f & BT_E) ? 0.5 * (uc + U[o + 1]) : 0.0;
+        const double fw = (f & BT_W) ? 0.5 * (U[o - 1] + uc) : 0.0;
+        const double fn = (f & BT_N) ? 0.5 * (vc + V[o + PX]) * cfp[r] : 0.0;
+        const double fs = (f & BT_S) ? 0.5 * (V[o - PX] + vc) * cfp[r - 1] : 0.0;
+        en = E[o] - a.dtH * ((fe - fw) * ixs[o] + (fn - fs) * iyc[r]);
+      }
+      E[o] = en;
     }
     __syncthreads();
     // 2b: lateral sponge, then eta relaxation, each with its volume refill
-    if (a.sponge && !refill(d, a, t, a.es, a.part_s[pout], nblocks)) return;
-    if (a.relax && !refill(d, a, t, a.er, a.part_r[pout], nblocks)) return;
+    if (a.sponge && !refill(a.es)) return;
+    if (a.relax && !refill(a.er)) return;
     // 3: polar cap of eta*
     if (cap) {
-      band_partials(d, a, t, t.E, a.part_e[pout], xt);
+      band_partials(E, a.part_e[pout]);
       if (!grid_barrier(a.bar, a.err, nblocks, ZM_BT_BARRIER_POLLS)) return;
-      band_means(a, t, 0, a.part_e[pout]);
+      band_means(0, a.part_e[pout]);
       __syncthreads();
-      for (int e = tid; e < NR; e += nt) {
-        const int r = 1 + e / (BT_TX + 2), c = 1 + e % (BT_TX + 2);
-        if (t.gj[r] >= 0) t.E[r][c] = cap_val(a, t, d.ny, 0, t.gj[r], t.w[r][c], t.E[r][c]);
-      }
+#pragma unroll
+      for (int q = 0; q < K; ++q)
+        if (fl[q] & BT_LIVE) E[at[q]] = cap_val(0, j0 + (int)(fl[q] >> BT_ROW) - BT_H, fl[q] & BT_WET, E[at[q]]);
       __syncthreads();
     }
-    // 4: momentum on the owned cells; publish eta*, u, v
-    for (int e = tid; e < NT; e += nt) {
-      const int r = BT_H + e / BT_TX, c = BT_H + e % BT_TX;
-      const int j = t.gj[r];
-      if (j < 0 || !t.own_c[c]) continue;
-      const int g = idx2(d, j, t.gx[c]);
-      const double w0 = t.w[r][c];
-      const double e0 = t.E[r][c];
-      const double gx = t.ix[r][c] * 0.5 *
-                        ((t.E[r][c + 1] - e0) * (w0 * t.w[r][c + 1]) + (e0 - t.E[r][c - 1]) * (w0 * t.w[r][c - 1]));
-      double dyp = 0.0, dym = 0.0;
-      if (j < d.ny - 1) dyp = (t.E[r + 1][c] - e0) * (w0 * t.w[r + 1][c]) * t.cfp[r];
-      if (j > 0) dym = (e0 - t.E[r - 1][c]) * (w0 * t.w[r - 1][c]) * t.cfm[r];
-      const double gy = t.iyc[r] * 0.5 * (dyp + dym);
-      const double us = t.U[r][c] + a.dtb * (-g9 * gx + t.fx[r - BT_H][c - BT_H]);
-      const double vs = t.V[r][c] + a.dtb * (-g9 * gy + t.fy[r - BT_H][c - BT_H]);
-      const double fd = t.fd[r - BT_H][c - BT_H], rd = t.rd[r - BT_H][c - BT_H];
-      double un = (us + fd * vs) * rd * w0;
-      double vn = (vs - fd * us) * rd * w0;
-      if (a.sponge) {
-        un *= a.es[g];
-        vn *= a.es[g];
+    // 4: momentum on the owned cells; publish eta*, u, v along the edges
+    const unsigned long long seq = base + n + 1;
+    Word* out = words + (seq & 1) * set;
+    const bool more = n + 1 < a.nsub;
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+      const unsigned f = fl[q];
+      if (!(f & BT_OWN)) continue;
+      const int o = at[q], e = tid + q * nt;
+      double un = 0.0, vn = 0.0;
+      const double e0 = E[o];
+      if (f & BT_WET) {
+        const int r = (int)(f >> BT_ROW);
+        const double de = (f & BT_E) ? E[o + 1] - e0 : 0.0, dw = (f & BT_W) ? e0 - E[o - 1] : 0.0;
+        const double dn = (f & BT_N) ? (E[o + PX] - e0) * cfp[r] : 0.0, ds = (f & BT_S) ? (e0 - E[o - PX]) * cfm[r] : 0.0;
+        const double gx = ixs[o] * 0.5 * (de + dw);
+        const double gy = iyc[r] * 0.5 * (dn + ds);
+        const double us = U[o] + a.dtb * (-g9 * gx + fxs[e]);
+        const double vs = V[o] + a.dtb * (-g9 * gy + fys[e]);
+        const double fd = fds[e], rd = rds[e];
+        un = (us + fd * vs) * rd;
+        vn = (vs - fd * us) * rd;
+        if (a.sponge) {
+          un *= a.es[gi[q]];
+          vn *= a.es[gi[q]];
+        }
       }
-      t.U[r][c] = un;
-      t.V[r][c] = vn;
-      a.pub_u[pout][g] = un;
-      a.pub_v[pout][g] = vn;
-      a.pub_e[pout][g] = e0;
+      U[o] = un;
+      V[o] = vn;
+      if ((f & BT_PUB) && more) {
+        st_word(out + gi[q], e0, seq);
+        st_word(out + d.plane + gi[q], un, seq);
+        st_word(out + 2 * d.plane + gi[q], vn, seq);
+      }
     }
-    __syncthreads();
+    __syncthreads();  // the halo is overwritten next
     if (cap) {
-      band_partials(d, a, t, t.U, a.part_u[pout], xt);
-      band_partials(d, a, t, t.V, a.part_v[pout], xt);
+      band_partials(U, a.part_u[pout]);
+      band_partials(V, a.part_v[pout]);
+      if (!grid_barrier(a.bar, a.err, nblocks, ZM_BT_BARRIER_POLLS)) return;
     }
-    // 5: the published fields are complete
-    if (!grid_barrier(a.bar, a.err, nblocks, ZM_BT_BARRIER_POLLS)) return;
   }
   // ---- outputs: capped velocities and the float32 free surface
-  const int plast = a.nsub & 1;
   if (cap) {
-    band_means(a, t, 1, a.part_u[plast]);
-    band_means(a, t, 2, a.part_v[plast]);
+    const int plast = (a.nsub - 1) & 1;
+    band_means(1, a.part_u[plast]);
+    band_means(2, a.part_v[plast]);
+    __syncthreads();
   }
-  __syncthreads();
-  for (int e = tid; e < NT; e += nt) {
-    const int r = BT_H + e / BT_TX, c = BT_H + e % BT_TX;
-    const int j = t.gj[r];
-    if (j < 0 || !t.own_c[c]) continue;
-    const int g = idx2(d, j, t.gx[c]);
-    double u = t.U[r][c], v = t.V[r][c];
+#pragma unroll
+  for (int q = 0; q < K; ++q) {
+    if (!(fl[q] & BT_OWN)) continue;
+    const int o = at[q];
+    double u = U[o], v = V[o];
     if (cap) {
-      u = cap_val(a, t, d.ny, 1, j, t.w[r][c], u);
-      v = cap_val(a, t, d.ny, 2, j, t.w[r][c], v);
+      const int j = j0 + (int)(fl[q] >> BT_ROW) - BT_H;
+      u = cap_val(1, j, fl[q] & BT_WET, u);
+      v = cap_val(2, j, fl[q] & BT_WET, v);
     }
-    a.ubt_out[g] = u;
-    a.vbt_out[g] = v;
-    a.eta_out[g] = (float)t.E[r][c];
+    a.ubt_out[gi[q]] = u;
+    a.vbt_out[gi[q]] = v;
+    a.eta_out[gi[q]] = (float)E[o];
   }
+}
+
+// After a launch that may have given up: the sequence number moves past every
+// word it may have left, the barrier and error words are cleared.
+__global__ void k_bt_reset(unsigned long long* seq, unsigned long long by, unsigned* sync) {
+  *seq += by;
+  for (int q = 0; q < 4; ++q) sync[q] = 0u;
+}
+
+void (*bt_loop_kernel(int k))(Dev, BtArgs) {
+  return k <= 1 ? k_bt_loop<1> : k == 2 ? k_bt_loop<2> : k == 3 ? k_bt_loop<3> : k_bt_loop<4>;
+}
+
+// The tile of the resident kernel: at most one block per SM, its cells and ring
+// sides on BT_THREADS threads of at most four, its arrays in shared memory.
+// Fewest cells per block, but no fewer than `least`; blocks 0 if none fits.
+BtTile bt_tile(int nx, int ny, int sms, size_t smem_max, int least) {
+  BtTile best{};
+  for (int nty = 1; nty <= ny; ++nty)
+    for (int ntx = 1; ntx <= nx && ntx * nty <= min(sms, 32 * WORD_CHUNKS); ++ntx) {
+      BtTile t{};
+      t.x = (nx + ntx - 1) / ntx;
+      t.y = (ny + nty - 1) / nty;
+      t.tiles_x = (nx + t.x - 1) / t.x;
+      t.blocks = t.tiles_x * ((ny + t.y - 1) / t.y);
+      const int cells = t.x * t.y, n_eta = cells + 2 * (t.x + t.y);
+      t.k = (n_eta + BT_THREADS - 1) / BT_THREADS;
+      if (t.k > 4 || (t.blocks > 1 && cells < least)) continue;
+      t.threads = ((n_eta + t.k - 1) / t.k + 31) / 32 * 32;
+      t.smem = bt_tile_smem(t.x, t.y);
+      if (t.smem > smem_max) continue;
+      if (best.blocks == 0 || 8 * cells + t.x + t.y < 8 * best.x * best.y + best.x + best.y) best = t;
+    }
+  return best;
 }
 
 // ---- streaming path: one subcycle as three plain kernels

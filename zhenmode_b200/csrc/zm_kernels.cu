@@ -1972,8 +1972,13 @@ __global__ void __launch_bounds__(256) k_final(Dev d, const float* __restrict__ 
                                                const float* __restrict__ T0, const float* __restrict__ S0,
                                                const float* __restrict__ means, const float* __restrict__ wts,
                                                int nb_rows, float* __restrict__ uo, float* __restrict__ vo,
-                                               float* __restrict__ To, float* __restrict__ So) {
+                                               float* __restrict__ To, float* __restrict__ So,
+                                               unsigned long long* __restrict__ seq, int seq_by) {
   pdl_trigger();
+  if (seq && blockIdx.x + blockIdx.y + blockIdx.z + threadIdx.x + threadIdx.y == 0) {
+    pdl_wait();  // the barotropic loop's blocks have all read it
+    *seq += seq_by;
+  }
   ZM_POINT_IDX
   const int c = idx2(d, j, i);
   const bool wet = wetb(wb(d, j, i), k);

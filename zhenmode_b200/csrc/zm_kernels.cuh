@@ -81,16 +81,19 @@ constexpr int NB_T = 6;
 #define ZM_BT_MAX_NB 64
 #define ZM_BT_BARRIER_POLLS (1u << 24)
 #define ZM_BT_ERR_BARRIER 1u
-// barotropic tile of the resident kernel: owned cells, halo width, threads
-constexpr int BT_TX = 32, BT_TY = 16, BT_H = 2, BT_THREADS = 128;
+// most threads of a block of the resident kernel
+constexpr int BT_THREADS = 768;
 struct BtArgs {
-  const double *eta0, *ubt0, *vbt0, *Fx, *Fy, *count;
-  double *pub_e[2], *pub_u[2], *pub_v[2];  // published fields by subcycle parity
+  const float *eta_in, *frx, *fry;     // free surface and F_rho at the start of the loop
+  const double *ubt0, *vbt0, *count;
+  void *pub, *sums;                    // exchange words: fields [2][3][ny][P], sums [2][blocks][blocks]
+  unsigned long long* seq;             // sequence number before this launch
   double *ubt_out, *vbt_out;
-  double *part_e[2], *part_u[2], *part_v[2];
+  double *part_e[2], *part_u[2], *part_v[2];  // cap active: band-row partial sums by subcycle parity
   float* eta_out;
   const float* wts;
   unsigned *bar, *err;
+  int tile_x, tile_y;
   int ntx, nb, nsub, cap_active;
   double dtH, dtb, drag;
   // lateral sponge and eta relaxation (barotropic.py:22-41); off when the flags are 0
@@ -98,10 +101,15 @@ struct BtArgs {
   const double *es, *er;     // exp(-sponge_rate dt_bt), exp(-eta_relax_rate dt_bt mask)
   const double* area;        // dx dy
   double ocean;              // max(sum area wet, 1)
-  double *part_s[2], *part_r[2];  // per-block refill partials by subcycle parity
+  double* part_s;            // streaming path: per-block refill partials
 };
-size_t bt_tile_smem();
-__global__ void k_bt_loop(Dev d, BtArgs a);
+struct BtTile {
+  int x, y, tiles_x, blocks, k, threads;  // blocks 0: no tile fits
+  size_t smem;
+};
+BtTile bt_tile(int nx, int ny, int sms, size_t smem_max, int least);
+void (*bt_loop_kernel(int k))(Dev, BtArgs);
+__global__ void k_bt_reset(unsigned long long* seq, unsigned long long by, unsigned* sync);
 __global__ void k_bt_eta(Dev d, const double* eta, const double* ubt, const double* vbt, double* eta_o, double dtH);
 __global__ void k_bt_vel(Dev d, const double* eta, const double* ubt, const double* vbt, const double* Fx,
                          const double* Fy, double* ubt_o, double* vbt_o, double dtb, double drag, const double* sv);
@@ -183,7 +191,7 @@ __global__ void k_cap3_means(Dev d, const float* u, const float* v, const float*
 __global__ void k_final(Dev d, const float* u3, const float* v3, const float* T3, const float* S3, const double* ubt,
                         const double* ubt0, const double* vbt, const double* vbt0, const float* u0, const float* v0,
                         const float* T0, const float* S0, const float* means, const float* wts, int nb_rows,
-                        float* uo, float* vo, float* To, float* So);
+                        float* uo, float* vo, float* To, float* So, unsigned long long* seq, int seq_by);
 // column-divergence projection of the stage-2 advective velocity (zm_projection.cu)
 constexpr int PJ_THREADS = 1024;
 #define ZM_PJ_SUMS 4

@@ -448,49 +448,14 @@ __global__ void __launch_bounds__(256) k_proj_correct(Dev d, float* __restrict__
 
 namespace {
 
-struct alignas(16) SumWord {
-  double v;
-  unsigned long long seq;
-};
-
-__device__ __forceinline__ void st_word(SumWord* p, double v, unsigned long long seq) {
-  asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}\n" ::"l"(p),
-               "l"(__double_as_longlong(v)), "l"(seq)
-               : "memory");
-}
-
-__device__ __forceinline__ SumWord ld_word(const SumWord* p) {
-  long long v;
-  unsigned long long q;
-  asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}\n"
-               : "=l"(v), "=l"(q)
-               : "l"(p)
-               : "memory");
-  return SumWord{__longlong_as_double(v), q};
-}
-
-// Polls a word until it carries seq; bounded, false after the limit or when another block gave up.
-__device__ __forceinline__ bool wait_word(const SumWord* p, unsigned long long seq, const ProjArgs& a, double& v) {
-  SumWord w = ld_word(p);
-  for (unsigned polls = 0; w.seq != seq; w = ld_word(p))
-    if (++polls > a.max_polls || ((polls & 255u) == 0u && ld_acquire(a.err) != 0u)) {
-      atomicOr(a.err, ZM_BT_ERR_BARRIER);
-      return false;
-    }
-  v = w.v;
-  return true;
-}
-
 template <int N>
 struct PjInt {
   static constexpr int value = N;
 };
 
-constexpr int PJ_CHUNKS = 5;  // at most 32 * PJ_CHUNKS blocks
-
 struct ResShared {  // fixed part of the block's shared memory
   double red[ZM_PJ_SUMS][32];
-  double tot[ZM_PJ_SUMS], part[ZM_PJ_SUMS][PJ_CHUNKS];
+  double tot[ZM_PJ_SUMS], part[ZM_PJ_SUMS][WORD_CHUNKS];
   double pad;  // an even number of doubles, for what follows
 };
 
@@ -521,7 +486,7 @@ __global__ void __launch_bounds__(PJ_RES_THREADS, 1) k_proj_res(Dev d, ProjArgs 
   double* cy = cx + 3 * (tx + 1) * ty;     // [3][ty + 1][tx]: north faces of rows -1 .. ty - 1
   double* sx = cy + 3 * tx * (ty + 1);     // [ty][tx] area / dx
   double* sy = sx + tx * ty;               // [ty][tx] area / (dy cos)
-  SumWord* words = reinterpret_cast<SumWord*>(a.words);
+  Word* words = reinterpret_cast<Word*>(a.words);
   const bool ident = a.minv == nullptr;
   const long long n2 = d.plane;
   const int i0 = (int)(blockIdx.x % a.tiles_x) * tx, j0 = (int)(blockIdx.x / a.tiles_x) * ty;
@@ -555,7 +520,7 @@ __global__ void __launch_bounds__(PJ_RES_THREADS, 1) k_proj_res(Dev d, ProjArgs 
   const int o0 = (ly0 + 2) * PX + lx + 2, g0 = idx2(d, j0 + ly0, i0 + lx);
   auto own = [&](int q) { return q < rows; };
   auto edge = [&](int q) { return lx < 2 || lx >= w_own - 2 || ly0 + q < 2 || ly0 + q >= h_own - 2; };
-  SumWord* const pub0 = reinterpret_cast<SumWord*>(a.pub) + g0;
+  Word* const pub0 = reinterpret_cast<Word*>(a.pub) + g0;
   // ---- halo: the cells two deep around the tile that the stencil reads, two
   // columns west and east, two rows south and north (none beyond the walls);
   // cell h as its place e in the padded tile and its 2-D index g
@@ -634,18 +599,18 @@ __global__ void __launch_bounds__(PJ_RES_THREADS, 1) k_proj_res(Dev d, ProjArgs 
       const int q = t / nb, dst = t - q * nb;
       st_word(words + ((size_t)((seq & 1) * nb + dst) * ZM_PJ_SUMS + q) * nb + blockIdx.x, sh.tot[q], seq);
     }
-    const SumWord* mine = words + (size_t)((seq & 1) * nb + blockIdx.x) * ZM_PJ_SUMS * nb;
+    const Word* mine = words + (size_t)((seq & 1) * nb + blockIdx.x) * ZM_PJ_SUMS * nb;
     for (int c = warp; c < NQ * nchunk; c += nw) {
       const int q = c / nchunk, blk = (c - q * nchunk) * 32 + lane;
       double y = 0.0;
-      if (blk < nb) ok = wait_word(mine + q * nb + blk, seq, a, y) && ok;
+      if (blk < nb) ok = wait_word(mine + q * nb + blk, seq, a.err, a.max_polls, y) && ok;
       __syncwarp();
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) y += __shfl_down_sync(0xffffffffu, y, o);
       if (lane == 0) sh.part[q][c - q * nchunk] = y;
     }
-    const SumWord* pub = reinterpret_cast<const SumWord*>(a.pub) + (seq & 1) * n2;
-    each_halo([&](int, int g, int h) { ok = ok && wait_word(pub + g, seq, a, hv[h]); });
+    const Word* pub = reinterpret_cast<const Word*>(a.pub) + (seq & 1) * n2;
+    each_halo([&](int, int g, int h) { ok = ok && wait_word(pub + g, seq, a.err, a.max_polls, hv[h]); });
     ++seq;
     if (__syncthreads_or(!ok)) return false;
 #pragma unroll
@@ -865,7 +830,7 @@ void (*proj_res_kernel(int cpt))(Dev, ProjArgs) {
 bool proj_res_tile(int nx, int ny, int sms, size_t smem_max, int least, ProjTile& best) {
   best = ProjTile{};
   for (int nty = 1; nty <= ny; ++nty)
-    for (int ntx = 1; ntx <= nx && ntx * nty <= std::min(sms, 32 * PJ_CHUNKS); ++ntx) {
+    for (int ntx = 1; ntx <= nx && ntx * nty <= std::min(sms, 32 * WORD_CHUNKS); ++ntx) {
       ProjTile t{};
       t.x = (nx + ntx - 1) / ntx;
       t.y = (ny + nty - 1) / nty;

@@ -102,6 +102,8 @@ struct zm_solver {
   double *eta64[2] = {nullptr, nullptr}, *Fx = nullptr, *Fy = nullptr, *wts_d = nullptr;
   BtArgs bt{};          // persistent barotropic kernel arguments
   int bt_blocks = 0;
+  BtTile btt{};
+  unsigned long long* bt_seq = nullptr;  // sequence number of the loop's exchange words
   unsigned* bt_sync = nullptr;  // [0..1] barrier counter/generation, [2] error flags
   // reference-layout staging (zm_step_host)
   Fields4 ref;
@@ -206,6 +208,14 @@ struct zm_solver {
     k_nu_class<<<(strips + 7) / 8, dim3(32, 8)>>>(d, nu_class_buf, warps, halo, (int)g.x, (int)g.y);
     check_launch();
     ZM_CUDA(cudaDeviceSynchronize());
+  }
+
+  // Clear the barotropic loop's barrier and error words.  The sequence number
+  // moves past every word that a launch which gave up may have left behind.
+  void reset_sync(cudaStream_t s) {
+    if (bt_seq) k_bt_reset<<<1, 1, 0, s>>>(bt_seq, 1ull << 20, bt_sync);
+    else ZM_CUDA(cudaMemsetAsync(bt_sync, 0, 4 * sizeof(unsigned), s));
+    check_launch();
   }
 
   // ---------------------------------------------------------------- stages
@@ -475,17 +485,18 @@ struct zm_solver {
     a.mode = 0;
     pgf(s, a);
     const dim3 c(32, 8);
-    pb(ZM_K_BAROTROPIC, s);
-    ZM_CUDA(launch_pdl(k_bt_forcing, grid2(c), c, 0, s, d, frx, fry, Fx, Fy, eta_in, eta64[0]));
-    pe(s);
     double *ubt_fin, *vbt_fin;
     if (bt_blocks > 0) {
       BtArgs a2 = bt;
+      a2.eta_in = eta_in;
       a2.eta_out = eta_out;
-      coop_launch(s, ZM_K_BAROTROPIC, k_bt_loop, bt_blocks, BT_THREADS, bt_tile_smem(), d, a2);
+      coop_launch(s, ZM_K_BAROTROPIC, bt_loop_kernel(btt.k), bt_blocks, btt.threads, btt.smem, d, a2);
       ubt_fin = bt.ubt_out;
       vbt_fin = bt.vbt_out;
     } else {
+      pb(ZM_K_BAROTROPIC, s);
+      ZM_CUDA(launch_pdl(k_bt_forcing, grid2(c), c, 0, s, d, frx, fry, Fx, Fy, eta_in, eta64[0]));
+      pe(s);
       ZM_CUDA(cudaMemcpyAsync(ubt[0], ubt0, n2 * sizeof(double), cudaMemcpyDeviceToDevice, s));
       ZM_CUDA(cudaMemcpyAsync(vbt[0], vbt0, n2 * sizeof(double), cudaMemcpyDeviceToDevice, s));
       const bool cap = bt.cap_active != 0;
@@ -499,10 +510,10 @@ struct zm_solver {
           const double* fac = f == 0 ? bt.es : bt.er;
           const dim3 g2 = grid2(c);
           pb(ZM_K_BAROTROPIC, s);
-          k_refill_part<<<g2, c, 0, s>>>(d, eta64[a1], fac, bt.area, bt.part_s[0]);
+          k_refill_part<<<g2, c, 0, s>>>(d, eta64[a1], fac, bt.area, bt.part_s);
           pe(s);
           pb(ZM_K_BAROTROPIC, s);
-          k_refill_apply<<<g2, c, 0, s>>>(d, eta64[a1], fac, bt.part_s[0], (int)(g2.x * g2.y), bt.ocean);
+          k_refill_apply<<<g2, c, 0, s>>>(d, eta64[a1], fac, bt.part_s, (int)(g2.x * g2.y), bt.ocean);
           pe(s);
         }
         if (cap) {
@@ -535,7 +546,8 @@ struct zm_solver {
     }
     pb(ZM_K_FINAL, s);
     ZM_CUDA(launch_pdl(k_final, grid3(c), c, 0, s, d, s3.u, s3.v, s3.T, s3.S, ubt_fin, ubt0, vbt_fin, vbt0, held.u,
-                       held.v, held.T, held.S, means, wts, cap_rows > 0 ? cap_nb : 0, out.u, out.v, out.T, out.S));
+                       held.v, held.T, held.S, means, wts, cap_rows > 0 ? cap_nb : 0, out.u, out.v, out.T, out.S,
+                       bt_blocks > 0 ? bt_seq : nullptr, 2 * n_subcyc + 2));
     pe(s);
     check_launch();
   }
@@ -1063,31 +1075,38 @@ void build(zm_solver* s, const zm_grid* g, const zm_params* p) {
     }
     a.count = s->upload(cnt);
     a.wts = s->wts;
-    a.eta0 = s->eta64[0];
     a.ubt0 = s->ubt0;
     a.vbt0 = s->vbt0;
-    a.Fx = s->Fx;
-    a.Fy = s->Fy;
-    const size_t smem = bt_tile_smem();
-    ZM_CUDA(cudaFuncSetAttribute(k_bt_loop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 0, sms = 0, coop = 0;
-    ZM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bt_loop, BT_THREADS, smem));
+    a.frx = s->frx;
+    a.fry = s->fry;
+    int sms = 0, coop = 0, optin = 0;
     ZM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
     ZM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, s->device));
-    a.ntx = (nx + BT_TX - 1) / BT_TX;
-    const int nty = (ny + BT_TY - 1) / BT_TY;
-    const long long tiles = (long long)a.ntx * nty;
+    ZM_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
     require(p->bt_kernel >= ZM_BT_AUTO && p->bt_kernel <= ZM_BT_STREAMING, ZM_ERR_INVALID, "unknown bt_kernel");
-    const bool fits = coop && tiles <= (long long)per_sm * sms;
-    require(fits || p->bt_kernel != ZM_BT_RESIDENT, ZM_ERR_UNSUPPORTED,
+    optin -= 64;  // the barrier's own static words
+    s->btt = bt_tile(nx, ny, sms, (size_t)optin, 128);
+    bool fits = coop && s->btt.blocks > 0;
+    if (fits) {
+      auto kern = bt_loop_kernel(s->btt.k);
+      int per_sm = 0;
+      ZM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+      ZM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, s->btt.threads, s->btt.smem));
+      fits = s->btt.blocks <= per_sm * sms;
+    }
+    // the documented limit of an explicit request: four 32 x 16 tiles per SM
+    const bool named = (long long)((nx + 31) / 32) * ((ny + 15) / 16) <= 4ll * sms;
+    require((fits && named) || p->bt_kernel != ZM_BT_RESIDENT, ZM_ERR_UNSUPPORTED,
             "barotropic tiles do not fit on the GPU at once (bt_kernel = ZM_BT_RESIDENT)");
-    s->bt_blocks = (fits && p->bt_kernel != ZM_BT_STREAMING) ? (int)tiles : 0;
+    s->bt_blocks = (fits && p->bt_kernel != ZM_BT_STREAMING) ? s->btt.blocks : 0;
     if (s->bt_blocks > 0) {
-      for (int q = 0; q < 2; ++q) {
-        a.pub_e[q] = s->alloc<double>(s->n2);
-        a.pub_u[q] = s->alloc<double>(s->n2);
-        a.pub_v[q] = s->alloc<double>(s->n2);
-      }
+      a.tile_x = s->btt.x;
+      a.tile_y = s->btt.y;
+      a.ntx = s->btt.tiles_x;
+      a.pub = s->alloc<double>((size_t)2 * 2 * 3 * s->n2);  // 16-byte words
+      a.sums = s->alloc<double>((size_t)2 * 2 * s->bt_blocks * s->bt_blocks);
+      s->bt_seq = s->alloc<unsigned long long>(1);
+      a.seq = s->bt_seq;
       a.ubt_out = s->alloc<double>(s->n2);
       a.vbt_out = s->alloc<double>(s->n2);
       const size_t np = (size_t)std::max(1, 2 * a.nb) * a.ntx;
@@ -1137,12 +1156,7 @@ void build(zm_solver* s, const zm_grid* g, const zm_params* p) {
       a.relax = relax ? 1 : 0;
       a.es = s->upload(es);
       a.er = s->upload(er);
-      const size_t np = std::max<size_t>((size_t)std::max(s->bt_blocks, 1),
-                                         (size_t)((nx + 31) / 32) * ((ny + 7) / 8));
-      for (int q = 0; q < 2; ++q) {
-        a.part_s[q] = s->alloc<double>(np);
-        a.part_r[q] = s->alloc<double>(np);
-      }
+      a.part_s = s->alloc<double>((size_t)((nx + 31) / 32) * ((ny + 7) / 8));
     }
     if (sponge) {
       require(p->T_clim && p->S_clim, ZM_ERR_INVALID, "the sponge needs T_clim and S_clim");
@@ -1317,7 +1331,7 @@ int zm_info(const zm_solver* s, int32_t* out, int32_t n) {
 int zm_load_state(zm_solver* s, void* stream, const zm_state* in) {
   if (!s || !in || !in->u || !in->v || !in->T || !in->S || !in->eta) return ZM_ERR_INVALID;
   try {
-    ZM_CUDA(cudaMemsetAsync(s->bt_sync, 0, 4 * sizeof(unsigned), (cudaStream_t)stream));
+    s->reset_sync((cudaStream_t)stream);
     s->load((cudaStream_t)stream, in, s->st[s->cur], s->eta[s->cur]);
   } catch (const Err& e) {
     return fail(s, e);

@@ -70,4 +70,44 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned* err, unsig
   return ok != 0;
 }
 
+// ---- exchange words: a value and the sequence number of its exchange in 16
+// bytes that are stored and loaded whole.  A reader polls the word itself, so
+// no fence, atomic or second load stands between a value and its use.  Words
+// alternate between two sets by the parity of the sequence number.
+struct alignas(16) Word {
+  double v;
+  unsigned long long seq;
+};
+
+__device__ __forceinline__ void st_word(Word* p, double v, unsigned long long seq) {
+  asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}\n" ::"l"(p),
+               "l"(__double_as_longlong(v)), "l"(seq)
+               : "memory");
+}
+
+__device__ __forceinline__ Word ld_word(const Word* p) {
+  long long v;
+  unsigned long long q;
+  asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}\n"
+               : "=l"(v), "=l"(q)
+               : "l"(p)
+               : "memory");
+  return Word{__longlong_as_double(v), q};
+}
+
+// Polls a word until it carries seq; bounded, false after the limit or when another block gave up.
+__device__ __forceinline__ bool wait_word(const Word* p, unsigned long long seq, unsigned* err, unsigned max_polls,
+                                          double& v) {
+  Word w = ld_word(p);
+  for (unsigned polls = 0; w.seq != seq; w = ld_word(p))
+    if (++polls > max_polls || ((polls & 255u) == 0u && ld_acquire(err) != 0u)) {
+      atomicOr(err, ZM_BT_ERR_BARRIER);
+      return false;
+    }
+  v = w.v;
+  return true;
+}
+
+constexpr int WORD_CHUNKS = 5;  // sums over at most 32 * WORD_CHUNKS blocks
+
 }  // namespace zm
