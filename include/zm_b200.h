@@ -278,6 +278,16 @@ int zm_diagnostics(zm_solver* s, void* stream, const zm_state* in, const float* 
 int zm_mlp_forward_bf16(void* stream, int32_t ncol, const void* X, const void* W1, const float* b1, const void* W2,
                         const float* b2, const void* W3, const float* b3, float* Y, uint32_t* err);
 
+/* The weights as the inference reads them: one BF16 array of
+ * ZM_MLP_PACKED values (16-byte aligned) from the float32 parameters.  Stream ordered. */
+#define ZM_MLP_PACKED 147456
+int zm_mlp_pack_tc(void* stream, const float* params, void* packed);
+
+/* Inference with packed weights on rows X [ncol][256] (16-byte aligned): BF16
+ * when x_bf16 is set, else float32 that is rounded to BF16 on the way in. */
+int zm_mlp_forward_packed(void* stream, int32_t ncol, const void* X, int32_t x_bf16, const void* packed,
+                          const float* b1, const float* b2, const float* b3, float* Y, uint32_t* err);
+
 /* float32 parameters -> BF16 W1, W2, W3 (device arrays). Stream ordered. */
 int zm_mlp_pack_bf16(void* stream, const float* params, void* W1, void* W2, void* W3);
 

@@ -108,3 +108,31 @@ def test_gradients_at_tile_edges(B, offset):
     for name in omlp.OFF:
         sl = slice(omlp.OFF[name], omlp.OFF[name] + int(np.prod(omlp.SHAPES[name])))
         assert _rel(g[sl], want_g[sl]) < GRAD_TOL, (name, _rel(g[sl], want_g[sl]))
+
+
+@pytest.mark.parametrize("ncol", [1, 31, 127, 128, 129, 37889])
+@pytest.mark.parametrize("kind", ["float32", "bfloat16", "float64", "offset"])
+def test_inference_rows_and_types(ncol, kind):
+    """Ragged row counts (one wave of CTAs and a row) and every way the rows may
+    come: float32 rows are rounded to BF16 in the kernel, others before it, so
+    all give the same bits; against the oracle at the bound above."""
+    import torch
+    from zhenmode_b200.closure import ClosureMLP, init_params
+    p = init_params(seed=3, out_bias=0.5)
+    p[:] += np.random.default_rng(4).standard_normal(p.size).astype(np.float32) * 0.01
+    net = ClosureMLP(p)
+    X = 2.0 * np.random.default_rng(ncol).standard_normal((ncol, 256)).astype(np.float32)
+    X[0, :8] = [60.0, -60.0, 0.0, -0.0, 1e-30, -1e-30, 9.0, -9.0]
+    Xd = torch.as_tensor(X, device="cuda")
+    base = net.forward_bf16(Xd)
+    if kind == "offset":
+        flat = torch.zeros(X.size + 1, device="cuda")
+        flat[1:] = Xd.reshape(-1)
+        got = net.forward_bf16(flat[1:].view(ncol, 256))
+    else:
+        got = net.forward_bf16(Xd.to(getattr(torch, kind)))
+    net.check_error()
+    assert torch.equal(got, base)
+    rows = np.unique(np.concatenate([np.arange(min(ncol, 300)), np.arange(max(0, ncol - 300), ncol)]))
+    want = omlp.forward_bf16(p, X[rows], _bf16)
+    assert _rel(got.cpu().numpy()[rows], want) < INFER_TOL

@@ -87,19 +87,25 @@ class ClosureMLP:
         self.W3 = torch.empty((64, 256), dtype=torch.bfloat16, device=dev)
         _check(self.lib.zm_mlp_pack_bf16(_stream(self.params), _ptr(self.params), _ptr(self.W1), _ptr(self.W2),
                                          _ptr(self.W3)), "zm_mlp_pack_bf16")
+        self.Wp = torch.empty(2 * 256 * 256 + 64 * 256, dtype=torch.bfloat16, device=dev)  # as the inference reads them
+        _check(self.lib.zm_mlp_pack_tc(_stream(self.params), _ptr(self.params), _ptr(self.Wp)), "zm_mlp_pack_tc")
         blocks = unpack(self.params)
         self.b1, self.b2, self.b3 = (blocks[k].contiguous() for k in ("b1", "b2", "b3"))
 
     def forward_bf16(self, X):
         """Tensor-core inference: X [n][256] (any float dtype, CUDA) -> [n][64] float32."""
         import torch
-        Xb = X.to(torch.bfloat16).contiguous()
-        if Xb.dim() != 2 or Xb.shape[1] != N_IN:
+        if X.dim() != 2 or X.shape[1] != N_IN:
             raise ValueError("X must be [n][256]")
-        Y = torch.empty((Xb.shape[0], N_OUT), dtype=torch.float32, device=Xb.device)
-        _check(self.lib.zm_mlp_forward_bf16(_stream(Xb), int(Xb.shape[0]), _ptr(Xb), _ptr(self.W1), _ptr(self.b1),
-                                            _ptr(self.W2), _ptr(self.b2), _ptr(self.W3), _ptr(self.b3), _ptr(Y),
-                                            _ptr(self.err)), "zm_mlp_forward_bf16")
+        if X.dtype != torch.float32 or not X.is_cuda or not X.is_contiguous() or X.data_ptr() % 16:
+            X = X.to(torch.bfloat16).contiguous()
+            if X.data_ptr() % 16:
+                X = X.clone()
+        # float32 rows are rounded to BF16 as the kernel reads them
+        Y = torch.empty((X.shape[0], N_OUT), dtype=torch.float32, device=X.device)
+        _check(self.lib.zm_mlp_forward_packed(_stream(X), int(X.shape[0]), _ptr(X), int(X.dtype == torch.bfloat16),
+                                              _ptr(self.Wp), _ptr(self.b1), _ptr(self.b2), _ptr(self.b3), _ptr(Y),
+                                              _ptr(self.err)), "zm_mlp_forward_packed")
         return Y
 
     def check_error(self):

@@ -119,12 +119,13 @@ __global__ void k_sponge(Dev d, float* u, float* v, float* T, float* S, const fl
                          const float* Sc);
 __global__ void k_cap2d(Dev d, double* f0, double* f1, const float* wts, const double* count, int nb_rows);
 __global__ void k_eta_to_float(Dev d, const double* e64, float* e32);
-// per-column MLP of the learned closure (zm_mlp.cu); BF16 weights [out][in]
-struct MlpBf16 {
-  const __nv_bfloat16 *W1, *W2, *W3;
+// per-column MLP of the learned closure (zm_mlp.cu): packed BF16 weights, float32 biases
+struct MlpTc {
+  const __nv_bfloat16* packed;
   const float *b1, *b2, *b3;
 };
 size_t mlp_tc_smem();
+constexpr int MLP_TC_THREADS = 288;
 // learned closure in the step: features of a column, the plain closure per
 // interface, and the fused tensor-core inference writing kappa per interface
 struct ClosureArgs {
@@ -135,7 +136,7 @@ struct ClosureArgs {
   float bound;                  // largest |feature| the network is trusted with
 };
 __global__ void k_closure_features(Dev d, ClosureArgs a);
-__global__ void k_mlp_closure(MlpBf16 w, Dev d, ClosureArgs a, unsigned* err);
+__global__ void k_mlp_closure(MlpTc w, Dev d, ClosureArgs a, unsigned* err);
 __global__ void k_kappa_rows(Dev d, const float* kap3, float* out);
 // diagnostics outside the step (zm_diagnostics.cu)
 #define ZM_BUDGET_SUMS 7

@@ -5,17 +5,25 @@
 // with W[out][in] (the input index contiguous).
 //
 // Inference (k_mlp_tc): BF16 operands on the 5th-generation tensor cores with
-// float32 accumulation in tensor memory.  A CTA of 128 threads owns 128
-// columns: thread t owns column t, which is row t of the A operand and lane t
-// of the accumulator.  The activations stay in shared memory as BF16 in the
-// canonical K-major layout without swizzle (8-row x 16-byte core matrices;
-// the two core matrices of one K=16 step are LBO = 128 B apart, 8-row groups
-// SBO = 16 * K bytes apart).  Weights stream through shared memory in K
-// chunks of 64; one thread issues the four tcgen05.mma of a chunk and commits
-// them to an mbarrier that every thread waits on with a poll limit.  The
-// epilogue of a layer reads the accumulator row with tcgen05.ld, adds the
-// bias, applies GELU and writes BF16 back into the activation tile, which is
-// the next layer's A operand.
+// float32 accumulation in tensor memory.  A CTA owns 128 columns: column t is
+// row t of the A operand and lane t of the accumulator.  The activations stay
+// in shared memory as BF16 in the canonical K-major layout without swizzle
+// (8-row x 16-byte core matrices; the two core matrices of one K=16 step are
+// LBO = 128 B apart, 8-row groups SBO = 16 * K bytes apart).  The weights are
+// packed once in that layout, in K chunks of 32 (zm_mlp_pack_tc), so that one
+// bulk copy brings a chunk; three buffers, filled two chunks ahead.
+//  * A control thread waits for a chunk, issues its two tcgen05.mma, commits
+//    them to the buffer's mbarrier and refills the buffer before last; the
+//    last commit of a layer goes to the epilogue's mbarrier.
+//  * Eight warps run the epilogue of a layer: the accumulator by tcgen05.ld
+//    (warp w the rows 32 (w mod 4) .., the columns of half w / 4), bias, GELU,
+//    BF16 back into the activation tile, which is the next layer's A operand.
+// Every wait has a poll limit; one that runs out sets the error word, and the
+// CTA waits (again bounded) for its copies and products before it frees TMEM.
+//
+// The products of a tile take 2.4 us of an SM's tensor core, GELU on 65536
+// values 4.3 us of its FMA pipes: that is the bound, so two CTAs share an SM and
+// one's products and loads run under the other's epilogue.  MEASURED_INFER
 //
 // Training: float32 SIMT kernels (tiled GEMM with optional transposes, GELU
 // and its derivative, masked mean-square loss, bias gradients, Adam), driven
@@ -36,10 +44,14 @@ namespace {
 constexpr int MT = 128;                          // columns per CTA
 constexpr int MK = ZM_MLP_IN;                    // 256: input and hidden width
 constexpr int MO = ZM_MLP_OUT;                   // 64: padded output width
-constexpr int KC = 64;                           // K chunk of a weight stage
+constexpr int MEPI = 256;                        // epilogue threads per CTA
+static_assert(MLP_TC_THREADS == MEPI + 32, "one more warp for the control thread");
+constexpr int KC = 32;                           // K chunk of a weight stage
+constexpr int WSTAGES = 3;                       // weight buffers
+constexpr int KCHUNKS = MK / KC;                 // chunks per layer
 constexpr uint32_t ACT_BYTES = MT * MK * 2;      // 64 KiB
-constexpr uint32_t WB_BYTES = MK * KC * 2;       // 32 KiB
-constexpr uint32_t TC_SMEM = ACT_BYTES + WB_BYTES + 64;
+constexpr uint32_t WB_BYTES = MK * KC * 2;       // 16 KiB
+constexpr uint32_t TC_SMEM = ACT_BYTES + WSTAGES * WB_BYTES + 128 + MT * 4;  // two CTAs per SM
 constexpr unsigned WAIT_POLLS = 1u << 22;
 
 __device__ __forceinline__ uint32_t su32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -84,22 +96,34 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
         : "r"(bar), "r"(parity)
         : "memory");
     if (ok) return true;
-    __nanosleep(20);
   }
   return false;
 }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
-  uint32_t r[16];
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
+  uint32_t r[32];
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-  for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+  for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+}
+
+// bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned) that completes on an mbarrier
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -107,6 +131,35 @@ __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::aft
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.f + erff(x * 0.70710678118654752f)); }
+// GELU of two values for the BF16 inference: x Phi(x) with Phi = 0.5 + 0.5 erf
+// and erf(t) = t P(t^2) / Q(t^2), a rational minimax fit of degrees 5 and 5 on
+// |t| <= 4 (weighted linearised least squares, own fit: 2.1e-8 off in exact
+// arithmetic, the value 1.1e-6 in float32, where BF16 rounds to 2^-9 of it);
+// beyond, P / Q stays at its end value and the saturation gives 0 or 1.  On
+// paired instructions this is 13 issue slots a value, erff about 30.
+__device__ __forceinline__ float2 gelu2(float2 x) {
+  auto c = [](float a) { return make_float2(a, a); };
+  auto rcp = [](float a) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+  };
+  const float2 t = __fmul2_rn(x, c(0.70710678118654752f));
+  float2 s = __fmul2_rn(t, t);
+  s = make_float2(fminf(s.x, 16.f), fminf(s.y, 16.f));
+  float2 p = __ffma2_rn(s, c(1.974827910089516e-06f), c(0.00028804215253330767f));
+  p = __ffma2_rn(s, p, c(0.00400366960093379f));
+  p = __ffma2_rn(s, p, c(0.05346754938364029f));
+  p = __ffma2_rn(s, p, c(0.19624949991703033f));
+  p = __ffma2_rn(s, p, c(1.128378987312317f));
+  float2 q = __ffma2_rn(s, c(3.748088056454435e-05f), c(0.0012163660721853375f));
+  q = __ffma2_rn(s, q, c(0.015444467775523663f));
+  q = __ffma2_rn(s, q, c(0.1164766475558281f));
+  q = __ffma2_rn(s, q, c(0.5072527527809143f));
+  q = __ffma2_rn(s, q, c(1.f));
+  p = __fmul2_rn(p, __fmul2_rn(t, c(0.5f)));
+  return make_float2(x.x * __saturatef(fmaf(p.x, rcp(q.x), 0.5f)), x.y * __saturatef(fmaf(p.y, rcp(q.y), 0.5f)));
+}
 __device__ __forceinline__ float gelu_grad(float x) {
   return 0.5f * (1.f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
 }
@@ -115,94 +168,142 @@ __device__ __forceinline__ float gelu_grad(float x) {
 
 size_t mlp_tc_smem() { return TC_SMEM; }
 
-// One MLP pass over BF16 rows that `stage(t, act)` writes as row t of the
-// activation tile (core_off layout), writing the 64 raw outputs of each row
-// through `emit`.  Shared by the standalone and the fused kernels.
+// Packed weights: the chunks of W1, W2, W3 in turn, KCHUNKS each, [out][32] in
+// the canonical layout.
+constexpr int PACK_ELEMS = (2 * MK + MO) * MK;
+__device__ __forceinline__ size_t pack_chunk(int i) {  // first element of chunk i
+  return i < 2 * KCHUNKS ? (size_t)i * (MK * KC) : (size_t)2 * MK * MK + (size_t)(i - 2 * KCHUNKS) * (MO * KC);
+}
+
+// One MLP pass over the 128 BF16 rows that `stage(act, scratch)` writes into the
+// activation tile (core_off layout; called by the MEPI epilogue threads,
+// scratch holds 128 words), writing the raw outputs of each row through
+// `emit(row, c0, v)`, 32 at a time.  Shared by the standalone and the fused kernels.
 template <class Stage, class Emit>
-__device__ __forceinline__ void mlp_tc_body(const MlpBf16& w, uint8_t* msm, unsigned* err, Stage stage, Emit emit) {
+__device__ __forceinline__ void mlp_tc_body(const MlpTc& w, uint8_t* msm, unsigned* err, Stage stage, Emit emit) {
   uint8_t* act = msm;
   uint8_t* wb = msm + ACT_BYTES;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(msm + ACT_BYTES + WB_BYTES);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(msm + ACT_BYTES + WB_BYTES + 8);
-  int* abort_flag = reinterpret_cast<int*>(msm + ACT_BYTES + WB_BYTES + 16);
+  uint64_t* full = reinterpret_cast<uint64_t*>(msm + ACT_BYTES + WSTAGES * WB_BYTES);  // a chunk has landed
+  uint64_t* empty = full + WSTAGES;   // a chunk's products are done
+  uint64_t* ready = empty + WSTAGES;  // the activation tile is written
+  uint64_t* done = ready + 1;         // a layer's products are done
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
+  uint32_t* scratch = reinterpret_cast<uint32_t*>(msm + ACT_BYTES + WSTAGES * WB_BYTES + 128);
   const int t = threadIdx.x, warp = t >> 5;
-  if (t == 0) {
-    *abort_flag = 0;
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(su32(bar)) : "memory");
+  constexpr int CHUNKS = 3 * KCHUNKS;
+  if (t == MEPI) {
+    for (int b = 0; b < WSTAGES; ++b) {
+      mbar_init(su32(full + b), 1);
+      mbar_init(su32(empty + b), 1);
+    }
+    mbar_init(su32(ready), MEPI);
+    mbar_init(su32(done), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(tslot)), "r"(256u)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  // the inputs of this thread's column as row t of the A tile
-  stage(t, act);
-  fence_async_smem();
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tmem = *tslot;
-  const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
-  uint32_t phase = 0;
-  bool failed = false;
-  for (int layer = 0; layer < 3 && !failed; ++layer) {
-    const __nv_bfloat16* W = layer == 0 ? w.W1 : (layer == 1 ? w.W2 : w.W3);
-    const float* bias = layer == 0 ? w.b1 : (layer == 1 ? w.b2 : w.b3);
-    const int N = layer < 2 ? MK : MO;
-    const uint32_t id = layer < 2 ? idesc_bf16(MT, MK) : idesc_bf16(MT, MO);
-    for (int kc = 0; kc < MK / KC; ++kc) {
-      for (int p = t; p < N * (KC / 8); p += MT) {
-        const int n = p / (KC / 8), kp = p - n * (KC / 8);
-        const uint4 v = *reinterpret_cast<const uint4*>(W + (size_t)n * MK + kc * KC + kp * 8);
-        *reinterpret_cast<uint4*>(wb + core_off(n, kp * 8, KC)) = v;
-      }
-      fence_async_smem();
-      __syncthreads();
-      if (t == 0) {
+  bool ok = true;
+  if (warp == MEPI / 32) {
+    if (t == MEPI) {  // control thread
+      int loaded = 0, issued = 0;  // chunks whose copy, whose products were started
+      auto load = [&]() {
+        const uint32_t bytes = (uint32_t)(loaded < 2 * KCHUNKS ? MK : MO) * KC * 2u;
+        bulk_load(su32(wb) + (uint32_t)(loaded % WSTAGES) * WB_BYTES, w.packed + pack_chunk(loaded), bytes,
+                  su32(full + loaded % WSTAGES));
+        ++loaded;
+      };
+      for (int b = 0; b < WSTAGES; ++b) load();
+      for (int i = 0; i < CHUNKS && ok; ++i) {
+        const int layer = i / KCHUNKS, kc = i - layer * KCHUNKS, buf = i % WSTAGES;
+        if (kc == 0) ok = mbar_wait(su32(ready), (uint32_t)layer & 1u, WAIT_POLLS);
+        ok = ok && mbar_wait(su32(full + buf), (uint32_t)(i / WSTAGES) & 1u, WAIT_POLLS);
+        if (!ok) break;
         fence_after();
+        const uint32_t id = layer < 2 ? idesc_bf16(MT, MK) : idesc_bf16(MT, MO);
+        const uint32_t wsrc = su32(wb) + (uint32_t)buf * WB_BYTES;
 #pragma unroll
         for (int s = 0; s < KC / 16; ++s) {
           const uint64_t da = sdesc(su32(act) + (uint32_t)((kc * KC + s * 16) / 8) * 128u, 128u, (uint32_t)MK * 16u);
-          const uint64_t db = sdesc(su32(wb) + (uint32_t)s * 256u, 128u, (uint32_t)KC * 16u);
+          const uint64_t db = sdesc(wsrc + (uint32_t)s * 256u, 128u, (uint32_t)KC * 16u);
           umma_bf16(tmem, da, db, id, (kc | s) != 0 ? 1u : 0u);
         }
-        umma_commit(su32(bar));
+        umma_commit(su32(empty + buf));
+        if (kc + 1 == KCHUNKS) umma_commit(su32(done));
+        ++issued;
+        // the buffer of the chunk before this one is free once its products are done
+        if (i > 0 && loaded < CHUNKS) {
+          ok = mbar_wait(su32(empty + (i - 1) % WSTAGES), (uint32_t)((i - 1) / WSTAGES) & 1u, WAIT_POLLS);
+          if (ok) load();
+        }
       }
-      // the chunk's products are done before the weight buffer is refilled
-      if (!mbar_wait(su32(bar), phase, WAIT_POLLS)) atomicOr(abort_flag, 1);
-      __syncthreads();
-      if (*abort_flag) {  // phase still names the outstanding commit
-        failed = true;
+      // every copy and product that was started ends before the memory goes
+      for (int i = issued; i < loaded; ++i)
+        ok = mbar_wait(su32(full + i % WSTAGES), (uint32_t)(i / WSTAGES) & 1u, WAIT_POLLS) && ok;
+      if (issued > 0)
+        ok = mbar_wait(su32(empty + (issued - 1) % WSTAGES), (uint32_t)((issued - 1) / WSTAGES) & 1u, WAIT_POLLS) && ok;
+      ok = ok && issued == CHUNKS;
+    }
+    __syncwarp();
+  } else {
+    stage(act, scratch);
+    fence_async_smem();
+    mbar_arrive(su32(ready));
+    const int quarter = warp & 3, half = warp >> 2, row = quarter * 32 + (t & 31);
+    const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+    for (int layer = 0; layer < 3; ++layer) {
+      const int N = layer < 2 ? MK : MO;
+      if (!mbar_wait(su32(done), (uint32_t)layer & 1u, WAIT_POLLS)) ok = false;
+      if (!__all_sync(0xffffffffu, ok)) {  // tcgen05.ld is a warp's
+        ok = false;
         break;
       }
-      phase ^= 1u;
-    }
-    if (failed) break;
-    fence_after();
-    for (int c0 = 0; c0 < N; c0 += 16) {
-      float v[16];
-      tmem_ld16(tmem + lane_base + (uint32_t)c0, v);
-      if (layer < 2) {
-        __align__(16) __nv_bfloat16 h[16];
+      fence_after();
+      const float* bias = layer == 0 ? w.b1 : (layer == 1 ? w.b2 : w.b3);
+      const bool vb = ((uintptr_t)bias & 15u) == 0;
+      for (int c0 = half * (N / 2); c0 < (half + 1) * (N / 2); c0 += 32) {
+        float v[32];
+        tmem_ld32(tmem + lane_base + (uint32_t)c0, v);
+        auto bias4 = [&](int e) {
+          const float* b = bias + c0 + e;
+          return vb ? __ldg(reinterpret_cast<const float4*>(b))
+                    : make_float4(__ldg(b), __ldg(b + 1), __ldg(b + 2), __ldg(b + 3));
+        };
+        if (layer < 2) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) h[j] = __float2bfloat16(gelu(v[j] + __ldg(bias + c0 + j)));
-        *reinterpret_cast<uint4*>(act + core_off(t, c0, MK)) = *reinterpret_cast<const uint4*>(h);
-        *reinterpret_cast<uint4*>(act + core_off(t, c0 + 8, MK)) = *reinterpret_cast<const uint4*>(h + 8);
-      } else {
+          for (int e = 0; e < 32; e += 8) {
+            const float4 ba = bias4(e), bb = bias4(e + 4);
+            __align__(16) __nv_bfloat162 h[4];
+            h[0] = __float22bfloat162_rn(gelu2(__fadd2_rn(make_float2(v[e], v[e + 1]), make_float2(ba.x, ba.y))));
+            h[1] = __float22bfloat162_rn(gelu2(__fadd2_rn(make_float2(v[e + 2], v[e + 3]), make_float2(ba.z, ba.w))));
+            h[2] = __float22bfloat162_rn(gelu2(__fadd2_rn(make_float2(v[e + 4], v[e + 5]), make_float2(bb.x, bb.y))));
+            h[3] = __float22bfloat162_rn(gelu2(__fadd2_rn(make_float2(v[e + 6], v[e + 7]), make_float2(bb.z, bb.w))));
+            *reinterpret_cast<uint4*>(act + core_off(row, c0 + e, MK)) = *reinterpret_cast<const uint4*>(h);
+          }
+        } else {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] += __ldg(bias + c0 + j);
-        emit(t, c0, v);
+          for (int e = 0; e < 32; e += 4) {
+            const float4 ba = bias4(e);
+            v[e] += ba.x;
+            v[e + 1] += ba.y;
+            v[e + 2] += ba.z;
+            v[e + 3] += ba.w;
+          }
+          emit(row, c0, v);
+        }
       }
+      fence_before();
+      fence_async_smem();
+      if (layer < 2) mbar_arrive(su32(ready));
     }
-    fence_before();
-    fence_async_smem();
-    __syncthreads();
   }
-  if (failed) {
-    // let the outstanding products finish (bounded) before the memory goes
-    mbar_wait(su32(bar), phase, WAIT_POLLS);
-    if (t == 0) atomicOr(err, 1u);
-  }
+  if (!ok) atomicOr(err, 1u);
   fence_before();
   __syncthreads();
   if (warp == 0) {
@@ -211,23 +312,57 @@ __device__ __forceinline__ void mlp_tc_body(const MlpBf16& w, uint8_t* msm, unsi
   }
 }
 
-// Standalone inference on BF16 feature rows X [ncol][256] -> Y [ncol][64].
-__global__ void __launch_bounds__(MT, 1) k_mlp_tc(MlpBf16 w, const __nv_bfloat16* __restrict__ X,
-                                                  float* __restrict__ Y, int ncol, unsigned* err) {
+// Standalone inference on feature rows X [ncol][256] (BF16, or float32 that is
+// rounded to BF16 on the way in) -> Y [ncol][64].
+template <class In>
+__global__ void __launch_bounds__(MLP_TC_THREADS, 2) k_mlp_tc(MlpTc w, const In* __restrict__ X, float* __restrict__ Y,
+                                                        int ncol, unsigned* err) {
   extern __shared__ __align__(1024) uint8_t msm[];
-  const long long col = (long long)blockIdx.x * MT + threadIdx.x;
+  const long long col0 = (long long)blockIdx.x * MT;
   mlp_tc_body(
       w, msm, err,
-      [&](int t, uint8_t* act) {
-        for (int kp = 0; kp < MK / 8; ++kp) {
-          uint4 v = make_uint4(0u, 0u, 0u, 0u);
-          if (col < ncol) v = *reinterpret_cast<const uint4*>(X + col * MK + kp * 8);
-          *reinterpret_cast<uint4*>(act + core_off(t, kp * 8, MK)) = v;
+      [&](uint8_t* act, uint32_t*) {
+        // a warp takes 8 rows x 4 groups of 8 features at a time: rows in full
+        // 128-byte (64-byte) pieces, shared stores without bank conflicts
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll 1
+        for (int oct = 0; oct < MT / 8 / (MEPI / 32); ++oct) {
+          const int r = (oct * (MEPI / 32) + warp) * 8 + (lane & 7);
+          const long long col = col0 + r;
+          uint4 v[MK / 32];
+#pragma unroll
+          for (int g = 0; g < MK / 32; ++g) {
+            const int k = g * 32 + (lane >> 3) * 8;
+            v[g] = make_uint4(0u, 0u, 0u, 0u);
+            if (col >= ncol) continue;
+            if constexpr (sizeof(In) == 2) {
+              v[g] = __ldg(reinterpret_cast<const uint4*>(X + col * MK + k));
+            } else {
+              const float4 a = __ldg(reinterpret_cast<const float4*>(X + col * MK + k));
+              const float4 b = __ldg(reinterpret_cast<const float4*>(X + col * MK + k) + 1);
+              __align__(16) const __nv_bfloat162 h[4] = {
+                  __float22bfloat162_rn(make_float2(a.x, a.y)), __float22bfloat162_rn(make_float2(a.z, a.w)),
+                  __float22bfloat162_rn(make_float2(b.x, b.y)), __float22bfloat162_rn(make_float2(b.z, b.w))};
+              v[g] = *reinterpret_cast<const uint4*>(h);
+            }
+          }
+#pragma unroll
+          for (int g = 0; g < MK / 32; ++g)
+            *reinterpret_cast<uint4*>(act + core_off(r, g * 32 + (lane >> 3) * 8, MK)) = v[g];
         }
       },
-      [&](int, int c0, const float* v) {
-        if (col < ncol)
-          for (int j = 0; j < 16; ++j) Y[col * MO + c0 + j] = v[j];
+      [&](int row, int c0, const float* v) {
+        const long long col = col0 + row;
+        if (col >= ncol) return;
+        float* y = Y + col * MO + c0;
+        if (((uintptr_t)Y & 15u) == 0) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 4)
+            *reinterpret_cast<float4*>(y + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) y[j] = v[j];
+        }
       });
 }
 
@@ -313,72 +448,92 @@ __global__ void __launch_bounds__(128) k_closure_features(Dev d, ClosureArgs a) 
 // the tensor-core MLP; kappa = 10^y at the wet interfaces, clipped to
 // [1e-7, 1] m^2/s, or the plain closure for a column whose features exceed
 // the trusted bound (or are not finite).
-__global__ void __launch_bounds__(MT, 1) k_mlp_closure(MlpBf16 w, Dev d, ClosureArgs a, unsigned* err) {
+__global__ void __launch_bounds__(MLP_TC_THREADS, 2) k_mlp_closure(MlpTc w, Dev d, ClosureArgs a, unsigned* err) {
   extern __shared__ __align__(1024) uint8_t msm[];
   const long long ncol = (long long)d.nx * d.ny;
-  const long long col = (long long)blockIdx.x * MT + threadIdx.x;
-  const bool act = col < ncol;
-  const int j = act ? (int)(col / d.nx) : 0, i = act ? (int)(col - (long long)j * d.nx) : 0;
-  const long long base = idx2(d, j, i);
-  const uint64_t bits = act ? __ldg(d.wbits + base) : 0ull;
-  bool trusted = true;
-  int unstable = -1;  // column gate of the plain closure, formed on first use
+  // threads 0..127 take T, S and N^2 of column t, threads 128..255 u, v and the forcing of column t - 128
+  const int c = threadIdx.x & (MT - 1), part = threadIdx.x / MT;
+  auto place = [&](int r, long long& base, uint64_t& bits) {
+    const long long col = (long long)blockIdx.x * MT + r;
+    if (col >= ncol) {
+      base = 0;
+      bits = 0ull;
+      return false;
+    }
+    const int j = (int)(col / d.nx), i = (int)(col - (long long)j * d.nx);
+    base = idx2(d, j, i);
+    bits = __ldg(d.wbits + base);
+    return true;
+  };
+  const uint32_t* largest = reinterpret_cast<const uint32_t*>(msm + ACT_BYTES + WSTAGES * WB_BYTES + 128);
   mlp_tc_body(
       w, msm, err,
-      [&](int t, uint8_t* tile) {
-        // the row is zero, then the features level by level: four loads per
-        // level, coalesced over the CTA's consecutive columns; N^2 from the
-        // level above kept in registers
-        for (int kp = 0; kp < MK / 8; ++kp)
-          *reinterpret_cast<uint4*>(tile + core_off(t, kp * 8, MK)) = make_uint4(0u, 0u, 0u, 0u);
-        float amax = 0.f;
-        auto put = [&](int q, float f) {
-          amax = fmaxf(amax, fabsf(f));
-          if (!(f == f) || isinf(f)) amax = INFINITY;
-          *reinterpret_cast<__nv_bfloat16*>(tile + core_off(t, q, MK)) = __float2bfloat16(f);
-        };
-        if (act) {
+      [&](uint8_t* tile, uint32_t* amax_bits) {
+        // the rows are zero, then the features level by level: loads coalesced
+        // over the CTA's consecutive columns; N^2 from the level above kept in registers
+        for (int kp = part * (MK / 16); kp < (part + 1) * (MK / 16); ++kp)
+          *reinterpret_cast<uint4*>(tile + core_off(c, kp * 8, MK)) = make_uint4(0u, 0u, 0u, 0u);
+        if (part == 0) amax_bits[c] = 0u;
+        asm volatile("bar.sync 1, %0;" ::"n"(MEPI) : "memory");
+        long long base;
+        uint64_t bits;
+        if (place(c, base, bits)) {
+          float amax = 0.f;
+          auto put = [&](int q, float f) {
+            amax = fmaxf(amax, fabsf(f));
+            if (!(f == f) || isinf(f)) amax = INFINITY;
+            *reinterpret_cast<__nv_bfloat16*>(tile + core_off(c, q, MK)) = __float2bfloat16(f);
+          };
+          const int nk = levels_of(bits);
+          const float *pa = part ? a.u : a.T, *pb = part ? a.v : a.S;
           float Tu = 0.f, Su = 0.f;
           bool wu = false;
-#pragma unroll 4
-          for (int k = 0; k < d.nz; ++k) {
+#pragma unroll 5
+          for (int k = 0; k < nk; ++k) {
             const long long id = base + (long long)k * d.plane;
-            const float Tk = ld(a.T, id), Sk = ld(a.S, id), uk = ld(a.u, id), vk = ld(a.v, id);
+            const float fa = ld(pa, id), fb = ld(pb, id);
             const bool wk = wetb(bits, k);
             if (wk) {
-              put(k, Tk * 0.1f);
-              put(50 + k, Sk);
-              put(100 + k, uk * 2.f);
-              put(150 + k, vk * 2.f);
-              if (k > 0 && wu)
-                put(199 + k, asinhf(kG * (-kAlpha * (Tk - Tu) + kBeta * (Sk - Su)) * d.vc.inv_dz_iface[k - 1] * 1e8f) *
+              put(100 * part + k, fa * (part ? 2.f : 0.1f));
+              put(100 * part + 50 + k, part ? fb * 2.f : fb);
+              if (part == 0 && k > 0 && wu)
+                put(199 + k, asinhf(kG * (-kAlpha * (fa - Tu) + kBeta * (fb - Su)) * d.vc.inv_dz_iface[k - 1] * 1e8f) *
                                  0.25f);
             }
-            Tu = Tk;
-            Su = Sk;
+            Tu = fa;
+            Su = fb;
             wu = wk;
           }
-          const float tx = __ldg(d.tau_x + base), ty = __ldg(d.tau_y + base);
-          put(250, sqrtf(tx * tx + ty * ty) * 10.f);
-          put(251, __ldg(d.qheat + base) * 0.01f);
-        }
-        trusted = amax <= a.bound;
-      },
-      [&](int, int c0, const float* y) {
-        if (!act) return;
-        if (!trusted && unstable < 0) {
-          unstable = column_unstable(d, a, base, bits) ? 1 : 0;
-          atomicAdd(a.fallback, 1u);
-        }
-        for (int e = 0; e < 16; ++e) {
-          const int m = c0 + e;
-          if (m + 1 >= d.nz) break;
-          float k = 0.f;
-          if (wetb(bits, m) && wetb(bits, m + 1)) {
-            if (trusted) k = fminf(fmaxf(exp10f(y[e]), 1e-7f), 1.f);
-            else k = plain_kappa(d, a, base, bits, m, unstable == 1);
+          if (part) {
+            const float tx = __ldg(d.tau_x + base), ty = __ldg(d.tau_y + base);
+            put(250, sqrtf(tx * tx + ty * ty) * 10.f);
+            put(251, __ldg(d.qheat + base) * 0.01f);
           }
-          a.kappa3[(long long)m * d.plane + base] = k;
+          atomicMax(amax_bits + c, __float_as_uint(amax));  // non-negative: ordered like the bits
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(MEPI) : "memory");
+      },
+      [&](int row, int c0, const float* y) {
+        long long base;
+        uint64_t bits;
+        if (!place(row, base, bits)) return;
+        const bool trusted = __uint_as_float(largest[row]) <= a.bound;
+        bool unstable = false;  // column gate of the plain closure
+        if (!trusted) {
+          unstable = column_unstable(d, a, base, bits);
+          if (c0 == 0) atomicAdd(a.fallback, 1u);
+        }
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+          const int m = c0 + e;
+          if (m + 1 < d.nz) {
+            float k = 0.f;
+            if (wetb(bits, m) && wetb(bits, m + 1)) {
+              if (trusted) k = fminf(fmaxf(exp10f(y[e]), 1e-7f), 1.f);
+              else k = plain_kappa(d, a, base, bits, m, unstable);
+            }
+            a.kappa3[(long long)m * d.plane + base] = k;
+          }
         }
       });
 }
@@ -401,6 +556,18 @@ __global__ void k_mlp_pack(const float* __restrict__ params, __nv_bfloat16* __re
     W1[i] = __float2bfloat16(params[i]);
     W2[i] = __float2bfloat16(params[n1 + MK + i]);
     if (i < n3) W3[i] = __float2bfloat16(params[2 * (n1 + MK) + i]);
+  }
+}
+
+// float32 parameters, or BF16 weights [out][in], -> packed BF16 weights
+template <class In>
+__global__ void k_mlp_pack_tc(const In* __restrict__ W1, const In* __restrict__ W2, const In* __restrict__ W3,
+                              __nv_bfloat16* __restrict__ out) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < PACK_ELEMS; i += gridDim.x * blockDim.x) {
+    const int layer = i < MK * MK ? 0 : (i < 2 * MK * MK ? 1 : 2), e = i - layer * MK * MK;
+    const int n = e / MK, k = e - n * MK;
+    const In* W = layer == 0 ? W1 : (layer == 1 ? W2 : W3);
+    out[pack_chunk(layer * KCHUNKS + k / KC) + core_off(n, k % KC, KC) / 2] = __float2bfloat16((float)W[e]);
   }
 }
 
@@ -704,6 +871,14 @@ bool launch_ok(const char* what) {
 
 bool vec16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
+template <class In>
+int forward_tc(cudaStream_t st, int ncol, const In* X, const MlpTc& w, float* Y, uint32_t* err) {
+  if (cudaFuncSetAttribute(k_mlp_tc<In>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM) != cudaSuccess)
+    return ZM_ERR_CUDA;
+  k_mlp_tc<In><<<(ncol + MT - 1) / MT, MLP_TC_THREADS, TC_SMEM, st>>>(w, X, Y, ncol, err);
+  return launch_ok("mlp forward") ? ZM_OK : ZM_ERR_CUDA;
+}
+
 // splits of the weight gradients' batch sums: with 14 the 10 tiles fill the 148 SMs once
 constexpr int GRAD_SPLITS = 14;
 
@@ -724,11 +899,31 @@ extern "C" int zm_mlp_forward_bf16(void* stream, int32_t ncol, const void* X, co
   if (ncol < 0 || !X || !W1 || !b1 || !W2 || !b2 || !W3 || !b3 || !Y || !err) return ZM_ERR_INVALID;
   if (ncol == 0) return ZM_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  if (cudaFuncSetAttribute(k_mlp_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM) != cudaSuccess)
-    return ZM_ERR_CUDA;
-  MlpBf16 w{(const __nv_bfloat16*)W1, (const __nv_bfloat16*)W2, (const __nv_bfloat16*)W3, b1, b2, b3};
-  k_mlp_tc<<<(ncol + MT - 1) / MT, MT, TC_SMEM, st>>>(w, (const __nv_bfloat16*)X, Y, ncol, err);
-  return launch_ok("zm_mlp_forward_bf16") ? ZM_OK : ZM_ERR_CUDA;
+  // the weights in the layout of the bulk copies, in memory of this call's own
+  __nv_bfloat16* packed = nullptr;
+  if (cudaMallocAsync(&packed, PACK_ELEMS * sizeof(__nv_bfloat16), st) != cudaSuccess) return ZM_ERR_CUDA;
+  k_mlp_pack_tc<<<288, 256, 0, st>>>((const __nv_bfloat16*)W1, (const __nv_bfloat16*)W2, (const __nv_bfloat16*)W3,
+                                     packed);
+  const int rc = forward_tc(st, ncol, (const __nv_bfloat16*)X, MlpTc{packed, b1, b2, b3}, Y, err);
+  cudaFreeAsync(packed, st);
+  return rc;
+}
+
+extern "C" int zm_mlp_forward_packed(void* stream, int32_t ncol, const void* X, int32_t x_bf16, const void* packed,
+                                     const float* b1, const float* b2, const float* b3, float* Y, uint32_t* err) {
+  if (ncol < 0 || !X || !packed || !b1 || !b2 || !b3 || !Y || !err || !vec16(X) || !vec16(packed))
+    return ZM_ERR_INVALID;
+  if (ncol == 0) return ZM_OK;
+  const MlpTc w{(const __nv_bfloat16*)packed, b1, b2, b3};
+  if (x_bf16) return forward_tc((cudaStream_t)stream, ncol, (const __nv_bfloat16*)X, w, Y, err);
+  return forward_tc((cudaStream_t)stream, ncol, (const float*)X, w, Y, err);
+}
+
+extern "C" int zm_mlp_pack_tc(void* stream, const float* params, void* packed) {
+  if (!params || !packed) return ZM_ERR_INVALID;
+  k_mlp_pack_tc<<<288, 256, 0, (cudaStream_t)stream>>>(params + Off::W1, params + Off::W2, params + Off::W3,
+                                                       (__nv_bfloat16*)packed);
+  return launch_ok("zm_mlp_pack_tc") ? ZM_OK : ZM_ERR_CUDA;
 }
 
 extern "C" int zm_mlp_pack_bf16(void* stream, const float* params, void* W1, void* W2, void* W3) {

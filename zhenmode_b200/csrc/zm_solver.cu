@@ -79,7 +79,7 @@ struct zm_solver {
   bool want_tune = false;
   bool tuned = false;
   bool closure_on = false;
-  MlpBf16 cw{};
+  MlpTc cw{};
   float* kappa3 = nullptr;       // [nz-1][ny][P] diffusivity per interface
   unsigned* cl_count = nullptr;  // [0] fallback columns of the last step, [1] tensor-core wait errors
   float cl_bound = 8.f;
@@ -145,14 +145,30 @@ struct zm_solver {
     if (profiling) ZM_CUDA(cudaEventRecord(prof.back().b, s));
   }
 
+  // Zeroed device memory.  Small arrays come from shared pieces of 16 MB: a
+  // handle holds some eighty arrays, and one cudaMalloc and cudaMemset each
+  // were most of the time to create one for a small grid.
+  char* piece = nullptr;
+  size_t piece_left = 0;
   template <class T>
   T* alloc(size_t count) {
-    void* p = nullptr;
-    ZM_CUDA(cudaMalloc(&p, count * sizeof(T)));
-    ZM_CUDA(cudaMemset(p, 0, count * sizeof(T)));
-    allocs.push_back(p);
-    bytes += count * sizeof(T);
-    return static_cast<T*>(p);
+    constexpr size_t PIECE = 16u << 20;
+    const size_t need = (std::max<size_t>(count, 1) * sizeof(T) + 255) / 256 * 256;
+    if (need > piece_left) {
+      void* p = nullptr;
+      const size_t take = std::max(need, PIECE);
+      ZM_CUDA(cudaMalloc(&p, take));
+      allocs.push_back(p);
+      ZM_CUDA(cudaMemset(p, 0, take));
+      bytes += take;
+      if (take - need <= piece_left) return static_cast<T*>(p);  // the current piece has more left
+      piece = static_cast<char*>(p);
+      piece_left = take;
+    }
+    T* out = reinterpret_cast<T*>(piece);
+    piece += need;
+    piece_left -= need;
+    return out;
   }
   float* f3() { return alloc<float>(n3); }
   float* f2() { return alloc<float>(n2); }
@@ -559,7 +575,7 @@ struct zm_solver {
     a.T = in.T; a.S = in.S; a.u = in.u; a.v = in.v; a.kappa3 = kappa3; a.fallback = cl_count; a.bound = cl_bound;
     const long long ncol = (long long)nx * ny;
     pb(ZM_K_CLOSURE, s);
-    k_mlp_closure<<<(unsigned)((ncol + 127) / 128), 128, mlp_tc_smem(), s>>>(cw, d, a, cl_count + 1);
+    k_mlp_closure<<<(unsigned)((ncol + 127) / 128), MLP_TC_THREADS, mlp_tc_smem(), s>>>(cw, d, a, cl_count + 1);
     pe(s);
     check_launch();
   }
@@ -1784,14 +1800,12 @@ int zm_set_closure(zm_solver* s, void* stream, const float* params, float bound)
       if (!s->kappa3) {
         s->kappa3 = s->alloc<float>((size_t)std::max(1, s->nz - 1) * s->d.plane);
         s->cl_count = s->alloc<unsigned>(2);
-        __nv_bfloat16* W1 = s->alloc<__nv_bfloat16>((size_t)ZM_MLP_IN * ZM_MLP_IN);
-        __nv_bfloat16* W2 = s->alloc<__nv_bfloat16>((size_t)ZM_MLP_IN * ZM_MLP_IN);
-        __nv_bfloat16* W3 = s->alloc<__nv_bfloat16>((size_t)ZM_MLP_OUT * ZM_MLP_IN);
+        __nv_bfloat16* W = s->alloc<__nv_bfloat16>((size_t)(2 * ZM_MLP_IN + ZM_MLP_OUT) * ZM_MLP_IN);
         float* b = s->alloc<float>(2 * ZM_MLP_IN + ZM_MLP_OUT);
-        s->cw = MlpBf16{W1, W2, W3, b, b + ZM_MLP_IN, b + 2 * ZM_MLP_IN};
+        s->cw = MlpTc{W, b, b + ZM_MLP_IN, b + 2 * ZM_MLP_IN};
         ZM_CUDA(cudaFuncSetAttribute(k_mlp_closure, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_tc_smem()));
       }
-      const int rc = zm_mlp_pack_bf16(stream, params, (void*)s->cw.W1, (void*)s->cw.W2, (void*)s->cw.W3);
+      const int rc = zm_mlp_pack_tc(stream, params, (void*)s->cw.packed);
       if (rc != ZM_OK) return fail(s, Err{rc, "packing the closure weights failed"});
       const long long off_b1 = (long long)ZM_MLP_IN * ZM_MLP_IN, off_b2 = 2 * off_b1 + ZM_MLP_IN,
                       off_b3 = off_b2 + ZM_MLP_IN + (long long)ZM_MLP_OUT * ZM_MLP_IN;
