@@ -125,7 +125,8 @@ struct MlpTc {
   const float *b1, *b2, *b3;
 };
 size_t mlp_tc_smem();
-constexpr int MLP_TC_THREADS = 288;
+int mlp_tc_blocks(long long ncol);
+constexpr int MLP_TC_THREADS = 576;
 // learned closure in the step: features of a column, the plain closure per
 // interface, and the fused tensor-core inference writing kappa per interface
 struct ClosureArgs {

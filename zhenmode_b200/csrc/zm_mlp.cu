@@ -12,10 +12,11 @@
 // LBO = 128 B apart, 8-row groups SBO = 16 * K bytes apart).  The weights are
 // packed once in that layout, in K chunks of 32 (zm_mlp_pack_tc), so that one
 // bulk copy brings a chunk; three buffers, filled two chunks ahead.
-//  * A control thread waits for a chunk, issues its two tcgen05.mma, commits
-//    them to the buffer's mbarrier and refills the buffer before last; the
-//    last commit of a layer goes to the epilogue's mbarrier.
-//  * Eight warps run the epilogue of a layer: the accumulator by tcgen05.ld
+//  * A copy thread fills the buffers; a product thread waits for a chunk, issues
+//    its tcgen05.mma and commits them to the buffer's mbarrier, the last commit
+//    of a layer to the epilogue's (one thread for both, with its index
+//    arithmetic, took 850 cycles a chunk where the products take 540).
+//  * Sixteen warps run the epilogue of a layer: the accumulator by tcgen05.ld
 //    (warp w the rows 32 (w mod 4) .., the columns of half w / 4), bias, GELU,
 //    BF16 back into the activation tile, which is the next layer's A operand.
 // Every wait has a poll limit; one that runs out sets the error word, and the
@@ -31,6 +32,7 @@
 // workspaces.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <string>
 
@@ -41,17 +43,25 @@ namespace zm {
 
 namespace {
 
-constexpr int MT = 128;                          // columns per CTA
+constexpr int MT = 128;                          // columns per accumulator (rows of one product)
+constexpr int TILES = 2;                         // accumulators per CTA
+constexpr int MROWS = TILES * MT;                // columns per pass of a CTA
 constexpr int MK = ZM_MLP_IN;                    // 256: input and hidden width
 constexpr int MO = ZM_MLP_OUT;                   // 64: padded output width
-constexpr int MEPI = 256;                        // epilogue threads per CTA
-static_assert(MLP_TC_THREADS == MEPI + 32, "one more warp for the control thread");
+constexpr int MEPI = 512;                        // epilogue threads per CTA
+static_assert(MLP_TC_THREADS == MEPI + 64, "two more warps: the copy and the product thread");
 constexpr int KC = 32;                           // K chunk of a weight stage
-constexpr int WSTAGES = 3;                       // weight buffers
-constexpr int KCHUNKS = MK / KC;                 // chunks per layer
+constexpr int WSTAGES = 4;                       // weight buffers (a power of two)
+constexpr int KCHUNKS = MK / KC;                 // chunks of a hidden layer
+constexpr int KC3 = 128, KCHUNKS3 = MK / KC3;    // of the output layer: as many bytes a chunk
+constexpr int CHUNKS = 2 * KCHUNKS + KCHUNKS3;
 constexpr uint32_t ACT_BYTES = MT * MK * 2;      // 64 KiB
 constexpr uint32_t WB_BYTES = MK * KC * 2;       // 16 KiB
-constexpr uint32_t TC_SMEM = ACT_BYTES + WSTAGES * WB_BYTES + 128 + MT * 4;  // two CTAs per SM
+constexpr int BIASES = 2 * MK + MO;
+constexpr uint32_t BAR_OFF = TILES * ACT_BYTES + WSTAGES * WB_BYTES;   // mbarriers, 128 bytes
+constexpr uint32_t BIAS_OFF = BAR_OFF + 128;                           // float32 biases
+constexpr uint32_t SCRATCH_OFF = BIAS_OFF + BIASES * 4;                // one word per column
+constexpr uint32_t TC_SMEM = SCRATCH_OFF + MROWS * 4;                  // one CTA per SM
 constexpr unsigned WAIT_POLLS = 1u << 22;
 
 __device__ __forceinline__ uint32_t su32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -130,13 +140,18 @@ __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::be
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+template <int N>
+struct Int {
+  static constexpr int value = N;
+};
+
 __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.f + erff(x * 0.70710678118654752f)); }
-// GELU of two values for the BF16 inference: x Phi(x) with Phi = 0.5 + 0.5 erf
-// and erf(t) = t P(t^2) / Q(t^2), a rational minimax fit of degrees 5 and 5 on
-// |t| <= 4 (weighted linearised least squares, own fit: 2.1e-8 off in exact
-// arithmetic, the value 1.1e-6 in float32, where BF16 rounds to 2^-9 of it);
-// beyond, P / Q stays at its end value and the saturation gives 0 or 1.  On
-// paired instructions this is 13 issue slots a value, erff about 30.
+// GELU of two values for the BF16 inference: x Phi(x) with
+// Phi = 0.5 + x P(x^2) / Q(x^2), a rational minimax fit of degrees 5 and 5 on
+// x^2 <= 32 (weighted linearised least squares, own fit: 3.2e-8 off in exact
+// arithmetic, the value 9e-7 in float32, where BF16 rounds to 2^-9 of it);
+// beyond, P / Q stays at its end value and the saturation gives 0 or 1.  The
+// epilogue is bound by the FMA pipes: 15 operations a value, erff takes about 30.
 __device__ __forceinline__ float2 gelu2(float2 x) {
   auto c = [](float a) { return make_float2(a, a); };
   auto rcp = [](float a) {
@@ -144,20 +159,19 @@ __device__ __forceinline__ float2 gelu2(float2 x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
     return r;
   };
-  const float2 t = __fmul2_rn(x, c(0.70710678118654752f));
-  float2 s = __fmul2_rn(t, t);
-  s = make_float2(fminf(s.x, 16.f), fminf(s.y, 16.f));
-  float2 p = __ffma2_rn(s, c(1.974827910089516e-06f), c(0.00028804215253330767f));
-  p = __ffma2_rn(s, p, c(0.00400366960093379f));
-  p = __ffma2_rn(s, p, c(0.05346754938364029f));
-  p = __ffma2_rn(s, p, c(0.19624949991703033f));
-  p = __ffma2_rn(s, p, c(1.128378987312317f));
-  float2 q = __ffma2_rn(s, c(3.748088056454435e-05f), c(0.0012163660721853375f));
-  q = __ffma2_rn(s, q, c(0.015444467775523663f));
-  q = __ffma2_rn(s, q, c(0.1164766475558281f));
-  q = __ffma2_rn(s, q, c(0.5072527527809143f));
+  float2 s = __fmul2_rn(x, x);
+  s = make_float2(fminf(s.x, 32.f), fminf(s.y, 32.f));
+  float2 p = __ffma2_rn(s, c(2.1449805487350204e-08f), c(6.633825250901282e-06f));
+  p = __ffma2_rn(s, p, c(0.00019462825730443f));
+  p = __ffma2_rn(s, p, c(0.0048324111849069595f));
+  p = __ffma2_rn(s, p, c(0.03627265989780426f));
+  p = __ffma2_rn(s, p, c(0.39894184470176697f));
+  float2 q = __ffma2_rn(s, c(1.1807725286416826e-06f), c(8.251606777776033e-05f));
+  q = __ffma2_rn(s, q, c(0.002028433606028557f));
+  q = __ffma2_rn(s, q, c(0.030050016939640045f));
+  q = __ffma2_rn(s, q, c(0.25758427381515503f));
   q = __ffma2_rn(s, q, c(1.f));
-  p = __fmul2_rn(p, __fmul2_rn(t, c(0.5f)));
+  p = __fmul2_rn(p, x);
   return make_float2(x.x * __saturatef(fmaf(p.x, rcp(q.x), 0.5f)), x.y * __saturatef(fmaf(p.y, rcp(q.y), 0.5f)));
 }
 __device__ __forceinline__ float gelu_grad(float x) {
@@ -167,30 +181,40 @@ __device__ __forceinline__ float gelu_grad(float x) {
 }  // namespace
 
 size_t mlp_tc_smem() { return TC_SMEM; }
-
-// Packed weights: the chunks of W1, W2, W3 in turn, KCHUNKS each, [out][32] in
-// the canonical layout.
-constexpr int PACK_ELEMS = (2 * MK + MO) * MK;
-__device__ __forceinline__ size_t pack_chunk(int i) {  // first element of chunk i
-  return i < 2 * KCHUNKS ? (size_t)i * (MK * KC) : (size_t)2 * MK * MK + (size_t)(i - 2 * KCHUNKS) * (MO * KC);
+int mlp_tc_blocks(long long ncol) {  // one CTA per SM at most, each with its passes
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return (int)std::min<long long>((ncol + MROWS - 1) / MROWS, std::max(sms, 1));
 }
 
-// One MLP pass over the 128 BF16 rows that `stage(act, scratch)` writes into the
-// activation tile (core_off layout; called by the MEPI epilogue threads,
-// scratch holds 128 words), writing the raw outputs of each row through
-// `emit(row, c0, v)`, 32 at a time.  Shared by the standalone and the fused kernels.
-template <class Stage, class Emit>
-__device__ __forceinline__ void mlp_tc_body(const MlpTc& w, uint8_t* msm, unsigned* err, Stage stage, Emit emit) {
+// Packed weights: the chunks of W1, W2 ([256][32] each) and W3 ([64][128]) in
+// turn, all of WB_BYTES, in the canonical layout.
+constexpr int PACK_ELEMS = (2 * MK + MO) * MK;
+static_assert(MO * KC3 * 2 == WB_BYTES && PACK_ELEMS * 2 == CHUNKS * WB_BYTES, "chunks of one size");
+
+// The MLP over passes of MROWS rows, pass blockIdx.x, blockIdx.x + gridDim.x, ...
+// of `passes`: stage(pass, act, scratch) writes the pass's BF16 rows into the
+// activation tiles (row r at act + (r / MT) ACT_BYTES + core_off(r % MT, ..);
+// called by the MEPI epilogue threads, scratch holds MROWS words), next(pass)
+// may prefetch a later pass's inputs, emit(pass, row, c0, v) takes the raw
+// outputs of a row, 32 at a time, with EMIT_BYTES of shared memory of its warp's.
+// Shared by the standalone and the fused kernels.
+constexpr int EMIT_STRIDE = 36, EMIT_BYTES = 32 * EMIT_STRIDE * 4;
+template <class Stage, class Next, class Emit>
+__device__ __forceinline__ void mlp_tc_body(const MlpTc& w, uint8_t* msm, unsigned* err, int passes, Stage stage,
+                                            Next next, Emit emit) {
   uint8_t* act = msm;
-  uint8_t* wb = msm + ACT_BYTES;
-  uint64_t* full = reinterpret_cast<uint64_t*>(msm + ACT_BYTES + WSTAGES * WB_BYTES);  // a chunk has landed
+  uint8_t* wb = msm + TILES * ACT_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(msm + BAR_OFF);  // a chunk has landed
   uint64_t* empty = full + WSTAGES;   // a chunk's products are done
-  uint64_t* ready = empty + WSTAGES;  // the activation tile is written
+  uint64_t* ready = empty + WSTAGES;  // the activation tiles are written
   uint64_t* done = ready + 1;         // a layer's products are done
   uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
-  uint32_t* scratch = reinterpret_cast<uint32_t*>(msm + ACT_BYTES + WSTAGES * WB_BYTES + 128);
+  float* sbias = reinterpret_cast<float*>(msm + BIAS_OFF);
+  uint32_t* scratch = reinterpret_cast<uint32_t*>(msm + SCRATCH_OFF);
   const int t = threadIdx.x, warp = t >> 5;
-  constexpr int CHUNKS = 3 * KCHUNKS;
+  const int mine = passes > (int)blockIdx.x ? (passes - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   if (t == MEPI) {
     for (int b = 0; b < WSTAGES; ++b) {
       mbar_init(su32(full + b), 1);
@@ -201,106 +225,128 @@ __device__ __forceinline__ void mlp_tc_body(const MlpTc& w, uint8_t* msm, unsign
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(tslot)), "r"(256u)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(tslot)), "r"(512u)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  for (int e = t; e < BIASES; e += MLP_TC_THREADS)
+    sbias[e] = e < MK ? __ldg(w.b1 + e) : (e < 2 * MK ? __ldg(w.b2 + e - MK) : __ldg(w.b3 + e - 2 * MK));
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tmem = *tslot;
   bool ok = true;
   if (warp == MEPI / 32) {
-    if (t == MEPI) {  // control thread
-      int loaded = 0, issued = 0;  // chunks whose copy, whose products were started
-      auto load = [&]() {
-        const uint32_t bytes = (uint32_t)(loaded < 2 * KCHUNKS ? MK : MO) * KC * 2u;
-        bulk_load(su32(wb) + (uint32_t)(loaded % WSTAGES) * WB_BYTES, w.packed + pack_chunk(loaded), bytes,
-                  su32(full + loaded % WSTAGES));
-        ++loaded;
-      };
-      for (int b = 0; b < WSTAGES; ++b) load();
-      for (int i = 0; i < CHUNKS && ok; ++i) {
-        const int layer = i / KCHUNKS, kc = i - layer * KCHUNKS, buf = i % WSTAGES;
-        if (kc == 0) ok = mbar_wait(su32(ready), (uint32_t)layer & 1u, WAIT_POLLS);
-        ok = ok && mbar_wait(su32(full + buf), (uint32_t)(i / WSTAGES) & 1u, WAIT_POLLS);
-        if (!ok) break;
-        fence_after();
-        const uint32_t id = layer < 2 ? idesc_bf16(MT, MK) : idesc_bf16(MT, MO);
-        const uint32_t wsrc = su32(wb) + (uint32_t)buf * WB_BYTES;
-#pragma unroll
-        for (int s = 0; s < KC / 16; ++s) {
-          const uint64_t da = sdesc(su32(act) + (uint32_t)((kc * KC + s * 16) / 8) * 128u, 128u, (uint32_t)MK * 16u);
-          const uint64_t db = sdesc(wsrc + (uint32_t)s * 256u, 128u, (uint32_t)KC * 16u);
-          umma_bf16(tmem, da, db, id, (kc | s) != 0 ? 1u : 0u);
-        }
-        umma_commit(su32(empty + buf));
-        if (kc + 1 == KCHUNKS) umma_commit(su32(done));
-        ++issued;
-        // the buffer of the chunk before this one is free once its products are done
-        if (i > 0 && loaded < CHUNKS) {
-          ok = mbar_wait(su32(empty + (i - 1) % WSTAGES), (uint32_t)((i - 1) / WSTAGES) & 1u, WAIT_POLLS);
-          if (ok) load();
+    if (t == MEPI) {  // copy thread: weight chunks in turn, WSTAGES ahead of the products
+      int n = 0;  // copies started
+      for (int m = 0; m < mine && ok; ++m) {
+        const __nv_bfloat16* src = w.packed;
+        for (int c = 0; c < CHUNKS && ok; ++c, ++n) {
+          const int b = n & (WSTAGES - 1);
+          if (n >= WSTAGES) ok = mbar_wait(su32(empty + b), (uint32_t)(n / WSTAGES - 1) & 1u, WAIT_POLLS);
+          if (!ok) break;
+          bulk_load(su32(wb) + (uint32_t)b * WB_BYTES, src, WB_BYTES, su32(full + b));
+          src += WB_BYTES / 2;
         }
       }
-      // every copy and product that was started ends before the memory goes
-      for (int i = issued; i < loaded; ++i)
-        ok = mbar_wait(su32(full + i % WSTAGES), (uint32_t)(i / WSTAGES) & 1u, WAIT_POLLS) && ok;
-      if (issued > 0)
-        ok = mbar_wait(su32(empty + (issued - 1) % WSTAGES), (uint32_t)((issued - 1) / WSTAGES) & 1u, WAIT_POLLS) && ok;
-      ok = ok && issued == CHUNKS;
+      // every copy that was started ends before the memory goes
+      for (int i = n > WSTAGES ? n - WSTAGES : 0; i < n; ++i)
+        ok = mbar_wait(su32(full + (i & (WSTAGES - 1))), (uint32_t)(i / WSTAGES) & 1u, WAIT_POLLS) && ok;
+    }
+    __syncwarp();
+  } else if (warp == MEPI / 32 + 1) {
+    if (t == MEPI + 32) {  // product thread; descriptors advance by constants: a chunk is short
+      const uint64_t da0 = sdesc(su32(act), 128u, (uint32_t)MK * 16u);
+      int n = 0, phase = 0;  // chunks taken, layers begun
+      // one layer: K chunks of kc from a row of `id`'s N weights
+      auto products = [&](auto kc_, uint32_t id) {
+        constexpr int K = decltype(kc_)::value;
+        const uint64_t db0 = sdesc(su32(wb), 128u, (uint32_t)K * 16u);
+        ok = mbar_wait(su32(ready), (uint32_t)(phase++) & 1u, WAIT_POLLS);
+#pragma unroll
+        for (int kc = 0; kc < MK / K; ++kc) {
+          const int b = n & (WSTAGES - 1);
+          ok = ok && mbar_wait(su32(full + b), (uint32_t)(n / WSTAGES) & 1u, WAIT_POLLS);
+          if (!ok) return;
+          fence_after();
+          const uint64_t db = db0 + (uint64_t)b * (WB_BYTES / 16);
+#pragma unroll
+          for (int q = 0; q < TILES; ++q)
+#pragma unroll
+            for (int s = 0; s < K / 16; ++s)
+              umma_bf16(tmem + (uint32_t)q * 256u, da0 + (uint64_t)(q * (ACT_BYTES / 16) + (kc * K + s * 16) / 8 * 8),
+                        db + (uint64_t)(s * 16), id, (kc | s) != 0 ? 1u : 0u);
+          umma_commit(su32(empty + b));
+          ++n;
+        }
+        umma_commit(su32(done));
+      };
+      for (int m = 0; m < mine && ok; ++m) {
+        products(Int<KC>{}, idesc_bf16(MT, MK));
+        if (ok) products(Int<KC>{}, idesc_bf16(MT, MK));
+        if (ok) products(Int<KC3>{}, idesc_bf16(MT, MO));
+      }
+      // the last products end before the memory goes
+      if (n > 0) ok = mbar_wait(su32(empty + ((n - 1) & (WSTAGES - 1))), (uint32_t)((n - 1) / WSTAGES) & 1u, WAIT_POLLS) && ok;
     }
     __syncwarp();
   } else {
-    stage(act, scratch);
-    fence_async_smem();
-    mbar_arrive(su32(ready));
-    const int quarter = warp & 3, half = warp >> 2, row = quarter * 32 + (t & 31);
-    const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-    for (int layer = 0; layer < 3; ++layer) {
-      const int N = layer < 2 ? MK : MO;
-      if (!mbar_wait(su32(done), (uint32_t)layer & 1u, WAIT_POLLS)) ok = false;
-      if (!__all_sync(0xffffffffu, ok)) {  // tcgen05.ld is a warp's
-        ok = false;
-        break;
-      }
-      fence_after();
-      const float* bias = layer == 0 ? w.b1 : (layer == 1 ? w.b2 : w.b3);
-      const bool vb = ((uintptr_t)bias & 15u) == 0;
-      for (int c0 = half * (N / 2); c0 < (half + 1) * (N / 2); c0 += 32) {
-        float v[32];
-        tmem_ld32(tmem + lane_base + (uint32_t)c0, v);
-        auto bias4 = [&](int e) {
-          const float* b = bias + c0 + e;
-          return vb ? __ldg(reinterpret_cast<const float4*>(b))
-                    : make_float4(__ldg(b), __ldg(b + 1), __ldg(b + 2), __ldg(b + 3));
-        };
+    // warp w: rows 32 (w mod 4) .. of accumulator w / 8, columns of half (w / 4) mod 2
+    const int quarter = warp & 3, half = (warp >> 2) & 1, tile = warp >> 3;
+    const int row = quarter * 32 + (t & 31);
+    const uint32_t lane_base = tmem + (uint32_t)tile * 256u + ((uint32_t)(quarter * 32) << 16);
+    uint8_t* my_act = act + (size_t)tile * ACT_BYTES;
+    int phase = 0;
+    for (int n = 0; n < mine && ok; ++n) {
+      const int pass = (int)blockIdx.x + n * (int)gridDim.x;
+      if (n > 0) asm volatile("bar.sync 1, %0;" ::"n"(MEPI) : "memory");  // emit may use the tiles
+      stage(pass, act, scratch);
+      fence_async_smem();
+      mbar_arrive(su32(ready));
+      if (n + 1 < mine) next(pass + (int)gridDim.x);
+      for (int layer = 0; layer < 3; ++layer) {
+        const int N = layer < 2 ? MK : MO;
+        if (!mbar_wait(su32(done), (uint32_t)(phase++) & 1u, WAIT_POLLS)) ok = false;
+        if (!__all_sync(0xffffffffu, ok)) {  // tcgen05.ld is a warp's
+          ok = false;
+          break;
+        }
+        fence_after();
+        const float* bias = sbias + layer * MK;
+        for (int c0 = half * (N / 2); c0 < (half + 1) * (N / 2); c0 += 32) {
+          float v[32];
+          tmem_ld32(lane_base + (uint32_t)c0, v);
+          const float4* b4 = reinterpret_cast<const float4*>(bias + c0);
+          if (layer < 2) {
+#pragma unroll
+            for (int e = 0; e < 32; e += 8) {
+              const float4 ba = b4[e / 4], bb = b4[e / 4 + 1];
+              __align__(16) __nv_bfloat162 h[4];
+              h[0] = __float22bfloat162_rn(gelu2(__fadd2_rn(make_float2(v[e], v[e + 1]), make_float2(ba.x, ba.y))));
+              h[1] = __float22bfloat162_rn(gelu2(__fadd2_rn(make_float2(v[e + 2], v[e + 3]), make_float2(ba.z, ba.w))));
+              h[2] = __float22bfloat162_rn(gelu2(__fadd2_rn(make_float2(v[e + 4], v[e + 5]), make_float2(bb.x, bb.y))));
+              h[3] = __float22bfloat162_rn(gelu2(__fadd2_rn(make_float2(v[e + 6], v[e + 7]), make_float2(bb.z, bb.w))));
+              *reinterpret_cast<uint4*>(my_act + core_off(row, c0 + e, MK)) = *reinterpret_cast<const uint4*>(h);
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 32; e += 4) {
+              const float4 ba = b4[e / 4];
+              v[e] += ba.x;
+              v[e + 1] += ba.y;
+              v[e + 2] += ba.z;
+              v[e + 3] += ba.w;
+            }
+            // this warp's part of the tile, which no product reads any more
+            emit(pass, tile * MT + row, c0, v, reinterpret_cast<float*>(my_act + (warp & 7) * EMIT_BYTES));
+          }
+        }
+        fence_before();
         if (layer < 2) {
-#pragma unroll
-          for (int e = 0; e < 32; e += 8) {
-            const float4 ba = bias4(e), bb = bias4(e + 4);
-            __align__(16) __nv_bfloat162 h[4];
-            h[0] = __float22bfloat162_rn(gelu2(__fadd2_rn(make_float2(v[e], v[e + 1]), make_float2(ba.x, ba.y))));
-            h[1] = __float22bfloat162_rn(gelu2(__fadd2_rn(make_float2(v[e + 2], v[e + 3]), make_float2(ba.z, ba.w))));
-            h[2] = __float22bfloat162_rn(gelu2(__fadd2_rn(make_float2(v[e + 4], v[e + 5]), make_float2(bb.x, bb.y))));
-            h[3] = __float22bfloat162_rn(gelu2(__fadd2_rn(make_float2(v[e + 6], v[e + 7]), make_float2(bb.z, bb.w))));
-            *reinterpret_cast<uint4*>(act + core_off(row, c0 + e, MK)) = *reinterpret_cast<const uint4*>(h);
-          }
-        } else {
-#pragma unroll
-          for (int e = 0; e < 32; e += 4) {
-            const float4 ba = bias4(e);
-            v[e] += ba.x;
-            v[e + 1] += ba.y;
-            v[e + 2] += ba.z;
-            v[e + 3] += ba.w;
-          }
-          emit(row, c0, v);
+          fence_async_smem();
+          mbar_arrive(su32(ready));
         }
       }
-      fence_before();
-      fence_async_smem();
-      if (layer < 2) mbar_arrive(su32(ready));
     }
   }
   if (!ok) atomicOr(err, 1u);
@@ -308,27 +354,27 @@ __device__ __forceinline__ void mlp_tc_body(const MlpTc& w, uint8_t* msm, unsign
   __syncthreads();
   if (warp == 0) {
     fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   }
 }
 
 // Standalone inference on feature rows X [ncol][256] (BF16, or float32 that is
 // rounded to BF16 on the way in) -> Y [ncol][64].
 template <class In>
-__global__ void __launch_bounds__(MLP_TC_THREADS, 2) k_mlp_tc(MlpTc w, const In* __restrict__ X, float* __restrict__ Y,
-                                                        int ncol, unsigned* err) {
+__global__ void __launch_bounds__(MLP_TC_THREADS, 1) k_mlp_tc(MlpTc w, const In* __restrict__ X,
+                                                              float* __restrict__ Y, int ncol, unsigned* err) {
   extern __shared__ __align__(1024) uint8_t msm[];
-  const long long col0 = (long long)blockIdx.x * MT;
+  const bool y16 = ((uintptr_t)Y & 15u) == 0;
   mlp_tc_body(
-      w, msm, err,
-      [&](uint8_t* act, uint32_t*) {
+      w, msm, err, (ncol + MROWS - 1) / MROWS,
+      [&](int pass, uint8_t* act, uint32_t*) {
         // a warp takes 8 rows x 4 groups of 8 features at a time: rows in full
         // 128-byte (64-byte) pieces, shared stores without bank conflicts
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll 1
-        for (int oct = 0; oct < MT / 8 / (MEPI / 32); ++oct) {
+        for (int oct = 0; oct < MROWS / 8 / (MEPI / 32); ++oct) {
           const int r = (oct * (MEPI / 32) + warp) * 8 + (lane & 7);
-          const long long col = col0 + r;
+          const long long col = (long long)pass * MROWS + r;
           uint4 v[MK / 32];
 #pragma unroll
           for (int g = 0; g < MK / 32; ++g) {
@@ -346,22 +392,38 @@ __global__ void __launch_bounds__(MLP_TC_THREADS, 2) k_mlp_tc(MlpTc w, const In*
               v[g] = *reinterpret_cast<const uint4*>(h);
             }
           }
+          uint8_t* a = act + (size_t)(r / MT) * ACT_BYTES;
 #pragma unroll
           for (int g = 0; g < MK / 32; ++g)
-            *reinterpret_cast<uint4*>(act + core_off(r, g * 32 + (lane >> 3) * 8, MK)) = v[g];
+            *reinterpret_cast<uint4*>(a + core_off(r % MT, g * 32 + (lane >> 3) * 8, MK)) = v[g];
         }
       },
-      [&](int row, int c0, const float* v) {
-        const long long col = col0 + row;
-        if (col >= ncol) return;
-        float* y = Y + col * MO + c0;
-        if (((uintptr_t)Y & 15u) == 0) {
+      [&](int pass) {  // the next pass's rows into L2 while this one computes
+        constexpr int LINE = 128 / sizeof(In);  // elements of a cache line
+        for (int e = threadIdx.x; e < MROWS * MK / LINE; e += MEPI) {
+          const long long o = (long long)pass * MROWS * MK + (long long)e * LINE;
+          if (o < (long long)ncol * MK) asm volatile("prefetch.global.L2 [%0];" ::"l"(X + o));
+        }
+      },
+      [&](int pass, int row, int c0, const float* v, float* area) {
+        // rows side by side through shared memory: stores of whole 128-byte lines
+        const int lane = threadIdx.x & 31;
 #pragma unroll
-          for (int j = 0; j < 32; j += 4)
-            *reinterpret_cast<float4*>(y + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-        } else {
+        for (int j = 0; j < 32; j += 4)
+          *reinterpret_cast<float4*>(area + lane * EMIT_STRIDE + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        __syncwarp();
+        const long long col0 = (long long)pass * MROWS + row - lane;
 #pragma unroll
-          for (int j = 0; j < 32; ++j) y[j] = v[j];
+        for (int it = 0; it < 8; ++it) {
+          const int r = it * 4 + (lane >> 3), j = (lane & 7) * 4;
+          if (col0 + r >= ncol) break;
+          const float4 y = *reinterpret_cast<const float4*>(area + r * EMIT_STRIDE + j);
+          float* o = Y + (col0 + r) * MO + c0 + j;
+          if (y16) {
+            *reinterpret_cast<float4*>(o) = y;
+          } else {
+            o[0] = y.x; o[1] = y.y; o[2] = y.z; o[3] = y.w;
+          }
         }
       });
 }
@@ -448,13 +510,13 @@ __global__ void __launch_bounds__(128) k_closure_features(Dev d, ClosureArgs a) 
 // the tensor-core MLP; kappa = 10^y at the wet interfaces, clipped to
 // [1e-7, 1] m^2/s, or the plain closure for a column whose features exceed
 // the trusted bound (or are not finite).
-__global__ void __launch_bounds__(MLP_TC_THREADS, 2) k_mlp_closure(MlpTc w, Dev d, ClosureArgs a, unsigned* err) {
+__global__ void __launch_bounds__(MLP_TC_THREADS, 1) k_mlp_closure(MlpTc w, Dev d, ClosureArgs a, unsigned* err) {
   extern __shared__ __align__(1024) uint8_t msm[];
   const long long ncol = (long long)d.nx * d.ny;
-  // threads 0..127 take T, S and N^2 of column t, threads 128..255 u, v and the forcing of column t - 128
-  const int c = threadIdx.x & (MT - 1), part = threadIdx.x / MT;
-  auto place = [&](int r, long long& base, uint64_t& bits) {
-    const long long col = (long long)blockIdx.x * MT + r;
+  // the first MROWS threads take T, S and N^2 of column t, the others u, v and the forcing of column t - MROWS
+  const int c = threadIdx.x & (MROWS - 1), part = threadIdx.x / MROWS;
+  auto place = [&](int pass, int r, long long& base, uint64_t& bits) {
+    const long long col = (long long)pass * MROWS + r;
     if (col >= ncol) {
       base = 0;
       bits = 0ull;
@@ -465,24 +527,26 @@ __global__ void __launch_bounds__(MLP_TC_THREADS, 2) k_mlp_closure(MlpTc w, Dev 
     bits = __ldg(d.wbits + base);
     return true;
   };
-  const uint32_t* largest = reinterpret_cast<const uint32_t*>(msm + ACT_BYTES + WSTAGES * WB_BYTES + 128);
+  const uint32_t* largest = reinterpret_cast<const uint32_t*>(msm + SCRATCH_OFF);
   mlp_tc_body(
-      w, msm, err,
-      [&](uint8_t* tile, uint32_t* amax_bits) {
+      w, msm, err, (int)((ncol + MROWS - 1) / MROWS),
+      [&](int pass, uint8_t* act, uint32_t* amax_bits) {
+        uint8_t* tile = act + (size_t)(c / MT) * ACT_BYTES;
+        const int r = c % MT;
         // the rows are zero, then the features level by level: loads coalesced
         // over the CTA's consecutive columns; N^2 from the level above kept in registers
         for (int kp = part * (MK / 16); kp < (part + 1) * (MK / 16); ++kp)
-          *reinterpret_cast<uint4*>(tile + core_off(c, kp * 8, MK)) = make_uint4(0u, 0u, 0u, 0u);
+          *reinterpret_cast<uint4*>(tile + core_off(r, kp * 8, MK)) = make_uint4(0u, 0u, 0u, 0u);
         if (part == 0) amax_bits[c] = 0u;
         asm volatile("bar.sync 1, %0;" ::"n"(MEPI) : "memory");
         long long base;
         uint64_t bits;
-        if (place(c, base, bits)) {
+        if (place(pass, c, base, bits)) {
           float amax = 0.f;
           auto put = [&](int q, float f) {
             amax = fmaxf(amax, fabsf(f));
             if (!(f == f) || isinf(f)) amax = INFINITY;
-            *reinterpret_cast<__nv_bfloat16*>(tile + core_off(c, q, MK)) = __float2bfloat16(f);
+            *reinterpret_cast<__nv_bfloat16*>(tile + core_off(r, q, MK)) = __float2bfloat16(f);
           };
           const int nk = levels_of(bits);
           const float *pa = part ? a.u : a.T, *pb = part ? a.v : a.S;
@@ -513,10 +577,11 @@ __global__ void __launch_bounds__(MLP_TC_THREADS, 2) k_mlp_closure(MlpTc w, Dev 
         }
         asm volatile("bar.sync 1, %0;" ::"n"(MEPI) : "memory");
       },
-      [&](int row, int c0, const float* y) {
+      [](int) {},
+      [&](int pass, int row, int c0, const float* y, float*) {
         long long base;
         uint64_t bits;
-        if (!place(row, base, bits)) return;
+        if (!place(pass, row, base, bits)) return;
         const bool trusted = __uint_as_float(largest[row]) <= a.bound;
         bool unstable = false;  // column gate of the plain closure
         if (!trusted) {
@@ -567,7 +632,8 @@ __global__ void k_mlp_pack_tc(const In* __restrict__ W1, const In* __restrict__ 
     const int layer = i < MK * MK ? 0 : (i < 2 * MK * MK ? 1 : 2), e = i - layer * MK * MK;
     const int n = e / MK, k = e - n * MK;
     const In* W = layer == 0 ? W1 : (layer == 1 ? W2 : W3);
-    out[pack_chunk(layer * KCHUNKS + k / KC) + core_off(n, k % KC, KC) / 2] = __float2bfloat16((float)W[e]);
+    const int kc = layer < 2 ? KC : KC3, chunk = layer * KCHUNKS + k / kc;
+    out[(size_t)chunk * (WB_BYTES / 2) + core_off(n, k % kc, kc) / 2] = __float2bfloat16((float)W[e]);
   }
 }
 
@@ -875,7 +941,7 @@ template <class In>
 int forward_tc(cudaStream_t st, int ncol, const In* X, const MlpTc& w, float* Y, uint32_t* err) {
   if (cudaFuncSetAttribute(k_mlp_tc<In>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM) != cudaSuccess)
     return ZM_ERR_CUDA;
-  k_mlp_tc<In><<<(ncol + MT - 1) / MT, MLP_TC_THREADS, TC_SMEM, st>>>(w, X, Y, ncol, err);
+  k_mlp_tc<In><<<mlp_tc_blocks(ncol), MLP_TC_THREADS, TC_SMEM, st>>>(w, X, Y, ncol, err);
   return launch_ok("mlp forward") ? ZM_OK : ZM_ERR_CUDA;
 }
 

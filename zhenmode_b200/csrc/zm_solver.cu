@@ -575,7 +575,7 @@ struct zm_solver {
     a.T = in.T; a.S = in.S; a.u = in.u; a.v = in.v; a.kappa3 = kappa3; a.fallback = cl_count; a.bound = cl_bound;
     const long long ncol = (long long)nx * ny;
     pb(ZM_K_CLOSURE, s);
-    k_mlp_closure<<<(unsigned)((ncol + 127) / 128), MLP_TC_THREADS, mlp_tc_smem(), s>>>(cw, d, a, cl_count + 1);
+    k_mlp_closure<<<mlp_tc_blocks(ncol), MLP_TC_THREADS, mlp_tc_smem(), s>>>(cw, d, a, cl_count + 1);
     pe(s);
     check_launch();
   }
