@@ -28,6 +28,8 @@ constexpr float kRho0 = 1025.0f;
 constexpr float kAlpha = 2.0e-4f;
 constexpr float kBeta = 7.6e-4f;
 constexpr float kCp = 3992.0f;
+// limits of the state classification (runtime/monitor.py:20-30)
+constexpr float kMonitorVelocity = 10.f, kMonitorEta = 15.f;
 
 // Per-level coefficients of the non-uniform vertical grid, passed by value.
 struct Vert {

@@ -57,6 +57,7 @@ struct PgfArgs {
   double *ubt0, *vbt0;
   float dt, bottom_decay;
   int mode;
+  unsigned int* flags;  // mode 0: the step's classification of its result, cleared here
 };
 
 struct RestArgs {
@@ -193,7 +194,8 @@ __global__ void k_cap3_means(Dev d, const float* u, const float* v, const float*
 __global__ void k_final(Dev d, const float* u3, const float* v3, const float* T3, const float* S3, const double* ubt,
                         const double* ubt0, const double* vbt, const double* vbt0, const float* u0, const float* v0,
                         const float* T0, const float* S0, const float* means, const float* wts, int nb_rows,
-                        float* uo, float* vo, float* To, float* So, unsigned long long* seq, int seq_by);
+                        float* uo, float* vo, float* To, float* So, unsigned long long* seq, int seq_by,
+                        const float* eta, unsigned int* flags);
 // column-divergence projection of the stage-2 advective velocity (zm_projection.cu)
 constexpr int PJ_THREADS = 1024;
 #define ZM_PJ_SUMS 4
@@ -262,10 +264,15 @@ __global__ void k_led_disp(Dev d, const float* eb, const float* Tb, const float*
                            const float* Sa, const double* area, double* part);
 __global__ void k_led_fold(const double* part, int nblocks, int nq, LedFold f, double* acc);
 __global__ void k_led_proj(const double* norms, double* acc);
-__global__ void k_ref_to_int3(Dev d, const float* src, float* dst, float offset);
-__global__ void k_int_to_ref3(Dev d, const float* src, float* dst, float offset);
+// layout change of n3 3-D fields, then n2 (0 or 1) 2-D fields; offset is subtracted inward, added outward
+struct LayoutArgs {
+  const float* src[5];
+  float* dst[5];
+  float offset[5];
+  int n3, n2;
+};
+void launch_layout(cudaStream_t s, const Dev& d, const LayoutArgs& a, bool to_internal);
 __global__ void k_ref_to_int2(Dev d, const float* src, float* dst);
-__global__ void k_int_to_ref2(Dev d, const float* src, float* dst);
 __global__ void k_monitor(Dev d, const float* u, const float* v, const float* T, const float* S, const float* eta,
                           float umax, float etamax, unsigned int* flags);
 

@@ -5,26 +5,29 @@
 // with W[out][in] (the input index contiguous).
 //
 // Inference (k_mlp_tc): BF16 operands on the 5th-generation tensor cores with
-// float32 accumulation in tensor memory.  A CTA owns 128 columns: column t is
-// row t of the A operand and lane t of the accumulator.  The activations stay
-// in shared memory as BF16 in the canonical K-major layout without swizzle
-// (8-row x 16-byte core matrices; the two core matrices of one K=16 step are
-// LBO = 128 B apart, 8-row groups SBO = 16 * K bytes apart).  The weights are
-// packed once in that layout, in K chunks of 32 (zm_mlp_pack_tc), so that one
-// bulk copy brings a chunk; three buffers, filled two chunks ahead.
+// float32 accumulation in tensor memory.  One persistent CTA per SM takes 256
+// columns a pass: column t is row t of one of two A operands and lane t of its
+// accumulator.  The activations stay in shared memory as BF16 in the canonical
+// K-major layout without swizzle (8-row x 16-byte core matrices; the two core
+// matrices of one K=16 step are LBO = 128 B apart, 8-row groups SBO = 16 * K bytes
+// apart).  The weights are packed once in that layout, in K chunks of 16 KB
+// (zm_mlp_pack_tc), so that one bulk copy brings a chunk for both operands; four
+// buffers.  The rows of the next pass are prefetched into L2.
 //  * A copy thread fills the buffers; a product thread waits for a chunk, issues
 //    its tcgen05.mma and commits them to the buffer's mbarrier, the last commit
 //    of a layer to the epilogue's (one thread for both, with its index
 //    arithmetic, took 850 cycles a chunk where the products take 540).
 //  * Sixteen warps run the epilogue of a layer: the accumulator by tcgen05.ld
-//    (warp w the rows 32 (w mod 4) .., the columns of half w / 4), bias, GELU,
+//    (warp w the rows 32 (w mod 4) .., accumulator w / 8, columns of half (w / 4) mod 2), bias, GELU,
 //    BF16 back into the activation tile, which is the next layer's A operand.
 // Every wait has a poll limit; one that runs out sets the error word, and the
 // CTA waits (again bounded) for its copies and products before it frees TMEM.
 //
-// The products of a tile take 2.4 us of an SM's tensor core, GELU on 65536
-// values 4.3 us of its FMA pipes: that is the bound, so two CTAs share an SM and
-// one's products and loads run under the other's epilogue.  MEASURED_INFER
+// Of the 42k cycles of a pass the epilogues take 29k (GELU on 131072 values, 15
+// FMA-pipe operations each, is the bound), the products that nothing overlaps 12k.
+// 259200 columns: 558 us with weights fetched by all threads between barriers, 377
+// with two such CTAs per SM, 249 with packed weights and a control thread, 220 as
+// it stands (64800 columns 66 us, 4000 columns 35).
 //
 // Training: float32 SIMT kernels (tiled GEMM with optional transposes, GELU
 // and its derivative, masked mean-square loss, bias gradients, Adam), driven

@@ -110,7 +110,7 @@ struct zm_solver {
   float* ref_eta = nullptr;
   // mutable forcing fields
   float *tau_x = nullptr, *tau_y = nullptr, *qheat = nullptr;
-  unsigned int* flags = nullptr;
+  unsigned int* flags = nullptr;  // [0] the classification zm_status reports, [1] that of the last step's result
   cudaStream_t cap_stream = nullptr;  // graphs are captured here, launched on the caller's stream
   cudaStream_t side = nullptr;        // the second branch of the N step (momentum advection)
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -499,6 +499,7 @@ struct zm_solver {
     PgfArgs a{};
     a.T = s3.T; a.S = s3.S; a.u1 = s3.u; a.v1 = s3.v; a.frx = frx; a.fry = fry; a.ubt0 = ubt0; a.vbt0 = vbt0;
     a.mode = 0;
+    a.flags = flags + 1;
     pgf(s, a);
     const dim3 c(32, 8);
     double *ubt_fin, *vbt_fin;
@@ -563,7 +564,7 @@ struct zm_solver {
     pb(ZM_K_FINAL, s);
     ZM_CUDA(launch_pdl(k_final, grid3(c), c, 0, s, d, s3.u, s3.v, s3.T, s3.S, ubt_fin, ubt0, vbt_fin, vbt0, held.u,
                        held.v, held.T, held.S, means, wts, cap_rows > 0 ? cap_nb : 0, out.u, out.v, out.T, out.S,
-                       bt_blocks > 0 ? bt_seq : nullptr, 2 * n_subcyc + 2));
+                       bt_blocks > 0 ? bt_seq : nullptr, 2 * n_subcyc + 2, eta_out, flags + 1));
     pe(s);
     check_launch();
   }
@@ -603,10 +604,16 @@ struct zm_solver {
     }
   }
 
-  void monitor(cudaStream_t s, int which) {
+  // The classification of the state an advance ends with: its last step's own, or, where no
+  // step ran, one pass over the state (72 us at 720 x 360 x 50, against 4 for the copy).
+  void monitor(cudaStream_t s, int which, bool stepped) {
+    if (stepped) {
+      ZM_CUDA(cudaMemcpyAsync(flags, flags + 1, sizeof(unsigned int), cudaMemcpyDeviceToDevice, s));
+      return;
+    }
     ZM_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned int), s));
-    k_monitor<<<4 * 148, 256, 0, s>>>(d, st[which].u, st[which].v, st[which].T, st[which].S, eta[which], 10.f, 15.f,
-                                      flags);
+    k_monitor<<<4 * 148, 256, 0, s>>>(d, st[which].u, st[which].v, st[which].T, st[which].S, eta[which],
+                                      kMonitorVelocity, kMonitorEta, flags);
     check_launch();
   }
 
@@ -725,28 +732,20 @@ struct zm_solver {
 
   // layout conversion between reference arrays and internal fields
   void to_int3(cudaStream_t s, const float* src, float* dst, float offset) {
-    k_ref_to_int3<<<dim3((nx + 31) / 32, (nz + 31) / 32, ny), dim3(32, 8), 0, s>>>(d, src, dst, offset);
+    launch_layout(s, d, LayoutArgs{{src}, {dst}, {offset}, 1, 0}, true);
   }
   void to_ref3(cudaStream_t s, const float* src, float* dst, float offset) {
-    k_int_to_ref3<<<dim3((nx + 31) / 32, (nz + 31) / 32, ny), dim3(32, 8), 0, s>>>(d, src, dst, offset);
+    launch_layout(s, d, LayoutArgs{{src}, {dst}, {offset}, 1, 0}, false);
   }
   // tracers enter as anomalies from (T_ref, S_ref)
   void load(cudaStream_t s, const zm_state* in, const Fields4& f, float* e) {
-    to_int3(s, in->u, f.u, 0.f);
-    to_int3(s, in->v, f.v, 0.f);
-    to_int3(s, in->T, f.T, d.T_ref);
-    to_int3(s, in->S, f.S, d.S_ref);
-    const dim3 c(32, 8);
-    k_ref_to_int2<<<grid2(c), c, 0, s>>>(d, in->eta, e);
+    launch_layout(s, d, LayoutArgs{{in->u, in->v, in->T, in->S, in->eta}, {f.u, f.v, f.T, f.S, e},
+                                   {0.f, 0.f, d.T_ref, d.S_ref, 0.f}, 4, 1}, true);
     check_launch();
   }
   void store(cudaStream_t s, const Fields4& f, const float* e, zm_state* out) {
-    to_ref3(s, f.u, out->u, 0.f);
-    to_ref3(s, f.v, out->v, 0.f);
-    to_ref3(s, f.T, out->T, d.T_ref);
-    to_ref3(s, f.S, out->S, d.S_ref);
-    const dim3 c(32, 8);
-    k_int_to_ref2<<<grid2(c), c, 0, s>>>(d, e, out->eta);
+    launch_layout(s, d, LayoutArgs{{f.u, f.v, f.T, f.S, e}, {out->u, out->v, out->T, out->S, out->eta},
+                                   {0.f, 0.f, d.T_ref, d.S_ref, 0.f}, 4, 1}, false);
     check_launch();
   }
 };
@@ -1279,7 +1278,7 @@ void build(zm_solver* s, const zm_grid* g, const zm_params* p) {
   const size_t nref3 = (size_t)nx * ny * nz;
   s->ref = Fields4{s->alloc<float>(nref3), s->alloc<float>(nref3), s->alloc<float>(nref3), s->alloc<float>(nref3)};
   s->ref_eta = s->alloc<float>((size_t)nx * ny);
-  s->flags = s->alloc<unsigned int>(1);
+  s->flags = s->alloc<unsigned int>(2);
   {
     // budget snapshot (diagnostics/snapshot.py:42-64, 67-128)
     std::vector<double> area((size_t)nx * ny), width(nz);
@@ -1375,7 +1374,7 @@ int zm_advance(zm_solver* s, void* stream, int32_t nsteps) {
       ZM_CUDA(cudaGraphLaunch(s->graph[s->cur], st));
       s->cur = 1 - s->cur;
     }
-    s->monitor(st, s->cur);
+    s->monitor(st, s->cur, nsteps > 0);
   } catch (const Err& e) {
     return fail(s, e);
   }
@@ -1505,7 +1504,7 @@ int zm_ensemble_advance(zm_ensemble* e, void* stream, int32_t nsteps, int32_t* k
       for (auto* s : e->m) s->cur = 1 - s->cur;
       rel = 1 - rel;
     }
-    for (auto* s : e->m) s->monitor(st, s->cur);
+    for (auto* s : e->m) s->monitor(st, s->cur, nsteps > 0);
     if (kernels_per_step) *kernels_per_step = e->launches;
   } catch (const Err& err) {
     std::fprintf(stderr, "zm_ensemble_advance: %s\n", err.msg.c_str());
@@ -1548,11 +1547,10 @@ int zm_step_host(zm_solver* s, void* stream, const zm_state* in, zm_state* out, 
       ZM_CUDA(cudaMemcpyAsync(ref[f], hin[f], f < 4 ? b3 : b2, cudaMemcpyHostToDevice, cs));
       ZM_CUDA(cudaEventRecord(ev[1 + f], cs));
     }
-    const dim3 c(32, 8);
     for (int f = 0; f < 5; ++f) {
       ZM_CUDA(cudaStreamWaitEvent(st, ev[1 + f], 0));
       if (f < 4) s->to_int3(st, ref[f], fin[f], offs[f]);
-      else k_ref_to_int2<<<s->grid2(c), c, 0, st>>>(s->d, ref[4], s->eta[s->cur]);
+      else launch_layout(st, s->d, LayoutArgs{{ref[4]}, {s->eta[s->cur]}, {0.f}, 0, 1}, true);
     }
     s->check_launch();
     int rc = zm_advance(s, stream, nsteps);
@@ -1561,7 +1559,7 @@ int zm_step_host(zm_solver* s, void* stream, const zm_state* in, zm_state* out, 
     float* fout[4] = {b.u, b.v, b.T, b.S};
     for (int f = 0; f < 5; ++f) {
       if (f < 4) s->to_ref3(st, fout[f], ref[f], offs[f]);
-      else k_int_to_ref2<<<s->grid2(c), c, 0, st>>>(s->d, s->eta[s->cur], ref[4]);
+      else launch_layout(st, s->d, LayoutArgs{{s->eta[s->cur]}, {ref[4]}, {0.f}, 0, 1}, false);
       ZM_CUDA(cudaEventRecord(ev[6 + f], st));
       ZM_CUDA(cudaStreamWaitEvent(cs, ev[6 + f], 0));
       ZM_CUDA(cudaMemcpyAsync(hout[f], ref[f], f < 4 ? b3 : b2, cudaMemcpyDeviceToHost, cs));
@@ -1734,9 +1732,7 @@ int zm_diagnostics(zm_solver* s, void* stream, const zm_state* in, const float* 
     launch_fz(st, s->d, s->L.u, s->L.v, s->Fz);
     k_diagnostics<<<s->grid2(c), c, 0, st>>>(s->d, s->L.T, s->L.S, s->frx, s->Fz, sp, s->W1.u, s->W1.v, s->W2.u);
     s->check_launch();
-    s->to_ref3(st, s->W1.u, rho, 0.f);
-    s->to_ref3(st, s->W1.v, pressure, 0.f);
-    s->to_ref3(st, s->W2.u, w, 0.f);
+    launch_layout(st, s->d, LayoutArgs{{s->W1.u, s->W1.v, s->W2.u}, {rho, pressure, w}, {}, 3, 0}, false);
     s->check_launch();
   } catch (const Err& e) {
     return fail(s, e);
@@ -1754,8 +1750,8 @@ int zm_tracer_terms(zm_solver* s, void* stream, const zm_state* in, float* terms
     launch_fz(st, s->d, s->L.u, s->L.v, s->Fz);
     launch_tracer_terms(st, s->d, s->L.T, s->L.S, s->L.u, s->L.v, s->Fz, s->W1.u, s->W1.v, s->W1.T, s->W1.S);
     s->check_launch();
-    const float* src[4] = {s->W1.u, s->W1.v, s->W1.T, s->W1.S};
-    for (int q = 0; q < 4; ++q) s->to_ref3(st, src[q], terms + q * nref, 0.f);
+    launch_layout(st, s->d, LayoutArgs{{s->W1.u, s->W1.v, s->W1.T, s->W1.S},
+                                       {terms, terms + nref, terms + 2 * nref, terms + 3 * nref}, {}, 4, 0}, false);
     s->check_launch();
     ZM_CUDA(cudaMemsetAsync(terms + 4 * nref, 0, 2 * nref * sizeof(float), st));  // GM, Redi: off
   } catch (const Err& e) {
