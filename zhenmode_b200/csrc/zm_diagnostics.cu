@@ -46,36 +46,67 @@ __global__ void __launch_bounds__(128) k_diagnostics(Dev d, const float* __restr
 
 // sums: 0 wet volume, 1 T volume, 2 S volume, 3 wet surface area,
 // 4 T_top surface area, 5 S_top surface area, 6 total cell area.
-__global__ void __launch_bounds__(256) k_budget_partials(Dev d, const float* __restrict__ T,
+__global__ void __launch_bounds__(256, 3) k_budget_partials(Dev d, const float* __restrict__ T,
                                                          const float* __restrict__ S,
                                                          const double* __restrict__ area,
                                                          const double* __restrict__ width,
                                                          double* __restrict__ partial) {
   __shared__ DD red[ZM_BUDGET_SUMS][8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long ncol = (long long)d.nx * d.ny;
+  const int ncol = d.nx * d.ny, step = gridDim.x * 8;
   DD acc[ZM_BUDGET_SUMS];
 #pragma unroll
   for (int q = 0; q < ZM_BUDGET_SUMS; ++q) acc[q] = DD{0.0, 0.0};
-  // one warp per column of the reference layout (nx, ny, nz): contiguous in z
-  for (long long col = (long long)blockIdx.x * 8 + warp; col < ncol; col += (long long)gridDim.x * 8) {
-    const int i = (int)(col / d.ny), j = (int)(col - (long long)i * d.ny);
-    const double a = area[col];
-    const uint64_t bits = __ldg(d.wbits + idx2(d, j, i));
-    const float* Tc = T + col * d.nz;
-    const float* Sc = S + col * d.nz;
-    for (int k = lane; k < d.nz; k += 32) {
-      const double vol = (a * width[k]) * (double)((bits >> k) & 1ull);
-      neumaier(acc[0], vol);
-      neumaier(acc[1], (double)Tc[k] * vol);
-      neumaier(acc[2], (double)Sc[k] * vol);
+  const double wd0 = lane < d.nz ? width[lane] : 0.0, wd1 = lane + 32 < d.nz ? width[lane + 32] : 0.0;
+  // One warp per column of the reference layout (nx, ny, nz), contiguous in z, BC of them in flight;
+  // the float64 additions are the bound (fp64 pipe 46 %).  720 x 360 x 50: 175 us with one column
+  // at a time and the surface sums on lane 0, 127 with four in flight (100 registers, two waves), 83 so.
+  constexpr int BC = 2;
+  for (int c0 = blockIdx.x * 8 + warp; c0 < ncol; c0 += BC * step) {
+    double a[BC];
+    float top[BC];
+    uint64_t bits[BC];
+    float t[BC][2], e[BC][2];
+#pragma unroll
+    for (int n = 0; n < BC; ++n) {
+      const int col = c0 + n * step;
+      a[n] = 0.0;
+      top[n] = 0.f;
+      bits[n] = 0ull;
+      t[n][0] = t[n][1] = e[n][0] = e[n][1] = 0.f;
+      if (col >= ncol) continue;
+      const int i = col / d.ny, j = col - i * d.ny;
+      a[n] = __ldg(area + col);
+      bits[n] = wb(d, j, i);
+      top[n] = __ldg(d.wet2 + idx2(d, j, i));
+      const long long o = (long long)col * d.nz + lane;
+      if (lane < d.nz) t[n][0] = __ldg(T + o), e[n][0] = __ldg(S + o);
+      if (lane + 32 < d.nz) t[n][1] = __ldg(T + o + 32), e[n][1] = __ldg(S + o + 32);
     }
-    if (lane == 0) {
-      const double sa = a * (double)__ldg(d.wet2 + idx2(d, j, i));
+#pragma unroll
+    for (int n = 0; n < BC; ++n) {  // past the last column: area and bits are zero
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const double vol = (a[n] * (h ? wd1 : wd0)) * (double)((bits[n] >> (lane + 32 * h)) & 1ull);
+        neumaier(acc[0], vol);
+        neumaier(acc[1], (double)t[n][h] * vol);
+        neumaier(acc[2], (double)e[n][h] * vol);
+      }
+    }
+    // the surface sums: lane n takes column n
+    double a1 = a[0];
+    float w1 = top[0], t1 = __shfl_sync(0xffffffffu, t[0][0], 0), e1 = __shfl_sync(0xffffffffu, e[0][0], 0);
+#pragma unroll
+    for (int n = 1; n < BC; ++n) {
+      const float tn = __shfl_sync(0xffffffffu, t[n][0], 0), en = __shfl_sync(0xffffffffu, e[n][0], 0);
+      if (lane == n) a1 = a[n], w1 = top[n], t1 = tn, e1 = en;
+    }
+    if (lane < BC) {
+      const double sa = a1 * (double)w1;
       neumaier(acc[3], sa);
-      neumaier(acc[4], (double)Tc[0] * sa);
-      neumaier(acc[5], (double)Sc[0] * sa);
-      neumaier(acc[6], a);
+      neumaier(acc[4], (double)t1 * sa);
+      neumaier(acc[5], (double)e1 * sa);
+      neumaier(acc[6], a1);
     }
   }
 #pragma unroll
@@ -93,14 +124,20 @@ __global__ void __launch_bounds__(256) k_budget_partials(Dev d, const float* __r
   }
 }
 
-__global__ void k_budget_final(const double* __restrict__ partial, int nblocks, double* __restrict__ out) {
-  const int q = threadIdx.x;
-  if (q >= ZM_BUDGET_SUMS) return;
+// One warp per sum: lanes take every 32nd partial, then a tree; one thread per sum
+// walked the 592 partials in 135 us.
+__global__ void __launch_bounds__(32 * ZM_BUDGET_SUMS) k_budget_final(const double* __restrict__ partial, int nblocks,
+                                                                      double* __restrict__ out) {
+  const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
   DD x{0.0, 0.0};
-  for (int b = 0; b < nblocks; ++b)
-    x = dd_add(x, DD{partial[(b * ZM_BUDGET_SUMS + q) * 2], partial[(b * ZM_BUDGET_SUMS + q) * 2 + 1]});
-  out[2 * q] = x.hi;
-  out[2 * q + 1] = x.lo;
+#pragma unroll 4
+  for (int b = lane; b < nblocks; b += 32)
+    x = dd_add(x, DD{__ldg(partial + (b * ZM_BUDGET_SUMS + q) * 2), __ldg(partial + (b * ZM_BUDGET_SUMS + q) * 2 + 1)});
+  for (int o = 16; o > 0; o >>= 1) x = dd_add(x, shfl_dd(x, o));
+  if (lane == 0) {
+    out[2 * q] = x.hi;
+    out[2 * q + 1] = x.lo;
+  }
 }
 
 }  // namespace zm

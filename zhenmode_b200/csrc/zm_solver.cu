@@ -1298,7 +1298,7 @@ void build(zm_solver* s, const zm_grid* g, const zm_params* p) {
     s->led_dzn = s->upload(width);
     int sms = 0;
     ZM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
-    s->bblocks = std::max(1, std::min(4 * sms, (int)(((long long)nx * ny + 7) / 8)));
+    s->bblocks = std::max(1, std::min(3 * sms, (int)(((long long)nx * ny + 7) / 8)));
     s->bpart = s->alloc<double>((size_t)s->bblocks * ZM_BUDGET_SUMS * 2);
     s->bout = s->alloc<double>(ZM_BUDGET_SUMS * 2);
   }
@@ -1766,7 +1766,7 @@ int zm_budgets(zm_solver* s, void* stream, const float* T, const float* S, doubl
   double sums[2 * ZM_BUDGET_SUMS];
   try {
     k_budget_partials<<<s->bblocks, 256, 0, st>>>(s->d, T, S, s->area64, s->width64, s->bpart);
-    k_budget_final<<<1, 32, 0, st>>>(s->bpart, s->bblocks, s->bout);
+    k_budget_final<<<1, 32 * ZM_BUDGET_SUMS, 0, st>>>(s->bpart, s->bblocks, s->bout);
     s->check_launch();
     ZM_CUDA(cudaMemcpyAsync(sums, s->bout, sizeof(sums), cudaMemcpyDeviceToHost, st));
     ZM_CUDA(cudaStreamSynchronize(st));
