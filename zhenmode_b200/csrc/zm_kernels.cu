@@ -751,136 +751,199 @@ void launch_lin_t(cudaStream_t s, const Dev& d, const float* usub, const float* 
 // Thomas algorithm in FP32 plus one step of iterative refinement, residual
 // formed in FP32 against the original right-hand side.  Rows below the
 // deepest wet level are untouched.
-__device__ __forceinline__ void vcoef(const Dev& d, int k, int kb, float s, float& a, float& b, float& c) {
-  a = 0.f; c = 0.f; b = 1.f;
-  if (k == 0) { b += s * d.vc.d2_top; c = -s * d.vc.d2_top; return; }
-  if (k == d.nz - 1) { a = -s * d.vc.d2_bot; b += s * d.vc.d2_bot; return; }
-  a = -s * d.vc.d2_lo[k];
-  b += s * (d.vc.d2_lo[k] + d.vc.d2_hi[k]);
-  if (k < kb) c = -s * d.vc.d2_hi[k]; else b -= s * d.vc.d2_hi[k];
-}
-
-// One thread per (column, field); lanes 2c and 2c+1 hold u and v (blockIdx.z
-// = 0: nu_v, node form of d2z with the ghost fill, then the land hold and the
-// exact Coriolis rotation, which swaps values within the lane pair) or T and S
-// (blockIdx.z = 1: kappa_v + coastal in the node form, or the learned
-// closure's diffusivity per interface kap3 in the interface-flux form, then
-// the land hold).  Each thread runs its own sequential Thomas sweeps (the two
-// fields of a pair repeat the same pivots).  The sweeps are latency-bound, so
-// the kernel is held to 32 registers for full occupancy: more independent
-// column chains in flight per SM outweigh a few spilled scalars and the
-// per-thread level arrays in local memory.  Passes over the n = kbot + 1 wet
-// levels:
+//
+// One thread per column and pair of fields that share the matrix: u and v
+// (blockIdx.z = 0: nu_v, node form of d2z with the ghost fill, then the land
+// hold and the exact Coriolis rotation) or T and S (blockIdx.z = 1: kappa_v +
+// coastal in the node form, or the learned closure's diffusivity per interface
+// kap3 in the interface-flux form, then the land hold).  Passes over the
+// n = kbot + 1 wet levels, each a serial chain along the column:
 //   1. forward elimination, keeping 1 / pivot;
 //   2. back substitution: the FP32 solution x;
-//   3. the residual r - A x (r read again) and its forward elimination;
+//   3. the residual r - A x and its forward elimination;
 //   4. back substitution of the correction e; x + e, hold, rotation, store.
-// The factor up / pivot is formed again where it is needed.
+// The factor up / pivot is formed again where it is needed.  A block is one
+// warp, its columns' r (later e), x and 1 / pivot in shared memory (20 bytes a
+// level and column, 24 with kap3: six or five blocks per SM at 50 levels), the
+// right-hand sides fetched by asynchronous copies all at once; a thread reads
+// back only what it wrote, so the kernel has no barrier.  Bound by the length of
+// the four chains at the six warps per SM that shared memory leaves (issue 38 %).
+// 800 x 400 x 50: 526 us a launch with one thread per column and field and the
+// levels in local memory, 252 so; 360 x 180 x 50 with kap3: 230 and 106.
 template <bool KAP>
-__global__ void __launch_bounds__(IV_T, 32) k_implicit_vdiff(Dev d, float* __restrict__ u, float* __restrict__ v,
-                                                        float* __restrict__ T, float* __restrict__ S,
-                                                        const float* __restrict__ u0, const float* __restrict__ v0,
-                                                        const float* __restrict__ T0, const float* __restrict__ S0,
-                                                        float dth, const float* __restrict__ kap3) {
-  const int f = threadIdx.x & 1;
-  const int i = blockIdx.x * (IV_T / 2) + (threadIdx.x >> 1);
-  const int j = blockIdx.y;
+__global__ void __launch_bounds__(32) k_implicit_vdiff(Dev d, float* __restrict__ u, float* __restrict__ v,
+                                                       float* __restrict__ T, float* __restrict__ S,
+                                                       const float* __restrict__ u0, const float* __restrict__ v0,
+                                                       float dth, const float* __restrict__ kap3) {
+  pdl_trigger();
+  extern __shared__ __align__(16) float2 iv_sm[];
+  const int lane = threadIdx.x, j = blockIdx.y;
+  const bool in = blockIdx.x * 32 + lane < d.nx;
+  const int i = in ? blockIdx.x * 32 + lane : d.nx - 1;
   const bool tracers = blockIdx.z == 1;
-  const bool in = i < d.nx;  // lanes past the last column run along (the pair exchange needs every lane) unstored
-  const long long base = idx2(d, j, in ? i : d.nx - 1);
-  float* __restrict__ fld = tracers ? (f ? S : T) : (f ? v : u);
-  const float* __restrict__ hold = tracers ? (f ? S0 : T0) : (f ? v0 : u0);
   const bool kap = KAP && tracers;  // the u, v blocks of a closure launch keep nu_v
-  const uint64_t bits = wb(d, j, in ? i : d.nx - 1);
+  const int base = idx2(d, j, i);
+  const uint64_t bits = wb(d, j, i);
   const int kb = kbot_of(bits);
-  const int n = kb > 0 && wetb(bits, 0) ? kb + 1 : 0;
+  const int n = in && kb > 0 && wetb(bits, 0) ? kb + 1 : 0;
+  // the warp's longest column: every loop runs all lanes over the same levels, so that they access whole lines
+  const int nm = __reduce_max_sync(0xffffffffu, n);
+  if (tracers && nm == 0) return;
+  float2* const e = iv_sm + lane;                                  // level k at [32 k]
+  float2* const x = e + 32 * d.nz;
+  float* const inv = reinterpret_cast<float*>(iv_sm + 64 * d.nz) + lane;
+  float* const kq = inv + 32 * d.nz;
+  float* fa = (tracers ? T : u) + base;
+  float* fb = (tracers ? S : v) + base;
+  const float *__restrict__ ha = u0 + base, *__restrict__ hb = v0 + base;
   const float sc = tracers ? __ldg(d.kv2 + base) * dth : d.nu_v * dth;
+  const float rc = tracers ? 0.f : __ldg(d.rot_c + base), rs = tracers ? 0.f : __ldg(d.rot_s + base);
   const long long pl = d.plane;
-  float x[ZM_MAXZ], inv[ZM_MAXZ], e[ZM_MAXZ], kq[KAP ? ZM_MAXZ : 1];
-  for (int k = 0; k < n; ++k) {
-    x[k] = fld[base + k * pl];
-    if (KAP && kap && k + 1 < n) kq[k] = __ldg(kap3 + base + k * pl);
+  pdl_wait();  // the fields and kap3 come from the preceding kernels
+  for (int k = 0; k < nm; ++k) {  // beyond a column's own system: what it keeps there
+    const bool own = tracers || k < n || wetb(bits, k);
+    if (tracers && k >= n) continue;
+    cp_async4(&e[32 * k].x, (own ? fa : ha) + k * pl);
+    cp_async4(&e[32 * k].y, (own ? fb : hb) + k * pl);
+    if (KAP && kap && k + 1 < n) cp_async4(&kq[32 * k], kap3 + base + k * pl);
   }
-  // tridiagonal row k: lower lo, diagonal dg, upper up
+  cp_async_commit();
+  auto store_uv = [&](int k, float a, float b) {
+    fa[k * pl] = rc * a + rs * b;
+    fb[k * pl] = -rs * a + rc * b;
+  };
+  if (!tracers && in) {  // levels below every system of the warp: held where dry (dry T, S are never read)
+    for (int k = nm; k < d.nz; k += 8) {
+      float a[8], b[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        if (k + q >= d.nz) continue;
+        const bool wet = wetb(bits, k + q);
+        a[q] = *((wet ? fa : ha) + (k + q) * pl);
+        b[q] = *((wet ? fb : hb) + (k + q) * pl);
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (k + q < d.nz) store_uv(k + q, a[q], b[q]);
+    }
+  }
+  cp_async_wait<0>();
+  // Tridiagonal row k <= kb: lower lo, diagonal dg, upper up (lo = 0 in row 0, up = 0 in row kb).  Lanes
+  // whose column ends above k run along; nothing of theirs at k > kb goes back up.
   auto row = [&](int k, float& lo, float& dg, float& up) {
     if (KAP && kap) {
-      lo = k > 0 ? -dth * kq[k - 1] * d.vc.inv_dz_iface[k - 1] * d.vc.inv_dz_node[k] : 0.f;
-      up = k + 1 < n ? -dth * kq[k] * d.vc.inv_dz_iface[k] * d.vc.inv_dz_node[k] : 0.f;
+      lo = k > 0 ? -dth * kq[32 * (k - 1)] * d.vc.inv_dz_iface[k - 1] * d.vc.inv_dz_node[k] : 0.f;
+      up = k < kb ? -dth * kq[32 * k] * d.vc.inv_dz_iface[k] * d.vc.inv_dz_node[k] : 0.f;
       dg = 1.f - lo - up;
     } else {
-      vcoef(d, k, kb, sc, lo, dg, up);
+      const float dl = d.vc.d2_lo[k], dh = d.vc.d2_hi[k];
+      lo = -sc * dl;
+      dg = 1.f + sc * (dl + dh);
+      up = -sc * dh;
+      if (k >= kb) {
+        dg += up;
+        up = 0.f;
+      }
     }
   };
-  // 1. forward elimination (lo = 0 in row 0, so its pivot is dg)
+  // 1. forward elimination
   {
-    float cpp = 0.f, y = 0.f;
-    for (int k = 0; k < n; ++k) {
+    float cpp = 0.f, ya = 0.f, yb = 0.f;
+#pragma unroll 4
+    for (int k = 0; k < nm; ++k) {
       float lo, dg, up;
       row(k, lo, dg, up);
+      const float2 r = e[32 * k];
       const float iv = 1.f / (dg - lo * cpp);
       cpp = up * iv;
-      y = (x[k] - lo * y) * iv;
-      x[k] = y;
-      inv[k] = iv;
+      ya = (r.x - lo * ya) * iv;
+      yb = (r.y - lo * yb) * iv;
+      x[32 * k] = make_float2(ya, yb);
+      inv[32 * k] = iv;
     }
   }
   // 2. back substitution
-  for (int k = n - 2; k >= 0; --k) {
-    float lo, dg, up;
-    row(k, lo, dg, up);
-    x[k] -= (up * inv[k]) * x[k + 1];
+  {
+    float2 xn = make_float2(0.f, 0.f);
+#pragma unroll 4
+    for (int k = nm - 1; k >= 0; --k) {
+      float lo, dg, up;
+      row(k, lo, dg, up);
+      const float c = up * inv[32 * k];
+      float2 y = x[32 * k];
+      if (k < kb) {
+        y.x -= c * xn.x;
+        y.y -= c * xn.y;
+      }
+      x[32 * k] = xn = y;
+    }
   }
   // 3. residual of the FP32 solution, eliminated with the same factorization
   {
-    float ep = 0.f, xm = 0.f, x0 = n > 0 ? x[0] : 0.f;
-    for (int k = 0; k < n; ++k) {
+    float2 ep = make_float2(0.f, 0.f), xm = ep, x0 = nm > 0 ? x[0] : ep;
+#pragma unroll 4
+    for (int k = 0; k < nm; ++k) {
       float lo, dg, up;
       row(k, lo, dg, up);
-      const float xp = k + 1 < n ? x[k + 1] : 0.f;
-      float a = dg * x0;
-      if (k > 0) a += lo * xm;
-      if (k + 1 < n) a += up * xp;
-      ep = ((fld[base + k * pl] - a) - lo * ep) * inv[k];
-      e[k] = ep;
+      const float2 xp = k < kb ? x[32 * (k + 1)] : make_float2(0.f, 0.f);
+      const float2 r = e[32 * k];
+      const float iv = inv[32 * k];
+      float2 a = make_float2(dg * x0.x, dg * x0.y);
+      if (k > 0) {
+        a.x += lo * xm.x;
+        a.y += lo * xm.y;
+      }
+      a.x += up * xp.x;
+      a.y += up * xp.y;
+      ep.x = ((r.x - a.x) - lo * ep.x) * iv;
+      ep.y = ((r.y - a.y) - lo * ep.y) * iv;
+      if (k < n) e[32 * k] = ep;
       xm = x0;
       x0 = xp;
     }
   }
   // 4. back substitution of the correction; x + e, land hold, rotation
-  const float rc = tracers ? 0.f : __ldg(d.rot_c + base), rs = tracers ? 0.f : __ldg(d.rot_s + base);
-  float en = 0.f;
-  for (int k = (tracers ? n : d.nz) - 1; k >= 0; --k) {  // dry T, S are never read (u, v: every lane runs all levels)
-    const long long id = base + k * pl;
-    const bool wet = wetb(bits, k);
-    float val = 0.f;
+  if (!in) return;
+  fa += (nm - 1) * pl;
+  fb += (nm - 1) * pl;
+  float2 en = make_float2(0.f, 0.f);
+#pragma unroll 4
+  for (int k = nm - 1; k >= 0; --k, fa -= pl, fb -= pl) {
+    float lo, dg, up;
+    row(k, lo, dg, up);
+    const float c = up * inv[32 * k];
+    const float2 xk = x[32 * k];
+    float2 o = e[32 * k];
     if (k < n) {
-      float ek = e[k];
-      if (k + 1 < n) {
-        float lo, dg, up;
-        row(k, lo, dg, up);
-        ek -= (up * inv[k]) * en;
+      if (k < kb) {
+        o.x -= c * en.x;
+        o.y -= c * en.y;
       }
-      en = ek;
-      val = x[k] + ek;
-    } else if (!tracers && wet) {
-      val = fld[id];
+      en = o;
+      o.x = xk.x + o.x;
+      o.y = xk.y + o.y;
     }
-    if (!wet) val = ld(hold, id);
+    const bool wet = wetb(bits, k);
     if (tracers) {
-      if (in && wet) fld[id] = val;
+      if (wet && k < n) {
+        *fa = o.x;
+        *fb = o.y;
+      }
     } else {
-      const float other = __shfl_xor_sync(0xffffffffu, val, 1);
-      const float uu = f ? other : val, vv = f ? val : other;
-      if (in) fld[id] = f ? -rs * uu + rc * vv : rc * uu + rs * vv;
+      if (!wet && k < n) o = make_float2(ld(ha, k * pl), ld(hb, k * pl));  // a dry level between wet ones
+      *fa = rc * o.x + rs * o.y;
+      *fb = -rs * o.x + rc * o.y;
     }
   }
 }
 
-void launch_implicit_vdiff(cudaStream_t s, const Dev& d, float* u, float* v, float* T, float* S, const float* u0,
-                           const float* v0, const float* T0, const float* S0, float dth, const float* kap3) {
-  const dim3 g((d.nx + IV_T / 2 - 1) / (IV_T / 2), d.ny, 2);
-  if (kap3) k_implicit_vdiff<true><<<g, IV_T, 0, s>>>(d, u, v, T, S, u0, v0, T0, S0, dth, kap3);
-  else k_implicit_vdiff<false><<<g, IV_T, 0, s>>>(d, u, v, T, S, u0, v0, T0, S0, dth, kap3);
+cudaError_t launch_implicit_vdiff(cudaStream_t s, const Dev& d, float* u, float* v, float* T, float* S,
+                                  const float* u0, const float* v0, float dth, const float* kap3) {
+  const dim3 g((d.nx + 31) / 32, d.ny, 2);
+  const size_t sm = (size_t)32 * d.nz * (kap3 ? 24 : 20);
+  static_assert(32 * ZM_MAXZ * 24 <= 48 * 1024, "columns within the default dynamic shared memory");
+  if (kap3) return launch_pdl(k_implicit_vdiff<true>, g, dim3(32), sm, s, d, u, v, T, S, u0, v0, dth, kap3);
+  return launch_pdl(k_implicit_vdiff<false>, g, dim3(32), sm, s, d, u, v, T, S, u0, v0, dth, kap3);
 }
 
 // ------------------------------------------------------------------ transport

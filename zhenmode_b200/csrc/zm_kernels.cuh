@@ -165,10 +165,8 @@ __global__ void k_nu_gates(Dev d, unsigned char* gate);
 void launch_lin_t(cudaStream_t s, const Dev& d, const float* usub, const float* vsub, const float* u0,
                   const float* v0, const float* T0, const float* S0, float* uo, float* vo, float* To, float* So,
                   float dth, int implicit_v);
-// threads per block of k_implicit_vdiff (two per column) and its launch
-constexpr int IV_T = 64;
-void launch_implicit_vdiff(cudaStream_t s, const Dev& d, float* u, float* v, float* T, float* S, const float* u0,
-                           const float* v0, const float* T0, const float* S0, float dth, const float* kap3);
+cudaError_t launch_implicit_vdiff(cudaStream_t s, const Dev& d, float* u, float* v, float* T, float* S,
+                                  const float* u0, const float* v0, float dth, const float* kap3);
 void launch_fz(cudaStream_t s, const Dev& d, const float* u, const float* v, float* Fz);
 void launch_tracer_terms(cudaStream_t s, const Dev& d, const float* T, const float* S, const float* u,
                          const float* v, const float* Fz, float* adv, float* dh, float* dv, float* conv);

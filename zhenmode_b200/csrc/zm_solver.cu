@@ -265,8 +265,7 @@ struct zm_solver {
     pe(s);
     if (vdiff || closure_on) {
       pb(ZM_K_IMPLICIT, s);
-      launch_implicit_vdiff(s, d, dst.u, dst.v, dst.T, dst.S, src.u, src.v, src.T, src.S, dth,
-                            closure_on ? kappa3 : nullptr);
+      ZM_CUDA(launch_implicit_vdiff(s, d, dst.u, dst.v, dst.T, dst.S, src.u, src.v, dth, closure_on ? kappa3 : nullptr));
       pe(s);
     }
     if (ledger_on) led_stage(s, 0, src.T, src.S, nullptr, dst.T, dst.S, nullptr);  // step.py:138-140
@@ -981,6 +980,10 @@ void build(zm_solver* s, const zm_grid* g, const zm_params* p) {
   vc.ddz_inv[nz - 1] = (float)(1.0 / (z[nz - 1] - z[nz - 2]));
   vc.d2_top = (float)(2.0 / (gap[0] * gap[0]));
   vc.d2_bot = (float)(2.0 / (gap[nz - 2] * gap[nz - 2]));
+  // the end rows in the interior form
+  vc.d2_lo[0] = vc.d2_hi[nz - 1] = 0.f;
+  vc.d2_hi[0] = vc.d2_top;
+  vc.d2_lo[nz - 1] = vc.d2_bot;
   // ---- polar cap weights (numerics/horizontal.py:362-385), pole-inward
   std::vector<float> w(std::max(nb, 1), 0.f);
   for (int r = 0; r < p->polar_cap_rows; ++r) w[r] = 1.f;
