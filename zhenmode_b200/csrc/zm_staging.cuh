@@ -1,0 +1,216 @@
+// Host copies of a state that lives in ordinary (pageable) memory.
+//
+// The driver stages a pageable copy itself, on the calling thread, at the speed of
+// one core's memcpy, and the first touch of a fresh result array (page faults and
+// their zeroing) falls into the same serial copy.  Here several threads stage the
+// chunks through pinned slots of their own, two each, so that a thread fills or
+// empties one slot while the other is on the bus, and they let the kernel map the
+// result's pages while the device computes.  A whole host step: 31 MB of state
+// 12.4 -> 3.7 ms, 207 MB 69.5 -> 22.4 ms, 1 MB 0.67 -> 0.55 ms (six threads; chunks
+// of 256 KB 4.4 and 27.0 ms).
+#pragma once
+
+#include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
+
+#include <algorithm>
+#include <atomic>
+#include <condition_variable>
+#include <cstdint>
+#include <cstring>
+#include <mutex>
+#include <system_error>
+#include <thread>
+#include <vector>
+
+namespace zm {
+
+class HostStage {
+ public:
+  struct Piece {
+    char* host;
+    char* dev;
+    size_t bytes;
+  };
+  static constexpr size_t CHUNK = 512 << 10;
+  static constexpr int MAX_WORKERS = 6;
+
+  HostStage() = default;
+  HostStage(const HostStage&) = delete;
+  HostStage& operator=(const HostStage&) = delete;
+  ~HostStage() {
+    for (auto& w : ev_)
+      for (cudaEvent_t e : w)
+        if (e) cudaEventDestroy(e);
+    if (pin_) cudaFreeHost(pin_);
+  }
+
+  // Whether every array is pageable host memory that the driver knows nothing of.
+  static bool pageable(const void* const* p, int n) {
+    for (int q = 0; q < n; ++q) {
+      cudaPointerAttributes a{};
+      if (cudaPointerGetAttributes(&a, p[q]) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+      }
+      if (a.type != cudaMemoryTypeUnregistered) return false;
+    }
+    return true;
+  }
+
+  // Pinned slots and events, kept with the solver; false where they cannot be had.
+  bool ready() {
+    if (pin_) return true;
+    workers_ = std::max(1, std::min(MAX_WORKERS, (int)std::thread::hardware_concurrency() / 2));
+    if (cudaHostAlloc(reinterpret_cast<void**>(&pin_), 2 * CHUNK * workers_, cudaHostAllocDefault) != cudaSuccess) {
+      (void)cudaGetLastError();
+      pin_ = nullptr;
+      return false;
+    }
+    for (int w = 0; w < workers_; ++w)
+      for (cudaEvent_t& e : ev_[w])
+        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+          (void)cudaGetLastError();
+          cudaFreeHost(pin_);
+          pin_ = nullptr;
+          return false;
+        }
+    return true;
+  }
+
+  // in -> device on `cs`; then compute(), which queues the work and makes `cs` wait for it and returns
+  // whether to go on; then device -> out.  Returns the first CUDA error of the copies; on any return
+  // nothing of this call is in flight on `cs` any more.
+  template <class Compute>
+  cudaError_t run(int device, cudaStream_t cs, const std::vector<Piece>& in, const std::vector<Piece>& out,
+                  Compute&& compute) {
+    Job job{device, cs, chunks(in), chunks(out)};
+    std::vector<std::thread> team;
+    try {
+      team.reserve(workers_ - 1);
+      for (int w = 1; w < workers_; ++w)
+        team.emplace_back([this, &job, w] {
+          note(job, cudaSetDevice(job.device));
+          upload(job, w);
+          populate(job);
+          {
+            std::unique_lock<std::mutex> lock(job.m);
+            job.turn.wait(lock, [&job] { return job.phase.load() != 0; });
+          }
+          if (job.phase.load() == 1) download(job, w);
+        });
+    } catch (...) {  // fewer threads, or none, do the same work
+    }
+    bool go = false;
+    try {
+      upload(job, 0);
+      while (job.sent.load(std::memory_order_acquire) < job.up.size() && !job.err.load()) std::this_thread::yield();
+      go = !job.err.load() && compute();
+    } catch (...) {
+      finish(job, team);
+      throw;
+    }
+    if (go) {
+      note(job, cudaStreamSynchronize(cs));  // one thread waits for the device; the others sleep
+      begin(job, 1);
+      download(job, 0);
+    }
+    finish(job, team);
+    return (cudaError_t)job.err.load();
+  }
+
+ private:
+  struct Job {
+    int device;
+    cudaStream_t cs;
+    std::vector<Piece> up, down;
+    std::atomic<size_t> next_up{0}, sent{0}, next_page{0}, next_down{0};
+    std::atomic<int> phase{0};  // 1: the results may be fetched, 2: there are none
+    std::atomic<int> err{0};
+    std::mutex m;
+    std::condition_variable turn;
+    Job(int dv, cudaStream_t s, std::vector<Piece> u, std::vector<Piece> d)
+        : device(dv), cs(s), up(std::move(u)), down(std::move(d)) {}
+  };
+
+  static std::vector<Piece> chunks(const std::vector<Piece>& fields) {
+    std::vector<Piece> c;
+    for (const Piece& f : fields)
+      for (size_t o = 0; o < f.bytes; o += CHUNK) c.push_back({f.host + o, f.dev + o, std::min(CHUNK, f.bytes - o)});
+    return c;
+  }
+  static void note(Job& job, cudaError_t e) {
+    int none = 0;
+    if (e != cudaSuccess) job.err.compare_exchange_strong(none, (int)e);
+  }
+  char* slot(int w, int s) const { return pin_ + (size_t)(2 * w + s) * CHUNK; }
+
+  void upload(Job& job, int w) {
+    bool used[2] = {false, false};
+    int s = 0;
+    for (size_t c; !job.err.load() && (c = job.next_up.fetch_add(1)) < job.up.size(); s ^= 1) {
+      const Piece& p = job.up[c];
+      if (used[s]) note(job, cudaEventSynchronize(ev_[w][s]));
+      std::memcpy(slot(w, s), p.host, p.bytes);
+      note(job, cudaMemcpyAsync(p.dev, slot(w, s), p.bytes, cudaMemcpyHostToDevice, job.cs));
+      note(job, cudaEventRecord(ev_[w][s], job.cs));
+      used[s] = true;
+      job.sent.fetch_add(1, std::memory_order_release);
+    }
+    for (int q = 0; q < 2; ++q)
+      if (used[q]) note(job, cudaEventSynchronize(ev_[w][q]));
+  }
+
+  // Maps the whole pages of the results; their contents stay as they are, and where the system knows no
+  // such request the download faults them in.
+  void populate(Job& job) {
+#ifdef MADV_POPULATE_WRITE
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    for (size_t c; job.phase.load() == 0 && (c = job.next_page.fetch_add(1)) < job.down.size();) {
+      const uintptr_t a = ((uintptr_t)job.down[c].host + page - 1) / page * page;
+      const uintptr_t b = ((uintptr_t)job.down[c].host + job.down[c].bytes) / page * page;
+      if (b > a && madvise(reinterpret_cast<void*>(a), b - a, MADV_POPULATE_WRITE) != 0) return;
+    }
+#else
+    (void)job;
+#endif
+  }
+
+  void download(Job& job, int w) {
+    const Piece* pending = nullptr;
+    int s = 0;
+    for (;;) {
+      const size_t c = job.err.load() ? job.down.size() : job.next_down.fetch_add(1);
+      const Piece* p = c < job.down.size() ? &job.down[c] : nullptr;
+      if (p) {
+        note(job, cudaMemcpyAsync(slot(w, s), p->dev, p->bytes, cudaMemcpyDeviceToHost, job.cs));
+        note(job, cudaEventRecord(ev_[w][s], job.cs));
+      }
+      if (pending) {
+        note(job, cudaEventSynchronize(ev_[w][s ^ 1]));
+        if (!job.err.load()) std::memcpy(pending->host, slot(w, s ^ 1), pending->bytes);
+      }
+      pending = p;
+      if (!p) return;
+      s ^= 1;
+    }
+  }
+
+  static void begin(Job& job, int phase) {
+    std::lock_guard<std::mutex> lock(job.m);
+    job.phase.store(phase);
+    job.turn.notify_all();
+  }
+  void finish(Job& job, std::vector<std::thread>& team) {
+    if (job.phase.load() == 0) begin(job, 2);
+    for (std::thread& t : team) t.join();
+    note(job, cudaStreamSynchronize(job.cs));
+  }
+
+  char* pin_ = nullptr;
+  int workers_ = 1;
+  cudaEvent_t ev_[MAX_WORKERS][2] = {};
+};
+
+}  // namespace zm
