@@ -1533,10 +1533,13 @@ void launch_tracer_terms(cudaStream_t s, const Dev& d, const float* T, const flo
 // Tracer residual of the N step (dynamics/tendencies.py:94-245) without the
 // diffusion pair that the residual adds and removes again: mean advection
 // rate + interface-flux convective mixing (physics/vertical.py:13-37, 63-82)
-// + surface sources at k = 0.  One column per thread.
+// + surface sources at k = 0.  TR_K threads per column, each a run of its levels:
+// only the gates need the whole column, one bit per interface, exchanged in shared
+// memory.  Bound by memory latency: one thread per column took 32 us a launch at
+// 180 x 90 x 50 and 117 at 720 x 360 x 50, four take 15 and 101.
 //   stage 1: dT1 = r(T1), Tp = T1 + dt dT1
 //   stage 2: T2 = T1 + dt (dT1 + r(Tp)) / 2
-
+constexpr int TR_Y = 2, TR_K = 4;
 
 __device__ __forceinline__ void rest_store(const Dev& d, const RestArgs& a, long long id, long long base, int k,
                                            float w, float rT, float rS) {
@@ -1562,44 +1565,57 @@ __device__ __forceinline__ void rest_store(const Dev& d, const RestArgs& a, long
 }
 
 template <bool ST2>
-__global__ void __launch_bounds__(128) k_tracer_rest(Dev d, RestArgs a) {
+__global__ void __launch_bounds__(32 * TR_Y * TR_K) k_tracer_rest(Dev d, RestArgs a) {
   pdl_trigger();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= d.nx || j >= d.ny) return;
-  const long long base = idx2(d, j, i);
-  const uint64_t bits = wb(d, j, i);
+  __shared__ unsigned long long gate[TR_K][TR_Y][32];
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * TR_Y + threadIdx.y, kg = threadIdx.z;
+  const bool in = i < d.nx && j < d.ny;
+  const long long base = in ? idx2(d, j, i) : 0;
+  const uint64_t bits = in ? wb(d, j, i) : 0ull;
   const int nz = levels_of(bits);  // dry levels below keep their values: nothing reads them
+  // this thread's levels k0 .. k1 - 1, the same for the 32 columns of the warp
+  const int share = (__reduce_max_sync(0xffffffffu, nz) + TR_K - 1) / TR_K;
+  const int k0 = kg * share, k1 = min(nz, k0 + share);
   pdl_wait();  // the evaluation state and the advection rates come from the preceding kernels
-  if (nz == 0) return;
   // static-instability gates of the evaluation state, in difference form:
   // rho[m] > rho[m+1]  <=>  beta (S[m]-S[m+1]) > alpha (T[m]-T[m+1]).
-  uint64_t unstable = 0ull, wetpair = 0ull;
-  float Tu = ld(a.Tev, base), Su = ld(a.Sev, base);
+  const uint64_t wetpair = bits & (bits >> 1);
+  uint64_t unstable = 0ull;
+  if (k0 < k1) {
+    float Tu = ld(a.Tev, base + (long long)k0 * d.plane), Su = ld(a.Sev, base + (long long)k0 * d.plane);
 #pragma unroll 8
-  for (int m = 0; m + 1 < nz; ++m) {
-    const long long idn = base + (long long)(m + 1) * d.plane;
-    const float Tl = ld(a.Tev, idn), Sl = ld(a.Sev, idn);
-    if (wetb(bits, m) && wetb(bits, m + 1)) {
-      wetpair |= 1ull << m;
+    for (int m = k0; m < k1 && m + 1 < nz; ++m) {
+      const long long idn = base + (long long)(m + 1) * d.plane;
+      const float Tl = ld(a.Tev, idn), Sl = ld(a.Sev, idn);
       if (kBeta * (Su - Sl) > kAlpha * (Tu - Tl)) unstable |= 1ull << m;
+      Tu = Tl;
+      Su = Sl;
     }
-    Tu = Tl;
-    Su = Sl;
   }
+  gate[kg][threadIdx.y][threadIdx.x] = unstable;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < TR_K; ++q) unstable |= gate[q][threadIdx.y][threadIdx.x];
+  unstable &= wetpair;
   uint64_t allow = 0ull;
   if (unstable && d.kappa_conv > 0.f && !a.no_conv) allow = d.localize_conv ? unstable : wetpair;
   if (a.nc == 1 || allow == 0ull) {
+    if (k0 >= k1) return;
     const float kc = d.kappa_conv;
-    float fT = 0.f, fS = 0.f;
-    float cT = ld(a.Tev, base), cS = ld(a.Sev, base);
+    const long long top = base + (long long)k0 * d.plane;
+    float fT = 0.f, fS = 0.f;  // convective flux through the interface above
+    float cT = ld(a.Tev, top), cS = ld(a.Sev, top);
+    if (k0 > 0 && ((allow >> (k0 - 1)) & 1ull)) {
+      fT = -kc * (cT - ld(a.Tev, top - d.plane)) * d.vc.inv_dz_iface[k0 - 1];
+      fS = -kc * (cS - ld(a.Sev, top - d.plane)) * d.vc.inv_dz_iface[k0 - 1];
+    }
     // the next level's inputs are loaded before this level's stores: the
     // argument pointers may alias, so loads issued after a store would wait
     constexpr bool st2 = ST2;  // stage 2 reads the stage-1 tendency
-    float qaT = ld(a.accT, base), qaS = ld(a.accS, base), qbT = ld(a.Tbase, base), qbS = ld(a.Sbase, base);
-    float qdT = st2 ? ld(a.dT1, base) : 0.f, qdS = st2 ? ld(a.dS1, base) : 0.f;
+    float qaT = ld(a.accT, top), qaS = ld(a.accS, top), qbT = ld(a.Tbase, top), qbS = ld(a.Sbase, top);
+    float qdT = st2 ? ld(a.dT1, top) : 0.f, qdS = st2 ? ld(a.dS1, top) : 0.f;
 #pragma unroll 2
-    for (int k = 0; k < nz; ++k) {
+    for (int k = k0; k < k1; ++k) {
       const long long id = base + (long long)k * d.plane;
       float nT = 0.f, nS = 0.f, gT = 0.f, gS = 0.f;
       float naT = 0.f, naS = 0.f, nbT = 0.f, nbS = 0.f, ndT = 0.f, ndS = 0.f;
@@ -1653,7 +1669,8 @@ __global__ void __launch_bounds__(128) k_tracer_rest(Dev d, RestArgs a) {
     }
     return;
   }
-  // several convective substeps (legacy: kappa and time both divided by nc)
+  if (kg != 0) return;
+  // several convective substeps (legacy: kappa and time both divided by nc): the column is one chain
   float cT[ZM_MAXZ], cS[ZM_MAXZ], sT[ZM_MAXZ], sS[ZM_MAXZ];
   for (int k = 0; k < nz; ++k) {
     cT[k] = ld(a.Tev, base + (long long)k * d.plane);
@@ -1697,7 +1714,8 @@ __global__ void __launch_bounds__(128) k_tracer_rest(Dev d, RestArgs a) {
 }
 
 // The RK stage is a template argument (stage 2 also reads dT1, dS1).
-void launch_tracer_rest(dim3 g, dim3 b, cudaStream_t s, const Dev& d, const RestArgs& a) {
+void launch_tracer_rest(cudaStream_t s, const Dev& d, const RestArgs& a) {
+  const dim3 b(32, TR_Y, TR_K), g((d.nx + 31) / 32, (d.ny + TR_Y - 1) / TR_Y);
   (void)launch_pdl(a.stage == 1 ? k_tracer_rest<false> : k_tracer_rest<true>, g, b, 0, s, d, a);
 }
 

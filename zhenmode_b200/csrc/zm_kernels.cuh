@@ -183,7 +183,7 @@ bool fft_reg_split(int n, int& r1, int& r2, int& r3);
 void launch_tracer_adv(cudaStream_t s, const Dev& d, const float* T, const float* S, const float* u, const float* v,
                        const float* Fz, float* accT, float* accS, float* Tn, float* Sn, float dts, int first, int last,
                        float* topT, float* topS);
-void launch_tracer_rest(dim3 g, dim3 b, cudaStream_t s, const Dev& d, const RestArgs& a);
+void launch_tracer_rest(cudaStream_t s, const Dev& d, const RestArgs& a);
 void launch_pgf(cudaStream_t s, const Dev& d, const PgfArgs& a);
 __global__ void k_bt_forcing(Dev d, const float* frx, const float* fry, double* Fx, double* Fy, const float* eta32,
                              double* eta64);

@@ -305,9 +305,8 @@ struct zm_solver {
     }
     RestArgs a{T, S, accT, accS, Tbase, Sbase, dT1, dS1, To, So, (float)dt, 1.f / (float)adv_nsub, conv_nsub, stage,
                closure_on ? 1 : 0, ledger_on ? led_convT : nullptr, ledger_on ? led_convS : nullptr};
-    const dim3 c(32, 4);
     pb(ZM_K_TRACER_REST, s);
-    launch_tracer_rest(grid2(c), c, s, d, a);
+    launch_tracer_rest(s, d, a);
     pe(s);
     check_launch();
     if (ledger_on) led_rk(s, T, S);  // tendencies.py:211-214
