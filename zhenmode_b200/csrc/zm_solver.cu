@@ -686,11 +686,11 @@ struct zm_solver {
       };
       const float dts = (float)(dt / adv_nsub);
       launch_fz(s, d, in.u, in.v, Fz);
-      tune(d.ta_kc, {5, 8, 10, 13, 17, 25}, [&] {
+      tune(d.ta_kc, {2, 3, 5, 8, 10, 13, 17, 25}, [&] {
         launch_tracer_adv(s, d, in.T, in.S, in.u, in.v, Fz, accT, accS, TsA, SsA, dts, 1, 0, nullptr, nullptr);
       });
       const float dth = (float)(dt / 2.0);
-      tune(d.lt_kc, {5, 8, 10, 13, 17, 25}, [&] {
+      tune(d.lt_kc, {2, 3, 5, 8, 10, 13, 17, 25}, [&] {
         launch_lin_t(s, d, in.u, in.v, in.u, in.v, in.T, in.S, s1.u, s1.v, s1.T, s1.S, dth, vdiff || closure_on);
       });
       tune(d.fz_rows, {4, 8}, [&] { launch_fz(s, d, in.u, in.v, Fz); });
@@ -898,8 +898,18 @@ void build(zm_solver* s, const zm_grid* g, const zm_params* p) {
     if (lines.empty()) lines.push_back(0);
     plan.lines = s->upload(lines);
   }
-  d.ta_kc = 10;
-  d.lt_kc = 10;
+  int sms = 0;
+  ZM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
+  {
+    // Levels per block of the tracer-advection and linear-finish marches (one tile shape): ten, which spread a block's
+    // first loads best, unless that leaves fewer than eight blocks per SM (two waves); then as many as
+    // give eight, down to two.  Per step at 90 x 45 x 15: 113 us with ten, 90 with two; 180 x 90 x 50:
+    // 488 with ten, 443 with six (four blocks per SM), 412 with three (eight).
+    const long long tiles = (long long)((nx + TA_X - 1) / TA_X) * ((ny + TA_Y - 1) / TA_Y);
+    int kc = 10;
+    while (kc > 2 && tiles * ((nz + kc - 1) / kc) < 8ll * sms) --kc;
+    d.ta_kc = d.lt_kc = kc;
+  }
   d.pg_rows = 4;
   d.fz_rows = 4;
   {
@@ -1039,7 +1049,11 @@ void build(zm_solver* s, const zm_grid* g, const zm_params* p) {
     plan.tw_full = s->upload(tw);
   }
   s->fft = plan;
+  // Lines per block of the filter: four, fewer where shared memory or the number of lines (eight blocks
+  // per SM) asks for it.  90 x 45 x 15: the filter takes 15 us with four lines, 12 with one;
+  // 450 x 219 x 37: 1.131 ms a step with four, 1.139 with two, 1.158 with one.
   s->fft_lines = std::max(1, std::min(4, (int)((200 * 1024 / sizeof(float2)) / (2 * nx))));
+  while (s->fft_lines > 1 && plan.nlines / s->fft_lines < 8 * sms) s->fft_lines /= 2;
   s->fft_smem = (size_t)2 * s->fft_lines * nx * sizeof(float2);
   require(s->fft_smem <= 227 * 1024, ZM_ERR_UNSUPPORTED, "nx too large for the shared-memory FFT filter");
   {
