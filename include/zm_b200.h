@@ -56,10 +56,11 @@ typedef struct {
   const double* wet_mask_3d;  /* (nx, ny, nz) or NULL: column-uniform from wet_mask */
 } zm_grid;
 
-/* Barotropic subcycle kernels: AUTO takes the resident kernel (every tile in
- * shared memory, one cooperative launch) when all tiles fit on the GPU at
- * once and the streaming kernels (three launches per subcycle) otherwise;
- * RESIDENT fails zm_create with ZM_ERR_UNSUPPORTED when they do not fit. */
+/* Barotropic subcycle kernels: AUTO takes the resident kernel (one tile per SM,
+ * one cooperative launch) when the tiles fit and the streaming kernels (three
+ * launches per subcycle) otherwise; RESIDENT fails zm_create with
+ * ZM_ERR_UNSUPPORTED when they do not fit or the grid has more than four
+ * 32 x 16 tiles per SM. */
 #define ZM_BT_AUTO 0
 #define ZM_BT_RESIDENT 1
 #define ZM_BT_STREAMING 2
