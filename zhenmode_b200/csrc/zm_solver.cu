@@ -204,28 +204,24 @@ struct zm_solver {
     if (e != cudaSuccess) throw Err{ZM_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e)};
   }
 
-  // Set the nu_h launch shape and form its strip classes.  Runs at creation and
-  // between the autotuner's trials; waits, so that any stream sees the table.
-  unsigned char* nu_class_buf = nullptr;
+  // Set the nu_h launch shape.  Its strip classes are formed on the shape's first
+  // use (at creation, between the autotuner's trials) and kept as they are: a
+  // captured step holds its shape and the table of that shape, also after the
+  // tuner has picked another one (an ensemble's graphs outlive its members' tuning).
+  unsigned char* nu_tables[2][NB_T + 1] = {};  // [8 or 16 warps][halo]
   void set_nu_shape(int halo, int warps) {
     nu_halo = halo;
     nu_warps = warps;
-    if (!nu_class_buf) {
-      size_t most = 0;
-      for (int w : {8, 16})
-        for (int h = 3; h <= NB_T; ++h) {
-          const dim3 g = nu_grid(d, w, h);
-          most = std::max(most, (size_t)g.x * g.y * g.z * w);
-        }
-      nu_class_buf = alloc<unsigned char>(most);
-      d.nu_class = nu_class_buf;
+    unsigned char*& table = nu_tables[warps == 16][halo];
+    if (!table) {
+      const dim3 g = nu_grid(d, warps, halo);
+      const unsigned strips = g.x * g.y * g.z * warps;
+      table = alloc<unsigned char>(strips);
+      k_nu_class<<<(strips + 7) / 8, dim3(32, 8)>>>(d, table, warps, halo, (int)g.x, (int)g.y);
+      check_launch();
+      ZM_CUDA(cudaStreamSynchronize(nullptr));  // any stream sees the table
     }
-    const dim3 g = nu_grid(d, warps, halo);
-    const unsigned strips = g.x * g.y * g.z * warps;
-    ZM_CUDA(cudaDeviceSynchronize());  // no launch reads the old table any more
-    k_nu_class<<<(strips + 7) / 8, dim3(32, 8)>>>(d, nu_class_buf, warps, halo, (int)g.x, (int)g.y);
-    check_launch();
-    ZM_CUDA(cudaDeviceSynchronize());
+    d.nu_class = table;
   }
 
   // Clear the barotropic loop's barrier and error words.  The sequence number
