@@ -1,14 +1,46 @@
-"""The strip classes of the nu_h kernel: every launch shape has its own class
-table."""
+"""The strip classes of the nu_h kernel: strips with every face open take
+another form of the update than the others, and every launch shape has its own
+class table."""
 import ctypes
+import dataclasses
 
 import numpy as np
 import pytest
 
+from tests.gpu_util import f32, run_stage
 from zhenmode_b200 import JaxStateG, make_solver_global, workloads
 from zhenmode_b200.ensemble import Ensemble
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nx,ny", [(192, 96), (75, 47)])
+def test_open_and_gated_strips_give_the_same_bits(nx, ny):
+    """One dry column turns the open strips around it into gated ones.  Cells
+    further from it than the stencils reach (3 subcycles, the finish's two
+    cells) have the same inputs and coefficients in both runs; both forms add
+    the same products in the same order, so the results are equal."""
+    nz, i0, j0 = 4, nx // 2, ny // 2
+    rng = np.random.default_rng(nx)
+    out = []
+    for island in (False, True):
+        depth = np.full((nx, ny), 4900.0)
+        depth[:, :3] = depth[:, -3:] = 0.0
+        if island:
+            depth[i0, j0] = 0.0
+        grid = workloads.build_grid(nx, ny, nz, depth=depth)
+        phys = dataclasses.replace(workloads.PLAIN_PHYSICS, nu_h=1.0e6)
+        kw = dict(workloads.PLAIN_OPTIONS, forcing=workloads.wind_forcing(grid), dt_bt=75.0, nu_nsub=3,
+                  dtype="float32")
+        if not out:
+            T, S = workloads.initial_fields(grid)
+            state = f32(dict(u=rng.standard_normal((nx, ny, nz)), v=rng.standard_normal((nx, ny, nz)), T=T, S=S,
+                             eta=np.zeros((nx, ny))))
+        out.append(run_stage(make_solver_global(grid, phys, 1800.0, **kw)[0], 1, state))
+    i, j = np.meshgrid(np.arange(nx), np.arange(ny), indexing="ij")
+    far = np.maximum(np.minimum(abs(i - i0), nx - abs(i - i0)), abs(j - j0)) > 6
+    for k in ("u", "v"):
+        assert np.array_equal(out[0][k][far], out[1][k][far]), k
 
 
 def _member(seed):

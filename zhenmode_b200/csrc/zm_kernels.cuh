@@ -156,7 +156,7 @@ inline dim3 nu_grid(const Dev& d, int warps, int halo) {
   const int TI = NB_W - 2 * halo, TJ = warps * NB_R - 2 * halo;
   return dim3((d.nx + TI - 1) / TI, (d.ny + TJ - 1) / TJ, d.nz);
 }
-inline size_t nu_smem_bytes(int warps) { return (size_t)warps * (2 * 2 * 32 * 16 + NB_R * 24); }
+inline size_t nu_smem_bytes(int warps) { return (size_t)warps * (2 * 2 * 32 * 16 + NB_R * 32); }
 cudaError_t launch_nu_tb(cudaStream_t s, const Dev& d, int warps, const float* u, const float* v, float* uo,
                          float* vo, float c, int nsub, int halo, int left);
 __global__ void k_nu_class(Dev d, unsigned char* cls, int nw, int halo, int gxn, int gyn);
