@@ -129,3 +129,27 @@ def test_trained_closure_tracks_the_plain_run():
     print(f"daily-mean SST RMSE vs plain: learned {rmse(learned):.4f} K, without the network {rmse(without):.4f} K")
     assert rmse(learned) <= 0.05
     assert rmse(without) > 4.0 * rmse(learned)
+
+
+def test_51_levels_leave_the_last_one_out_of_the_features():
+    """51 levels have 50 interfaces; the features hold 50 levels, so the last
+    one enters through its interface alone, in the fused inference as in the
+    feature rows."""
+    import torch
+    from zhenmode_b200.closure import ClosureMLP
+    nx, ny, nz = 40, 20, 51
+    grid = workloads.build_grid(nx, ny, nz, depth=np.full((nx, ny), 5000.0))
+    assert np.asarray(grid.wet_mask_3d)[:, :, -1].all()
+    kw = dict(workloads.PLAIN_OPTIONS, forcing=workloads.wind_forcing(grid), dt_bt=75.0, dtype="float32")
+    step, init, _ = make_solver_global(grid, workloads.PLAIN_PHYSICS, 1800.0, **kw)
+    st = init(*workloads.initial_fields(grid))
+    g = torch.Generator(device="cuda").manual_seed(3)
+    rn = lambda: 0.2 * torch.randn((nx, ny, nz), generator=g, device="cuda")  # noqa: E731
+    st = JaxStateG(rn(), rn(), st.T + rn(), st.S + rn(), st.eta, st.ice)
+    net = ClosureMLP(seed=5)
+    step.set_closure(net, bound=1e6)
+    K = step.closure_kappa(st).cpu().numpy()
+    X, _, M = step.closure_features(st)
+    want = np.clip(10.0 ** net.forward_bf16(X).cpu().numpy().astype(np.float64), 1e-7, 1.0) * M.cpu().numpy()
+    assert M[:, 49].all()
+    assert np.max(np.abs(K - want) / np.maximum(want, 1e-30) * (want > 0)) < 1e-3

@@ -561,8 +561,10 @@ __global__ void __launch_bounds__(MLP_TC_THREADS, 1) k_mlp_closure(MlpTc w, Dev 
             const float fa = ld(pa, id), fb = ld(pb, id);
             const bool wk = wetb(bits, k);
             if (wk) {
-              put(100 * part + k, fa * (part ? 2.f : 0.1f));
-              put(100 * part + 50 + k, part ? fb * 2.f : fb);
+              if (k < 50) {  // a 51st level has no feature of its own, only its interface
+                put(100 * part + k, fa * (part ? 2.f : 0.1f));
+                put(100 * part + 50 + k, part ? fb * 2.f : fb);
+              }
               if (part == 0 && k > 0 && wu)
                 put(199 + k, asinhf(kG * (-kAlpha * (fa - Tu) + kBeta * (fb - Su)) * d.vc.inv_dz_iface[k - 1] * 1e8f) *
                                  0.25f);
