@@ -85,3 +85,21 @@ def test_autotuned_shapes_change_no_result():
     assert 3 <= halo <= 6 and lines in (1, 2, 4, 8)
     for k in ("u", "v", "T", "S", "eta"):
         assert torch.equal(getattr(a, k), getattr(b, k)), k
+
+
+def test_a_members_closure_reaches_the_ensemble():
+    """A closure set on a member after the ensemble captured its steps, and the
+    member stepped on its own in between: the ensemble's next step has it."""
+    import torch
+    from zhenmode_b200.closure import ClosureMLP
+    members = [_member(48, 24, 10, 1), _member(48, 24, 10, 2)]
+    ens = Ensemble([m[0] for m in members])
+    ens.load([m[1] for m in members])
+    ens.advance(1)
+    members[0][0].set_closure(ClosureMLP(seed=1))
+    want = members[0][0].advance(members[0][1], 2)
+    ens.load([m[1] for m in members])
+    ens.advance(2)
+    got = ens.store()[0]
+    for k in ("u", "v", "T", "S", "eta"):
+        assert torch.equal(getattr(got, k), getattr(want, k)), k

@@ -122,6 +122,7 @@ struct zm_solver {
   cudaEvent_t ev_copy[11] = {};
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   bool graphs_ready = false;
+  unsigned graphs_built = 0;  // captures so far: who holds a copy of the step compares it
   // set while an ensemble captures this member: the cooperative barotropic
   // kernel waits for bt_wait and records bt_done, so that the members'
   // grid-barrier kernels never run at the same time
@@ -724,6 +725,7 @@ struct zm_solver {
       cudaGraphDestroy(graph_def);
     }
     graphs_ready = true;
+    ++graphs_built;
   }
 
   // layout conversion between reference arrays and internal fields
@@ -1399,7 +1401,8 @@ int zm_advance(zm_solver* s, void* stream, int32_t nsteps) {
 
 struct zm_ensemble {
   std::vector<zm_solver*> m;
-  std::vector<int> parity;  // members' state index when graph[0] was captured
+  std::vector<int> parity;      // members' state index when graph[0] was captured
+  std::vector<unsigned> built;  // their own captures then
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   bool ready = false;
   cudaStream_t cap = nullptr;
@@ -1424,7 +1427,11 @@ struct zm_ensemble {
       }
     }
     parity.resize(m.size());
-    for (size_t q = 0; q < m.size(); ++q) parity[q] = m[q]->cur;
+    built.resize(m.size());
+    for (size_t q = 0; q < m.size(); ++q) {
+      parity[q] = m[q]->cur;
+      built[q] = m[q]->graphs_built;
+    }
     for (int g = 0; g < 2; ++g) {
       cudaGraph_t def = nullptr;
       ZM_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
@@ -1491,14 +1498,14 @@ int zm_ensemble_advance(zm_ensemble* e, void* stream, int32_t nsteps, int32_t* k
   if (!e || nsteps < 0) return ZM_ERR_INVALID;
   cudaStream_t st = (cudaStream_t)stream;
   try {
-    // a capture exists, every member still has its own graphs (no closure
-    // change), and all members stepped alike since the capture
+    // a capture exists, every member still has the graphs it had then (no
+    // closure change, no tuning), and all members stepped alike since
     bool stale = !e->ready || e->parity.size() != e->m.size();
     int rel = 0;
     if (!stale) {
       rel = -1;
       for (size_t q = 0; q < e->m.size(); ++q) {
-        if (!e->m[q]->graphs_ready) stale = true;
+        if (!e->m[q]->graphs_ready || e->m[q]->graphs_built != e->built[q]) stale = true;
         const int r = e->m[q]->cur == e->parity[q] ? 0 : 1;
         if (rel < 0) rel = r;
         else if (r != rel) stale = true;
