@@ -153,3 +153,16 @@ def test_51_levels_leave_the_last_one_out_of_the_features():
     want = np.clip(10.0 ** net.forward_bf16(X).cpu().numpy().astype(np.float64), 1e-7, 1.0) * M.cpu().numpy()
     assert M[:, 49].all()
     assert np.max(np.abs(K - want) / np.maximum(want, 1e-30) * (want > 0)) < 1e-3
+
+
+def test_a_new_bound_reaches_the_next_step():
+    """The trusted bound of a closure that is set again counts from the next step on."""
+    from zhenmode_b200.closure import ClosureMLP
+    grid, p, step, st = _case(48, 24, 10)
+    net = ClosureMLP(seed=1)
+    step.set_closure(net, bound=1e6)
+    step(st)
+    assert step.closure_stats()[0] == 0
+    step.set_closure(net, bound=1e-30)
+    step(st)
+    assert step.closure_stats()[0] > 0

@@ -1860,10 +1860,10 @@ int zm_set_closure(zm_solver* s, void* stream, const float* params, float bound)
       ZM_CUDA(cudaMemcpyAsync(b + 2 * ZM_MLP_IN, params + off_b3, ZM_MLP_OUT * sizeof(float),
                               cudaMemcpyDeviceToDevice, st));
       ZM_CUDA(cudaMemsetAsync(s->cl_count, 0, 2 * sizeof(unsigned), st));
-      s->cl_bound = bound;
     }
     const bool on = params != nullptr;
-    if (on != s->closure_on) {  // the captured steps change shape
+    if (on != s->closure_on || (on && bound != s->cl_bound)) {  // the captured steps change shape or hold the old bound
+      if (on) s->cl_bound = bound;
       s->closure_on = on;
       ZM_CUDA(cudaStreamSynchronize(st));
       for (int g = 0; g < 2; ++g)
