@@ -220,6 +220,13 @@ int zm_profile(zm_solver* s, void* stream, float* ms, int32_t* launches, int32_t
  * 1 <= blocks <= the SM count, expected >= blocks.  Synchronizes. */
 int zm_barrier_probe(zm_solver* s, void* stream, int32_t blocks, int32_t expected, int32_t max_polls);
 
+/* Poll limit of the waits between the blocks of the barotropic loop and the
+ * column projection, for the following steps; negative: the default (2^24).
+ * With 0 a block gives up at the first word that is not there yet, which
+ * exercises the error path: zm_status then returns ZM_ERR_TIMEOUT until
+ * zm_load_state.  Synchronizes the device; the steps are captured anew. */
+int zm_set_wait_limit(zm_solver* s, int32_t max_polls);
+
 /* Monitor of the resident state after the last zm_advance (runtime/monitor.py:20-30):
  * 0 accepted, 1 non-finite, 3 velocity above 10 m/s, 4 |eta| above 15 m.
  * Returns ZM_ERR_TIMEOUT if a grid barrier of the barotropic or the column

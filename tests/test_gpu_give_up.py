@@ -1,0 +1,53 @@
+"""Steps whose kernels gave up waiting for one another: the poll limit is set to
+zero, so that the first word or barrier that is not there yet ends the wait.
+Every block returns, the status names the timeout, and a reloaded state runs as
+on a fresh handle: no word or barrier count of the broken launch is taken."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from zhenmode_b200 import JaxStateG, _native, make_solver_global, workloads
+
+pytestmark = pytest.mark.gpu
+
+
+def _make(nx, ny, nz, land_lat, **extra):
+    import torch
+    grid = workloads.build_grid(nx, ny, nz, land_lat=land_lat)
+    kw = dict(workloads.PLAIN_OPTIONS, forcing=workloads.wind_forcing(grid), dt_bt=75.0, dtype="float32", **extra)
+    step, init, _ = make_solver_global(grid, workloads.PLAIN_PHYSICS, 1800.0, **kw)
+    st = init(*workloads.initial_fields(grid))
+    wet = torch.as_tensor(np.asarray(grid.wet_mask_3d, np.float32), device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(nx)
+    rn = lambda: 0.05 * torch.randn(st.u.shape, generator=g, device="cuda") * wet  # noqa: E731
+    return step, [JaxStateG(rn(), rn(), st.T + rn(), st.S, st.eta, st.ice) for _ in range(2)]
+
+
+def _status(step):
+    sv, code = step.solver, ctypes.c_int32()
+    return sv.lib.zm_status(sv.handle, ctypes.byref(code))
+
+
+@pytest.mark.parametrize("nx,ny,nz,land_lat,extra", [
+    (96, 48, 6, 65.0, {}),                                                     # words between neighbours
+    (96, 48, 6, 90.0, {}),                                                     # and the polar cap's barriers
+    (96, 48, 6, 65.0, dict(sponge_days=5.0, sponge_cells=8)),                  # and the sums over the grid
+    (96, 48, 6, 65.0, dict(project_adv_vel=True, projection_niter=20)),        # the projection, resident
+    (1000, 400, 3, 65.0, dict(project_adv_vel=True, projection_niter=5)),      # and streamed
+])
+def test_a_reloaded_state_runs_as_on_a_fresh_handle(nx, ny, nz, land_lat, extra):
+    import torch
+    step, (first, second) = _make(nx, ny, nz, land_lat, **extra)
+    sv = step.solver
+    step(first)
+    assert _status(step) == _native.ZM_OK
+    sv.check(sv.lib.zm_set_wait_limit(sv.handle, 0), "zm_set_wait_limit")
+    step(first)
+    assert _status(step) == _native.ZM_ERR_TIMEOUT
+    sv.check(sv.lib.zm_set_wait_limit(sv.handle, -1), "zm_set_wait_limit")
+    got = step(second)
+    assert _status(step) == _native.ZM_OK
+    want = _make(nx, ny, nz, land_lat, **extra)[0](second)
+    for k in ("u", "v", "T", "S", "eta"):
+        assert torch.equal(getattr(got, k), getattr(want, k)), k

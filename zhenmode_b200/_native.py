@@ -78,6 +78,7 @@ EXPORTS = {
                                   ctypes.POINTER(ctypes.c_int32), ctypes.c_int32]),
     "zm_barrier_probe": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32,
                                         ctypes.c_int32]),
+    "zm_set_wait_limit": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32]),
     "zm_status": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int32)]),
     "zm_projection_stats": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_int32), ctypes.c_int32]),
     "zm_ledger_step": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.POINTER(ZmState), ctypes.POINTER(ZmState),

@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(BT_THREADS, 1) k_bt_loop(Dev d, BtArgs a) {
     for (int c = warp; c < chunks; c += nw) {
       const int b = 32 * c + lane;
       double y = 0.0;
-      if (b < (int)nblocks) ok = wait_word(lists + (size_t)blockIdx.x * nblocks + b, sums, a.err, ZM_BT_BARRIER_POLLS, y) && ok;
+      if (b < (int)nblocks) ok = wait_word(lists + (size_t)blockIdx.x * nblocks + b, sums, a.err, a.max_polls, y) && ok;
       __syncwarp();
       for (int o = 16; o > 0; o >>= 1) y += __shfl_down_sync(0xffffffffu, y, o);
       if (lane == 0) sh.part[c] = y;
@@ -307,11 +307,11 @@ __global__ void __launch_bounds__(BT_THREADS, 1) k_bt_loop(Dev d, BtArgs a) {
       bool ok = true;
 #pragma unroll
       for (int s = 0; s < BT_HS; ++s)
-        if (hp[s] >= 0) ok = wait_word(in + hx[s], seq, a.err, ZM_BT_BARRIER_POLLS, E[hp[s]]) && ok;
+        if (hp[s] >= 0) ok = wait_word(in + hx[s], seq, a.err, a.max_polls, E[hp[s]]) && ok;
       for (int h = tid + BT_HS * nt; h < n_halo && ok; h += nt) {
         int place;
         long long index;
-        if (halo_word(h, place, index)) ok = wait_word(in + index, seq, a.err, ZM_BT_BARRIER_POLLS, E[place]);
+        if (halo_word(h, place, index)) ok = wait_word(in + index, seq, a.err, a.max_polls, E[place]);
       }
       if (cap) {
         band_means(1, a.part_u[pout ^ 1]);
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(BT_THREADS, 1) k_bt_loop(Dev d, BtArgs a) {
     // 3: polar cap of eta*
     if (cap) {
       band_partials(E, a.part_e[pout]);
-      if (!grid_barrier(a.bar, a.err, nblocks, ZM_BT_BARRIER_POLLS)) return;
+      if (!grid_barrier(a.bar, a.err, nblocks, a.max_polls)) return;
       band_means(0, a.part_e[pout]);
       __syncthreads();
 #pragma unroll
@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(BT_THREADS, 1) k_bt_loop(Dev d, BtArgs a) {
     if (cap) {
       band_partials(U, a.part_u[pout]);
       band_partials(V, a.part_v[pout]);
-      if (!grid_barrier(a.bar, a.err, nblocks, ZM_BT_BARRIER_POLLS)) return;
+      if (!grid_barrier(a.bar, a.err, nblocks, a.max_polls)) return;
     }
   }
   // ---- outputs: capped velocities and the float32 free surface
@@ -426,11 +426,17 @@ __global__ void __launch_bounds__(BT_THREADS, 1) k_bt_loop(Dev d, BtArgs a) {
   }
 }
 
-// After a launch that may have given up: the sequence number moves past every
-// word it may have left, the barrier and error words are cleared.
-__global__ void k_bt_reset(unsigned long long* seq, unsigned long long by, unsigned* sync) {
-  *seq += by;
-  for (int q = 0; q < 4; ++q) sync[q] = 0u;
+// After a launch that may have given up: the sequence numbers move past every
+// word that it may have left (a launch has fewer than 2^33 exchanges, and
+// 2^31 of these fit in a number), the barrier and error words are cleared.
+// Thread 0 for the loop, thread 1 for the projection; null: none.
+__global__ void k_sync_reset(unsigned long long* bt_seq, unsigned* bt_sync, unsigned long long* pj_seq,
+                             unsigned* pj_sync) {
+  unsigned long long* seq = threadIdx.x == 0 ? bt_seq : pj_seq;
+  unsigned* sync = threadIdx.x == 0 ? bt_sync : pj_sync;
+  if (seq) *seq += 1ull << 33;
+  if (sync)
+    for (int q = 0; q < 4; ++q) sync[q] = 0u;
 }
 
 void (*bt_loop_kernel(int k))(Dev, BtArgs) {

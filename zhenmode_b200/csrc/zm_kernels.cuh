@@ -94,6 +94,7 @@ struct BtArgs {
   float* eta_out;
   const float* wts;
   unsigned *bar, *err;
+  unsigned max_polls;
   int tile_x, tile_y;
   int ntx, nb, nsub, cap_active;
   double dtH, dtb, drag;
@@ -110,7 +111,8 @@ struct BtTile {
 };
 BtTile bt_tile(int nx, int ny, int sms, size_t smem_max, int least);
 void (*bt_loop_kernel(int k))(Dev, BtArgs);
-__global__ void k_bt_reset(unsigned long long* seq, unsigned long long by, unsigned* sync);
+__global__ void k_sync_reset(unsigned long long* bt_seq, unsigned* bt_sync, unsigned long long* pj_seq,
+                             unsigned* pj_sync);
 __global__ void k_bt_eta(Dev d, const double* eta, const double* ubt, const double* vbt, double* eta_o, double dtH);
 __global__ void k_bt_vel(Dev d, const double* eta, const double* ubt, const double* vbt, const double* Fx,
                          const double* Fy, double* ubt_o, double* vbt_o, double dtb, double drag, const double* sv);
@@ -217,7 +219,7 @@ struct ProjArgs {
   int tile_x, tile_y, tiles_x;
   void *pub, *words;
   unsigned long long* seq;
-  unsigned max_polls;
+  unsigned max_polls;  // of both forms
 };
 struct ProjTile {
   int x, y, tiles_x, tiles_y, cpt, blocks, threads;  // blocks 0: no tile fits

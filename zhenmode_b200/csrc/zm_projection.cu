@@ -111,7 +111,7 @@ __device__ __forceinline__ bool reduce(const ProjArgs& a, int& red, const double
   double* part = a.part + (size_t)(red & 1) * gridDim.x * ZM_PJ_SUMS;
   ++red;
   block_partials(v, part);
-  if (!grid_barrier(a.bar, a.err, gridDim.x, ZM_BT_BARRIER_POLLS)) return false;
+  if (!grid_barrier(a.bar, a.err, gridDim.x, a.max_polls)) return false;
   grid_totals(part, out);
   return true;
 }
@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(PJ_THREADS, 1) k_proj_cg(Dev d, ProjArgs a) {
     }
     // the next residual reads the neighbours' psi
     if (q + 1 < a.refinements || a.norms)
-      if (!grid_barrier(a.bar, a.err, gridDim.x, ZM_BT_BARRIER_POLLS)) return;
+      if (!grid_barrier(a.bar, a.err, gridDim.x, a.max_polls)) return;
   }
   if (a.norms) {
     // ledger mode: squared surface-transport norms of the input and of the

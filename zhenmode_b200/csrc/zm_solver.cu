@@ -225,13 +225,14 @@ struct zm_solver {
     d.nu_class = table;
   }
 
-  // Clear the barotropic loop's barrier and error words.  The sequence number
-  // moves past every word that a launch which gave up may have left behind.
+  // Clear the barrier and error words of the barotropic loop and the projection.  Their sequence
+  // numbers move past every word that a launch which gave up may have left behind.
   void reset_sync(cudaStream_t s) {
-    if (bt_seq) k_bt_reset<<<1, 1, 0, s>>>(bt_seq, 1ull << 20, bt_sync);
-    else ZM_CUDA(cudaMemsetAsync(bt_sync, 0, 4 * sizeof(unsigned), s));
+    k_sync_reset<<<1, 2, 0, s>>>(bt_seq, bt_sync, pj.seq, proj_on ? pj.bar : nullptr);
     check_launch();
   }
+  // Poll limit of the waits between their blocks.  The captured steps hold it.
+  void set_wait_limit(unsigned polls) { bt.max_polls = pj.max_polls = polls; }
 
   // ---------------------------------------------------------------- stages
   // Linear half step L(dt/2): src -> dst (dst must not alias src).
@@ -706,6 +707,13 @@ struct zm_solver {
     tuned = true;
   }
 
+  void drop_graphs() {
+    for (cudaGraphExec_t& g : graph) {
+      if (g) cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
+    graphs_ready = false;
+  }
   void build_graphs() {
     cudaStream_t s = cap_stream;
     for (int g = 0; g < 2; ++g) {
@@ -1285,12 +1293,12 @@ void build(zm_solver* s, const zm_grid* g, const zm_params* p) {
       a.pub = s->alloc<double>(4 * s->n2);
       a.words = s->alloc<double>((size_t)2 * ZM_PJ_SUMS * s->pj_tile.blocks * s->pj_tile.blocks * 2);
       a.seq = s->alloc<unsigned long long>(1);
-      a.max_polls = ZM_BT_BARRIER_POLLS;
     }
     s->pj_dtg = p->dt * 9.81;
     a.dtg = s->pj_dtg;
     s->proj_on = true;
   }
+  s->set_wait_limit(ZM_BT_BARRIER_POLLS);
   const size_t nref3 = (size_t)nx * ny * nz;
   s->ref = Fields4{s->alloc<float>(nref3), s->alloc<float>(nref3), s->alloc<float>(nref3), s->alloc<float>(nref3)};
   s->ref_eta = s->alloc<float>((size_t)nx * ny);
@@ -1764,6 +1772,18 @@ int zm_barrier_probe(zm_solver* s, void* stream, int32_t blocks, int32_t expecte
   return ZM_OK;
 }
 
+int zm_set_wait_limit(zm_solver* s, int32_t max_polls) {
+  if (!s) return ZM_ERR_INVALID;
+  try {
+    s->set_wait_limit(max_polls < 0 ? ZM_BT_BARRIER_POLLS : (unsigned)max_polls);
+    ZM_CUDA(cudaDeviceSynchronize());
+    s->drop_graphs();
+  } catch (const Err& e) {
+    return fail(s, e);
+  }
+  return ZM_OK;
+}
+
 int zm_diagnostics(zm_solver* s, void* stream, const zm_state* in, const float* surface_pressure_pa, float* rho,
                    float* pressure, float* w) {
   if (!s || !in || !in->u || !in->v || !in->T || !in->S || !in->eta || !rho || !pressure || !w)
@@ -1866,12 +1886,7 @@ int zm_set_closure(zm_solver* s, void* stream, const float* params, float bound)
       if (on) s->cl_bound = bound;
       s->closure_on = on;
       ZM_CUDA(cudaStreamSynchronize(st));
-      for (int g = 0; g < 2; ++g)
-        if (s->graph[g]) {
-          cudaGraphExecDestroy(s->graph[g]);
-          s->graph[g] = nullptr;
-        }
-      s->graphs_ready = false;
+      s->drop_graphs();
     }
   } catch (const Err& e) {
     return fail(s, e);
@@ -1884,12 +1899,7 @@ int zm_autotune(zm_solver* s, void* stream, int32_t* nu_halo, int32_t* fft_lines
   cudaStream_t st = (cudaStream_t)stream;
   try {
     s->autotune(st);
-    for (int g = 0; g < 2; ++g)
-      if (s->graph[g]) {
-        cudaGraphExecDestroy(s->graph[g]);
-        s->graph[g] = nullptr;
-      }
-    s->graphs_ready = false;
+    s->drop_graphs();
   } catch (const Err& e) {
     return fail(s, e);
   }
