@@ -1577,14 +1577,14 @@ int zm_step_host(zm_solver* s, void* stream, const zm_state* in, zm_state* out, 
     // Pageable arrays are staged by several threads from one chunk of state on: a call at 1.0 MB of state
     // takes 545 us so and 595 copied directly, at 4.1 MB 897 and 1098.  Pinned arrays copy directly.
     if (4 * b3 + b2 > HostStage::CHUNK && HostStage::pageable(all, 10) && s->stage.ready()) {
-      std::vector<HostStage::Piece> up, down;
+      HostStage::Piece up[5], down[5];
       for (int f = 0; f < 5; ++f) {
         const size_t n = f < 4 ? b3 : b2;
-        up.push_back({const_cast<char*>(reinterpret_cast<const char*>(hin[f])), reinterpret_cast<char*>(ref[f]), n});
-        down.push_back({reinterpret_cast<char*>(hout[f]), reinterpret_cast<char*>(ref[f]), n});
+        up[f] = {const_cast<char*>(reinterpret_cast<const char*>(hin[f])), reinterpret_cast<char*>(ref[f]), n};
+        down[f] = {reinterpret_cast<char*>(hout[f]), reinterpret_cast<char*>(ref[f]), n};
       }
       int rc = ZM_OK;
-      ZM_CUDA(s->stage.run(s->device, cs, up, down, [&] {
+      ZM_CUDA(s->stage.run(s->device, cs, up, down, 5, [&] {
         ZM_CUDA(cudaEventRecord(ev[1], cs));
         ZM_CUDA(cudaStreamWaitEvent(st, ev[1], 0));
         const zm_state r{ref[0], ref[1], ref[2], ref[3], ref[4]};

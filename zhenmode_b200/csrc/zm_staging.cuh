@@ -20,9 +20,7 @@
 #include <cstdint>
 #include <cstring>
 #include <mutex>
-#include <system_error>
 #include <thread>
-#include <vector>
 
 namespace zm {
 
@@ -39,12 +37,7 @@ class HostStage {
   HostStage() = default;
   HostStage(const HostStage&) = delete;
   HostStage& operator=(const HostStage&) = delete;
-  ~HostStage() {
-    for (auto& w : ev_)
-      for (cudaEvent_t e : w)
-        if (e) cudaEventDestroy(e);
-    if (pin_) cudaFreeHost(pin_);
-  }
+  ~HostStage() { release(); }
 
   // Whether every array is pageable host memory that the driver knows nothing of.
   static bool pageable(const void* const* p, int n) {
@@ -71,26 +64,24 @@ class HostStage {
     for (int w = 0; w < workers_; ++w)
       for (cudaEvent_t& e : ev_[w])
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+          e = nullptr;
           (void)cudaGetLastError();
-          cudaFreeHost(pin_);
-          pin_ = nullptr;
+          release();
           return false;
         }
     return true;
   }
 
-  // in -> device on `cs`; then compute(), which queues the work and makes `cs` wait for it and returns
-  // whether to go on; then device -> out.  Returns the first CUDA error of the copies; on any return
-  // nothing of this call is in flight on `cs` any more.
+  // Fields in[0 .. n) -> device on `cs`; then compute(), which queues the work and makes `cs` wait for it and
+  // returns whether to go on; then device -> out[0 .. n).  Returns the first CUDA error of the copies; on any
+  // return nothing of this call is in flight on `cs` any more.  Throws only what compute() throws.
   template <class Compute>
-  cudaError_t run(int device, cudaStream_t cs, const std::vector<Piece>& in, const std::vector<Piece>& out,
-                  Compute&& compute) {
-    Job job{device, cs, chunks(in), chunks(out)};
-    std::vector<std::thread> team;
+  cudaError_t run(int device, cudaStream_t cs, const Piece* in, const Piece* out, int n, Compute&& compute) {
+    Job job(device, cs, in, out, n);
+    std::thread team[MAX_WORKERS];
     try {
-      team.reserve(workers_ - 1);
       for (int w = 1; w < workers_; ++w)
-        team.emplace_back([this, &job, w] {
+        team[w] = std::thread([this, &job, w] {
           note(job, cudaSetDevice(job.device));
           upload(job, w);
           populate(job);
@@ -105,7 +96,7 @@ class HostStage {
     bool go = false;
     try {
       upload(job, 0);
-      while (job.sent.load(std::memory_order_acquire) < job.up.size() && !job.err.load()) std::this_thread::yield();
+      while (job.sent.load(std::memory_order_acquire) < job.up.count && !job.err.load()) std::this_thread::yield();
       go = !job.err.load() && compute();
     } catch (...) {
       finish(job, team);
@@ -121,36 +112,53 @@ class HostStage {
   }
 
  private:
+  // The chunks of some fields, in order.
+  struct Chunks {
+    const Piece* field;
+    size_t count = 0;
+    Chunks(const Piece* f, int n) : field(f) {
+      for (int q = 0; q < n; ++q) count += (f[q].bytes + CHUNK - 1) / CHUNK;
+    }
+    Piece operator[](size_t c) const {
+      const Piece* f = field;
+      for (size_t m; c >= (m = (f->bytes + CHUNK - 1) / CHUNK); c -= m) ++f;
+      const size_t o = c * CHUNK;
+      return {f->host + o, f->dev + o, std::min(CHUNK, f->bytes - o)};
+    }
+  };
   struct Job {
     int device;
     cudaStream_t cs;
-    std::vector<Piece> up, down;
+    Chunks up, down;
     std::atomic<size_t> next_up{0}, sent{0}, next_page{0}, next_down{0};
     std::atomic<int> phase{0};  // 1: the results may be fetched, 2: there are none
     std::atomic<int> err{0};
     std::mutex m;
     std::condition_variable turn;
-    Job(int dv, cudaStream_t s, std::vector<Piece> u, std::vector<Piece> d)
-        : device(dv), cs(s), up(std::move(u)), down(std::move(d)) {}
+    Job(int dv, cudaStream_t s, const Piece* in, const Piece* out, int n) : device(dv), cs(s), up(in, n), down(out, n) {}
   };
 
-  static std::vector<Piece> chunks(const std::vector<Piece>& fields) {
-    std::vector<Piece> c;
-    for (const Piece& f : fields)
-      for (size_t o = 0; o < f.bytes; o += CHUNK) c.push_back({f.host + o, f.dev + o, std::min(CHUNK, f.bytes - o)});
-    return c;
-  }
   static void note(Job& job, cudaError_t e) {
     int none = 0;
     if (e != cudaSuccess) job.err.compare_exchange_strong(none, (int)e);
   }
+  void release() {
+    for (auto& w : ev_)
+      for (cudaEvent_t& e : w) {
+        if (e) cudaEventDestroy(e);
+        e = nullptr;
+      }
+    if (pin_) cudaFreeHost(pin_);
+    pin_ = nullptr;
+  }
+
   char* slot(int w, int s) const { return pin_ + (size_t)(2 * w + s) * CHUNK; }
 
   void upload(Job& job, int w) {
     bool used[2] = {false, false};
     int s = 0;
-    for (size_t c; !job.err.load() && (c = job.next_up.fetch_add(1)) < job.up.size(); s ^= 1) {
-      const Piece& p = job.up[c];
+    for (size_t c; !job.err.load() && (c = job.next_up.fetch_add(1)) < job.up.count; s ^= 1) {
+      const Piece p = job.up[c];
       if (used[s]) note(job, cudaEventSynchronize(ev_[w][s]));
       std::memcpy(slot(w, s), p.host, p.bytes);
       note(job, cudaMemcpyAsync(p.dev, slot(w, s), p.bytes, cudaMemcpyHostToDevice, job.cs));
@@ -167,9 +175,10 @@ class HostStage {
   void populate(Job& job) {
 #ifdef MADV_POPULATE_WRITE
     const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
-    for (size_t c; job.phase.load() == 0 && (c = job.next_page.fetch_add(1)) < job.down.size();) {
-      const uintptr_t a = ((uintptr_t)job.down[c].host + page - 1) / page * page;
-      const uintptr_t b = ((uintptr_t)job.down[c].host + job.down[c].bytes) / page * page;
+    for (size_t c; job.phase.load() == 0 && (c = job.next_page.fetch_add(1)) < job.down.count;) {
+      const Piece p = job.down[c];
+      const uintptr_t a = ((uintptr_t)p.host + page - 1) / page * page;
+      const uintptr_t b = ((uintptr_t)p.host + p.bytes) / page * page;
       if (b > a && madvise(reinterpret_cast<void*>(a), b - a, MADV_POPULATE_WRITE) != 0) return;
     }
 #else
@@ -178,21 +187,22 @@ class HostStage {
   }
 
   void download(Job& job, int w) {
-    const Piece* pending = nullptr;
+    Piece pending{nullptr, nullptr, 0};
     int s = 0;
     for (;;) {
-      const size_t c = job.err.load() ? job.down.size() : job.next_down.fetch_add(1);
-      const Piece* p = c < job.down.size() ? &job.down[c] : nullptr;
-      if (p) {
-        note(job, cudaMemcpyAsync(slot(w, s), p->dev, p->bytes, cudaMemcpyDeviceToHost, job.cs));
+      const size_t c = job.err.load() ? job.down.count : job.next_down.fetch_add(1);
+      const bool more = c < job.down.count;
+      const Piece p = more ? job.down[c] : Piece{nullptr, nullptr, 0};
+      if (more) {
+        note(job, cudaMemcpyAsync(slot(w, s), p.dev, p.bytes, cudaMemcpyDeviceToHost, job.cs));
         note(job, cudaEventRecord(ev_[w][s], job.cs));
       }
-      if (pending) {
+      if (pending.bytes) {
         note(job, cudaEventSynchronize(ev_[w][s ^ 1]));
-        if (!job.err.load()) std::memcpy(pending->host, slot(w, s ^ 1), pending->bytes);
+        if (!job.err.load()) std::memcpy(pending.host, slot(w, s ^ 1), pending.bytes);
       }
       pending = p;
-      if (!p) return;
+      if (!more) return;
       s ^= 1;
     }
   }
@@ -202,9 +212,10 @@ class HostStage {
     job.phase.store(phase);
     job.turn.notify_all();
   }
-  void finish(Job& job, std::vector<std::thread>& team) {
+  void finish(Job& job, std::thread (&team)[MAX_WORKERS]) {
     if (job.phase.load() == 0) begin(job, 2);
-    for (std::thread& t : team) t.join();
+    for (std::thread& t : team)
+      if (t.joinable()) t.join();
     note(job, cudaStreamSynchronize(job.cs));
   }
 
