@@ -158,8 +158,9 @@ int zm_step(zm_solver* s, void* stream, const zm_state* in, zm_state* out, int32
  * copies run on a stream of the solver's own, ordered after the work already
  * queued on `stream`.  Pinned arrays are copied directly, each field's layout
  * change overlapping the next field's transfer; where all ten arrays are
- * pageable, up to six host threads stage them through pinned slots (6 MB) that
- * the solver keeps from the first such call on. */
+ * pageable and large (20 MB a state, or 3 MB once the handle has moved 32), up
+ * to six host threads stage them through pinned slots (6 MB) that the solver
+ * keeps from the first such call on. */
 int zm_step_host(zm_solver* s, void* stream, const zm_state* in, zm_state* out, int32_t nsteps);
 
 /* Replace the 2-D forcing fields (device float32 arrays, (nx, ny)); the

@@ -58,3 +58,18 @@ def test_every_kind_of_host_memory(shape, n):
 
     _host_step(step, ins, ins, n)                                # in place
     assert all(np.array_equal(a, b) for a, b in zip(ins, want))
+
+
+@pytest.mark.parametrize("shape", [(180, 90, 19), (200, 99, 53), (360, 180, 25)])
+def test_calls_before_and_after_the_slots_are_made(shape):
+    """States of 5 and 17 MB: the first calls of a handle copy directly, the
+    later ones are staged (from 32 MB in all on); 26 MB are staged at once.
+    All give the same results."""
+    step, st = _case(*shape)
+    ins = [st[k] for k in gu.FIELDS]
+    want = step.advance(JaxStateG(*gu.to_device(st), 0.0), 1)
+    want = [getattr(want, k).cpu().numpy() for k in gu.FIELDS]
+    for _ in range(9):
+        outs = [np.full_like(x, np.nan) for x in ins]
+        _host_step(step, ins, outs, 1)
+        assert all(np.array_equal(a, b) for a, b in zip(outs, want))

@@ -1,6 +1,7 @@
 """The threads that stage host states (zm_staging.cuh), compiled for the CPU
-against a stand-in for the CUDA runtime whose copies happen at once: what the
-threads move, and what is left after a failure."""
+against a stand-in for the CUDA runtime whose copies happen at once: when the
+pinned slots are made and given back, what the threads move, and what is left
+after a failure."""
 import os
 import subprocess
 
@@ -20,8 +21,8 @@ static std::set<void*> pinned;
 static std::atomic<int> events{0}, made{0}, copies{0};
 static int fail_event = -1, fail_copy = -1;
 extern "C" {
-cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { pinned.insert(*p = malloc(n)); return cudaSuccess; }
-cudaError_t cudaFreeHost(void* p) { assert(pinned.erase(p) == 1); free(p); return cudaSuccess; }
+cudaError_t cudaHostRegister(void* p, size_t, unsigned) { pinned.insert(p); return cudaSuccess; }
+cudaError_t cudaHostUnregister(void* p) { assert(pinned.erase(p) == 1); return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
   if (made++ == fail_event) return cudaErrorMemoryAllocation;
   ++events;
@@ -90,6 +91,22 @@ def _run(tmp_path, main, extra=""):
                     "-I" + os.path.join(ROOT, "zhenmode_b200", "csrc"), str(src), "-o", str(exe)], check=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_slots_are_made_when_they_pay_and_given_back(tmp_path):
+    _run(tmp_path, r"""
+  {
+    HostStage small, middle, large;
+    for (int n = 0; n < 100; ++n) CHECK(!small.wanted(1u << 20));
+    int first = 0;
+    while (!middle.wanted(5u << 20)) ++first;
+    CHECK(first == 6);  // the seventh call has moved 35 MB
+    CHECK(middle.ready() && middle.wanted(5u << 20) && !middle.wanted(1u << 20));
+    CHECK(large.wanted(20u << 20) && large.ready());
+    CHECK(pinned.size() == 2 && events > 0);
+  }
+  CHECK(pinned.empty() && events == 0);
+""")
 
 
 @pytest.mark.parametrize("size", [1, 4095, 512 << 10, (512 << 10) + 1, 3000001])

@@ -1574,9 +1574,8 @@ int zm_step_host(zm_solver* s, void* stream, const zm_state* in, zm_state* out, 
     ZM_CUDA(cudaStreamWaitEvent(cs, ev[0], 0));
     const void* all[10];
     for (int f = 0; f < 5; ++f) all[f] = hin[f], all[5 + f] = hout[f];
-    // Pageable arrays are staged by several threads from one chunk of state on: a call at 1.0 MB of state
-    // takes 545 us so and 595 copied directly, at 4.1 MB 897 and 1098.  Pinned arrays copy directly.
-    if (4 * b3 + b2 > HostStage::CHUNK && HostStage::pageable(all, 10) && s->stage.ready()) {
+    // Pageable arrays are staged by several threads, pinned ones copied directly.
+    if (HostStage::pageable(all, 10) && s->stage.wanted(4 * b3 + b2) && s->stage.ready()) {
       HostStage::Piece up[5], down[5];
       for (int f = 0; f < 5; ++f) {
         const size_t n = f < 4 ? b3 : b2;

@@ -5,9 +5,10 @@
 // their zeroing) falls into the same serial copy.  Here several threads stage the
 // chunks through pinned slots of their own, two each, so that a thread fills or
 // empties one slot while the other is on the bus, and they let the kernel map the
-// result's pages while the device computes.  A whole host step: 31 MB of state
-// 12.4 -> 3.7 ms, 207 MB 69.5 -> 22.4 ms, 1 MB 0.67 -> 0.55 ms (six threads; chunks
-// of 256 KB 4.4 and 27.0 ms).
+// result's pages while the device computes.  A whole host step on one machine, copied
+// directly and staged (six threads): 8 MB of state 1.53 and 1.21 ms, 15 MB 6.8 and
+// 1.77, 31 MB 8.2 and 4.0.  How long the driver's own staging takes differs from
+// machine to machine (31 MB: 5 to 12 ms).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -33,6 +34,11 @@ class HostStage {
   };
   static constexpr size_t CHUNK = 512 << 10;
   static constexpr int MAX_WORKERS = 6;
+  // Making the slots costs the handle's first staged call 1.3 ms.  A call of 20 MB gains that at once (31 MB: 6.6 ms
+  // with it, 10 to 13 copied directly; 15 MB 4.1, and 3.8 to 8 directly); from 3 MB on a handle gains 0.04 ms a MB in
+  // each call and makes them when it has moved 32 MB (8 MB: 1.21 ms staged, 1.53 directly, 3.5 with the slots);
+  // below, both take the same time.
+  static constexpr size_t LEAST = 3u << 20, AT_ONCE = 20u << 20, IN_ALL = 32u << 20;
 
   HostStage() = default;
   HostStage(const HostStage&) = delete;
@@ -52,15 +58,17 @@ class HostStage {
     return true;
   }
 
+  // Whether a call with pageable arrays of this many bytes is staged.
+  bool wanted(size_t bytes) {
+    moved_ = std::min(moved_, IN_ALL) + bytes;
+    return bytes >= LEAST && (pin_ || bytes >= AT_ONCE || moved_ >= IN_ALL);
+  }
+
   // Pinned slots and events, kept with the solver; false where they cannot be had.
   bool ready() {
     if (pin_) return true;
     workers_ = std::max(1, std::min(MAX_WORKERS, (int)std::thread::hardware_concurrency() / 2));
-    if (cudaHostAlloc(reinterpret_cast<void**>(&pin_), 2 * CHUNK * workers_, cudaHostAllocDefault) != cudaSuccess) {
-      (void)cudaGetLastError();
-      pin_ = nullptr;
-      return false;
-    }
+    if (!pin(2 * CHUNK * workers_)) return false;
     for (int w = 0; w < workers_; ++w)
       for (cudaEvent_t& e : ev_[w])
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
@@ -142,13 +150,36 @@ class HostStage {
     int none = 0;
     if (e != cudaSuccess) job.err.compare_exchange_strong(none, (int)e);
   }
+  // Page-locked memory of huge pages: the first host step of a handle pays for it.  cudaHostAlloc
+  // of 6 MB took 2.2 to 11 ms, a mapping of huge pages and its registration take 0.8.
+  bool pin(size_t bytes) {
+    constexpr size_t HUGE_PAGE = 2u << 20;
+    const size_t len = (bytes + HUGE_PAGE - 1) / HUGE_PAGE * HUGE_PAGE + HUGE_PAGE;
+    void* m = mmap(nullptr, len, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (m == MAP_FAILED) return false;
+    char* p = reinterpret_cast<char*>(((uintptr_t)m + HUGE_PAGE - 1) / HUGE_PAGE * HUGE_PAGE);
+#ifdef MADV_HUGEPAGE
+    (void)madvise(p, len - HUGE_PAGE, MADV_HUGEPAGE);  // where there are none, ordinary pages
+#endif
+    if (cudaHostRegister(p, bytes, cudaHostRegisterDefault) != cudaSuccess) {
+      (void)cudaGetLastError();
+      munmap(m, len);
+      return false;
+    }
+    map_ = m;
+    map_len_ = len;
+    pin_ = p;
+    return true;
+  }
   void release() {
     for (auto& w : ev_)
       for (cudaEvent_t& e : w) {
         if (e) cudaEventDestroy(e);
         e = nullptr;
       }
-    if (pin_) cudaFreeHost(pin_);
+    if (!pin_) return;
+    (void)cudaHostUnregister(pin_);
+    munmap(map_, map_len_);
     pin_ = nullptr;
   }
 
@@ -219,6 +250,9 @@ class HostStage {
     note(job, cudaStreamSynchronize(job.cs));
   }
 
+  size_t moved_ = 0;     // bytes of the calls so far
+  void* map_ = nullptr;  // the mapping that holds the slots
+  size_t map_len_ = 0;
   char* pin_ = nullptr;
   int workers_ = 1;
   cudaEvent_t ev_[MAX_WORKERS][2] = {};
