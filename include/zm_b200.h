@@ -299,6 +299,12 @@ int zm_mlp_pack_tc(void* stream, const float* params, void* packed);
 int zm_mlp_forward_packed(void* stream, int32_t ncol, const void* X, int32_t x_bf16, const void* packed,
                           const float* b1, const float* b2, const float* b3, float* Y, uint32_t* err);
 
+/* Exercise the give-up path of the inference on BF16 rows: half of a CTA's
+ * epilogue warps act as if the wait for their first pass's last layer had run
+ * out.  Every CTA returns, and *err is set. */
+int zm_mlp_wait_probe(void* stream, int32_t ncol, const void* X, const void* packed, const float* b1,
+                      const float* b2, const float* b3, float* Y, uint32_t* err);
+
 /* float32 parameters -> BF16 W1, W2, W3 (device arrays). Stream ordered. */
 int zm_mlp_pack_bf16(void* stream, const float* params, void* W1, void* W2, void* W3);
 

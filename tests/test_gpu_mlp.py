@@ -136,3 +136,28 @@ def test_inference_rows_and_types(ncol, kind):
     rows = np.unique(np.concatenate([np.arange(min(ncol, 300)), np.arange(max(0, ncol - 300), ncol)]))
     want = omlp.forward_bf16(p, X[rows], _bf16)
     assert _rel(got.cpu().numpy()[rows], want) < INFER_TOL
+
+
+@pytest.mark.parametrize("ncol", [100, 37889, 150000])
+def test_a_wait_that_runs_out_ends_every_warp(ncol):
+    """Half of the epilogue warps give up in the first pass: the kernel ends (one
+    pass a CTA, a second one in one CTA, several in all), sets its error word, and
+    the next inference is right."""
+    import ctypes
+    import torch
+    from zhenmode_b200.closure import ClosureMLP
+    net = ClosureMLP(seed=2)
+    X = torch.randn((ncol, 256), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda").bfloat16()
+    want = net.forward_bf16(X)
+    net.check_error()
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    Y = torch.empty((ncol, 64), device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert net.lib.zm_mlp_wait_probe(stream, ncol, p(X), p(net.Wp), p(net.b1), p(net.b2), p(net.b3), p(Y),
+                                     p(net.err)) == 0
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError):
+        net.check_error()
+    net.err.zero_()
+    assert torch.equal(net.forward_bf16(X), want)
+    net.check_error()

@@ -89,6 +89,7 @@ EXPORTS = {
                             + [ctypes.c_void_p]),
     "zm_mlp_forward_packed": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_int32]
                               + [ctypes.c_void_p] * 6),
+    "zm_mlp_wait_probe": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32] + [ctypes.c_void_p] * 7),
     "zm_mlp_pack_tc": (ctypes.c_int, [ctypes.c_void_p] * 3),
     "zm_mlp_pack_bf16": (ctypes.c_int, [ctypes.c_void_p] * 5),
     "zm_mlp_trainer_create": (ctypes.c_int, [ctypes.c_int32, ctypes.POINTER(ctypes.c_void_p)]),

@@ -20,8 +20,11 @@
 //  * Sixteen warps run the epilogue of a layer: the accumulator by tcgen05.ld
 //    (warp w the rows 32 (w mod 4) .., accumulator w / 8, columns of half (w / 4) mod 2), bias, GELU,
 //    BF16 back into the activation tile, which is the next layer's A operand.
-// Every wait has a poll limit; one that runs out sets the error word, and the
-// CTA waits (again bounded) for its copies and products before it frees TMEM.
+// Every wait has a poll limit; one that runs out sets the error word.  Before the
+// next pass the epilogue warps agree whether to go on (a warp that left alone would
+// leave the others at their barrier); when not, they wake the product thread, it
+// leaves after one more layer and wakes the copy thread, and the CTA waits (again
+// bounded) for its copies and products before it frees TMEM.
 //
 // Of the 42k cycles of a pass the epilogues take 29k (GELU on 131072 values, 15
 // FMA-pipe operations each, is the bound), the products that nothing overlaps 12k.
@@ -138,6 +141,14 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ uint32_t get_quit(const uint32_t* q) {
+  uint32_t v;
+  asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(su32(q)) : "memory");
+  return v;
+}
+__device__ __forceinline__ void set_quit(uint32_t* q, uint32_t v) {
+  asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(su32(q)), "r"(v) : "memory");
+}
 
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -203,8 +214,10 @@ static_assert(MO * KC3 * 2 == WB_BYTES && PACK_ELEMS * 2 == CHUNKS * WB_BYTES, "
 // may prefetch a later pass's inputs, emit(pass, row, c0, v) takes the raw
 // outputs of a row, 32 at a time, with EMIT_BYTES of shared memory of its warp's.
 // Shared by the standalone and the fused kernels.
+// With LOSE the second tile's warps give up at the first pass's last layer, where
+// the first tile's see the same products done: the path after a wait ran out.
 constexpr int EMIT_STRIDE = 36, EMIT_BYTES = 32 * EMIT_STRIDE * 4;
-template <class Stage, class Next, class Emit>
+template <bool LOSE, class Stage, class Next, class Emit>
 __device__ __forceinline__ void mlp_tc_body(const MlpTc& w, uint8_t* msm, unsigned* err, int passes, Stage stage,
                                             Next next, Emit emit) {
   uint8_t* act = msm;
@@ -214,6 +227,7 @@ __device__ __forceinline__ void mlp_tc_body(const MlpTc& w, uint8_t* msm, unsign
   uint64_t* ready = empty + WSTAGES;  // the activation tiles are written
   uint64_t* done = ready + 1;         // a layer's products are done
   uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
+  uint32_t* quit = tslot + 1;  // 1: the epilogue leaves after a wait ran out, 2: the product thread does
   float* sbias = reinterpret_cast<float*>(msm + BIAS_OFF);
   uint32_t* scratch = reinterpret_cast<uint32_t*>(msm + SCRATCH_OFF);
   const int t = threadIdx.x, warp = t >> 5;
@@ -225,6 +239,7 @@ __device__ __forceinline__ void mlp_tc_body(const MlpTc& w, uint8_t* msm, unsign
     }
     mbar_init(su32(ready), MEPI);
     mbar_init(su32(done), 1);
+    set_quit(quit, 0u);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -246,7 +261,7 @@ __device__ __forceinline__ void mlp_tc_body(const MlpTc& w, uint8_t* msm, unsign
         const __nv_bfloat16* src = w.packed;
         for (int c = 0; c < CHUNKS && ok; ++c, ++n) {
           const int b = n & (WSTAGES - 1);
-          if (n >= WSTAGES) ok = mbar_wait(su32(empty + b), (uint32_t)(n / WSTAGES - 1) & 1u, WAIT_POLLS);
+          if (n >= WSTAGES) ok = mbar_wait(su32(empty + b), (uint32_t)(n / WSTAGES - 1) & 1u, WAIT_POLLS) && get_quit(quit) < 2u;
           if (!ok) break;
           bulk_load(su32(wb) + (uint32_t)b * WB_BYTES, src, WB_BYTES, su32(full + b));
           src += WB_BYTES / 2;
@@ -286,11 +301,16 @@ __device__ __forceinline__ void mlp_tc_body(const MlpTc& w, uint8_t* msm, unsign
       };
       for (int m = 0; m < mine && ok; ++m) {
         products(Int<KC>{}, idesc_bf16(MT, MK));
+        if (get_quit(quit)) ok = false;  // once a pass; the epilogue leaves before a pass's rows are staged
         if (ok) products(Int<KC>{}, idesc_bf16(MT, MK));
         if (ok) products(Int<KC3>{}, idesc_bf16(MT, MO));
       }
       // the last products end before the memory goes
       if (n > 0) ok = mbar_wait(su32(empty + ((n - 1) & (WSTAGES - 1))), (uint32_t)((n - 1) / WSTAGES) & 1u, WAIT_POLLS) && ok;
+      if (!ok) {  // wake the copy thread
+        set_quit(quit, 2u);
+        for (int b = 0; b < WSTAGES; ++b) mbar_arrive(su32(empty + b));
+      }
     }
     __syncwarp();
   } else {
@@ -300,9 +320,17 @@ __device__ __forceinline__ void mlp_tc_body(const MlpTc& w, uint8_t* msm, unsign
     const uint32_t lane_base = tmem + (uint32_t)tile * 256u + ((uint32_t)(quarter * 32) << 16);
     uint8_t* my_act = act + (size_t)tile * ACT_BYTES;
     int phase = 0;
-    for (int n = 0; n < mine && ok; ++n) {
+    for (int n = 0; n < mine; ++n) {
       const int pass = (int)blockIdx.x + n * (int)gridDim.x;
-      if (n > 0) asm volatile("bar.sync 1, %0;" ::"n"(MEPI) : "memory");  // emit may use the tiles
+      if (n > 0) {  // emit may use the tiles until here
+        if (!ok) set_quit(quit, 1u);
+        asm volatile("bar.sync 1, %0;" ::"n"(MEPI) : "memory");
+        if (get_quit(quit)) {  // all leave together and wake the product thread
+          ok = false;
+          mbar_arrive(su32(ready));
+          break;
+        }
+      }
       stage(pass, act, scratch);
       fence_async_smem();
       mbar_arrive(su32(ready));
@@ -310,6 +338,7 @@ __device__ __forceinline__ void mlp_tc_body(const MlpTc& w, uint8_t* msm, unsign
       for (int layer = 0; layer < 3; ++layer) {
         const int N = layer < 2 ? MK : MO;
         if (!mbar_wait(su32(done), (uint32_t)(phase++) & 1u, WAIT_POLLS)) ok = false;
+        if (LOSE && n == 0 && layer == 2 && tile == 1) ok = false;
         if (!__all_sync(0xffffffffu, ok)) {  // tcgen05.ld is a warp's
           ok = false;
           break;
@@ -363,12 +392,12 @@ __device__ __forceinline__ void mlp_tc_body(const MlpTc& w, uint8_t* msm, unsign
 
 // Standalone inference on feature rows X [ncol][256] (BF16, or float32 that is
 // rounded to BF16 on the way in) -> Y [ncol][64].
-template <class In>
+template <class In, bool LOSE = false>
 __global__ void __launch_bounds__(MLP_TC_THREADS, 1) k_mlp_tc(MlpTc w, const In* __restrict__ X,
                                                               float* __restrict__ Y, int ncol, unsigned* err) {
   extern __shared__ __align__(1024) uint8_t msm[];
   const bool y16 = ((uintptr_t)Y & 15u) == 0;
-  mlp_tc_body(
+  mlp_tc_body<LOSE>(
       w, msm, err, (ncol + MROWS - 1) / MROWS,
       [&](int pass, uint8_t* act, uint32_t*) {
         // a warp takes 8 rows x 4 groups of 8 features at a time: rows in full
@@ -531,7 +560,7 @@ __global__ void __launch_bounds__(MLP_TC_THREADS, 1) k_mlp_closure(MlpTc w, Dev 
     return true;
   };
   const uint32_t* largest = reinterpret_cast<const uint32_t*>(msm + SCRATCH_OFF);
-  mlp_tc_body(
+  mlp_tc_body<false>(
       w, msm, err, (int)((ncol + MROWS - 1) / MROWS),
       [&](int pass, uint8_t* act, uint32_t* amax_bits) {
         uint8_t* tile = act + (size_t)(c / MT) * ACT_BYTES;
@@ -942,11 +971,12 @@ bool launch_ok(const char* what) {
 
 bool vec16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
-template <class In>
+template <class In, bool LOSE = false>
 int forward_tc(cudaStream_t st, int ncol, const In* X, const MlpTc& w, float* Y, uint32_t* err) {
-  if (cudaFuncSetAttribute(k_mlp_tc<In>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM) != cudaSuccess)
+  if (cudaFuncSetAttribute(k_mlp_tc<In, LOSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM) !=
+      cudaSuccess)
     return ZM_ERR_CUDA;
-  k_mlp_tc<In><<<mlp_tc_blocks(ncol), MLP_TC_THREADS, TC_SMEM, st>>>(w, X, Y, ncol, err);
+  k_mlp_tc<In, LOSE><<<mlp_tc_blocks(ncol), MLP_TC_THREADS, TC_SMEM, st>>>(w, X, Y, ncol, err);
   return launch_ok("mlp forward") ? ZM_OK : ZM_ERR_CUDA;
 }
 
@@ -988,6 +1018,14 @@ extern "C" int zm_mlp_forward_packed(void* stream, int32_t ncol, const void* X, 
   const MlpTc w{(const __nv_bfloat16*)packed, b1, b2, b3};
   if (x_bf16) return forward_tc((cudaStream_t)stream, ncol, (const __nv_bfloat16*)X, w, Y, err);
   return forward_tc((cudaStream_t)stream, ncol, (const float*)X, w, Y, err);
+}
+
+extern "C" int zm_mlp_wait_probe(void* stream, int32_t ncol, const void* X, const void* packed, const float* b1,
+                                 const float* b2, const float* b3, float* Y, uint32_t* err) {
+  if (ncol < 1 || !X || !packed || !b1 || !b2 || !b3 || !Y || !err || !vec16(X) || !vec16(packed))
+    return ZM_ERR_INVALID;
+  return forward_tc<__nv_bfloat16, true>((cudaStream_t)stream, ncol, (const __nv_bfloat16*)X,
+                                         MlpTc{(const __nv_bfloat16*)packed, b1, b2, b3}, Y, err);
 }
 
 extern "C" int zm_mlp_pack_tc(void* stream, const float* params, void* packed) {
