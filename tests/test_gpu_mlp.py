@@ -161,3 +161,51 @@ def test_a_wait_that_runs_out_ends_every_warp(ncol):
     net.err.zero_()
     assert torch.equal(net.forward_bf16(X), want)
     net.check_error()
+
+
+def test_gelu_of_the_inference_on_both_sides():
+    """One feature through one unit of each hidden layer, scaled between them by
+    2^23, where GELU is the identity (exactly, in BF16) or vanishes: output 0 is
+    |gelu(x)| for negative x, output 1 gelu(x) for positive.  The hidden value is
+    rounded to BF16 once and the rest is exact, so the outputs are BF16 numbers:
+    the one nearest to the float64 value, or its neighbour where the kernel's GELU
+    (well below a step of 2^-8 off) falls to the other side of a rounding boundary."""
+    import math
+    import torch
+    from zhenmode_b200.closure import N_PARAMS, ClosureMLP, unpack
+    p = np.zeros(N_PARAMS, np.float32)
+    w = unpack(p)
+    s = 2.0 ** 23
+    w["W1"][0, 0] = 1.0
+    w["W2"][0, 0], w["W2"][1, 0] = -s, s
+    w["W3"][0, 0] = w["W3"][1, 1] = 1.0 / s
+    net = ClosureMLP(p)
+    x = torch.cat([-torch.linspace(2.0 ** -7, 5.0, 4000), torch.linspace(2.0 ** -7, 60.0, 4000)]).bfloat16()
+    X = torch.zeros((x.numel(), 256), dtype=torch.bfloat16)
+    X[:, 0] = x
+    y = net.forward_bf16(X.cuda()).double().cpu().numpy()
+    net.check_error()
+    x = x.double().numpy()
+    want = x * np.array([0.5 * math.erfc(-v / math.sqrt(2.0)) for v in x])
+    got = np.where(x < 0, -y[:, 0], y[:, 1])
+    step = torch.as_tensor(want).bfloat16().view(torch.int16).int() - torch.as_tensor(got).bfloat16().view(torch.int16).int()
+    assert np.array_equal(torch.as_tensor(got).bfloat16().double().numpy(), got)
+    assert int(step.abs().max()) <= 1
+    assert np.max(np.abs(np.where(x < 0, y[:, 1], y[:, 0]))) < 1e-30  # |gelu(z)| <= 12 Phi(-12) = 2e-32
+
+
+def test_rows_with_nan_and_infinities_stay_alone():
+    """Non-finite features make their own row NaN (a hidden value of -inf has none) and no other."""
+    import torch
+    from zhenmode_b200.closure import ClosureMLP
+    net = ClosureMLP(seed=2)
+    X = torch.randn((300, 256), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda")
+    want = net.forward_bf16(X)
+    bad = X.clone()
+    bad[5, 3], bad[130, 7], bad[299, 0] = float("nan"), float("inf"), float("-inf")
+    got = net.forward_bf16(bad)
+    net.check_error()
+    rows = torch.ones(300, dtype=torch.bool, device="cuda")
+    rows[[5, 130, 299]] = False
+    assert torch.equal(got[rows], want[rows])
+    assert got[~rows].isnan().all()
