@@ -284,7 +284,8 @@ int zm_diagnostics(zm_solver* s, void* stream, const zm_state* in, const float* 
 #define ZM_MLP_NPARAMS 148032
 
 /* Inference on the tensor cores: X [ncol][256] BF16 rows, W1/W2/W3 BF16 as
- * above, float32 biases; Y [ncol][64] float32 (raw outputs).  *err gets bit 0
+ * above (X and the weights 16-byte aligned), float32 biases; Y [ncol][64]
+ * float32 (raw outputs).  *err gets bit 0
  * set if a wait on the tensor cores ran out of polls.  Stream ordered. */
 int zm_mlp_forward_bf16(void* stream, int32_t ncol, const void* X, const void* W1, const float* b1, const void* W2,
                         const float* b2, const void* W3, const float* b3, float* Y, uint32_t* err);

@@ -209,3 +209,34 @@ def test_rows_with_nan_and_infinities_stay_alone():
     rows[[5, 130, 299]] = False
     assert torch.equal(got[rows], want[rows])
     assert got[~rows].isnan().all()
+
+
+def _ptr(t):
+    import ctypes
+    return ctypes.c_void_p(t.data_ptr())
+
+
+@pytest.mark.parametrize("ncol", [0, 1, 129, 37889, 80000])
+def test_weights_in_rows_give_the_packed_ones_bits(ncol):
+    """The same chunks of the same BF16 weights, fetched from their rows: the same products in the same order."""
+    import ctypes
+    import torch
+    from zhenmode_b200.closure import ClosureMLP
+    net = ClosureMLP(seed=4)
+    X = torch.randn((max(ncol, 1), 256), generator=torch.Generator(device="cuda").manual_seed(ncol), device="cuda")
+    X = X.bfloat16()
+    want = net.forward_bf16(X)
+    W = [torch.empty(s, dtype=torch.bfloat16, device="cuda") for s in ((256, 256), (256, 256), (64, 256))]
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert net.lib.zm_mlp_pack_bf16(stream, _ptr(net.params), *[_ptr(w) for w in W]) == 0
+    Y = torch.full((max(ncol, 1), 64), 7.0, device="cuda")
+
+    def call(x, w1):
+        return net.lib.zm_mlp_forward_bf16(stream, ncol, x, w1, _ptr(net.b1), _ptr(W[1]), _ptr(net.b2), _ptr(W[2]),
+                                           _ptr(net.b3), _ptr(Y), _ptr(net.err))
+
+    assert call(_ptr(X), _ptr(W[0])) == 0
+    net.check_error()
+    assert torch.equal(Y, want) if ncol else bool((Y == 7.0).all())
+    off = ctypes.c_void_p(W[0].data_ptr() + 2)  # rows off a 16-byte boundary are refused
+    assert call(_ptr(X), off) != 0 and call(ctypes.c_void_p(X.data_ptr() + 2), _ptr(W[0])) != 0

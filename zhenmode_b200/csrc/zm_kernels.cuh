@@ -127,6 +127,10 @@ struct MlpTc {
   const __nv_bfloat16* packed;
   const float *b1, *b2, *b3;
 };
+struct MlpRows {  // BF16 weights [out][in]
+  const __nv_bfloat16 *W1, *W2, *W3;
+  const float *b1, *b2, *b3;
+};
 size_t mlp_tc_smem();
 int mlp_tc_blocks(long long ncol);
 constexpr int MLP_TC_THREADS = 576;

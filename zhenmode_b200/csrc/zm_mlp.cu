@@ -12,7 +12,8 @@
 // matrices of one K=16 step are LBO = 128 B apart, 8-row groups SBO = 16 * K bytes
 // apart).  The weights are packed once in that layout, in K chunks of 16 KB
 // (zm_mlp_pack_tc), so that one bulk copy brings a chunk for both operands; four
-// buffers.  The rows of the next pass are prefetched into L2.
+// buffers.  Weights that are not packed (zm_mlp_forward_bf16) are brought in the same
+// chunks by the asynchronous copies of one warp.  The rows of the next pass are prefetched into L2.
 //  * A copy thread fills the buffers; a product thread waits for a chunk, issues
 //    its tcgen05.mma and commits them to the buffer's mbarrier, the last commit
 //    of a layer to the epilogue's (one thread for both, with its index
@@ -42,6 +43,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <string>
+#include <type_traits>
 
 #include "../../include/zm_b200.h"
 #include "zm_kernels.cuh"
@@ -227,9 +229,10 @@ static_assert(MO * KC3 * 2 == WB_BYTES && PACK_ELEMS * 2 == CHUNKS * WB_BYTES, "
 // With LOSE the second tile's warps give up at the first pass's last layer, where
 // the first tile's see the same products done: the path after a wait ran out.
 constexpr int EMIT_STRIDE = 36, EMIT_BYTES = 32 * EMIT_STRIDE * 4;
-template <bool LOSE, class Stage, class Next, class Emit>
-__device__ __forceinline__ void mlp_tc_body(const MlpTc& w, uint8_t* msm, unsigned* err, int passes, Stage stage,
+template <bool LOSE, class Weights, class Stage, class Next, class Emit>
+__device__ __forceinline__ void mlp_tc_body(const Weights& w, uint8_t* msm, unsigned* err, int passes, Stage stage,
                                             Next next, Emit emit) {
+  constexpr bool ROWS = std::is_same_v<Weights, MlpRows>;
   uint8_t* act = msm;
   uint8_t* wb = msm + TILES * ACT_BYTES;
   uint64_t* full = reinterpret_cast<uint64_t*>(msm + BAR_OFF);  // a chunk has landed
@@ -244,7 +247,7 @@ __device__ __forceinline__ void mlp_tc_body(const MlpTc& w, uint8_t* msm, unsign
   const int mine = passes > (int)blockIdx.x ? (passes - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   if (t == MEPI) {
     for (int b = 0; b < WSTAGES; ++b) {
-      mbar_init(su32(full + b), 1);
+      mbar_init(su32(full + b), ROWS ? 32 : 1);
       mbar_init(su32(empty + b), 1);
     }
     mbar_init(su32(ready), MEPI);
@@ -265,7 +268,38 @@ __device__ __forceinline__ void mlp_tc_body(const MlpTc& w, uint8_t* msm, unsign
   const uint32_t tmem = *tslot;
   bool ok = true;
   if (warp == MEPI / 32) {
-    if (t == MEPI) {  // copy thread: weight chunks in turn, WSTAGES ahead of the products
+    if constexpr (ROWS) {  // the copy warp: the same chunks from the weights' rows, a lane 16 bytes at a time
+      const int lane = t & 31;
+      int n = 0;  // chunks begun
+      auto landed = [&](int i) {
+        fence_async_smem();
+        mbar_arrive(su32(full + (i & (WSTAGES - 1))));
+      };
+      for (int m = 0; m < mine && ok; ++m)
+        for (int c = 0; c < CHUNKS; ++c, ++n) {
+          const int b = n & (WSTAGES - 1);
+          if (n >= WSTAGES) ok = mbar_wait(su32(empty + b), (uint32_t)(n / WSTAGES - 1) & 1u, WAIT_POLLS) && get_quit(quit) < 2u;
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          const int layer = c < KCHUNKS ? 0 : (c < 2 * KCHUNKS ? 1 : 2), kw = layer < 2 ? KC : KC3;
+          const __nv_bfloat16* W = (layer == 0 ? w.W1 : (layer == 1 ? w.W2 : w.W3)) + (c - layer * KCHUNKS) * kw;
+          const uint32_t dst = su32(wb) + (uint32_t)b * WB_BYTES;
+          const int groups = kw / 32;  // 8 rows x 4 pieces at a time: whole sectors, no bank conflicts
+#pragma unroll 8
+          for (int e = 0; e < (int)(WB_BYTES / 512); ++e) {
+            const int r = e / groups * 8 + (lane & 7), k = e % groups * 32 + (lane >> 3) * 8;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + core_off(r, k, kw)), "l"(W + r * MK + k)
+                         : "memory");
+          }
+          asm volatile("cp.async.commit_group;" ::: "memory");
+          if (n >= 2) {  // two chunks on the way
+            asm volatile("cp.async.wait_group 2;" ::: "memory");
+            landed(n - 2);
+          }
+        }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      for (int i = n > 2 ? n - 2 : 0; i < n; ++i) landed(i);
+    } else if (t == MEPI) {  // copy thread: weight chunks in turn, WSTAGES ahead of the products
       int n = 0;  // copies started
       for (int m = 0; m < mine && ok; ++m) {
         const __nv_bfloat16* src = w.packed;
@@ -402,8 +436,8 @@ __device__ __forceinline__ void mlp_tc_body(const MlpTc& w, uint8_t* msm, unsign
 
 // Standalone inference on feature rows X [ncol][256] (BF16, or float32 that is
 // rounded to BF16 on the way in) -> Y [ncol][64].
-template <class In, bool LOSE = false>
-__global__ void __launch_bounds__(MLP_TC_THREADS, 1) k_mlp_tc(MlpTc w, const In* __restrict__ X,
+template <class In, class Weights, bool LOSE = false>
+__global__ void __launch_bounds__(MLP_TC_THREADS, 1) k_mlp_tc(Weights w, const In* __restrict__ X,
                                                               float* __restrict__ Y, int ncol, unsigned* err) {
   extern __shared__ __align__(1024) uint8_t msm[];
   const bool y16 = ((uintptr_t)Y & 15u) == 0;
@@ -668,16 +702,15 @@ __global__ void k_mlp_pack(const float* __restrict__ params, __nv_bfloat16* __re
   }
 }
 
-// float32 parameters, or BF16 weights [out][in], -> packed BF16 weights
-template <class In>
-__global__ void k_mlp_pack_tc(const In* __restrict__ W1, const In* __restrict__ W2, const In* __restrict__ W3,
-                              __nv_bfloat16* __restrict__ out) {
+// float32 weights [out][in] -> packed BF16 weights
+__global__ void k_mlp_pack_tc(const float* __restrict__ W1, const float* __restrict__ W2,
+                              const float* __restrict__ W3, __nv_bfloat16* __restrict__ out) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < PACK_ELEMS; i += gridDim.x * blockDim.x) {
     const int layer = i < MK * MK ? 0 : (i < 2 * MK * MK ? 1 : 2), e = i - layer * MK * MK;
     const int n = e / MK, k = e - n * MK;
-    const In* W = layer == 0 ? W1 : (layer == 1 ? W2 : W3);
+    const float* W = layer == 0 ? W1 : (layer == 1 ? W2 : W3);
     const int kc = layer < 2 ? KC : KC3, chunk = layer * KCHUNKS + k / kc;
-    out[(size_t)chunk * (WB_BYTES / 2) + core_off(n, k % kc, kc) / 2] = __float2bfloat16((float)W[e]);
+    out[(size_t)chunk * (WB_BYTES / 2) + core_off(n, k % kc, kc) / 2] = __float2bfloat16(W[e]);
   }
 }
 
@@ -981,12 +1014,12 @@ bool launch_ok(const char* what) {
 
 bool vec16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
-template <class In, bool LOSE = false>
-int forward_tc(cudaStream_t st, int ncol, const In* X, const MlpTc& w, float* Y, uint32_t* err) {
-  if (cudaFuncSetAttribute(k_mlp_tc<In, LOSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM) !=
+template <class In, class Weights, bool LOSE = false>
+int forward_tc(cudaStream_t st, int ncol, const In* X, const Weights& w, float* Y, uint32_t* err) {
+  if (cudaFuncSetAttribute(k_mlp_tc<In, Weights, LOSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM) !=
       cudaSuccess)
     return ZM_ERR_CUDA;
-  k_mlp_tc<In, LOSE><<<mlp_tc_blocks(ncol), MLP_TC_THREADS, TC_SMEM, st>>>(w, X, Y, ncol, err);
+  k_mlp_tc<In, Weights, LOSE><<<mlp_tc_blocks(ncol), MLP_TC_THREADS, TC_SMEM, st>>>(w, X, Y, ncol, err);
   return launch_ok("mlp forward") ? ZM_OK : ZM_ERR_CUDA;
 }
 
@@ -1007,17 +1040,13 @@ struct zm_mlp_trainer {
 extern "C" int zm_mlp_forward_bf16(void* stream, int32_t ncol, const void* X, const void* W1, const float* b1,
                                    const void* W2, const float* b2, const void* W3, const float* b3, float* Y,
                                    uint32_t* err) {
-  if (ncol < 0 || !X || !W1 || !b1 || !W2 || !b2 || !W3 || !b3 || !Y || !err) return ZM_ERR_INVALID;
+  if (ncol < 0 || !X || !W1 || !b1 || !W2 || !b2 || !W3 || !b3 || !Y || !err || !vec16(X) || !vec16(W1) ||
+      !vec16(W2) || !vec16(W3))
+    return ZM_ERR_INVALID;
   if (ncol == 0) return ZM_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  // the weights in the layout of the bulk copies, in memory of this call's own
-  __nv_bfloat16* packed = nullptr;
-  if (cudaMallocAsync(&packed, PACK_ELEMS * sizeof(__nv_bfloat16), st) != cudaSuccess) return ZM_ERR_CUDA;
-  k_mlp_pack_tc<<<288, 256, 0, st>>>((const __nv_bfloat16*)W1, (const __nv_bfloat16*)W2, (const __nv_bfloat16*)W3,
-                                     packed);
-  const int rc = forward_tc(st, ncol, (const __nv_bfloat16*)X, MlpTc{packed, b1, b2, b3}, Y, err);
-  cudaFreeAsync(packed, st);
-  return rc;
+  // 259200 columns 243 us, 4000 columns 47 (from packed weights 204 and 48)
+  const MlpRows w{(const __nv_bfloat16*)W1, (const __nv_bfloat16*)W2, (const __nv_bfloat16*)W3, b1, b2, b3};
+  return forward_tc((cudaStream_t)stream, ncol, (const __nv_bfloat16*)X, w, Y, err);
 }
 
 extern "C" int zm_mlp_forward_packed(void* stream, int32_t ncol, const void* X, int32_t x_bf16, const void* packed,
@@ -1034,7 +1063,7 @@ extern "C" int zm_mlp_wait_probe(void* stream, int32_t ncol, const void* X, cons
                                  const float* b2, const float* b3, float* Y, uint32_t* err) {
   if (ncol < 1 || !X || !packed || !b1 || !b2 || !b3 || !Y || !err || !vec16(X) || !vec16(packed))
     return ZM_ERR_INVALID;
-  return forward_tc<__nv_bfloat16, true>((cudaStream_t)stream, ncol, (const __nv_bfloat16*)X,
+  return forward_tc<__nv_bfloat16, MlpTc, true>((cudaStream_t)stream, ncol, (const __nv_bfloat16*)X,
                                          MlpTc{(const __nv_bfloat16*)packed, b1, b2, b3}, Y, err);
 }
 
