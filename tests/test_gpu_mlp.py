@@ -240,3 +240,29 @@ def test_weights_in_rows_give_the_packed_ones_bits(ncol):
     assert torch.equal(Y, want) if ncol else bool((Y == 7.0).all())
     off = ctypes.c_void_p(W[0].data_ptr() + 2)  # rows off a 16-byte boundary are refused
     assert call(_ptr(X), off) != 0 and call(ctypes.c_void_p(X.data_ptr() + 2), _ptr(W[0])) != 0
+
+
+def test_the_weights_of_a_network_may_be_replaced():
+    """W1, W2, W3 hold the BF16 weights of the last pack(); written in place or
+    set, the inference follows them, and pack() returns to the parameters."""
+    import torch
+    from zhenmode_b200.closure import ClosureMLP, unpack
+    net, other = ClosureMLP(seed=4), ClosureMLP(seed=9)
+    X = torch.randn((500, 256), device="cuda")
+    mine, theirs = net.forward_bf16(X), other.forward_bf16(X)
+    for a, b in zip((net.W1, net.W2, net.W3), ("W1", "W2", "W3")):
+        assert torch.equal(a, unpack(net.params)[b].bfloat16())
+    assert torch.equal(net.forward_bf16(X), mine)
+    net.W1 = other.W1.clone()
+    net.W2.copy_(other.W2)
+    net.W3 = other.W3
+    net.b3.copy_(other.b3)
+    assert torch.equal(net.forward_bf16(X), theirs)
+    net.params.mul_(1.0)
+    net.pack()
+    net.b3 = unpack(ClosureMLP(seed=4).params)["b3"].contiguous()
+    assert torch.equal(net.forward_bf16(X), mine)
+    # weights read before the parameters change are those of the last pack()
+    later = ClosureMLP(seed=4)
+    later.params.zero_()
+    assert torch.equal(later.W2, unpack(ClosureMLP(seed=4).params)["W2"].bfloat16())

@@ -9,7 +9,7 @@ outputs 0..nz-2 are log10 of the diffusivity at interfaces 0..nz-2 and the
 rest are unused.
 
 All arithmetic runs in ``libzm_b200.so``: inference on the tensor cores in
-BF16 with float32 accumulation (``zm_mlp_forward_bf16``), training in float32
+BF16 with float32 accumulation (``zm_mlp_forward_packed``), training in float32
 (``zm_mlp_grad``, ``zm_mlp_train_step``).  PyTorch only holds the device
 arrays.
 """
@@ -82,27 +82,46 @@ class ClosureMLP:
         """Refresh the BF16 weight copies from the float32 parameters."""
         import torch
         dev = self.params.device
-        self.W1 = torch.empty((256, 256), dtype=torch.bfloat16, device=dev)
-        self.W2 = torch.empty((256, 256), dtype=torch.bfloat16, device=dev)
-        self.W3 = torch.empty((64, 256), dtype=torch.bfloat16, device=dev)
-        _check(self.lib.zm_mlp_pack_bf16(_stream(self.params), _ptr(self.params), _ptr(self.W1), _ptr(self.W2),
-                                         _ptr(self.W3)), "zm_mlp_pack_bf16")
         self.Wp = torch.empty(2 * 256 * 256 + 64 * 256, dtype=torch.bfloat16, device=dev)  # as the inference reads them
         _check(self.lib.zm_mlp_pack_tc(_stream(self.params), _ptr(self.params), _ptr(self.Wp)), "zm_mlp_pack_tc")
+        self._rows = None
         blocks = unpack(self.params)
         self.b1, self.b2, self.b3 = (blocks[k].contiguous() for k in ("b1", "b2", "b3"))
+
+    # W1, W2, W3: the BF16 weights [out][in] as :meth:`pack` left them.  They may be
+    # written or replaced; the inference reads them from the first use on.
+    def _weights(self):
+        if self._rows is None:
+            # K chunks of 32 (32, 128) inputs in core matrices of 8 rows x 8 values (zm_mlp.cu)
+            hidden = self.Wp[:131072].view(2, 8, 32, 4, 8, 8).permute(0, 2, 4, 1, 3, 5).reshape(2, 256, 256)
+            out = self.Wp[131072:].view(2, 8, 16, 8, 8).permute(1, 3, 0, 2, 4).reshape(64, 256)
+            self._rows = [hidden[0].clone(), hidden[1].clone(), out.clone()]
+        return self._rows
+
+    def _replace(self, k, value):
+        self._weights()[k] = value
+
+    W1 = property(lambda self: self._weights()[0], lambda self, value: self._replace(0, value))
+    W2 = property(lambda self: self._weights()[1], lambda self, value: self._replace(1, value))
+    W3 = property(lambda self: self._weights()[2], lambda self, value: self._replace(2, value))
 
     def forward_bf16(self, X):
         """Tensor-core inference: X [n][256] (any float dtype, CUDA) -> [n][64] float32."""
         import torch
         if X.dim() != 2 or X.shape[1] != N_IN:
             raise ValueError("X must be [n][256]")
-        if X.dtype != torch.float32 or not X.is_cuda or not X.is_contiguous() or X.data_ptr() % 16:
+        if self._rows is not None or X.dtype != torch.float32 or not X.is_cuda or not X.is_contiguous() \
+                or X.data_ptr() % 16:
             X = X.to(torch.bfloat16).contiguous()
             if X.data_ptr() % 16:
                 X = X.clone()
         # float32 rows are rounded to BF16 as the kernel reads them
         Y = torch.empty((X.shape[0], N_OUT), dtype=torch.float32, device=X.device)
+        if self._rows is not None:
+            _check(self.lib.zm_mlp_forward_bf16(_stream(X), int(X.shape[0]), _ptr(X), _ptr(self.W1), _ptr(self.b1),
+                                                _ptr(self.W2), _ptr(self.b2), _ptr(self.W3), _ptr(self.b3), _ptr(Y),
+                                                _ptr(self.err)), "zm_mlp_forward_bf16")
+            return Y
         _check(self.lib.zm_mlp_forward_packed(_stream(X), int(X.shape[0]), _ptr(X), int(X.dtype == torch.bfloat16),
                                               _ptr(self.Wp), _ptr(self.b1), _ptr(self.b2), _ptr(self.b3), _ptr(Y),
                                               _ptr(self.err)), "zm_mlp_forward_packed")
