@@ -166,3 +166,30 @@ def test_a_new_bound_reaches_the_next_step():
     step.set_closure(net, bound=1e-30)
     step(st)
     assert step.closure_stats()[0] > 0
+
+
+@pytest.mark.parametrize("n", [(96, 48, 20), (180, 90, 50), (360, 180, 50)])
+def test_closure_set_on_a_stream_of_its_own(n):
+    """set_closure and the following calls on a stream that does not wait for the
+    default one, which is busy: what the handle allocates then is cleared before
+    it is filled."""
+    import torch
+    from zhenmode_b200.closure import ClosureMLP
+    grid, p, step, st = _case(*n)
+    net = ClosureMLP(seed=5)
+    other = _case(*n)[2]
+    other.set_closure(net)
+    want = other.closure_kappa(st)
+    assert bool((want > 0).any())
+    side = torch.cuda.Stream()
+    a = torch.randn((8192, 8192), device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(40):
+        a @ a
+    with torch.cuda.stream(side):
+        step.set_closure(net)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        got = step.closure_kappa(st)
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
