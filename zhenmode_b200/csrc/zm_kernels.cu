@@ -340,28 +340,49 @@ k_nu_tb(Dev d, const float* __restrict__ u, const float* __restrict__ v, float* 
 // launch shape: bits 0-3 half the distance in rows, rounded down and at most
 // 15, from the strip's nearest cell to the next wet cell of its column and
 // level (0: the strip holds a wet cell); bit 4 set when every face of its cells
-// is open and dx is constant along the rows.  One warp per strip; built once
-// per solver and launch shape.
+// is open and dx is constant along the rows.  One warp per strip of every level,
+// from the columns' wet words (one warp per level and strip read the masks 50
+// times over: NEW us at 720x360x50, now); built once per solver and launch shape.
 __global__ void k_nu_class(Dev d, unsigned char* __restrict__ cls, int nw, int halo, int gxn, int gyn) {
-  const int strip = blockIdx.x * blockDim.y + threadIdx.y;
-  if (strip >= d.nz * gyn * gxn * nw) return;
-  const int wp = strip % nw, bx = strip / nw % gxn, by = strip / nw / gxn % gyn, k = strip / nw / gxn / gyn;
+  const int strip = blockIdx.x * blockDim.y + threadIdx.y, lane = threadIdx.x;
+  if (strip >= gyn * gxn * nw) return;
+  const int wp = strip % nw, bx = strip / nw % gxn, by = strip / nw / gxn;
   const int gx0 = bx * (NB_W - 2 * halo) - halo, gy0 = by * (nw * NB_R - 2 * halo) - halo + wp * NB_R;
-  int dist = 30;
-  bool open = d.dx_rows != 0;
+  int i[2];
   for (int h = 0; h < 2; ++h) {
-    int i = (gx0 + 2 * threadIdx.x + h) % d.nx;
-    if (i < 0) i += d.nx;
-    for (int q = 0; q < NB_R; ++q) {
-      const int gj = gy0 + q, j = min(max(gj, 0), d.ny - 1);
-      open = open && gj == j && (__ldg(d.nu_gate + idx3(d, k, j, i)) & 15u) == 15u;
-      for (int m = 0; m < dist; ++m)
-        if (wetb(wb(d, max(j - m, 0), i), k) || wetb(wb(d, min(j + m, d.ny - 1), i), k)) dist = m;
-    }
+    i[h] = (gx0 + 2 * lane + h) % d.nx;
+    if (i[h] < 0) i[h] += d.nx;
   }
-  dist = __reduce_min_sync(0xffffffffu, dist);
-  open = __all_sync(0xffffffffu, open);
-  if (threadIdx.x == 0) cls[strip] = (unsigned char)((dist / 2) | (open ? NU_OPEN : 0u));
+  auto warp_or = [](uint64_t v) {
+    return (uint64_t)__reduce_or_sync(0xffffffffu, (unsigned)v) |
+           (uint64_t)__reduce_or_sync(0xffffffffu, (unsigned)(v >> 32)) << 32;
+  };
+  auto wet_row = [&](int j) { return wb(d, j, i[0]) | wb(d, j, i[1]); };
+  // levels with a closed face
+  uint64_t closed = d.dx_rows != 0 && gy0 >= 0 && gy0 + NB_R <= d.ny ? 0ull : ~0ull;
+  for (int j = max(gy0, 0); j < min(gy0 + NB_R, d.ny); ++j)
+    for (int h = 0; h < 2; ++h) {
+      const uint64_t n = j < d.ny - 1 ? wb(d, j + 1, i[h]) : 0ull, s = j > 0 ? wb(d, j - 1, i[h]) : 0ull;
+      closed |= ~(wb(d, j, i[h]) & wb(d, j, east(d, i[h])) & wb(d, j, west(d, i[h])) & n & s);
+    }
+  closed = warp_or(closed);
+  // levels with a wet cell within m rows, m = 0, 1, ..; lane l takes the levels l and l + 32
+  const int lo = min(max(gy0, 0), d.ny - 1), hi = min(max(gy0 + NB_R - 1, 0), d.ny - 1);
+  uint64_t any = 0ull;
+  for (int j = lo; j <= hi; ++j) any |= wet_row(j);
+  int dist[2] = {30, 30};
+  for (int m = 0; m < 30; ++m) {
+    if (m > 0 && lo - m >= 0) any |= wet_row(lo - m);
+    if (m > 0 && hi + m < d.ny) any |= wet_row(hi + m);
+    any = warp_or(any);
+    for (int h = 0; h < 2; ++h)
+      if (dist[h] == 30 && wetb(any, lane + 32 * h)) dist[h] = m;
+  }
+  for (int h = 0; h < 2; ++h) {
+    const int k = lane + 32 * h;
+    if (k < d.nz)
+      cls[((k * gyn + by) * gxn + bx) * nw + wp] = (unsigned char)((dist[h] / 2) | (wetb(closed, k) ? 0u : NU_OPEN));
+  }
 }
 
 // Union of the wet words over RY-row tiles of 32 columns and their two-cell

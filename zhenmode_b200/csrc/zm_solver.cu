@@ -218,11 +218,11 @@ struct zm_solver {
     unsigned char*& table = nu_tables[warps == 16][halo];
     if (!table) {
       const dim3 g = nu_grid(d, warps, halo);
-      const unsigned strips = g.x * g.y * g.z * warps;
-      table = alloc<unsigned char>(strips);
-      k_nu_class<<<(strips + 7) / 8, dim3(32, 8)>>>(d, table, warps, halo, (int)g.x, (int)g.y);
+      const unsigned strips = g.x * g.y * warps;  // of every level
+      table = alloc<unsigned char>((size_t)strips * g.z);
+      k_nu_class<<<(strips + 7) / 8, dim3(32, 8), 0, cap_stream>>>(d, table, warps, halo, (int)g.x, (int)g.y);
       check_launch();
-      ZM_CUDA(cudaStreamSynchronize(nullptr));  // any stream sees the table
+      ZM_CUDA(cudaStreamSynchronize(cap_stream));  // any stream sees the table
     }
     d.nu_class = table;
   }
