@@ -137,7 +137,9 @@ int zm_create(const zm_grid* grid, const zm_params* params, zm_solver** out);
  * FFT lines per block, out[11] levels per block of the tracer-advection
  * march, out[12] of the linear-finish march, out[13] tile rows of the
  * vertical-transport march, out[14] of the pressure-gradient march, out[15]
- * warps per nu_h tile (8 or 16).  Writes min(n, 16) values. */
+ * warps per nu_h tile (8 or 16), out[16] grid rows per thread of the column
+ * projection's resident form (0: streamed, or no projection).  Writes
+ * min(n, 17) values. */
 int zm_info(const zm_solver* s, int32_t* out, int32_t n);
 
 /* Copy a device state (reference layout) into the solver's resident state. */
@@ -285,8 +287,8 @@ int zm_diagnostics(zm_solver* s, void* stream, const zm_state* in, const float* 
 
 /* Inference on the tensor cores: X [ncol][256] BF16 rows, W1/W2/W3 BF16 as
  * above (X and the weights 16-byte aligned), float32 biases; Y [ncol][64]
- * float32 (raw outputs).  *err gets bit 0
- * set if a wait on the tensor cores ran out of polls.  Stream ordered. */
+ * float32 (raw outputs).  *err gets bit 0 set if a wait on the tensor cores
+ * ran out of polls.  Stream ordered. */
 int zm_mlp_forward_bf16(void* stream, int32_t ncol, const void* X, const void* W1, const float* b1, const void* W2,
                         const float* b2, const void* W3, const float* b3, float* Y, uint32_t* err);
 

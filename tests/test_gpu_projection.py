@@ -8,6 +8,8 @@ run in float64 arithmetic with those same tolerances for the tight
 comparison, and the reference's float64 goldens (tolerance 1e-12) bound the
 gap that the looser stopping rule leaves.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -156,3 +158,30 @@ def test_every_solver_form(shape, iters, pre):
     assert gu.rel_l2(got["u"], u, wet) < TIGHT and gu.rel_l2(got["v"], v, wet) < TIGHT
     again = gu.run_stage(step, 8, st)
     assert np.array_equal(got["u"], again["u"]) and np.array_equal(got["v"], again["v"])
+
+
+@pytest.mark.parametrize("shape,rows", [((180, 90, 3), 1), ((360, 180, 3), 1), ((450, 219, 3), 2), ((640, 320, 3), 3),
+                                        ((720, 360, 3), 4), ((800, 400, 3), 5)])
+@pytest.mark.parametrize("pre", ["none", "jacobi"])
+def test_every_tile_height_of_the_resident_solver(shape, rows, pre):
+    """Ten iterations on grids whose tiles give a thread one to five rows (148
+    SMs, 227 KB of shared memory), against the oracle at the tight bound."""
+    nx, ny, nz = shape
+    grid = workloads.build_grid(nx, ny, nz)
+    kw = dict(workloads.PLAIN_OPTIONS, forcing=workloads.wind_forcing(grid), dt_bt=75.0, project_adv_vel=True,
+              projection_niter=10, projection_preconditioner=pre, projection_max_refinements=1)
+    step = make_solver_global(grid, workloads.PLAIN_PHYSICS, 1800.0, dtype="float32", **kw)[0]
+    info = (ctypes.c_int32 * 17)()
+    step.solver.check(step.solver.lib.zm_info(step.solver.handle, info, 17), "zm_info")
+    assert info[16] == rows
+    p = oparams.build_params(grid, workloads.PLAIN_PHYSICS, 1800.0, dtype="float32", **kw)
+    rng = np.random.default_rng(6)
+    wet = np.asarray(grid.wet_mask_3d)
+    T, S = workloads.initial_fields(grid)
+    lon, lat = np.meshgrid(np.radians(grid.lon), np.radians(grid.lat), indexing="ij")
+    noise = 0.01 * rng.standard_normal(wet.shape)
+    st = gu.f32(dict(u=((0.1 * np.cos(3 * lon) * np.cos(2 * lat))[:, :, None] + noise) * wet,
+                     v=(0.1 * np.sin(2 * lon) * np.cos(3 * lat))[:, :, None] * wet, T=T, S=S, eta=np.zeros((nx, ny))))
+    got = gu.run_stage(step, 8, st)
+    u, v = ostep.project_column_divergence(st["u"], st["v"], p, 1800.0)
+    assert gu.rel_l2(got["u"], u, wet) < TIGHT and gu.rel_l2(got["v"], v, wet) < TIGHT

@@ -1362,10 +1362,11 @@ int zm_create(const zm_grid* grid, const zm_params* params, zm_solver** out) {
 
 int zm_info(const zm_solver* s, int32_t* out, int32_t n) {
   if (!s || !out) return ZM_ERR_INVALID;
-  const int32_t v[16] = {s->n_subcyc, s->n_nu, s->adv_nsub, s->conv_nsub, s->P, (int32_t)(s->bytes >> 20),
+  const int32_t v[17] = {s->n_subcyc, s->n_nu, s->adv_nsub, s->conv_nsub, s->P, (int32_t)(s->bytes >> 20),
                          s->kernels_per_step, s->bt_blocks, s->bt.cap_active, s->nu_halo, s->fft_lines,
-                         s->d.ta_kc, s->d.lt_kc, s->d.fz_rows, s->d.pg_rows, s->nu_warps};
-  for (int q = 0; q < n && q < 16; ++q) out[q] = v[q];
+                         s->d.ta_kc, s->d.lt_kc, s->d.fz_rows, s->d.pg_rows, s->nu_warps,
+                         s->pj_tile.blocks > 0 ? s->pj_tile.cpt : 0};
+  for (int q = 0; q < n && q < 17; ++q) out[q] = v[q];
   return ZM_OK;
 }
 
