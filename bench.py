@@ -53,7 +53,7 @@ PROFILE_STEPS = 5
 # DRAM bytes per launch measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum)
 # for a kernel class on a grid, as summarised under profiles/; null for others.
 # ncu dram__bytes_read.sum + dram__bytes_write.sum of one full-size k_nu_tb launch (6 subcycles)
-NCU_TRAFFIC_BYTES = {((720, 360, 50), "nu_sub"): 117752832 + 65883136}
+NCU_TRAFFIC_BYTES = {((720, 360, 50), "nu_sub"): 107450368 + 65228288}
 
 
 def algo_fields_per_launch(cls, launches_per_step, n_nu):

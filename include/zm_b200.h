@@ -329,11 +329,10 @@ int zm_mlp_train_step(zm_mlp_trainer* tr, void* stream, int32_t batch, const flo
 /* Autotuner: time, on the resident state and through stages that write only
  * work buffers, the launch shapes that change no result (the nu_h halo
  * width 3..6, i.e. subcycles per temporally blocked pass, with 8 or 16 warps
- * per nu_h tile, the FFT lines per
- * block 1..8, the levels per block of the tracer-advection and linear-finish
- * column marches 5..25, and the tile rows of the vertical-transport and
- * pressure-gradient marches 4 or 8) and keep the fastest; the next zm_advance recaptures its
- * graphs.  zm_params.autotune = 1 runs it at the first zm_advance.  Writes
+ * per nu_h tile, the FFT lines per block 1..8, the levels per block of the
+ * tracer-advection and linear-finish column marches 2..25, and the tile rows
+ * of the vertical-transport and pressure-gradient marches 4 or 8) and keep the
+ * fastest; the next zm_advance recaptures its graphs.  zm_params.autotune = 1 runs it at the first zm_advance.  Writes
  * the choices when the pointers are given.  Synchronizes. */
 int zm_autotune(zm_solver* s, void* stream, int32_t* nu_halo, int32_t* fft_lines);
 

@@ -20,8 +20,10 @@
 // barrier, no fence, and a block may run ahead of far ones.  The counter barrier
 // and the separate halo loads this replaces took 7.3 us per subcycle at every
 // grid size up to 360x180 (9.5 at 720x360); a subcycle takes 2.0 us at 180x90,
-// 3.2 at 360x180 and 4.7 at 720x360.  Grids between 300 and 480 thousand
+// 3.2 at 360x180 and 4.7 at 720x360.  Grids between 300 and 405 thousand
 // cells streamed before (three launches per subcycle, 0.49 ms at 800x400; now 0.165).
+// An active polar cap keeps two counter barriers a subcycle: a whole step 0.50 ms at
+// 90x45x15 (0.81 with the tiles and loads this replaces), 0.95 at 360x180x20 (1.18).
 // The polar cap (numerics/horizontal.py:387-451) needs the wet-point zonal mean
 // of each band row; blocks write per-tile partial row sums and every reader
 // folds them in tile order, so the result does not depend on timing.  When no

@@ -148,7 +148,7 @@ __device__ __forceinline__ float colv(const float* __restrict__ a, long long bas
 //    next wet one cannot change a wet point any more: it keeps its values and
 //    its warp leaves the barriers.
 // At 720x360x50 (40 % of the points dry: 37 % of the strips dead, 47 % open) a
-// launch of 6 subcycles went from 150 to 127 us, 98 to 72 M warp instructions;
+// launch of 6 subcycles went from 150 to 128 us, 98 to 64 M warp instructions;
 // issue-active fell from 60 to 47 %, barrier and shared-memory waits lead.
 // Strips of 4 rows with twice the warps took 138 us, coefficients formed from
 // gate bits at 64 registers (4 blocks per SM) 131 us: occupancy is not the bound.

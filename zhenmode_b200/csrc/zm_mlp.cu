@@ -729,7 +729,7 @@ __global__ void k_mlp_pack_tc(const float* __restrict__ W1, const float* __restr
 //    FP32 instructions;
 //  * the gradients of the weights are sums over the batch (16 output tiles of
 //    64 x 64 with a serial chain of 8192 rows filled 16 of 148 SMs): the batch
-//    is split over blockIdx.z, each split writes its partial sums and k_fold
+//    is split over blockIdx.y, each split writes its partial sums and k_fold
 //    adds them in split order; the bias gradients are the column sums of the
 //    same slabs (they took 0.47 ms each as one block's serial sums).
 // At 8192 rows a step went from 4.00 to 0.24 ms (one B200), 0.022 ms of it the host's

@@ -834,7 +834,7 @@ bool proj_res_tile(int nx, int ny, int sms, size_t smem_max, int least, ProjTile
       ProjTile t{};
       t.x = (nx + ntx - 1) / ntx;
       t.y = (ny + nty - 1) / nty;
-      // no empty tiles, and edges wide enough that a halo lies in the next tile alone
+      // no empty tiles; a halo may reach past the next tile, every block waits for all sums
       t.tiles_x = (nx + t.x - 1) / t.x;
       t.tiles_y = (ny + t.y - 1) / t.y;
       if (t.x > PJ_RES_THREADS) continue;
