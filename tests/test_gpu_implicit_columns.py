@@ -31,3 +31,17 @@ def test_linear_stage(kind, shape):
         assert rel_l2(got[k], want[k], wet) < 1e-5, (k, rel_l2(got[k], want[k], wet))
     again = run_stage(gpu, 1, st)
     assert all(np.array_equal(got[k], again[k]) for k in got)
+
+
+def test_no_diffusivity_leaves_the_explicit_forms_bits():
+    """With nu_v = kappa_v = 0 the solve is the identity, exactly, and the linear
+    stage differs from the explicit form in nothing: the same bits."""
+    import dataclasses
+    nx, ny, nz = 75, 31, 14
+    out = []
+    for extra in ({}, {"vertical_diffusion": "implicit"}):
+        grid, phys, dt, opts, st = _case(nx, ny, nz, "islands", **extra)
+        gpu, _ = build_pair(grid, dataclasses.replace(phys, nu_v=0.0, kappa_v=0.0), dt, opts)
+        out.append(run_stage(gpu, 1, st))
+    for k in ("u", "v", "T", "S"):
+        assert np.array_equal(out[0][k], out[1][k]), k
