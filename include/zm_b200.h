@@ -60,7 +60,8 @@ typedef struct {
  * one cooperative launch) when the tiles fit and the streaming kernels (three
  * launches per subcycle) otherwise; RESIDENT fails zm_create with
  * ZM_ERR_UNSUPPORTED when they do not fit or the grid has more than four
- * 32 x 16 tiles per SM. */
+ * 32 x 16 tiles per SM.  A wet_mask with values other than 0 and 1 always takes
+ * the streaming kernels. */
 #define ZM_BT_AUTO 0
 #define ZM_BT_RESIDENT 1
 #define ZM_BT_STREAMING 2

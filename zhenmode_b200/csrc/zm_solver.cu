@@ -1140,7 +1140,9 @@ void build(zm_solver* s, const zm_grid* g, const zm_params* p) {
     const bool named = (long long)((nx + 31) / 32) * ((ny + 15) / 16) <= 4ll * sms;
     require((fits && named) || p->bt_kernel != ZM_BT_RESIDENT, ZM_ERR_UNSUPPORTED,
             "barotropic tiles do not fit on the GPU at once (bt_kernel = ZM_BT_RESIDENT)");
-    s->bt_blocks = (fits && p->bt_kernel != ZM_BT_STREAMING) ? s->btt.blocks : 0;
+    // the loop knows wet and dry cells; a mask with weights between takes the streaming kernels, which multiply by it
+    const bool binary = std::all_of(g->wet_mask, g->wet_mask + (size_t)nx * ny, [](double w) { return w == 0.0 || w == 1.0; });
+    s->bt_blocks = (fits && binary && p->bt_kernel != ZM_BT_STREAMING) ? s->btt.blocks : 0;
     if (s->bt_blocks > 0) {
       a.tile_x = s->btt.x;
       a.tile_y = s->btt.y;
