@@ -429,7 +429,8 @@ __global__ void __launch_bounds__(256) k_proj_correct(Dev d, float* __restrict__
 //   alpha = gamma / (delta - beta gamma / alpha_old),
 //   p = z + beta p, s = w + beta s, x += alpha p, r -= alpha s, z = M r,
 // the recurrences of Chronopoulos and Gear (1989), equal to the loop above in
-// exact arithmetic; both sums are formed before either scalar is needed.  The
+// exact arithmetic for a symmetric A (zm_create checks the grid); both sums are formed
+// before either scalar is needed.  The
 // halo needs no second exchange: each block publishes its w along the tile's
 // edges with the sums, and carries s and z of its halo cells with the same
 // recurrences.

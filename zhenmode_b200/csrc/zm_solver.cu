@@ -1285,7 +1285,19 @@ void build(zm_solver* s, const zm_grid* g, const zm_params* p) {
     a.refinements = p->projection_max_refinements;
     int optin = 0;
     ZM_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
-    if (proj_res_tile(nx, ny, sms, (size_t)optin, 256, s->pj_tile)) {
+    // The resident form's recurrences take <p, A p> from <z, A z>, which holds for a symmetric A: dx / cos the
+    // same in every row (an area over dy cos is then a constant of the meridian), a mask of 0 and 1, no wet
+    // level where it is 0.  Other grids take k_proj_cg, which forms <p, A p> itself.
+    bool symmetric = true;
+    for (int i = 0; i < nx && symmetric; ++i)
+      for (int j = 0; j < ny; ++j) {
+        const size_t r = (size_t)i * ny + j;
+        const double w = g->wet_mask[r], q = g->dx_2d[r] / g->cos_lat[j], q0 = g->dx_2d[(size_t)i * ny] / g->cos_lat[0];
+        bool wet = false;
+        for (int k = 0; k < nz; ++k) wet = wet || (g->wet_mask_3d ? g->wet_mask_3d[r * nz + k] : w) == 1.0;
+        symmetric = symmetric && (w == 1.0 || (w == 0.0 && !wet)) && std::fabs(q - q0) <= 1e-10 * std::fabs(q0);
+      }
+    if (symmetric && proj_res_tile(nx, ny, sms, (size_t)optin, 256, s->pj_tile)) {
       auto kern = proj_res_kernel(s->pj_tile.cpt);
       ZM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
       ZM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, s->pj_tile.threads, s->pj_tile.smem));
