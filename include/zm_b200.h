@@ -227,8 +227,9 @@ int zm_barrier_probe(zm_solver* s, void* stream, int32_t blocks, int32_t expecte
 /* Poll limit of the waits between the blocks of the barotropic loop and the
  * column projection, for the following steps; negative: the default (2^24).
  * With 0 a block gives up at the first word that is not there yet, which
- * exercises the error path: zm_status then returns ZM_ERR_TIMEOUT until
- * zm_load_state.  Synchronizes the device; the steps are captured anew. */
+ * exercises the error path: zm_status then returns ZM_ERR_TIMEOUT until the
+ * next state is loaded (zm_load_state, zm_step, zm_step_host, zm_ledger_step,
+ * zm_run_stage).  Synchronizes the device; the steps are captured anew. */
 int zm_set_wait_limit(zm_solver* s, int32_t max_polls);
 
 /* Monitor of the resident state after the last zm_advance (runtime/monitor.py:20-30):

@@ -51,3 +51,31 @@ def test_a_reloaded_state_runs_as_on_a_fresh_handle(nx, ny, nz, land_lat, extra)
     want = _make(nx, ny, nz, land_lat, **extra)[0](second)
     for k in ("u", "v", "T", "S", "eta"):
         assert torch.equal(getattr(got, k), getattr(want, k)), k
+
+
+@pytest.mark.parametrize("extra", [{}, dict(project_adv_vel=True, projection_niter=20)])
+@pytest.mark.parametrize("call", ["host", "ledger", "stage"])
+def test_every_call_that_loads_a_state_starts_afresh(extra, call):
+    """The host step, the ledger step and a stage after a step that gave up."""
+    import torch
+    from tests.gpu_util import FIELDS, run_stage
+    from zhenmode_b200.ledger import make_budget_step
+
+    def run(step, st):
+        if call == "host":
+            return step.advance(JaxStateG(*[t.cpu().numpy() for t in st[:5]], 0.0), 2)[:5]
+        if call == "ledger":
+            return [t.cpu().numpy() for t in make_budget_step(step)(st)[0][:5]]
+        out = run_stage(step, 3, {k: getattr(st, k).double().cpu().numpy() for k in FIELDS})
+        return [out[k] for k in FIELDS]
+
+    step, (first, second) = _make(180, 90, 5, 65.0, **extra)
+    sv = step.solver
+    sv.check(sv.lib.zm_set_wait_limit(sv.handle, 0), "zm_set_wait_limit")
+    step(first)
+    torch.cuda.synchronize()
+    sv.check(sv.lib.zm_set_wait_limit(sv.handle, -1), "zm_set_wait_limit")
+    got = run(step, second)
+    assert _status(step) == _native.ZM_OK
+    for a, b in zip(got, run(_make(180, 90, 5, 65.0, **extra)[0], second)):
+        assert np.array_equal(a, b)

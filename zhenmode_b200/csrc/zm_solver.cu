@@ -228,8 +228,8 @@ struct zm_solver {
     d.nu_class = table;
   }
 
-  // Clear the barrier and error words of the barotropic loop and the projection.  Their sequence
-  // numbers move past every word that a launch which gave up may have left behind.
+  // Clear the barrier and error words of the barotropic loop and the projection, where a state is loaded.
+  // Their sequence numbers move past every word that a launch which gave up may have left behind.
   void reset_sync(cudaStream_t s) {
     k_sync_reset<<<1, 2, 0, s>>>(bt_seq, bt_sync, pj.seq, proj_on ? pj.bar : nullptr);
     check_launch();
@@ -1590,6 +1590,7 @@ int zm_step_host(zm_solver* s, void* stream, const zm_state* in, zm_state* out, 
     // the copies start after the work already queued on the caller's stream
     ZM_CUDA(cudaEventRecord(ev[0], st));
     ZM_CUDA(cudaStreamWaitEvent(cs, ev[0], 0));
+    s->reset_sync(st);
     const void* all[10];
     for (int f = 0; f < 5; ++f) all[f] = hin[f], all[5 + f] = hout[f];
     // Pageable arrays are staged by several threads, pinned ones copied directly.
@@ -1697,6 +1698,7 @@ int zm_run_stage(zm_solver* s, void* stream, int32_t stage, const zm_state* in, 
   if (stage == 8 && !s->proj_on) return fail(s, Err{ZM_ERR_INVALID, "stage 8 needs project_adv_vel"});
   cudaStream_t st = (cudaStream_t)stream;
   try {
+    s->reset_sync(st);
     s->load(st, in, s->st[s->cur], s->eta[s->cur]);
     const int a = s->cur, b = 1 - s->cur;
     if (stage <= 2) {  // the stages leave dry tracers alone; here they are part of the result
@@ -1997,6 +1999,7 @@ int zm_ledger_step(zm_solver* s, void* stream, const zm_state* in, zm_state* out
   try {
     s->ensure_ledger();
     ZM_CUDA(cudaMemsetAsync(s->led_acc, 0, ZM_LED_COUNT * sizeof(double), st));
+    s->reset_sync(st);
     s->load(st, in, s->st[s->cur], s->eta[s->cur]);
     const int a = s->cur, b = 1 - s->cur;
     s->ledger_on = true;
