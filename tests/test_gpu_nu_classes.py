@@ -44,11 +44,11 @@ def test_open_and_gated_strips_give_the_same_bits(nx, ny):
 
 
 def _member(seed):
+    import torch
     grid, physics, dt, kw, T, S = workloads.make_case("plain", 192, 96, 10, dtype="float32")
     step, init, _ = make_solver_global(grid, physics, dt, **dict(kw, nu_nsub=3))
     rng = np.random.default_rng(seed)
     st = init(T, S)
-    import torch
     wet = torch.as_tensor(np.asarray(grid.wet_mask_3d, np.float32), device="cuda")
     move = lambda: 0.1 * torch.as_tensor(rng.standard_normal(st.u.shape), dtype=torch.float32, device="cuda") * wet  # noqa: E731
     return step, JaxStateG(move(), move(), st.T, st.S, st.eta, st.ice)
@@ -64,16 +64,14 @@ def test_tuning_a_member_leaves_the_ensembles_steps_right():
     ens.load([m[1] for m in members])
     ens.advance(2)
     want = ens.store()
-    shape = lambda: [int(x) for x in info()]  # noqa: E731
+    sv = members[0][0].solver
 
-    def info():
-        sv = members[0][0].solver
+    def shape():
         out = (ctypes.c_int32 * 16)()
         sv.check(sv.lib.zm_info(sv.handle, out, 16), "zm_info")
         return out[9], out[15]
 
     before = shape()
-    sv = members[0][0].solver
     sv.check(sv.lib.zm_autotune(sv.handle, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), None, None),
              "zm_autotune")
     if shape() == before:
